@@ -102,6 +102,39 @@ def test_plain_gemm_rows_do_not_depend_on_the_batch():
     assert torch.equal(whole[37:38], one)
 
 
+@pytest.mark.parametrize("K", [4, 32, 36, 256, 260, 1100, 2048])
+@pytest.mark.parametrize("N", [7, 64, 130, 1000])
+@pytest.mark.parametrize("mode", ["store", "accumulate", "swiglu"])
+def test_float32_gemm_at_the_edges_of_its_kernels(mode, N, K):
+    """A few rows, tiles of 64 and 128 rows, the eighths of K in one CTA and in a cluster: within the bound of a sum of eight
+    chains of K / 8 products, and every row the same, bit for bit, whatever launch it is part of."""
+    from llmplayer_b200.kernels import ops
+    torch.manual_seed(N + K)
+    code = {"store": ops.STORE, "accumulate": ops.ACCUMULATE, "swiglu": ops.SWIGLU}[mode]
+    most = 1100 if N == 1000 else 300
+    a = torch.randn(most, K, device="cuda:0")
+    w = torch.randn(N * (2 if mode == "swiglu" else 1), K, device="cuda:0") / K ** 0.5
+    out0 = torch.randn(most, N, device="cuda:0")
+    ref = reference(a, w, code, out0)
+    # a chain of n products, and the eight additions behind it: at most (n + 9) units of 2^-24 of the sum of magnitudes
+    sums = (32 * -(-K // 256) + 9) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    if mode == "swiglu":
+        g, u = a.double() @ w[:N].double().T, a.double() @ w[N:].double().T
+        # |silu'| <= 1.1; exponential, division and product: a few units more of the result
+        bound = 1.1 * u.abs() * sums[:, :N] + (g * torch.sigmoid(g)).abs() * sums[:, N:] + 8 * 2.0 ** -24 * ref.abs() + 1e-30
+        bound = bound + sums[:, :N] * sums[:, N:]
+    else:
+        bound = sums + 2.0 ** -24 * ref.abs() + 2.0 ** -24 * out0.double().abs()
+    whole = out0.clone()
+    ops.gemm_plain(a, w, whole, code)
+    assert bool(((whole.double() - ref).abs() <= bound).all())
+    for M in (1, 2, 3, 5, 9, 17, 32, 33, 64, 65, 129, 200, 300, 777):
+        if M < most:
+            out = torch.cat([out0[:M], torch.full((1, N), 7.0, device="cuda:0")])
+            ops.gemm_plain(a[:M].contiguous(), w, out[:M], code)
+            assert torch.equal(out[:M], whole[:M]) and bool((out[M] == 7.0).all()), M
+
+
 def test_refusals():
     from llmplayer_b200.errors import KernelError
     from llmplayer_b200.kernels import ops
