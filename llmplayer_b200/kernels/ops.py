@@ -54,7 +54,7 @@ _SIGNATURES = {
         "lp_gemm_plain": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     },
     "attention_plain": {
-        "lp_attention_plain": [_P, _P, _I, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _F, _P, _I, _I, _P, _P, _P, _I, _P],
+        "lp_attention_plain": [_P, _P, _I, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _F, _P, _I, _I, _P, _P, _P, _I, _P, _I, _P],
     },
     "gemm_tcgen05": {
         "lp_gemm_tcgen05": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _F, _P, _P,
@@ -673,7 +673,7 @@ def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, angles: Optional[torch.Tenso
 
 # --------------------------------------------------------------------------- matrix products
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE) -> torch.Tensor:
-    """out (=|+=) a @ w.T with float32 multiply-adds in increasing k.
+    """out (=|+=) a @ w.T with float32 multiply-adds, each element in one fixed order whatever the number of rows.
 
     ``SWIGLU``: ``w`` is [2N, K], gate rows then up rows; out = silu(a gate^T) * (a up^T).
     """
@@ -900,17 +900,25 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = ST
 
 
 # --------------------------------------------------------------------------- attention
+PLAIN_KEY_BLOCK = 128               # keys that the plain kernels finish at a time
+PLAIN_PARTS_MOST = 32 << 20         # float32 values of scratch (128 MiB) beyond which the blocks are walked one behind the other
+PLAIN_PARTS_TOKENS = 8              # new tokens of a sequence up to which its blocks of keys are looked at side by side
+
+
 def attention_plain(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, page_table: torch.Tensor,
                     seq_ids: torch.Tensor, positions: torch.Tensor, *, num_heads: int, num_kv_heads: int,
                     head_dim: int, scale: float, window: Optional[int], softcap: Optional[float] = None,
-                    sinks: Optional[torch.Tensor] = None, keep_first: int = 0, chunk: int = 0, distance=None, gate=None) -> torch.Tensor:
+                    sinks: Optional[torch.Tensor] = None, keep_first: int = 0, chunk: int = 0, distance=None, gate=None,
+                    scratch=None, longest: int = 0) -> torch.Tensor:
     """Each query token attends over the cached keys of its sequence up to its own
     position (and within ``window``, if given). ``softcap``: scores become softcap * tanh(score / softcap) after the
     scale; ``sinks``: float32 [H], a logit per head that enters the softmax's denominator once. ``keep_first`` (with a
     window): the sequence's first ``keep_first`` tokens stay visible to every later query. ``chunk`` > 0: a query at
     position p sees keys of its own chunk only, from p // chunk * chunk on. ``distance`` = (scale, rate), float32 [H] each:
     the score of a key n positions back loses scale[h] * ln(1 + rate[h] * n). ``gate``: float32 [T, H] (may be a column
-    slice): head h's output of token t is multiplied by sigmoid(gate[t, h])."""
+    slice): head h's output of token t is multiplied by sigmoid(gate[t, h]). ``scratch(name, shape, dtype)`` and ``longest``
+    (no position reaches it): a step of a few tokens per sequence may then look at the blocks of its keys side by side
+    (float32; the result is the same, bit for bit)."""
     dist_scale, dist_rate = _distance_args(distance, num_heads, "attention")
     gate_ptr, gate_ld = _gate_args(gate, q.shape[0], num_heads, "attention")
     _check_sinks(sinks, num_heads, "attention")
@@ -927,11 +935,16 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, pag
     if pages.shape[1] != 2 or pages.shape[2] != G or pages.shape[4] != hd:
         raise KernelError(f"attention: pages {tuple(pages.shape)} do not fit {G} key heads of {hd}")
     lib = library("attention_plain")
+    parts, blocks = None, 0
+    if scratch is not None and longest > 0 and q.dtype == torch.float32 and pages.dtype == torch.float32:
+        blocks = -(-int(longest) // PLAIN_KEY_BLOCK)
+        if T * H * blocks * (hd + 2) <= PLAIN_PARTS_MOST:
+            parts = scratch("attention_parts", (T * H * blocks * (hd + 2),), torch.float32)
     _check(lib, lib.lp_attention_plain(
         q.data_ptr(), out.data_ptr(), _code(q, "attention q"), pages.data_ptr(), _code(pages, "attention pages"),
         page_table.data_ptr(), page_table.shape[1], seq_ids.data_ptr(), positions.data_ptr(), T, H, G, hd,
         pages.shape[3], float(scale), int(window) if window else 0, float(softcap or 0.0), _ptr(sinks),
-        int(keep_first) if window else 0, int(chunk or 0), dist_scale, dist_rate, gate_ptr, gate_ld, _stream()))
+        int(keep_first) if window else 0, int(chunk or 0), dist_scale, dist_rate, gate_ptr, gate_ld, _ptr(parts), blocks, _stream()))
     return out
 
 
@@ -1158,7 +1171,8 @@ def attention(ctx, q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, page
                                  keep_first=keep_first, chunk=chunk, distance=distance, gate=gate)
     return attention_plain(q, out, pages, page_table, ctx.seq_ids, ctx.positions, num_heads=num_heads,
                            num_kv_heads=num_kv_heads, head_dim=head_dim, scale=scale, window=window, softcap=softcap,
-                           sinks=sinks, keep_first=keep_first, chunk=chunk, distance=distance, gate=gate)
+                           sinks=sinks, keep_first=keep_first, chunk=chunk, distance=distance, gate=gate,
+                           scratch=ctx.buffer if ctx.max_new <= PLAIN_PARTS_TOKENS else None, longest=ctx.max_kv_len)
 
 
 # --------------------------------------------------------------------------- latent attention

@@ -379,3 +379,56 @@ def test_fused_decode_over_more_than_32_pages_in_one_share(H, G, hd):
     ops.check_kernel_status()
     assert torch.equal(pages_a, pages_b)
     assert float((got.float() - want.float()).abs().max()) <= 2e-2
+
+
+@pytest.mark.parametrize("H,G,hd", [(4, 2, 64), (9, 1, 48), (3, 3, 128), (2, 1, 256), (2, 2, 20)])
+@pytest.mark.parametrize("form", ["all", "window", "kept", "chunk"])
+def test_float32_attention_in_blocks(form, H, G, hd):
+    """Tiles of queries over blocks of keys, and blocks of keys side by side: against float64, and the same bits from both
+    however the sequences are cut into calls. Lengths at the edges of blocks (128), tiles (32, 64) and pages."""
+    from llmplayer_b200.kernels import ops
+    dev = "cuda:0"
+    g = torch.Generator().manual_seed(hd + H)
+    lengths, P = [300, 129, 1, 64], 64
+    width = -(-max(lengths) // P)
+    table = torch.randperm(len(lengths) * width, generator=g).reshape(len(lengths), width).to(torch.int32)
+    pages = torch.randn(len(lengths) * width, 2, G, P, hd, generator=g)
+    T = sum(lengths)
+    q = torch.randn(T, H * hd, generator=g) * 2
+    seq = torch.tensor([i for i, n in enumerate(lengths) for _ in range(n)], dtype=torch.int32)
+    pos = torch.tensor([p for n in lengths for p in range(n)], dtype=torch.int32)
+    window = 70 if form in ("window", "kept") else None
+    keep = 5 if form == "kept" else 0
+    chunk = 100 if form == "chunk" else 0
+    kw = dict(num_heads=H, num_kv_heads=G, head_dim=hd, scale=hd ** -0.5, window=window, keep_first=keep, chunk=chunk,
+              softcap=20.0 if form == "kept" else None)
+    sinks = torch.randn(H, generator=g) if form != "all" else None
+    ref = torch.empty(T, H, hd, dtype=torch.float64)
+    for t in range(T):
+        p, i = int(pos[t]), int(seq[t])
+        keys = [j for j in range(p + 1) if (window is None or j > p - window or j < keep) and (not chunk or j // chunk == p // chunk)]
+        for h in range(H):
+            kv = torch.stack([pages[table[i, j // P], :, h * G // H, j % P] for j in keys]).double()     # [keys, 2, hd]
+            s = kv[:, 0] @ q[t].reshape(H, hd)[h].double() * hd ** -0.5
+            if kw["softcap"]:
+                s = 20.0 * torch.tanh(s / 20.0)
+            w = torch.softmax(s if sinks is None else torch.cat([s, sinks[h:h + 1].double()]), 0)[:len(keys)]
+            ref[t, h] = w @ kv[:, 1]
+    if window is not None:          # pages that no query of the last call below reaches are gone
+        gone = table.clone()
+        gone[0, 1 if keep else 0:2] = -1
+    d = lambda t: t.to(dev)  # noqa: E731
+    whole = torch.empty(T, H * hd, device=dev)
+    scratch = lambda name, shape, dtype: torch.full(shape, float("nan"), dtype=dtype, device=dev)  # noqa: E731
+    sk = {"sinks": None if sinks is None else d(sinks)}
+    ops.attention_plain(d(q), whole, d(pages), d(table), d(seq), d(pos), **kw, **sk)
+    # scores carry hd products, exponentials and sums of up to 300 weights: a few hundred units of 2^-24 times scores of up to 20
+    assert float((whole.double().cpu().reshape(T, H, hd) - ref).abs().max()) < 2e-5 * float(ref.abs().max())
+    for rows in ([299, 300, 428, 429, 493], [0, 63, 64, 127, 128], list(range(250, 300))):
+        at = torch.tensor(rows)
+        late = window is not None and min(rows) >= 250 and max(rows) < 300
+        for use in (None, scratch):
+            out = torch.empty(len(rows), H * hd, device=dev)
+            ops.attention_plain(d(q[at]), out, d(pages), d(gone if late else table), d(seq[at]), d(pos[at]), **kw, **sk, scratch=use,
+                                longest=int(pos[at].max()) + 1)
+            assert torch.equal(out, whole[at.to(dev)]), (rows, use is None)
