@@ -31,6 +31,7 @@ LIBRARIES: Dict[str, str] = {
     "attention_plain": "attention_plain.cu",
     "sampling": "sampling.cu",
     "gemm_tcgen05": "gemm_tcgen05.cu",
+    "gemm_experts": "gemm_experts.cu",
     "attention_mma": "attention_mma.cu",
     "attention_tcgen05": "attention_tcgen05.cu",
     "host_loop": "host_loop.cu",

@@ -116,6 +116,9 @@ _SIGNATURES = {
     "stream_bundle": {
         "lp_stream_bundle": [_P, _I, _P, _P, _P, _F, _P, _P, _P, _F, _P, _I, _P, _I, _I, _I, _P, ctypes.c_longlong, _P],
     },
+    "gemm_experts": {
+        "lp_experts": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, ctypes.c_longlong, _P, _P],
+    },
     "host_loop": {
         "lp_decode_loop": [_P, _P, _P, _I, _I, _I, _P, _I, _I, _P, _P, _P, _P, _P],
         "lp_decode_loop_sampled": [_P, _P, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P,
@@ -721,7 +724,8 @@ def check_kernel_status() -> None:
         _status.zero_()
         raise KernelError(f"a tensor-core kernel gave up waiting on a barrier (code {code}: "
                           "1 = loader, 2 = MMA issuer, 3 = epilogue, 4-5 = operand maker; 2x the same in the "
-                          "persistent product; 6 = a page of the decode attention)")
+                          "persistent product, 5x in the experts' (55: more choices than announced); "
+                          "6 = a page of the decode attention)")
 
 
 def _token_tile(tokens: int, gated: bool) -> int:
@@ -2106,6 +2110,63 @@ def expert_scale(hidden: torch.Tensor, weights: torch.Tensor, expert_size: int, 
                                     weights.data_ptr(), ldw, T, E, int(expert_size), *_clear_args(clear, "expert_scale"),
                                     *id_args, _stream()))
     return hidden
+
+
+def expert_rows(tokens: int, num_experts: int, top: int, shared: bool) -> int:
+    """Rows that :func:`experts` needs at most: every expert's tokens rounded up to tiles of 128, and the shared expert's."""
+    tiles = -(-tokens // 128)
+    routed = min((tokens * min(top, num_experts) + 127 * num_experts) // 128, num_experts * tiles)
+    return 128 * (routed + (tiles if shared else 0))
+
+
+# What running experts for their own tokens only must save against running all tokens through all experts, and the
+# tokens below which the weights' bytes bound both. Measured on a B200 (us, all through all / own tokens; saved GFLOP):
+# width 2048, 8 experts of 2048 + a shared one, 2 chosen: 128 tokens 83 / 76 (6), 192: 95 / 87 (16), 512: 178 / 92, 2048: 374 / 173;
+# width 2048, 32 of 1024, 4 chosen: 96 tokens 111 / 113 (8), 128: 115 / 114 (19), 192: 178 / 112 (42), 2048: 653 / 211;
+# width 1024, 8 of 512 + 1024, 2 chosen: 384 tokens 63 / 68 (6), 512: 86 / 70 (8), 2048: 97 / 72.
+EXPERTS_GROUPED_MIN_TOKENS = 128
+EXPERTS_GROUPED_MIN_SAVED = 8e9
+
+
+def experts_grouped_pays(tokens: int, width: int, num_experts: int, top: int, expert_size: int) -> bool:
+    """Whether running every expert for its own tokens beats running all tokens through all experts."""
+    rows = tokens * num_experts - tokens * min(top, num_experts) - 64 * num_experts      # half a tile of padding per expert
+    return (tokens >= EXPERTS_GROUPED_MIN_TOKENS and num_experts <= 256
+            and 6.0 * width * expert_size * rows >= EXPERTS_GROUPED_MIN_SAVED)
+
+
+def experts(x: torch.Tensor, weights: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, out: torch.Tensor, scratch, *,
+            num_experts: int, top: int, expert_size: int, shared_size: int = 0, overwrite: bool = False) -> torch.Tensor:
+    """out[t] (+)= sum over the experts e that token t chose of down_e(weights[t, e] * silu(gate_e x) * (up_e x)), plus the
+    shared expert's (behind the others in ``w_up`` and ``w_down``, weight one), each expert run for its own tokens only.
+    ``x``: bfloat16 [T, d]; ``weights``: float32 [T, >= E], zero where a token did not choose an expert, at most ``top``
+    others per token; ``w_up``: the interleaved gate and up rows of all experts (:func:`interleave_gate_up`); ``w_down``:
+    bfloat16 [d, all hidden columns]; ``out``: float32 [T, d]. Hidden sizes are multiples of 128.
+    ``scratch(name, shape, dtype)`` gives the buffers."""
+    _want(x, "experts x", torch.bfloat16, 2)
+    _want(weights, "experts weights", torch.float32, 2)
+    _want(w_up, "experts w_up", torch.bfloat16, 2)
+    _want(w_down, "experts w_down", torch.bfloat16, 2)
+    _want(out, "experts out", torch.float32, 2)
+    T, d = x.shape
+    E, total = int(num_experts), int(num_experts) * int(expert_size) + int(shared_size)
+    if (weights.shape[0] != T or weights.shape[1] < E or w_up.shape != (2 * total, d) or w_down.shape != (d, total)
+            or out.shape != (T, d)):
+        raise KernelError(f"experts: x {tuple(x.shape)}, weights {tuple(weights.shape)}, w_up {tuple(w_up.shape)}, w_down "
+                          f"{tuple(w_down.shape)}, out {tuple(out.shape)} for {E} experts of {expert_size} and {shared_size}")
+    rows = expert_rows(T, E, top, shared_size > 0)
+    counts = scratch("expert_lists", (E * (T + 1),), torch.int32)
+    row_token = scratch("expert_row_tokens", (rows,), torch.int32)
+    row_weight = scratch("expert_row_weights", (rows,), torch.float32)
+    gathered = scratch("expert_rows", (rows, d), torch.bfloat16)
+    hidden = scratch("expert_hidden", (rows, max(int(expert_size), int(shared_size))), torch.bfloat16)
+    lib = library("gemm_experts")
+    _check(lib, lib.lp_experts(x.data_ptr(), weights.data_ptr(), weights.shape[1], w_up.data_ptr(), w_down.data_ptr(), out.data_ptr(), d,
+                               T, d, E, int(top), int(expert_size), int(shared_size), rows, counts.data_ptr(),
+                               counts.data_ptr() + 4 * E, gathered.data_ptr(), hidden.data_ptr(), row_token.data_ptr(),
+                               row_weight.data_ptr(), out.numel() if overwrite else 0, kernel_status().data_ptr(), _stream()))
+    count_launches(3)
+    return out
 
 
 def route_top(logits: torch.Tensor, bias: Optional[torch.Tensor], weights: torch.Tensor, *, num_experts: int, top: int,

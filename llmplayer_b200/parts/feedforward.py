@@ -267,7 +267,9 @@ class Mixture(Part):
     by rows), whose hidden activations are multiplied by the token's weight for their expert, and ONE down product
     over the experts' down matrices stacked by columns, which sums the weighted outputs: every token passes through
     every expert, so the cost does not depend on the routing and the step has no host-side decisions (it replays
-    from a captured graph); what a token did not choose is multiplied by zero.
+    from a captured graph); what a token did not choose is multiplied by zero. Steps of many tokens run silu experts as
+    products over each expert's own tokens instead (csrc/gemm_experts.cu), whose tiles the device lists: still no
+    host-side decision, and only the chosen experts' work.
 
     Squared-ReLU experts have one up matrix each instead of gate and up: one stacked up product with float32 sums, then a
     kernel that squares what is positive and applies the weights (to the expert's input or to its output). Where the
@@ -319,6 +321,7 @@ class Mixture(Part):
         self.up: Optional[Linear] = None
         self.down: Optional[Linear] = None
         self.stacked_router = False
+        self.grouped = False
 
     def _experts(self):
         s = self.spec
@@ -367,6 +370,9 @@ class Mixture(Part):
         # silu experts: the gated product applies the activation itself; clamped ones: float32 sums, then a kernel
         gate = torch.cat([tensors[p + "gate"] for p, _ in experts], dim=0)
         self.gate_up = Linear([gate, up], runtime, gated=s.activation == "silu")
+        # tiles of 128 hidden values that never hold two experts, rows that the tensor cores take
+        self.grouped = (s.activation == "silu" and self.gate_up.interleaved and self.down.tensor_cores()
+                        and s.expert_size % 128 == 0 and s.shared_size % 128 == 0)
 
     def buffer_to_clear(self, ctx, tokens: int):
         from ..kernels import ops
@@ -419,6 +425,15 @@ class Mixture(Part):
                                   scale=r.weight_scale)
             else:
                 ops.route(logits, weights, groups=r.groups, keep=r.keep_groups, top=r.top)
+        if (self.grouped and x.dtype == torch.bfloat16 and residual.dtype == torch.float32 and residual.is_contiguous()
+                and ops.experts_grouped_pays(T, s.hidden_size, r.num_experts, r.top, s.expert_size)):
+            with ops.section("ffn.experts"):
+                ops.experts(x, weights, self.gate_up.weight, self.down.weight, residual, ctx.buffer, num_experts=r.num_experts,
+                            top=r.top, expert_size=s.expert_size, shared_size=s.shared_size, overwrite=overwrite)
+            if r.identity_experts:
+                with ops.section("ffn.identity"):
+                    ops.identity_experts(residual, x, weights, r.num_experts, r.identity_experts)
+            return False
         h = ctx.buffer("ffn_hidden", (T, self.total), self.runtime.act_dtype)
         clear = residual if overwrite and residual.dtype == torch.float32 and self.down.needs_zero(T) else None
         rides = False
