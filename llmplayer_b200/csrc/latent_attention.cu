@@ -11,11 +11,13 @@
 //                       queries' rotated parts, write of the row into the paged cache
 //   lp_latent_absorb    q'[t, h] = [U_h^T q_n | q_r]
 //   lp_latent_attend    online-softmax attention of q' over the rows of the pages (float32 scores,
-//                       weights and sums), the keys of a sequence optionally shared out over several CTAs
+//                       weights and sums), the keys of a sequence optionally shared out over several CTAs;
+//                       over a bfloat16 cache the products run on the tensor cores, the queries and the
+//                       weights as sums of three bfloat16 numbers (24 bits), the rows as they are
 //   lp_latent_expand    merge of the shares, value map, output gate
 //
-// All arithmetic is float32; the cache and the weights may be bfloat16 or float32. Keys are visited in
-// blocks of 32 aligned to absolute positions, so a position's result does not depend on how its
+// All arithmetic is float32 (or products of its exact parts); the cache and the weights may be bfloat16 or float32. Keys
+// are visited in blocks of 32 (64 on the tensor cores) aligned to absolute positions, so a position's result does not depend on how its
 // sequence was cut into steps or batched (the number of shares changes only the last merge).
 #include "common.cuh"
 
@@ -362,6 +364,247 @@ latent_attend_kernel(const float* __restrict__ qa, const TKV* __restrict__ pages
     }
 }
 
+// ---------------------------------------------------------------- attend, on the tensor cores
+// A bfloat16 row of the cache is an exact operand; a float32 query (or softmax weight) is the sum of three bfloat16
+// numbers: 3 x 8 bits. So three mma.sync products per tile give the float32 scores and sums without rounding the query or
+// the weights to fewer than 24 bits.
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// x = part[0] + part[1] + part[2] to 24 bits; an infinity or a NaN stays in the first part alone
+__device__ __forceinline__ void three_parts(float x, __nv_bfloat16* part) {
+    part[0] = __float2bfloat16_rn(x);
+    const float head = __bfloat162float(part[0]);
+    const bool finite = fabsf(head) < INFINITY;
+    const float rest = finite ? x - head : 0.f;
+    part[1] = __float2bfloat16_rn(rest);
+    part[2] = __float2bfloat16_rn(rest - __bfloat162float(part[1]));
+}
+
+constexpr int TC_ROWS = 16;          // (token, head) rows of a CTA = MMA M
+constexpr int TC_KEYS = 64;          // keys per block
+constexpr int TC_PSTRIDE = TC_KEYS + 8, TC_SSTRIDE = TC_KEYS + 4;
+
+__host__ __device__ constexpr size_t tc_smem(int Dk) {
+    return (size_t)(3 * TC_ROWS + 2 * TC_KEYS) * (Dk + 8) * 2 + (size_t)4 * TC_ROWS * TC_SSTRIDE * 4 + (size_t)3 * TC_ROWS * TC_PSTRIDE * 2;
+}
+
+// A CTA takes 16 (token, head) rows of one sequence and one share of its blocks of 64 keys; the next block's rows are on
+// their way while a block is worked on. Scores: a warp takes 32 keys and a quarter of the row's width, the quarters meet in
+// shared memory; softmax: two rows per warp; sums: a warp takes an eighth of the latent's columns (NT tiles of 8). Row strides of
+// an odd multiple of 16 bytes keep ldmatrix free of bank conflicts.
+// Bound by the tensor instructions (3 x 36 + 3 x 32 per 16 keys and CTA at rank 512) and the latency of a block's steps:
+// 32 sequences of 750 to 1500 rows of 576, 16 heads, B200: 210 us with a lane per key (above) -> 39 (cold
+// caches); with three chains of products one behind the other and a division per 16 bytes copied it was 41.
+template <int NT>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__ pages, const int* __restrict__ page_table,
+                        int pt_stride, const int* __restrict__ q_start, const int* __restrict__ kv_len, float* __restrict__ part, int H,
+                        int dr, int page_size, float scale, int shares, int window) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    constexpr int rank = NT * 64;
+    const int Dk = rank + dr, stride = Dk + 8;
+    __nv_bfloat16* Qs = (__nv_bfloat16*)raw;                                  // [3][TC_ROWS][stride]
+    __nv_bfloat16* Ks = Qs + 3 * TC_ROWS * stride;                            // [2][TC_KEYS][stride]
+    float* Ss = (float*)(Ks + 2 * TC_KEYS * stride);                          // [4][TC_ROWS][TC_SSTRIDE]
+    __nv_bfloat16* Ps = (__nv_bfloat16*)(Ss + 4 * TC_ROWS * TC_SSTRIDE);      // [3][TC_ROWS][TC_PSTRIDE]
+    __shared__ float alphas[TC_ROWS];
+    lp_grid_release();
+    lp_grid_wait();
+    const int b = blockIdx.y, share = blockIdx.z;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int first_tok = q_start[b], n_new = q_start[b + 1] - first_tok;
+    const int rows_total = n_new * H, r0 = blockIdx.x * TC_ROWS;
+    if (r0 >= rows_total) return;
+    const int n_rows = min(TC_ROWS, rows_total - r0);
+    const int first_pos = kv_len[b] - n_new;
+    const int last_pos = first_pos + (r0 + n_rows - 1) / H;
+    const int blk_first = window > 0 ? max(0, first_pos + r0 / H - window + 1) / TC_KEYS : 0;
+    const int blk_end = last_pos / TC_KEYS + 1;
+    const int per = (blk_end - blk_first + shares - 1) / shares;
+    const int blk_lo = blk_first + share * per, blk_hi = min(blk_lo + per, blk_end);
+    const int* pt = page_table + (long long)b * pt_stride;
+    // a warp brings rows warp, warp + 8, ..., a lane 16 bytes of a row at a time: the addresses only count up
+    auto fetch = [&](int blk) {
+        if (blk < blk_hi) {
+            const int k0 = blk * TC_KEYS;
+            const __nv_bfloat16* from = pages + ((long long)pt[k0 / page_size] * page_size + k0 % page_size + warp) * Dk + lane * 8;
+            uint32_t to = smem_at(Ks + ((blk & 1) * TC_KEYS + warp) * stride + lane * 8);
+#pragma unroll
+            for (int u = 0; u < TC_KEYS / WARPS; ++u) {
+                const int bytes = k0 + warp + u * WARPS <= last_pos ? 16 : 0;          // rows beyond the last position are zero
+                const __nv_bfloat16* src = bytes ? from : pages;
+                for (int c = lane * 8, d = 0; c < Dk; c += 256, d += 256)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + d * 2), "l"(src + (bytes ? d : 0)), "r"(bytes) : "memory");
+                from += (long long)WARPS * Dk;
+                to += WARPS * stride * 2;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(blk_lo);
+    for (int r = warp; r < TC_ROWS; r += WARPS) {
+        const float* src = qa + ((long long)first_tok * H + r0 + r) * Dk;
+#pragma unroll 5
+        for (int e = lane * 4; e < Dk; e += 128) {
+            const float4 x = r < n_rows ? *(const float4*)(src + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float v[4] = {x.x, x.y, x.z, x.w};
+            __nv_bfloat16 p[4][3];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) three_parts(v[i], p[i]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                __nv_bfloat162* to = (__nv_bfloat162*)(Qs + (k * TC_ROWS + r) * stride + e);
+                to[0] = __halves2bfloat162(p[0][k], p[1][k]);
+                to[1] = __halves2bfloat162(p[2][k], p[3][k]);
+            }
+        }
+    }
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};        // of rows 2 warp, 2 warp + 1
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[n][k] = 0.f;
+    const int key_group = warp & 1, quarter = warp >> 1;
+    const int k_steps = Dk / 16, step_lo = quarter * k_steps / 4, step_hi = (quarter + 1) * k_steps / 4;
+    for (int blk = blk_lo; blk < blk_hi; ++blk) {
+        fetch(blk + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const __nv_bfloat16* K = Ks + (blk & 1) * TC_KEYS * stride;
+        {
+            // a chain of products per part and tile of 8 keys: none waits for another
+            float s[3][4][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[p][n][k] = 0.f;
+            const uint32_t a_at = smem_at(Qs + (lane & 15) * stride + (lane >> 4) * 8);
+            const uint32_t b_at = smem_at(K + (key_group * 32 + (lane >> 4) * 8 + (lane & 7)) * stride + ((lane >> 3) & 1) * 8);
+#pragma unroll 3
+            for (int step = step_lo; step < step_hi; ++step) {
+                uint32_t kf[2][4];
+                ldmatrix4(b_at + step * 32, kf[0]);
+                ldmatrix4(b_at + 16 * stride * 2 + step * 32, kf[1]);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    uint32_t qf[4];
+                    ldmatrix4(a_at + p * TC_ROWS * stride * 2 + step * 32, qf);
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) mma_bf16(s[p][n], qf, kf[n >> 1][(n & 1) * 2], kf[n >> 1][(n & 1) * 2 + 1]);
+                }
+            }
+            float* to = Ss + (quarter * TC_ROWS + (lane >> 2)) * TC_SSTRIDE + key_group * 32 + (lane & 3) * 2;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                float v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = s[0][n][k] + (s[1][n][k] + s[2][n][k]);
+                *(float2*)(to + n * 8) = make_float2(v[0], v[1]);
+                *(float2*)(to + 8 * TC_SSTRIDE + n * 8) = make_float2(v[2], v[3]);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = 2 * warp + i, pos = r < n_rows ? first_pos + (r0 + r) / H : -1;
+            float sc[2], p[2];
+            bool seen[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int key = blk * TC_KEYS + lane + 32 * k;
+                seen[k] = key <= pos && (window <= 0 || key > pos - window);
+                const float* from = Ss + r * TC_SSTRIDE + lane + 32 * k;
+                const float dot = (from[0] + from[TC_ROWS * TC_SSTRIDE]) + (from[2 * TC_ROWS * TC_SSTRIDE] + from[3 * TC_ROWS * TC_SSTRIDE]);
+                sc[k] = seen[k] ? dot * scale : -INFINITY;
+            }
+            const float m_new = fmaxf(m[i], lp_warp_max(fmaxf(sc[0], sc[1])));
+            float alpha = 1.f;
+            p[0] = p[1] = 0.f;
+            if (m_new != -INFINITY) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) p[k] = seen[k] ? expf(sc[k] - m_new) : 0.f;
+                alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+            }
+            l[i] = l[i] * alpha + lp_warp_sum(p[0] + p[1]);
+            m[i] = m_new;
+            if (lane == 0) alphas[r] = alpha;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                __nv_bfloat16 parts[3];
+                three_parts(p[k], parts);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) Ps[(q * TC_ROWS + r) * TC_PSTRIDE + lane + 32 * k] = parts[q];
+            }
+        }
+        __syncthreads();
+        const float f0 = alphas[lane >> 2], f1 = alphas[(lane >> 2) + 8];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            acc[n][0] *= f0;
+            acc[n][1] *= f0;
+            acc[n][2] *= f1;
+            acc[n][3] *= f1;
+        }
+        const uint32_t p_at = smem_at(Ps + (lane & 15) * TC_PSTRIDE + (lane >> 4) * 8);
+        const uint32_t c_at = smem_at(K + (lane & 15) * stride + warp * (NT * 8) + (lane >> 4) * 8);
+#pragma unroll
+        for (int step = 0; step < TC_KEYS / 16; ++step) {
+            uint32_t pf[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) ldmatrix4(p_at + p * TC_ROWS * TC_PSTRIDE * 2 + step * 32, pf[p]);
+#pragma unroll
+            for (int n = 0; n < NT; n += 2) {
+                uint32_t cf[4];
+                // (NT = 1: the second tile belongs to the next warp or to the key part; it is read and not used)
+                ldmatrix4_trans(c_at + step * 16 * stride * 2 + n * 16, cf);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    mma_bf16(acc[n], pf[p], cf[0], cf[1]);
+                    if (n + 1 < NT) mma_bf16(acc[n + 1 < NT ? n + 1 : n], pf[p], cf[2], cf[3]);
+                }
+            }
+        }
+        __syncthreads();                                  // the block's rows may be overwritten
+    }
+    const int row_a = lane >> 2, col = warp * (NT * 8) + (lane & 3) * 2;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int r = row_a + 8 * i;
+        if (r >= n_rows) continue;
+        float* dst = part + (((long long)first_tok * H + r0 + r) * shares + share) * (rank + 2) + col;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) *(float2*)(dst + n * 8) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = 2 * warp + i;
+            if (r >= n_rows) continue;
+            float* dst = part + (((long long)first_tok * H + r0 + r) * shares + share) * (rank + 2) + rank;
+            dst[0] = m[i];
+            dst[1] = l[i];
+        }
+}
+
+// Whether the tensor-core kernel serves these sizes: a rank of 64, 128, 256 or 512, rows of a multiple of 16 values that
+// fit shared memory, pages of whole blocks.
+inline bool attend_on_tensor_cores(int kv_dtype, int rank, int dr, int page_size) {
+    return kv_dtype == LP_BF16 && (rank == 64 || rank == 128 || rank == 256 || rank == 512) && dr % 16 == 0 &&
+           page_size % TC_KEYS == 0 && tc_smem(rank + dr) <= 227 * 1024 - 256;
+}
+
 // ---------------------------------------------------------------- merge
 // The shares of one (token, head) row become one: out = [sum_s o_s e^(m_s - M) / sum_s l_s e^(m_s - M) | 0 | 1],
 // the form of a single share whose sum of weights is one. One CTA per row; every warp forms the weights.
@@ -519,6 +762,176 @@ latent_expand_rows_kernel(const float* __restrict__ part, int shares, const TW* 
     }
 }
 
+// ---------------------------------------------------------------- absorb and expand on the tensor cores
+// Both maps are products per head with bfloat16 weights and a float32 operand: the weights are exact operands, the other is
+// split into three bfloat16 parts (24 bits), sums are float32. 16 tokens per CTA, so a head's weights are read once per 16
+// tokens, from L2.
+
+// qa[t, h, r] = sum over d of uk[h, d, r] q[t, h, d]: 64 columns of the latent per CTA, 16 per warp. Bound by latency: 32
+// tokens, 16 heads of 128, rank 512, B200: 28 us with a thread per column (above) -> 12 (cold caches).
+constexpr int AB_COLS = 64, AB_WARPS = 4;
+__global__ void __launch_bounds__(AB_WARPS * 32)
+latent_absorb_tc_kernel(const float* __restrict__ q, const __nv_bfloat16* __restrict__ uk, float* __restrict__ qa, int T, int H, int dn,
+                        int dr, int rank) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    const int stride = dn + 8;
+    constexpr int WSTRIDE = AB_COLS + 8;
+    __nv_bfloat16* Qs = (__nv_bfloat16*)raw;                  // [3][16][stride]
+    __nv_bfloat16* Ws = Qs + 3 * TC_ROWS * stride;            // [dn][WSTRIDE]
+    const int t0 = blockIdx.x * TC_ROWS, h = blockIdx.y, c0 = blockIdx.z * AB_COLS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int hd = dn + dr, Dk = rank + dr, nt = min(TC_ROWS, T - t0);
+    // weights are written by no kernel of a step: asked for before the wait
+    for (int i = tid; i < dn * (AB_COLS / 8); i += AB_WARPS * 32) {
+        const int d = i / (AB_COLS / 8), c = i % (AB_COLS / 8) * 8;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                     ::"r"(smem_at(Ws + d * WSTRIDE + c)), "l"(uk + ((long long)h * dn + d) * rank + c0 + c) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    lp_grid_release();
+    lp_grid_wait();
+    for (int e = tid; e < TC_ROWS * dn; e += AB_WARPS * 32) {
+        const int i = e / dn, d = e - i * dn;
+        __nv_bfloat16 p[3];
+        three_parts(i < nt ? q[((long long)(t0 + i) * H + h) * hd + d] : 0.f, p);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) Qs[(k * TC_ROWS + i) * stride + d] = p[k];
+    }
+    if (blockIdx.z == 0)
+        for (int e = tid; e < nt * dr; e += AB_WARPS * 32) {
+            const int i = e / dr, d = e - i * dr;
+            qa[((long long)(t0 + i) * H + h) * Dk + rank + d] = q[((long long)(t0 + i) * H + h) * hd + dn + d];
+        }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    const uint32_t a_at = smem_at(Qs + (lane & 15) * stride + (lane >> 4) * 8);
+    const uint32_t b_at = smem_at(Ws + (lane & 15) * WSTRIDE + warp * 16 + (lane >> 4) * 8);
+    for (int step = 0; step < dn / 16; ++step) {
+        uint32_t wf[4];
+        ldmatrix4_trans(b_at + step * 16 * WSTRIDE * 2, wf);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            uint32_t qf[4];
+            ldmatrix4(a_at + p * TC_ROWS * stride * 2 + step * 32, qf);
+            mma_bf16(acc[0], qf, wf[0], wf[1]);
+            mma_bf16(acc[1], qf, wf[2], wf[3]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int r = (lane >> 2) + 8 * i;
+        if (r >= nt) continue;
+        float* to = qa + ((long long)(t0 + r) * H + h) * Dk + c0 + warp * 16 + (lane & 3) * 2;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) *(float2*)(to + n * 8) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
+    }
+}
+
+// out[t, h * dv + v] = gate * sum over r of uv[h, v, r] latent[t, h, r], the latent being the merge of the shares: 32 value
+// features per CTA, 8 per pair of warps, each with half of the rank; the halves meet in shared memory. Every CTA merges the
+// shares of its 16 (token, head) rows itself. Bound by latency: 32 tokens, 16 heads of 128, rank 512, 4 shares, B200:
+// 26 us with a CTA per row (above) -> 19 (cold caches; 38 with
+// one row's shares asked for at a time).
+constexpr int EX_FEATURES = 32, EX_WARPS = 8;
+template <typename TOut>
+__global__ void __launch_bounds__(EX_WARPS * 32, 2)
+latent_expand_tc_kernel(const float* __restrict__ part, int shares, const __nv_bfloat16* __restrict__ uv, const float* __restrict__ gate,
+                        int ldg, TOut* __restrict__ out, int T, int H, int rank, int dv, float* __restrict__ zero, long long zero_count) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    const int stride = rank + 8;
+    __nv_bfloat16* Ls = (__nv_bfloat16*)raw;                  // [3][16][stride]
+    __nv_bfloat16* Ws = Ls + 3 * TC_ROWS * stride;            // [EX_FEATURES][stride]
+    float* ws = (float*)(Ws + EX_FEATURES * stride);          // [16][shares]
+    __shared__ float gs[TC_ROWS];
+    __shared__ float halves[TC_ROWS][EX_FEATURES];
+    const int t0 = blockIdx.x * TC_ROWS, h = blockIdx.y, v0 = blockIdx.z * EX_FEATURES;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nt = min(TC_ROWS, T - t0), width = rank + 2, nv = min(EX_FEATURES, dv - v0);
+    for (int i = tid; i < EX_FEATURES * (rank / 8); i += EX_WARPS * 32) {
+        const int v = i / (rank / 8), c = i % (rank / 8) * 8;
+        const int bytes = v < nv ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"(smem_at(Ws + v * stride + c)), "l"(v < nv ? uv + ((long long)h * dv + v0 + v) * rank + c : uv), "r"(bytes) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    lp_grid_release();
+    lp_grid_wait();
+    clear_on_the_side(zero, zero_count);
+    for (int i = warp; i < nt; i += EX_WARPS) {
+        const float* p = part + ((long long)(t0 + i) * H + h) * shares * width;
+        float M = -INFINITY;
+        for (int s = lane; s < shares; s += 32) M = fmaxf(M, p[s * width + rank]);
+        M = lp_warp_max(M);
+        float L = 0.f;
+        for (int s = lane; s < shares; s += 32) {
+            const float ms = p[s * width + rank];
+            const float e = ms == -INFINITY ? 0.f : expf(ms - M);
+            ws[i * shares + s] = e;
+            L += p[s * width + rank + 1] * e;
+        }
+        L = lp_warp_sum(L);
+        const float inv = 1.0f / L;
+        for (int s = lane; s < shares; s += 32) ws[i * shares + s] *= inv;
+        if (lane == 0) gs[i] = gate ? 1.0f / (1.0f + expf(-gate[(long long)(t0 + i) * ldg + h])) : 1.0f;
+    }
+    __syncthreads();
+    for (int r = tid * 2; r < rank; r += EX_WARPS * 64)
+#pragma unroll 4
+        for (int i = 0; i < TC_ROWS; ++i) {
+            float2 v = make_float2(0.f, 0.f);
+            if (i < nt) {
+                const float* p = part + ((long long)(t0 + i) * H + h) * shares * width + r;
+                const float* wi = ws + i * shares;
+#pragma unroll 4
+                for (int s = 0; s < shares; ++s) {
+                    const float2 x = *(const float2*)(p + (long long)s * width);
+                    v.x = fmaf(x.x, wi[s], v.x);
+                    v.y = fmaf(x.y, wi[s], v.y);
+                }
+            }
+            __nv_bfloat16 a[3], b[3];
+            three_parts(v.x, a);
+            three_parts(v.y, b);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) *(__nv_bfloat162*)(Ls + (k * TC_ROWS + i) * stride + r) = __halves2bfloat162(a[k], b[k]);
+        }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int group = warp & 3, half = warp >> 2;             // 8 features; half of the rank
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const int pairs = rank / 32;                              // steps of 32: two MMA steps per ldmatrix of the weights
+    const uint32_t a_at = smem_at(Ls + (lane & 15) * stride + (lane >> 4) * 8);
+    const uint32_t b_at = smem_at(Ws + (group * 8 + (lane & 7)) * stride + (lane >> 3) * 8);
+#pragma unroll 2
+    for (int step = half * pairs / 2; step < (half + 1) * pairs / 2; ++step) {
+        uint32_t wf[4];
+        ldmatrix4(b_at + step * 64, wf);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                uint32_t lf[4];
+                ldmatrix4(a_at + p * TC_ROWS * stride * 2 + step * 64 + k * 32, lf);
+                mma_bf16(acc, lf, wf[2 * k], wf[2 * k + 1]);
+            }
+    }
+    const int row = lane >> 2, col = group * 8 + (lane & 3) * 2;
+    if (half) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) halves[row + (i >> 1) * 8][col + (i & 1)] = acc[i];
+    }
+    __syncthreads();
+    if (!half) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = row + (i >> 1) * 8, v = col + (i & 1);
+            if (r < nt && v < nv)
+                out[((long long)(t0 + r) * H + h) * dv + v0 + v] = lp_from_float<TOut>((acc[i] + halves[r][v]) * gs[r]);
+        }
+    }
+}
+
 template <typename K>
 int grant_shared(K kernel, size_t bytes, const char* what) {
     if (bytes > 48 * 1024) {
@@ -590,6 +1003,15 @@ extern "C" int lp_latent_absorb(const float* q, const void* uk, int w_dtype, flo
                                 int rank, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (H <= 0 || H > 65535 || dn < 0 || dr < 0 || rank <= 0) LP_REFUSE("latent_absorb: %d heads of %d + %d over rank %d", H, dn, dr, rank);
+    // bfloat16 weights whose tiles can be read 16 bytes at a time go to the tensor cores
+    const size_t tc_bytes = ((size_t)3 * TC_ROWS * (dn + 8) + (size_t)dn * (AB_COLS + 8)) * 2;
+    if (w_dtype == LP_BF16 && dn > 0 && dn % 16 == 0 && rank % AB_COLS == 0 && dr % 2 == 0 && (uintptr_t)uk % 16 == 0 && (uintptr_t)qa % 8 == 0 &&
+        tc_bytes <= 200 * 1024) {
+        if (grant_shared(latent_absorb_tc_kernel, tc_bytes, "latent_absorb")) return -1;
+        lp_launch(latent_absorb_tc_kernel, dim3((T + TC_ROWS - 1) / TC_ROWS, H, rank / AB_COLS), AB_WARPS * 32, tc_bytes, stream, q,
+                  (const __nv_bfloat16*)uk, qa, T, H, dn, dr, rank);
+        return lp_check_launch("latent_absorb");
+    }
     dim3 grid((T + TOK_TILE - 1) / TOK_TILE, H, (rank + 127) / 128);
     const size_t smem = (size_t)TOK_TILE * (dn > 0 ? dn : 1) * sizeof(float);
     if (w_dtype == LP_F32) {
@@ -604,8 +1026,13 @@ extern "C" int lp_latent_absorb(const float* q, const void* uk, int w_dtype, flo
 
 constexpr int ATTEND_RW = 4;
 
-// How many (token, head) rows one CTA of lp_latent_attend takes.
-extern "C" int lp_latent_attend_rows() { return WARPS * ATTEND_RW; }
+// How many (token, head) rows one CTA of lp_latent_attend takes, and how many keys a block holds.
+extern "C" int lp_latent_attend_rows(int kv_dtype, int rank, int dr, int page_size) {
+    return attend_on_tensor_cores(kv_dtype, rank, dr, page_size) ? TC_ROWS : WARPS * ATTEND_RW;
+}
+extern "C" int lp_latent_attend_keys(int kv_dtype, int rank, int dr, int page_size) {
+    return attend_on_tensor_cores(kv_dtype, rank, dr, page_size) ? TC_KEYS : KEYS;
+}
 
 // qa: float32 [T, H, rank + dr]; part: float32 [T, H, shares, rank + 2] (unnormalised sums, maximum, sum of
 // weights); q_start [B + 1], kv_len [B] (lengths after the step); max_new: most new tokens of a sequence.
@@ -618,6 +1045,23 @@ extern "C" int lp_latent_attend(const float* qa, const void* pages, int kv_dtype
     if (rank > 512) LP_REFUSE("latent_attend: rank %d (supported: up to 512)", rank);
     if (page_size <= 0 || page_size % KEYS) LP_REFUSE("latent_attend: page size %d must be a multiple of %d", page_size, KEYS);
     if (shares <= 0 || shares > 65535 || B > 65535) LP_REFUSE("latent_attend: %d shares, %d sequences", shares, B);
+    if (attend_on_tensor_cores(kv_dtype, rank, dr, page_size) && (uintptr_t)pages % 16 == 0 && (uintptr_t)qa % 16 == 0 &&
+        (uintptr_t)part % 8 == 0) {
+        const size_t bytes = tc_smem(rank + dr);
+        const dim3 tc_grid((unsigned)(((long long)max_new * H + TC_ROWS - 1) / TC_ROWS), B, shares);
+#define LP_LAUNCH_TC(NT)                                                                                                     \
+    do {                                                                                                                     \
+        if (grant_shared(latent_attend_tc_kernel<NT>, bytes, "latent_attend")) return -1;                                    \
+        lp_launch(latent_attend_tc_kernel<NT>, tc_grid, WARPS * 32, bytes, stream, qa, (const __nv_bfloat16*)pages,          \
+                  page_table, pt_stride, q_start, kv_len, part, H, dr, page_size, scale, shares, window);                    \
+    } while (0)
+        if (rank == 64) LP_LAUNCH_TC(1);
+        else if (rank == 128) LP_LAUNCH_TC(2);
+        else if (rank == 256) LP_LAUNCH_TC(4);
+        else LP_LAUNCH_TC(8);
+#undef LP_LAUNCH_TC
+        return lp_check_launch("latent_attend");
+    }
     constexpr int ROWS = WARPS * ATTEND_RW;
     const int Dk = rank + dr;
     const size_t smem = ((size_t)ROWS * Dk + (size_t)KEYS * (Dk + 4)) * sizeof(float);
@@ -663,6 +1107,21 @@ extern "C" int lp_latent_expand(const float* part, int shares, const void* uv, i
                                 cudaStream_t stream) {
     if (T <= 0) return 0;
     if (H <= 0 || H > 65535 || rank <= 0 || dv <= 0 || shares <= 0) LP_REFUSE("latent_expand: %d heads, rank %d, values of %d, %d shares", H, rank, dv, shares);
+    const size_t tc_bytes = ((size_t)3 * TC_ROWS + EX_FEATURES) * (rank + 8) * 2 + (size_t)TC_ROWS * shares * sizeof(float);
+    if (w_dtype == LP_BF16 && rank % 64 == 0 && (uintptr_t)uv % 16 == 0 && (uintptr_t)part % 8 == 0 && tc_bytes <= 200 * 1024 &&
+        (out_dtype == LP_BF16 || out_dtype == LP_F32)) {
+        const dim3 tc_grid((T + TC_ROWS - 1) / TC_ROWS, H, (dv + EX_FEATURES - 1) / EX_FEATURES);
+#define LP_LAUNCH_TC(TOut)                                                                                           \
+    do {                                                                                                             \
+        if (grant_shared(latent_expand_tc_kernel<TOut>, tc_bytes, "latent_expand")) return -1;                       \
+        lp_launch(latent_expand_tc_kernel<TOut>, tc_grid, EX_WARPS * 32, tc_bytes, stream, part, shares,             \
+                  (const __nv_bfloat16*)uv, gate, ldg, (TOut*)out, T, H, rank, dv, zero, zero_count);                \
+    } while (0)
+        if (out_dtype == LP_BF16) LP_LAUNCH_TC(__nv_bfloat16);
+        else LP_LAUNCH_TC(float);
+#undef LP_LAUNCH_TC
+        return lp_check_launch("latent_expand");
+    }
     if (T <= ROWS_FORM_TOKENS) {
         const size_t bytes = (size_t)(rank + shares) * sizeof(float);
 #define LP_LAUNCH_ROWS(TW, TOut)                                                                                     \

@@ -81,7 +81,8 @@ _SIGNATURES = {
         "lp_latent_heads_to_pages": [_P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
         "lp_latent_gate_heads": [_P, _P, _I, _P, _I, _I, _I, _I, _P, ctypes.c_longlong, _P],
         "lp_latent_absorb": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _P],
-        "lp_latent_attend_rows": [],
+        "lp_latent_attend_rows": [_I, _I, _I, _I],
+        "lp_latent_attend_keys": [_I, _I, _I, _I],
         "lp_latent_attend": [_P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P],
         "lp_latent_merge": [_P, _I, _P, _I, _I, _P],
         "lp_latent_query_norm": [_P, _I, _I, _I, _P, _F, _P, _I, _I, _P],
@@ -1306,12 +1307,21 @@ def latent_absorb(q: torch.Tensor, k_up: torch.Tensor, out: torch.Tensor, *, nop
     return out
 
 
-def latent_shares(batch: int, max_new: int, num_heads: int, table_width: int, page_size: int) -> int:
+def latent_shares(batch: int, max_new: int, num_heads: int, table_width: int, page_size: int, pages: Optional[torch.Tensor] = None,
+                  kv_rank: int = 0, window: Optional[int] = None) -> int:
     """Into how many shares :func:`latent_attend` cuts a sequence's keys: one while the (token, head) rows
-    alone fill the SMs, else as many as the SMs have room for, down to shares of one block of 32 keys."""
-    rows = library("latent_attention").lp_latent_attend_rows()
+    alone fill the SMs, else as many as the SMs have room for, down to shares of one block of keys. ``pages`` and
+    ``kv_rank`` say which kernel will run (its rows per CTA and keys per block); ``window``: no row sees more keys."""
+    rows, keys = 32, 32
+    if pages is not None:
+        sizes = (_code(pages, "latent_attend pages"), kv_rank, pages.shape[2] - kv_rank, page_size)
+        lib = library("latent_attention")
+        rows, keys = lib.lp_latent_attend_rows(*sizes), lib.lp_latent_attend_keys(*sizes)
     ctas = batch * -(-max_new * num_heads // rows)
-    return max(1, min(num_sms() // max(ctas, 1), table_width * (page_size // 32)))
+    blocks = table_width * (page_size // keys)
+    if window is not None:
+        blocks = min(blocks, -(-window // keys) + 1)          # a row sees that many blocks at most
+    return max(1, min(num_sms() // max(ctas, 1), blocks))
 
 
 def latent_attend(q_abs: torch.Tensor, pages: torch.Tensor, page_table: torch.Tensor, q_start: torch.Tensor,

@@ -125,9 +125,8 @@ class LatentAttention(Part):
         q_abs = ctx.buffer("latent_q_absorbed", (T, H, rank + dr), torch.float32)
         with ops.section("attention.absorb"):
             ops.latent_absorb(q, self.k_up, q_abs, nope_dim=dn, rope_dim=dr)
-        shares = ops.latent_shares(ctx.num_sequences, ctx.max_new, H, table.shape[1], cache.pages.shape[1])
-        if s.window is not None:
-            shares = min(shares, -(-s.window // 32) + 1)        # a row sees that many blocks of 32 keys at most
+        shares = ops.latent_shares(ctx.num_sequences, ctx.max_new, H, table.shape[1], cache.pages.shape[1], cache.pages, rank,
+                                   s.window)
         partials = ctx.buffer("latent_partials", (T, H, shares, rank + 2), torch.float32)
         with ops.section("attention.scores"):
             ops.latent_attend(q_abs, cache.pages, table, ctx.q_start, ctx.kv_len, partials, max_new=ctx.max_new,

@@ -1,0 +1,86 @@
+"""Latent attention over a bfloat16 cache on the tensor cores: queries, weights and latents in three bfloat16 parts. Each kernel
+against float64, at the edges of its blocks of 64 keys and tiles of 16 rows, with windows, shares and several new tokens."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rel(got, ref):
+    return float((got.double() - ref).abs().max() / ref.abs().max())
+
+
+@pytest.mark.parametrize("rank,dr,H", [(64, 0, 3), (128, 16, 16), (256, 32, 8), (512, 64, 16), (512, 64, 40)])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("shares", [1, 3, 7])
+def test_attend(rank, dr, H, window, shares):
+    from llmplayer_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(rank + H)
+    before, new = [0, 63, 64, 200, 129], [5, 1, 1, 1, 3]
+    lengths = [a + b for a, b in zip(before, new)]
+    width, Dk = 5, rank + dr
+    pages = torch.randn(len(before) * width, 64, Dk, generator=g, device=DEV).to(torch.bfloat16)
+    order = torch.randperm(len(before) * width, generator=torch.Generator().manual_seed(1)).reshape(len(before), width)
+    for i, n in enumerate(lengths):                       # what lies behind a sequence's last row is no number
+        page = order[i, (n - 1) // 64]
+        pages[page, (n - 1) % 64 + 1:] = float("nan")
+    table = order.clone().to(torch.int32)
+    for i, b in enumerate(before):                        # pages that no row reaches any more are gone
+        if window is not None:
+            table[i, :max(0, b - window + 1) // 64] = -1
+    T = sum(new)
+    q = torch.randn(T, H, Dk, generator=g, device=DEV)
+    part = torch.full((T, H, shares, rank + 2), float("nan"), device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    starts = [sum(new[:i]) for i in range(len(new) + 1)]
+    scale = Dk ** -0.5
+    ops.latent_attend(q, pages, table.to(DEV), i32(starts), i32(lengths), part, max_new=max(new), kv_rank=rank, scale=scale, window=window)
+    assert bool(torch.isfinite(part[..., :rank]).all())
+    for i, n in enumerate(new):
+        rows = torch.cat([pages[order[i, p // 64], p % 64][None] for p in range(lengths[i])]).double()
+        for k in range(n):
+            t, pos = starts[i] + k, before[i] + k
+            lo = max(0, pos - window + 1) if window else 0
+            s = q[t].double() @ rows[lo:pos + 1].T * scale
+            w = torch.softmax(s, -1)
+            p = part[t].double()
+            m = p[:, :, rank].max(-1, keepdim=True).values
+            f = torch.exp(p[:, :, rank] - m)
+            got = (p[:, :, :rank] * f[..., None]).sum(1) / (p[:, :, rank + 1] * f).sum(-1, keepdim=True)
+            # float32 sums of 24-bit products
+            assert rel(got, w @ rows[lo:pos + 1, :rank]) < 3e-6, (i, k)
+
+
+@pytest.mark.parametrize("T,H,dn,dr,rank", [(1, 3, 16, 8, 64), (16, 2, 48, 0, 128), (33, 16, 128, 64, 512)])
+def test_absorb(T, H, dn, dr, rank):
+    from llmplayer_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    q = torch.randn(T, H, dn + dr, generator=g, device=DEV)
+    uk = torch.randn(H * dn, rank, generator=g, device=DEV).to(torch.bfloat16)
+    out = torch.full((T, H, rank + dr), float("nan"), device=DEV)
+    ops.latent_absorb(q, uk, out, nope_dim=dn, rope_dim=dr)
+    ref = torch.einsum("thd,hdr->thr", q[..., :dn].double(), uk.double().reshape(H, dn, rank))
+    assert rel(out[..., :rank], ref) < 2e-6 and torch.equal(out[..., rank:], q[..., dn:])
+
+
+@pytest.mark.parametrize("T,H,dv,rank,shares", [(1, 3, 8, 64, 1), (17, 2, 40, 192, 5), (33, 16, 128, 512, 4), (80, 4, 64, 256, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_expand(T, H, dv, rank, shares, dtype):
+    from llmplayer_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    part = torch.randn(T, H, shares, rank + 2, generator=g, device=DEV)
+    part[..., rank + 1] = 0.5 + part[..., rank + 1].abs()
+    if shares > 1:                                        # an empty share
+        part[:, :, 1] = 0.0
+        part[:, :, 1, rank] = -float("inf")
+    uv = torch.randn(H * dv, rank, generator=g, device=DEV).to(torch.bfloat16)
+    gate = torch.randn(T, H, generator=g, device=DEV)
+    out = torch.empty(T, H * dv, device=DEV, dtype=dtype)
+    junk = torch.ones(1000, device=DEV)
+    ops.latent_expand(part, uv, gate, out, value_dim=dv, clear=junk)
+    p = part.double()
+    f = torch.exp(p[..., rank] - p[..., rank].max(-1, keepdim=True).values)
+    latent = (p[..., :rank] * f[..., None]).sum(2) / (p[..., rank + 1] * f).sum(-1, keepdim=True)
+    ref = torch.einsum("thr,hvr->thv", latent, uv.double().reshape(H, dv, rank)) * torch.sigmoid(gate.double())[..., None]
+    assert rel(out.reshape(T, H, dv), ref) < (3e-6 if dtype == torch.float32 else 5e-3) and float(junk.abs().sum()) == 0.0
