@@ -1182,7 +1182,7 @@ def attention(ctx, q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, page
 
 # --------------------------------------------------------------------------- latent attention
 def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, gain: torch.Tensor, eps: float, rotation: Rotation,
-                   positions: torch.Tensor, seq_ids: torch.Tensor, page_table: torch.Tensor, q_out: torch.Tensor,
+                   positions: torch.Tensor, seq_ids: torch.Tensor, page_table: torch.Tensor, q_out: Optional[torch.Tensor],
                    pages: torch.Tensor, *, num_heads: int, nope_dim: int, rope_dim: int, kv_rank: int,
                    latent_out: Optional[torch.Tensor] = None, shared_out: Optional[torch.Tensor] = None,
                    q_half: Optional[torch.Tensor] = None, q_from: Optional[torch.Tensor] = None) -> None:
@@ -1191,21 +1191,22 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, gain: torch.Tens
     part and write both into ``pages`` [num_pages, page_size, rank + rope] at the tokens' positions; rotate the
     queries' rope parts and write the queries to ``q_out`` float32 [T, H, nope + rope]. Optional bfloat16 copies
     that lie together, for a step that forms every head's keys and values outright: ``latent_out`` [T, rank],
-    ``shared_out`` [T, rope], ``q_half`` [T, H * hd] with hd >= nope + rope (heads padded with zeros).
-    ``q_from``: float32 [T, H * (nope + rope)] (may be a column slice): the queries, when they come from a product
+    ``shared_out`` [T, rope], ``q_half`` [T, H * hd] with hd >= nope + rope (heads padded with zeros; ``q_out`` may then be
+    None). ``q_from``: float32 [T, H * (nope + rope)] (may be a column slice): the queries, when they come from a product
     of their own (queries formed through a latent) instead of from ``proj``."""
     _want(proj, "latent_prepare proj", torch.float32, 2)
     _want(gain, "latent_prepare gain", torch.float32, 1)
     _want(positions, "latent_prepare positions", torch.int32, 1)
     _want(seq_ids, "latent_prepare seq_ids", torch.int32, 1)
     _want(page_table, "latent_prepare page_table", torch.int32, 2)
-    _want(q_out, "latent_prepare q_out", torch.float32, 3)
+    if q_out is not None or q_half is None:
+        _want(q_out, "latent_prepare q_out", torch.float32, 3)
     _want(pages, "latent_prepare pages", ndim=3)
     T = proj.shape[0]
     H, dn, dr, rank = num_heads, nope_dim, rope_dim, kv_rank
-    if (q_out.shape != (T, H, dn + dr) or pages.shape[2] != rank + dr or gain.numel() != rank
+    if ((q_out is not None and q_out.shape != (T, H, dn + dr)) or pages.shape[2] != rank + dr or gain.numel() != rank
             or positions.numel() != T or seq_ids.numel() != T):
-        raise KernelError(f"latent_prepare: proj {tuple(proj.shape)}, q_out {tuple(q_out.shape)}, pages "
+        raise KernelError(f"latent_prepare: proj {tuple(proj.shape)}, q_out {None if q_out is None else tuple(q_out.shape)}, pages "
                           f"{tuple(pages.shape)} for {H} heads of {dn} + {dr} over rank {rank}")
     for extra, shape, what in ((latent_out, (T, rank), "latent_out"), (shared_out, (T, dr), "shared_out")):
         if extra is not None:
@@ -1227,7 +1228,7 @@ def latent_prepare(proj: torch.Tensor, q_off: int, kv_off: int, gain: torch.Tens
     lib = library("latent_attention")
     _check(lib, lib.lp_latent_prepare(
         proj.data_ptr(), proj.shape[1], int(q_off), int(kv_off), gain.data_ptr(), float(eps), freq_ptr, rot,
-        positions.data_ptr(), seq_ids.data_ptr(), page_table.data_ptr(), page_table.shape[1], q_out.data_ptr(),
+        positions.data_ptr(), seq_ids.data_ptr(), page_table.data_ptr(), page_table.shape[1], _ptr(q_out),
         pages.data_ptr(), _code(pages, "latent_prepare pages"), T, H, dn, dr, rank, pages.shape[1], _ptr(latent_out),
         _ptr(shared_out), _ptr(q_half), q_half_hd, q_ptr, ldq, interleaved, float(rotation.magnitude), _stream()))
 

@@ -116,9 +116,9 @@ class LatentAttention(Part):
                 ops.latent_query_norm(proj, q_off, self.q_gain, s.norm_eps, q_latent)
                 q_from = ctx.buffer("latent_q_proj", (T, H * (dn + dr)), torch.float32)
                 self.q_up.store(q_latent, q_from, ctx)
-        q = ctx.buffer("latent_q", (T, H, dn + dr), torch.float32)
         if self._forms_heads(ctx, cache):
-            return self._forward_heads(ctx, cache, proj, q_off, kv_off, gate_off, rotation, table, q, out, q_from, add)
+            return self._forward_heads(ctx, cache, proj, q_off, kv_off, gate_off, rotation, table, out, q_from, add)
+        q = ctx.buffer("latent_q", (T, H, dn + dr), torch.float32)
         with ops.section("attention.position"):
             ops.latent_prepare(proj, q_off, kv_off, self.latent_gain, s.norm_eps, rotation, ctx.positions, ctx.seq_ids,
                                table, q, cache.pages, num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank, q_from=q_from)
@@ -175,7 +175,7 @@ class LatentAttention(Part):
         need = self.spec.nope_dim + self.spec.rope_dim
         return next((size for size in (64, 128, 192, 256) if need <= size), None)
 
-    def _forward_heads(self, ctx, cache, proj, q_off, kv_off, gate_off, rotation, table, q, out, q_from=None, add=False):
+    def _forward_heads(self, ctx, cache, proj, q_off, kv_off, gate_off, rotation, table, out, q_from=None, add=False):
         s = self.spec
         T = proj.shape[0]
         H, dn, dr, dv, rank = s.num_heads, s.nope_dim, s.rope_dim, s.value_dim, s.kv_rank
@@ -186,7 +186,7 @@ class LatentAttention(Part):
         q_half = ctx.buffer("q", (T, H * hd), torch.bfloat16)
         with ops.section("attention.position"):
             ops.latent_prepare(proj, q_off, kv_off, self.latent_gain, s.norm_eps, rotation, ctx.positions, ctx.seq_ids,
-                               table, q, cache.pages, num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank,
+                               table, None, cache.pages, num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank,
                                latent_out=latent, shared_out=shared, q_half=q_half, q_from=q_from)
         if self._up is None:
             self._up = Linear([self._k_up_host, self._v_up_host], self.runtime)

@@ -84,3 +84,57 @@ def test_expand(T, H, dv, rank, shares, dtype):
     latent = (p[..., :rank] * f[..., None]).sum(2) / (p[..., rank + 1] * f).sum(-1, keepdim=True)
     ref = torch.einsum("thr,hvr->thv", latent, uv.double().reshape(H, dv, rank)) * torch.sigmoid(gate.double())[..., None]
     assert rel(out.reshape(T, H, dv), ref) < (3e-6 if dtype == torch.float32 else 5e-3) and float(junk.abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("dn,dr,rot,rank,dv", [(24, 16, 8, 40, 16), (128, 64, 64, 512, 128), (64, 32, 32, 256, 64)])
+def test_prompt_layouts_four_and_eight_at_a_time(dn, dr, rot, rank, dv, interleaved):
+    """The kernels that read and write several values at a time against the ones that take any size: a column to the right
+    moves the same projection off their alignment."""
+    from llmplayer_b200.kernels import ops
+    H, lengths = 3, [70, 1, 64]
+    g = torch.Generator(device=DEV).manual_seed(dn)
+    T, hd = sum(lengths), next(s for s in (64, 128, 192, 256) if dn + dr <= s)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, seq = i32([p for n in lengths for p in range(n)]), i32([i for i, n in enumerate(lengths) for _ in range(n)])
+    table = i32([[3, 1], [0, 0], [2, 0]])
+    wide = torch.randn(T, H * (dn + dr) + rank + dr + 4, generator=g, device=DEV)
+    rotation = ops.Rotation(torch.rand(rot // 2, generator=g, device=DEV), rot, interleaved, 1.25)
+    gain = torch.randn(rank, generator=g, device=DEV)
+    got = []
+    for shift in (0, 1):
+        proj = torch.cat([wide[:, wide.shape[1] - shift:], wide[:, :wide.shape[1] - shift]], dim=1).contiguous()
+        pages = torch.zeros(4, 64, rank + dr, device=DEV, dtype=torch.bfloat16)
+        latent, shared = torch.zeros(T, rank, device=DEV, dtype=torch.bfloat16), torch.zeros(T, dr, device=DEV, dtype=torch.bfloat16)
+        half = torch.full((T, H * hd), 7.0, device=DEV, dtype=torch.bfloat16)
+        q = torch.zeros(T, H, dn + dr, device=DEV)
+        kw = dict(num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank, latent_out=latent, shared_out=shared, q_half=half)
+        ops.latent_prepare(proj, shift, shift + H * (dn + dr), gain, 1e-5, rotation, pos, seq, table, q, pages, **kw)
+        first = half.clone()
+        ops.latent_prepare(proj, shift, shift + H * (dn + dr), gain, 1e-5, rotation, pos, seq, table, None, pages, **kw)
+        assert torch.equal(first, half)
+        got.append((q, half, shared, latent.float(), pages.float()))
+    for a, b in zip(got[0][:3], got[1][:3]):
+        assert torch.equal(a, b)
+    for a, b in zip(got[0][3:], got[1][3:]):              # the norm's sum is taken in another order: a last bit may round the other way
+        assert float((a - b).abs().max()) <= 2.0 ** -7 * float(b.abs().max())
+    kv = torch.randn(T, H * (dn + dv), generator=g, device=DEV).to(torch.bfloat16)
+    pages = torch.full((5, 2, H, 64, hd), float("nan"), device=DEV, dtype=torch.bfloat16)
+    table = i32([[4, 2], [0, 0], [3, 0]])
+    ops.latent_heads_to_pages(kv, got[0][2].to(torch.bfloat16), pos, seq, table, i32(lengths), pages, num_heads=H, nope_dim=dn, rope_dim=dr,
+                              value_dim=dv)
+    assert bool(torch.isnan(pages[1]).all())              # nobody's page
+    for i, n in enumerate(lengths):
+        t0 = sum(lengths[:i])
+        k = torch.cat([pages[int(p), 0] for p in table[i, :-(-n // 64)]], dim=1).transpose(0, 1)
+        v = torch.cat([pages[int(p), 1] for p in table[i, :-(-n // 64)]], dim=1).transpose(0, 1)
+        rows = kv[t0:t0 + n]
+        assert torch.equal(k[:n, :, :dn], rows[:, :H * dn].reshape(n, H, dn)) and torch.equal(v[:n, :, :dv], rows[:, H * dn:].reshape(n, H, dv))
+        assert torch.equal(k[:n, :, dn:dn + dr], got[0][2][t0:t0 + n, None].to(torch.bfloat16).expand(n, H, dr))
+        assert not k[:, :, dn + dr:].any() and not v[:, :, dv:].any() and not k[n:].any() and not v[n:].any()
+    heads = torch.randn(T, H * hd, generator=g, device=DEV).to(torch.bfloat16)
+    gate = torch.randn(T, H, generator=g, device=DEV)
+    out = torch.empty(T, H * dv, device=DEV, dtype=torch.bfloat16)
+    ops.latent_gate_heads(heads, gate, out, num_heads=H, head_dim=hd, value_dim=dv)
+    ref = heads.reshape(T, H, hd)[..., :dv].double() * torch.sigmoid(gate.double())[..., None]
+    assert rel(out.reshape(T, H, dv), ref) < 5e-3
