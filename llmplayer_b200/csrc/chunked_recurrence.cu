@@ -333,8 +333,14 @@ __device__ __forceinline__ float4 chains(const float (*acc)[4]) {
 
 // 16 warps. W S and Q S (32 x 16 each) share the warps, four per 16 rows with a quarter of the key channels each (without W,
 // eight per 16 rows of Q S); their parts meet in shared memory. Then warp m owns the state's key channels 16 m .. 16 m + 15:
-// its threads hold those entries in registers, shared memory holds them split for the products.
-// STAGES: records in flight (two, or one where two do not fit shared memory).
+// its threads hold those entries in registers, shared memory holds them split for the products; the last two warps add up
+// Q S for their rows, add B U and write the outputs.
+// Bound by the instructions of a chunk's steps (366 per warp, 48 % of the issue slots) and the barriers between them, one
+// chunk after another. With three records in flight a stage is free as soon as the next chunk begins, and the parts of Q S are read by the warps
+// that use them: three barriers per chunk for the delta rule, two without it (U is V then and is split beside the first
+// products), where four were. 2048 tokens, 8 heads of 128 x 256, B200: 117 -> 114 us; 3 sequences of 518 to 777, 8 heads of
+// 128 x 128, delta rule: 91 -> 88.
+// STAGES: records in flight (three, or fewer where they do not fit shared memory; then a barrier frees the stage).
 template <int STAGES>
 __global__ void __launch_bounds__(CARRY_THREADS)
 carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ q_start, int first_chunk, int chunks,
@@ -347,8 +353,7 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
     uint32_t* Uh = Sl + dkp * SROW;                      // [CT][SROW] twice
     uint32_t* Ul = Uh + CT * SROW;
     float4* parts = reinterpret_cast<float4*>(Ul + CT * SROW);           // [16 warps][2 tiles][32 lanes]
-    float4* qs = parts + 16 * 64;                                        // [2][2 tiles][32]: Q S
-    float* ring = reinterpret_cast<float*>(qs + 128);    // STAGES records, each followed by the chunk's 32 x 16 values
+    float* ring = reinterpret_cast<float*>(parts + 16 * 64);             // STAGES records, each followed by the chunk's 32 x 16 values
     const int stage = rec_n + CT * NC;
     lp_grid_release();
     lp_grid_wait();
@@ -370,8 +375,11 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // a stage that the previous chunk has left takes the next record when a chunk begins; with fewer than three stages a
+    // chunk's own stage does when it ends
+    constexpr bool EARLY = STAGES >= 3;
 #pragma unroll
-    for (int p = 0; p < STAGES; ++p) request(p);
+    for (int p = 0; p < (EARLY ? STAGES - 1 : STAGES); ++p) request(p);
     const int g8 = lane >> 2, t4 = lane & 3;
     const int kt = dkp >> 4, ks = dkp >> 3;
     const bool owns = warp < kt;
@@ -388,34 +396,39 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
     const int nk = delta ? 4 : 8, per = (ks + nk - 1) / nk;
     const int role = delta ? warp >> 3 : 1, mt = delta ? (warp >> 2) & 1 : warp >> 3;
     const int s0 = (warp & (nk - 1)) * per, s1 = min(ks, s0 + per);
+    // the parts of 16 rows of a product, added in order: the same lane of every part
+    auto gather = [&](int first, int w) {
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4* at = parts + first * 64 + w * 32 + lane;
+#pragma unroll 8
+        for (int k = 0; k < nk; ++k) {
+            const float4 v = at[k * 64];
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        return sum;
+    };
     for (int p = 0; p < used; ++p) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
-        __syncthreads();                            // the record is there, and S as the previous chunk left it
+        asm volatile("cp.async.wait_group %0;" ::"n"(EARLY ? STAGES - 2 : STAGES - 1) : "memory");
+        __syncthreads();                            // the record is there, S as the previous chunk left it, the chunk before done
+        if (EARLY) request(p + STAGES - 1);
         const float* rec = ring + (p % STAGES) * stage;
         const float* rec_q = rec + (delta ? CT * dkp : 0);
         const float* rec_k = rec_q + CT * dkp;
         const float* rec_b = rec_k + CT * dkp;
         const float* rec_p = rec_b + CT * CT;
         const float* val = rec + rec_n;
+        if (!delta) split_tf32(val[tid], Uh[(tid >> 4) * SROW + (tid & 15)], Ul[(tid >> 4) * SROW + (tid & 15)]);
         {
             float acc[2][3][4] = {};
             product(acc, (role == 1 ? rec_q : rec) + mt * ks * 128, Sh, Sl, s0, s1, lane);
             parts[warp * 64 + lane] = chains(acc[0]);
             parts[warp * 64 + 32 + lane] = chains(acc[1]);
         }
-        __syncthreads();
-        if (tid < 256) {                            // thread (product, row half, tile, lane): the parts added, in order
-            const int what = tid >> 7, half = (tid >> 6) & 1, w = (tid >> 5) & 1;
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (what == 1 || delta) {
-                const float4* at = parts + (delta ? what * 8 + half * 4 : half * 8) * 64 + w * 32 + lane;
-                for (int k = 0; k < nk; ++k) {
-                    const float4 v = at[k * 64];
-                    sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-                }
-            }
-            if (what == 1) qs[half * 64 + w * 32 + lane] = sum;
-            else {
+        __syncthreads();                            // S has been read
+        if (delta) {
+            if (warp < 4) {                         // warp (row half, tile): U = U0 - W S
+                const int half = warp >> 1, w = warp & 1;
+                const float4 sum = gather(half * 4, w);
                 const float x[4] = {sum.x, sum.y, sum.z, sum.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -423,8 +436,8 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
                     split_tf32(val[r * NC + c] - x[e], Uh[r * SROW + c], Ul[r * SROW + c]);
                 }
             }
+            __syncthreads();                        // U is there
         }
-        __syncthreads();                            // U and Q S are there; S has been read
         if (owns) {
             float up[2][3][4] = {};
             product(up, rec_k + warp * (CT >> 3) * 128, Uh, Ul, 0, CT >> 3, lane);
@@ -445,7 +458,7 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
             const int t = begin + p * CT;
 #pragma unroll
             for (int w = 0; w < 2; ++w) {
-                const float4 o = qs[half * 64 + w * 32 + lane], u = chains(acc[w]);
+                const float4 o = gather(delta ? 8 + half * 4 : half * 8, w), u = chains(acc[w]);
                 const float x[4] = {o.x + u.x, o.y + u.y, o.z + u.z, o.w + u.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -454,8 +467,10 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
                 }
             }
         }
-        __syncthreads();                            // the stage is free
-        request(p + STAGES);
+        if (!EARLY) {
+            __syncthreads();                        // the stage is free
+            request(p + STAGES);
+        }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
@@ -505,16 +520,16 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
     const int dkp = padded(dk), delta = beta ? 1 : 0;
     const size_t smem_p = ((size_t)(3 * CT + 3 * HB) * (dkp + 4) + 2 * CT * CT + CT) * sizeof(float);
     const size_t stage = (size_t)(record_floats(dkp, delta) + CT * NC) * sizeof(float);
-    const size_t kept = (size_t)(dkp + CT) * SROW * 2 * sizeof(float) + (16 * 64 + 128) * sizeof(float4);
-    const bool two = kept + 2 * stage <= MAX_SMEM;
-    const size_t smem_c = kept + (two ? 2 : 1) * stage;
+    const size_t kept = (size_t)(dkp + CT) * SROW * 2 * sizeof(float) + 16 * 64 * sizeof(float4);
+    const int stages = kept + 3 * stage <= MAX_SMEM ? 3 : kept + 2 * stage <= MAX_SMEM ? 2 : 1;
+    const size_t smem_c = kept + stages * stage;
     auto prepare = dk <= 64 ? prepare_kernel<4> : dk <= 128 ? prepare_kernel<8> : prepare_kernel<16>;
     const int size = dk <= 64 ? 0 : dk <= 128 ? 1 : 2;
-    auto carry = two ? carry_kernel<2> : carry_kernel<1>;
-    static size_t granted_p[3] = {}, granted_c[2] = {};       // what each kernel has been allowed so far
+    auto carry = stages == 3 ? carry_kernel<3> : stages == 2 ? carry_kernel<2> : carry_kernel<1>;
+    static size_t granted_p[3] = {}, granted_c[3] = {};       // what each kernel has been allowed so far
     int rc = reserve(prepare, smem_p, granted_p[size]);
     if (rc) return rc;
-    rc = reserve(carry, smem_c, granted_c[two ? 1 : 0]);
+    rc = reserve(carry, smem_c, granted_c[stages - 1]);
     if (rc) return rc;
     const int total = (max_new + CT - 1) / CT;
     for (int first = 0; first < total; first += chunks) {
