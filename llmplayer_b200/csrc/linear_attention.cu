@@ -17,32 +17,50 @@
 namespace {
 
 // ---------------------------------------------------------------- decay
-// low: float32 [T, ldl] slice with the R values A1 h; a2: [C, R]; bias: [C]; out: float32 [T, C].
-template <typename TW>
+// low: float32 [T, ldl] slice with the R values A1 h; a2: [C, R]; bias: [C]; out: float32 [T, C]. A thread owns one channel
+// of TT tokens: its weights are read once per TT tokens, the tokens' factors lie in shared memory (read by all lanes at
+// once). Bound by its arithmetic and its output: 2048 tokens, 1024 channels, rank 16, B200: 40 us with a thread per value,
+// which fetched both rows for every value -> 13. Steps of few tokens keep a block per token and 256 channels.
+constexpr int DECAY_R = 16;          // values of the factor per round
+template <typename TW, int TT>
 __global__ void __launch_bounds__(256)
 gla_decay_kernel(const float* __restrict__ low, int ldl, const TW* __restrict__ a2, const float* __restrict__ bias,
                  float* __restrict__ out, int T, int C, int R, float inv_tau, int form) {
+    __shared__ float x[TT][DECAY_R];
     lp_grid_release();
     lp_grid_wait();
-    const long long n = (long long)T * C;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long t = i / C;
-        const int c = (int)(i - t * C);
-        const float* x = low + t * ldl;
-        const TW* w = a2 + (long long)c * R;
-        float z = 0.f;
-        if (form == 1) {
-            // the time-mixing form: the factor's output passes through tanh, and the decay is exp(-exp(z))
-            for (int r = 0; r < R; ++r) z = fmaf(lp_to_float(w[r]), tanhf(x[r]), z);
-            z += bias ? bias[c] : 0.f;
-            out[i] = expf(-expf(z));
-            continue;
+    const int c = blockIdx.y * 256 + threadIdx.x;
+    const long long t0 = (long long)blockIdx.x * TT;
+    float z[TT];
+#pragma unroll
+    for (int i = 0; i < TT; ++i) z[i] = 0.f;
+    for (int r0 = 0; r0 < R; r0 += DECAY_R) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < TT * DECAY_R; e += 256) {
+            const int i = e / DECAY_R, r = r0 + e % DECAY_R;
+            float v = t0 + i < T && r < R ? low[(t0 + i) * ldl + r] : 0.f;
+            if (form == 1) v = tanhf(v);        // the time-mixing form: the factor's output passes through tanh
+            x[i][e % DECAY_R] = v;
         }
-        for (int r = 0; r < R; ++r) z = fmaf(lp_to_float(w[r]), x[r], z);
-        z += bias ? bias[c] : 0.f;
-        // log sigmoid(z) = -softplus(-z)
-        const float sp = fmaxf(-z, 0.f) + log1pf(expf(-fabsf(z)));
-        out[i] = expf(-sp * inv_tau);
+        __syncthreads();
+        if (c < C) {
+            float w[DECAY_R];
+#pragma unroll
+            for (int r = 0; r < DECAY_R; ++r) w[r] = r0 + r < R ? lp_to_float(a2[(long long)c * R + r0 + r]) : 0.f;
+#pragma unroll
+            for (int i = 0; i < TT; ++i)
+#pragma unroll
+                for (int r = 0; r < DECAY_R; ++r) z[i] = fmaf(w[r], x[i][r], z[i]);
+        }
+    }
+    if (c >= C) return;
+    const float add = bias ? bias[c] : 0.f;
+#pragma unroll
+    for (int i = 0; i < TT; ++i) {
+        if (t0 + i >= T) break;
+        const float v = z[i] + add;
+        // form 1: the decay is exp(-exp(z)); else log sigmoid(z) = -softplus(-z)
+        out[(t0 + i) * C + c] = form == 1 ? expf(-expf(v)) : expf(-(fmaxf(-v, 0.f) + log1pf(expf(-fabsf(v)))) * inv_tau);
     }
 }
 
@@ -519,6 +537,61 @@ gla_finish_kernel(const float* __restrict__ o, const float* __restrict__ gain, f
     }
 }
 
+// The same for rows of a multiple of four values, 16-byte aligned and at most 512 values (without a normaliser column): four
+// values per load, a row's values stay in registers between the norm and the gate. 16,384 rows of 256, B200: 21 -> 12 us.
+template <typename TOut, int N>
+__global__ void __launch_bounds__(256)
+gla_finish_vec4_kernel(const float* __restrict__ o, const float* __restrict__ gain, float eps, const float* __restrict__ gate,
+                       int ldg, TOut* __restrict__ out, int T, int H, int dv, float* __restrict__ zero, long long zero_count,
+                       int gain_per_head, int gate_sigmoid) {
+    lp_grid_release();
+    lp_grid_wait();
+    clear_on_the_side(zero, zero_count);
+    const int lane = threadIdx.x & 31;
+    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= (long long)T * H) return;
+    const long long t = row / H;
+    const int h = (int)(row - t * H);
+    const float* x = o + row * dv;
+    const float* g = gate ? gate + t * ldg + (long long)h * dv : nullptr;
+    const float* gn = gain && gain_per_head ? gain + (long long)h * dv : gain;
+    float v[N][4], z[N][4];
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int j = (lane + 32 * n) * 4;
+        const bool in = j < dv;
+        const float4 a = in ? *(const float4*)(x + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 b = in && g ? *(const float4*)(g + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[n][0] = a.x; v[n][1] = a.y; v[n][2] = a.z; v[n][3] = a.w;
+        z[n][0] = b.x; z[n][1] = b.y; z[n][2] = b.z; z[n][3] = b.w;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ss += v[n][k] * v[n][k];
+    }
+    ss = lp_warp_sum(ss);
+    const float factor = 1.0f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int j = (lane + 32 * n) * 4;
+        if (j >= dv) break;
+        const float4 a = gn ? *(const float4*)(gn + j) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const float w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[n][k] *= factor;
+            if (gn) v[n][k] *= w[k];
+            if (g) v[n][k] *= gate_sigmoid ? 1.0f / (1.0f + expf(-z[n][k])) : z[n][k] / (1.0f + expf(-z[n][k]));
+        }
+        TOut* to = out + row * dv + j;
+        if constexpr (sizeof(TOut) == 2) {
+            __nv_bfloat162 lo = __floats2bfloat162_rn(v[n][0], v[n][1]), hi = __floats2bfloat162_rn(v[n][2], v[n][3]);
+            *(uint2*)to = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+        } else {
+            *(float4*)to = make_float4(v[n][0], v[n][1], v[n][2], v[n][3]);
+        }
+    }
+}
+
 
 // ---------------------------------------------------------------- short causal convolution with a carried tail
 // out[t, c] = act(bias[c] + sum_j taps[c, j] * in[t - (K - 1) + j, c]), K taps per channel, the last one on the token
@@ -877,14 +950,20 @@ extern "C" int lp_gla_decay(const float* low, int ldl, const void* a2, int w_dty
     if (form < 0 || form > 1) LP_REFUSE("gla_decay: form %d", form);
     if (form == 1) tau = 1.0f;
     if (!(tau > 0.f)) LP_REFUSE("gla_decay: temperature %g", (double)tau);
-    const long long n = (long long)T * C;
-    long long blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (w_dtype == LP_F32)
-        lp_launch(gla_decay_kernel<float>, (unsigned)blocks, 256, 0, stream, low, ldl, (const float*)a2, bias, out, T, C, R, 1.0f / tau, form);
-    else if (w_dtype == LP_BF16)
-        lp_launch(gla_decay_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, stream, low, ldl, (const __nv_bfloat16*)a2, bias, out, T, C, R, 1.0f / tau, form);
+    // a tile of 16 tokens where that still leaves several blocks per SM
+    const unsigned columns = (unsigned)((C + 255) / 256);
+    const bool tiles = (long long)T * columns >= 16LL * 2 * lp_sm_count();
+    const dim3 grid((unsigned)((T + (tiles ? 15 : 0)) / (tiles ? 16 : 1)), columns);
+    if (grid.y > 65535) LP_REFUSE("gla_decay: %d channels exceed the grid", C);
+#define LP_LAUNCH_DECAY(TW)                                                                                                     \
+    do {                                                                                                                        \
+        if (tiles) lp_launch(gla_decay_kernel<TW, 16>, grid, 256, 0, stream, low, ldl, (const TW*)a2, bias, out, T, C, R, 1.0f / tau, form); \
+        else lp_launch(gla_decay_kernel<TW, 1>, grid, 256, 0, stream, low, ldl, (const TW*)a2, bias, out, T, C, R, 1.0f / tau, form);        \
+    } while (0)
+    if (w_dtype == LP_F32) LP_LAUNCH_DECAY(float);
+    else if (w_dtype == LP_BF16) LP_LAUNCH_DECAY(__nv_bfloat16);
     else LP_REFUSE("gla_decay: weight dtype code %d", w_dtype);
+#undef LP_LAUNCH_DECAY
     return lp_check_launch("gla_decay");
 }
 
@@ -973,6 +1052,21 @@ extern "C" int lp_gla_finish(const float* o, const float* gain, float eps, const
     if (xs < dv || (max_row && xs < dv + 1)) LP_REFUSE("gla_finish: rows %d apart for %d values", xs, dv);
     const long long rows = (long long)T * H;
     const unsigned blocks = (unsigned)((rows + 7) / 8);
+    if (!max_row && xs == dv && dv % 4 == 0 && dv <= 512 && (!gate || ldg % 4 == 0) && (out_dtype == LP_F32 || out_dtype == LP_BF16) &&
+        (((uintptr_t)o | (uintptr_t)gain | (uintptr_t)gate | (uintptr_t)out) & 15) == 0) {
+#define LP_LAUNCH_FINISH(N)                                                                                                          \
+    do {                                                                                                                             \
+        if (out_dtype == LP_F32) lp_launch(gla_finish_vec4_kernel<float, N>, blocks, 256, 0, stream, o, gain, eps, gate, ldg,        \
+                                           (float*)out, T, H, dv, zero, zero_count, gain_per_head, gate_sigmoid);                    \
+        else lp_launch(gla_finish_vec4_kernel<__nv_bfloat16, N>, blocks, 256, 0, stream, o, gain, eps, gate, ldg,                    \
+                       (__nv_bfloat16*)out, T, H, dv, zero, zero_count, gain_per_head, gate_sigmoid);                                \
+    } while (0)
+        if (dv <= 128) LP_LAUNCH_FINISH(1);
+        else if (dv <= 256) LP_LAUNCH_FINISH(2);
+        else LP_LAUNCH_FINISH(4);
+#undef LP_LAUNCH_FINISH
+        return lp_check_launch("gla_finish");
+    }
     if (out_dtype == LP_F32) lp_launch(gla_finish_kernel<float>, blocks, 256, 0, stream, o, gain, eps, gate, ldg, (float*)out, T, H, dv, zero, zero_count, xs, gain_per_head, gate_sigmoid, max_row);
     else if (out_dtype == LP_BF16)
         lp_launch(gla_finish_kernel<__nv_bfloat16>, blocks, 256, 0, stream, o, gain, eps, gate, ldg, (__nv_bfloat16*)out, T, H, dv, zero, zero_count, xs, gain_per_head, gate_sigmoid, max_row);

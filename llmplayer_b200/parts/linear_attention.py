@@ -77,9 +77,9 @@ class GatedLinearAttention(Part):
         """The matrices that multiply the mixer's input, in the order ``forward_projected`` expects their sums."""
         return list(self._inputs)
 
-    def forward_projected(self, ctx, cache, proj: torch.Tensor, offset: int, out: torch.Tensor) -> torch.Tensor:
+    def forward_projected(self, ctx, cache, proj: torch.Tensor, offset: int, out: torch.Tensor, add: bool = False) -> torch.Tensor:
         """``proj``: float32 [T, F] holding, from column ``offset``, the sums of :meth:`input_projections`;
-        writes the mixer's result (before any residual gate) to ``out`` float32 [T, hidden]."""
+        writes the mixer's result (before any residual gate) to ``out`` float32 [T, hidden] (``add``: adds it there)."""
         s, rt = self.spec, self.runtime
         if cache is None:
             raise ConfigError("gated linear attention needs its per-sequence state")
@@ -99,7 +99,7 @@ class GatedLinearAttention(Part):
                          key_dim=dk, value_dim=dv, q_scale=float(dk) ** -0.5, max_new=ctx.max_new, scratch=ctx.buffer, tensor_cores=rt.fast)
         o = ctx.buffer("attn_out", (T, H * dv), rt.act_dtype)
         # an output product that sums partial results into `out` wants it zero: the kernel before it clears it
-        clear = self.out.sums_into(ctx, T, "mixer_out", ops.STORE)
+        clear = None if add else self.out.sums_into(ctx, T, "mixer_out", ops.STORE)
         if clear is not None and clear.data_ptr() != out.data_ptr():
             clear = None
         with ops.section("recurrence.norm"):
@@ -108,7 +108,10 @@ class GatedLinearAttention(Part):
         if clear is not None:
             ctx.note_cleared()
         with ops.section("recurrence.out"):
-            self.out.store(o, out, ctx)
+            if add:
+                self.out.accumulate(o, out, ctx)
+            else:
+                self.out.store(o, out, ctx)
         return out
 
     def forward(self, ctx, cache, x, residual: torch.Tensor) -> bool:
@@ -120,9 +123,7 @@ class GatedLinearAttention(Part):
         proj = ctx.buffer("mixer_proj", (x.shape[0], self._own.out_features), torch.float32)
         with ops.section("recurrence.proj"):
             self._own.store(x, proj, ctx)
-        out = ctx.buffer("mixer_out", tuple(residual.shape), torch.float32)
-        self.forward_projected(ctx, cache, proj, 0, out)
-        ops.gated_sum(residual, out)
+        self.forward_projected(ctx, cache, proj, 0, residual, add=True)      # the output product adds into the stream itself
         return False
 
 
