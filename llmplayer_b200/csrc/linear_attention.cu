@@ -12,7 +12,7 @@
 //   lp_token_shift  per token the blends x_t + (x_(t-1) - x_t) * mu_s that such a layer's maps read
 //   lp_gla_scan     the recurrence over a step's tokens, sequence by sequence, in token order
 //   lp_gla_finish   per head: RMS norm over dv (gain shared by heads), times silu(gate)
-#include "common.cuh"
+#include "bf16_parts.cuh"
 
 namespace {
 
@@ -884,6 +884,122 @@ low_rank_gates_kernel(const float* __restrict__ proj, int ld, int T, int H, Rank
     }
 }
 
+// The same with bfloat16 maps whose ranks are multiples of 16, on the tensor cores: the factors' float32 values as three
+// bfloat16 parts, the map's rows as they are. 64 tokens x 128 channels per CTA over the whole rank; a warp takes 32 x 32.
+// Bound by splitting the factors (every column of CTAs does it again) and by its outputs: 1943 tokens, two maps of 1024
+// channels with rank 128, B200: 50 us with float32 multiply-adds (above) -> 36; half of
+// its instructions are the exponentials and logarithms of the decays.
+constexpr int LR_TOKENS = 64, LR_CHANNELS = 128;
+inline size_t low_rank_smem(int rank) { return (size_t)(3 * LR_TOKENS + LR_CHANNELS) * (rank + 8) * 2; }
+
+__global__ void __launch_bounds__(256, 2)
+low_rank_gates_tc_kernel(const float* __restrict__ proj, int ld, int T, int H, RankMap a, const float* __restrict__ dt_bias,
+                         const float* __restrict__ a_log, int dk, RankMap g, int a_tiles, int b_off, float* __restrict__ strength) {
+    extern __shared__ __align__(16) uint8_t raw[];
+    const bool decays = (int)blockIdx.x < a_tiles;
+    const RankMap m = decays ? a : g;
+    const int R = m.rank, stride = R + 8;
+    __nv_bfloat16* Xs = (__nv_bfloat16*)raw;                       // [3][LR_TOKENS][stride]
+    __nv_bfloat16* Ws = Xs + 3 * LR_TOKENS * stride;               // [LR_CHANNELS][stride]
+    const int t0 = blockIdx.y * LR_TOKENS, c0 = (decays ? blockIdx.x : blockIdx.x - a_tiles) * LR_CHANNELS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const __nv_bfloat16* up = (const __nv_bfloat16*)m.up;
+    // weights are written by no kernel of a step: asked for before the wait
+    for (int r = warp; r < LR_CHANNELS; r += 8) {
+        const bool real = c0 + r < m.channels;
+        const int bytes = real ? 16 : 0;
+        const __nv_bfloat16* from = real ? up + (long long)(c0 + r) * R : up;
+        for (int c = lane * 8; c < R; c += 256)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_at(Ws + r * stride + c)), "l"(real ? from + c : up), "r"(bytes) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    lp_grid_release();
+    lp_grid_wait();
+    const bool wide = ((m.off | ld) & 3) == 0;
+    for (int r = warp; r < LR_TOKENS; r += 8) {
+        const bool real = t0 + r < T;
+        const float* from = proj + (long long)(real ? t0 + r : 0) * ld + m.off;
+        for (int c = lane * 4; c < R; c += 128) {
+            float v[4];
+            if (wide) {
+                const float4 x = *(const float4*)(from + c);
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = from[c + i];
+            }
+            __nv_bfloat16 p[4][3];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) three_parts(real ? v[i] : 0.f, p[i]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                __nv_bfloat162* to = (__nv_bfloat162*)(Xs + (k * LR_TOKENS + r) * stride + c);
+                to[0] = __halves2bfloat162(p[0][k], p[1][k]);
+                to[1] = __halves2bfloat162(p[2][k], p[3][k]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int tm = (warp & 1) * 32, tn = (warp >> 1) * 32;
+    float acc[2][4][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[i][n][k] = 0.f;
+    const uint32_t x_at = smem_at(Xs + (tm + (lane & 15)) * stride + (lane >> 4) * 8);
+    const uint32_t w_at = smem_at(Ws + (tn + (lane >> 4) * 8 + (lane & 7)) * stride + ((lane >> 3) & 1) * 8);
+    for (int step = 0; step < R / 16; ++step) {
+        uint32_t wf[2][4];
+        ldmatrix4(w_at + step * 32, wf[0]);
+        ldmatrix4(w_at + 16 * stride * 2 + step * 32, wf[1]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                uint32_t xf[4];
+                ldmatrix4(x_at + (p * LR_TOKENS + i * 16) * stride * 2 + step * 32, xf);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) mma_bf16(acc[i][n], xf, wf[n >> 1][(n & 1) * 2], wf[n >> 1][(n & 1) * 2 + 1]);
+            }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        const int c = c0 + tn + n * 8 + (lane & 3) * 2;
+        float rate[2] = {0.f, 0.f}, bias[2] = {0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (decays && c + k < m.channels) {
+                rate[k] = expf(a_log[(c + k) / dk]);
+                bias[k] = dt_bias[c + k];
+            }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = t0 + tm + i * 16 + half * 8 + (lane >> 2);
+                if (t >= T) continue;
+                float v[2] = {acc[i][n][half * 2], acc[i][n][half * 2 + 1]};
+                if (decays)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) v[k] = expf(-rate[k] * lp_softplus(v[k] + bias[k]));
+                float* at = m.out + (long long)t * m.channels + c;
+                if ((m.channels & 1) == 0 && c + 1 < m.channels) *(float2*)at = make_float2(v[0], v[1]);
+                else
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        if (c + k < m.channels) at[k] = v[k];
+            }
+    }
+    if (blockIdx.x == 0 && strength)
+        for (int e = tid; e < LR_TOKENS * H; e += 256) {
+            const int t = t0 + e / H, h = e - e / H * H;
+            if (t < T) strength[(long long)t * H + h] = 1.0f / (1.0f + expf(-proj[(long long)t * ld + b_off + h]));
+        }
+}
+
 // ---------------------------------------------------------------- heads made unit vectors
 // x[t, off + h * dim + i] <- x / sqrt(sum_i x^2 + eps), in place, float32; the first `scaled` heads also times `scale`
 // (queries in front of keys). A warp per (token, head).
@@ -1169,6 +1285,16 @@ extern "C" int lp_low_rank_gates(const float* proj, int ld, int T, int H, int dk
     if ((a_dtype != LP_F32 && a_dtype != LP_BF16) || (g_up && g_dtype != LP_F32 && g_dtype != LP_BF16)) LP_REFUSE("low_rank_gates: dtype codes %d and %d", a_dtype, g_dtype);
     const RankMap a{a_off, a_rank, H * dk, a_up, a_dtype == LP_BF16, decay};
     const RankMap g{g_off, g_rank, g_up ? g_channels : 0, g_up, g_dtype == LP_BF16, gate};
+    const size_t tc_bytes = low_rank_smem(a_rank > g_rank || !g_up ? a_rank : g_rank);
+    if (T > 16 && a.up_bf16 && a_rank % 16 == 0 && (!g_up || (g.up_bf16 && g_rank % 16 == 0)) && tc_bytes <= 200 * 1024 &&
+        (((uintptr_t)proj | (uintptr_t)a_up | (uintptr_t)g_up | (uintptr_t)decay | (uintptr_t)gate) & 15) == 0 && T <= 65535 * LR_TOKENS) {
+        cudaError_t e = cudaFuncSetAttribute(low_rank_gates_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_bytes);
+        if (e != cudaSuccess) LP_REFUSE("low_rank_gates: cannot reserve %zu bytes of shared memory: %s", tc_bytes, cudaGetErrorString(e));
+        const int at = (a.channels + LR_CHANNELS - 1) / LR_CHANNELS, gt = (g.channels + LR_CHANNELS - 1) / LR_CHANNELS;
+        lp_launch(low_rank_gates_tc_kernel, dim3(at + gt, (T + LR_TOKENS - 1) / LR_TOKENS), 256, tc_bytes, stream, proj, ld, T, H, a, dt_bias,
+                  a_log, dk, g, at, b_off, strength);
+        return lp_check_launch("low_rank_gates");
+    }
     const int a_tiles = (a.channels + RM_TILE - 1) / RM_TILE, g_tiles = (g.channels + RM_TILE - 1) / RM_TILE;
     if ((((uintptr_t)decay | (uintptr_t)gate) & 15) != 0) LP_REFUSE("low_rank_gates: outputs must be aligned to 16 bytes");
     const int rows = (T + RM_TOKENS - 1) / RM_TOKENS;

@@ -42,7 +42,7 @@ LIBRARIES: Dict[str, str] = {
     "recurrent_step": "recurrent_step.cu",
     "stream_bundle": "stream_bundle.cu",
 }
-HEADERS = ("common.cuh", "attention_noalloc.h", "tcgen05_utils.cuh", "attention_decode.cuh")
+HEADERS = ("common.cuh", "attention_noalloc.h", "tcgen05_utils.cuh", "attention_decode.cuh", "bf16_parts.cuh")
 
 NVCC_FLAGS: List[str] = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -28,6 +28,26 @@ def test_decays(T, C, R, tanh, dtype):
     assert rel(out, ref) < 2e-6
 
 
+@pytest.mark.parametrize("T,H,dk,ra,dv,rg", [(17, 1, 16, 16, 8, 16), (64, 2, 40, 48, 129, 32), (129, 8, 128, 128, 128, 128), (200, 3, 96, 256, 64, 16)])
+def test_low_rank_gates(T, H, dk, ra, dv, rg):
+    from llmplayer_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    for shift in (0, 1):                                  # columns that start on 16 bytes, and columns that do not
+        proj = torch.randn(T, shift + ra + rg + H + (-(shift + ra + rg + H)) % 4, generator=g, device=DEV)
+        a_up = (torch.randn(H * dk, ra, generator=g, device=DEV) / ra ** 0.5).to(torch.bfloat16)
+        g_up = (torch.randn(H * dv, rg, generator=g, device=DEV) / rg ** 0.5).to(torch.bfloat16)
+        dt, a_log = torch.randn(H * dk, generator=g, device=DEV), 0.3 * torch.randn(H, generator=g, device=DEV)
+        decay, strength = torch.full((T, H * dk), 7.0, device=DEV), torch.full((T, H), 7.0, device=DEV)
+        gate = torch.full((T, H * dv), 7.0, device=DEV)
+        ops.low_rank_gates(proj, shift, a_up, dt, a_log, decay, shift + ra + rg, strength, key_dim=dk, g_off=shift + ra, g_up=g_up, gate=gate)
+        p = proj.double()
+        z = p[:, shift:shift + ra] @ a_up.double().T + dt.double()
+        ref = torch.exp(-torch.exp(a_log.double()).repeat_interleave(dk) * torch.nn.functional.softplus(z))
+        assert rel(decay, ref) < 3e-6
+        assert rel(gate, p[:, shift + ra:shift + ra + rg] @ g_up.double().T) < 2e-6
+        assert rel(strength, torch.sigmoid(p[:, shift + ra + rg:shift + ra + rg + H])) < 1e-6
+
+
 @pytest.mark.parametrize("T,H,dv", [(1, 1, 4), (37, 3, 100), (65, 2, 128), (20, 5, 132), (9, 2, 256), (11, 3, 300), (7, 2, 512), (5, 2, 516), (6, 2, 30)])
 @pytest.mark.parametrize("sigmoid,per_head", [(False, False), (True, True)])
 def test_finish(T, H, dv, sigmoid, per_head):
