@@ -1,5 +1,5 @@
-// Prefill attention on the Blackwell tensor cores, head sizes 64 and 128: scores and the
-// probabilities-times-values product run as tcgen05.mma with accumulators in tensor memory.
+// Prefill attention on the Blackwell tensor cores, head sizes 64 and 128, and 192 with values of 128: scores and
+// the probabilities-times-values product run as tcgen05.mma with accumulators in tensor memory.
 //
 // A CTA takes 128 consecutive new tokens of one sequence and one query head. Per page of 64
 // keys of the sequence's cache:
@@ -20,7 +20,13 @@
 // hardly ever after, so the softmax warps, which are bound by the instructions they issue, no longer
 // read and rescale a page's product on every page.
 // S and P are double-buffered: the scores of page i+1 are formed while the softmax of page i runs.
-// Two CTAs fit an SM at head size 64, one at head size 128.
+// Two CTAs fit an SM at head size 64, one at the others.
+//
+// SPLIT: weights that meet the values at float32 precision enter as hi = bf16(e) and lo = bf16(e - hi), 16 bits of mantissa, in two
+// tiles and two products per page; the sums use the float32 weights. It comes with everything else that may shape a score or an
+// output (a cap, sinks, kept first tokens, chunks, a gate per head) except a distance bias, which stays with the mma.sync kernel.
+// B200, one prompt of 2048 tokens, 16 heads of 128 on 4, capped scores and sinks: 174 us with mma.sync -> 89; 16 heads of
+// 192 with values of 128, sequences of 1100 and 825 tokens: 95 -> 39 (which also leaves out the values' 64 columns of zeros).
 //
 // Reference counterpart: src/main/resources/kernels/cuda/attention.cu:10-108 (one query at a
 // time, SIMT); the online-softmax recurrence is that of inference/Attention.java:161-207.
@@ -35,16 +41,32 @@ constexpr int P_BYTES = ROWS * PAGE * 2;          // 16 KB
 constexpr int XCHG_BYTES = 2 * 2 * ROWS * 4;      // row maxima of the two halves, double-buffered
 constexpr float RESCALE_ABOVE = 8.0f;             // in log2 units: the reference maximum may lag by a factor of 256
 
-template <int HD> struct Shape {
-    static constexpr int BLOCKS = HD / 64;                   // blocks of 64 features (one swizzle row each)
-    static constexpr int STAGES = 3;
+template <int HD, int VD, bool SPLIT> struct Shape {
+    static constexpr int BLOCKS = HD / 64, VBLOCKS = VD / 64;    // blocks of 64 features (one swizzle row each)
     static constexpr int Q_BYTES = ROWS * HD * 2;
-    static constexpr int KV_BYTES = PAGE * HD * 2;           // a K tile, or a V tile
-    static constexpr int STAGE_BYTES = 2 * KV_BYTES;
-    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * STAGE_BYTES + 2 * P_BYTES + XCHG_BYTES + 1024 + 256;
-    static constexpr int TMEM_COLS = 256;                    // S[2]: 0..127, O: 128 .. 128 + HD
+    static constexpr int K_BYTES = PAGE * HD * 2, V_BYTES = PAGE * VD * 2;
+    static constexpr int STAGE_BYTES = K_BYTES + V_BYTES;
+    // split weights at head size 64: one buffer for them and two stages, so that two CTAs still fit an SM
     static constexpr int CTAS_PER_SM = HD == 64 ? 2 : 1;
+    static constexpr int P_BUFFERS = SPLIT && HD == 64 ? 1 : 2;
+    static constexpr int STAGES = SPLIT && HD != 128 ? 2 : 3;
+    static constexpr int P_PAGE = (SPLIT ? 2 : 1) * P_BYTES;     // the weights of a page: hi, then lo
+    static constexpr int SMEM_BYTES = Q_BYTES + STAGES * STAGE_BYTES + P_BUFFERS * P_PAGE + XCHG_BYTES + 1024 + 256;
+    static constexpr int TMEM_COLS = 256;                        // S[2]: 0..127, O: 128 .. 128 + VD
+    static_assert(SMEM_BYTES * CTAS_PER_SM <= 227 * 1024 && VD <= 128 && HD % 64 == 0, "");
 };
+// What may shape a score or an output besides the scale (see ScoreExtras in attention_decode.cuh).
+struct Shaping {
+    float cap_log2, scale_over_cap;      // cap_log2 == 0: scores are not capped
+    const float* sinks;                  // [H] or null
+    int keep, chunk;
+    const float* gate;                   // rows of gate_ld values, or null
+    int gate_ld;
+};
+__device__ __forceinline__ int first_seen(int pos, int window, int chunk) {
+    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+    return chunk > 0 ? max(lo, pos / chunk * chunk) : lo;
+}
 // Two float32 operations in one instruction (Blackwell's packed f32x2 forms): the softmax warps are bound by
 // how many instructions they issue.
 __device__ __forceinline__ void fma2(float& x0, float& x1, float a, float b) {            // x = x * a + b
@@ -92,21 +114,22 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-template <int HD>
-__global__ void __launch_bounds__(THREADS, Shape<HD>::CTAS_PER_SM)
+template <int HD, int VD, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, Shape<HD, VD, SPLIT>::CTAS_PER_SM)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                             __nv_bfloat16* __restrict__ out, const int* __restrict__ page_table, int pt_stride,
                             const int* __restrict__ q_start, const int* __restrict__ kv_len, int H, int G,
-                            float scale_log2, int window, int* __restrict__ status) {
-    using SH = Shape<HD>;
-    constexpr int STAGES = SH::STAGES, STAGE_BYTES = SH::STAGE_BYTES, KV_BYTES = SH::KV_BYTES, BLOCKS = SH::BLOCKS;
+                            float scale_log2, int window, Shaping shaping, int* __restrict__ status) {
+    using SH = Shape<HD, VD, SPLIT>;
+    constexpr int STAGES = SH::STAGES, STAGE_BYTES = SH::STAGE_BYTES, K_BYTES = SH::K_BYTES;
+    constexpr int PB = SH::P_BUFFERS, P_PAGE = SH::P_PAGE;
     constexpr int O_COL = 2 * PAGE;                          // the output's first column of tensor memory
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* q_tile = smem;                                  // BLOCKS tiles of [ROWS x 64]
     uint8_t* ring = smem + SH::Q_BYTES;                      // per stage: K (BLOCKS tiles of [PAGE x 64]), then V likewise
     uint8_t* p_tile = ring + STAGES * STAGE_BYTES;
-    float* xchg = (float*)(p_tile + 2 * P_BYTES);            // [2 buffers][2 halves][ROWS]
+    float* xchg = (float*)(p_tile + PB * P_PAGE);            // [2 buffers][2 halves][ROWS]
     uint64_t* bars = (uint64_t*)((uint8_t*)xchg + XCHG_BYTES);
     uint64_t* q_full = bars;
     uint64_t* kv_full = bars + 1;                  // [STAGES]
@@ -153,9 +176,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int row0 = tile * ROWS;
     const int rows = has_work ? min(ROWS, n_new - row0) : 0;
     const int first_pos = pos0 + row0, last_pos = pos0 + row0 + rows - 1;
-    const int lo = window > 0 ? max(0, first_pos - window + 1) : 0;
-    const int page_lo = lo / PAGE, page_hi = last_pos / PAGE;
-    const int npages = has_work ? page_hi - page_lo + 1 : 0;
+    const int chunk = SPLIT ? shaping.chunk : 0;
+    const int page_lo = first_seen(first_pos, window, chunk) / PAGE, page_hi = last_pos / PAGE;
+    // the pages of the first tokens that stay visible beyond the window come first
+    const int keep = SPLIT ? shaping.keep : 0;
+    const int kept_pages = min((keep + PAGE - 1) / PAGE, page_lo);
+    auto page_of = [&](int i) { return i < kept_pages ? i : page_lo + i - kept_pages; };
+    const int npages = has_work ? page_hi - page_lo + 1 + kept_pages : 0;
     const int* table = page_table + (size_t)b * pt_stride;
 
     if (warp == 0) {
@@ -163,21 +190,21 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (lane == 0 && has_work) {
             mbar_expect_tx(q_full, SH::Q_BYTES);
 #pragma unroll
-            for (int c = 0; c < BLOCKS; ++c)
+            for (int c = 0; c < SH::BLOCKS; ++c)
                 tma_load_2d(q_tile + c * (ROWS * 128), &map_q, h * HD + c * 64, t_begin + row0, q_full);
             for (int i = 0; i < npages; ++i) {
                 const int s = i % STAGES;
                 const uint32_t phase = (i / STAGES) & 1;
                 if (!mbar_wait(&kv_empty[s], phase ^ 1)) { atomicExch(status, 11); *failed = 1; break; }
-                const int page = table[page_lo + i];
+                const int page = table[page_of(i)];
                 const int row = ((page * 2) * G + g) * PAGE;          // K rows; V rows lie G * PAGE further
                 mbar_expect_tx(&kv_full[s], STAGE_BYTES);
 #pragma unroll
-                for (int c = 0; c < BLOCKS; ++c) {
+                for (int c = 0; c < SH::BLOCKS; ++c)
                     tma_load_2d(ring + s * STAGE_BYTES + c * (PAGE * 128), &map_kv, c * 64, row, &kv_full[s]);
-                    tma_load_2d(ring + s * STAGE_BYTES + KV_BYTES + c * (PAGE * 128), &map_kv, c * 64, row + G * PAGE,
-                                &kv_full[s]);
-                }
+#pragma unroll
+                for (int c = 0; c < SH::VBLOCKS; ++c)
+                    tma_load_2d(ring + s * STAGE_BYTES + K_BYTES + c * (PAGE * 128), &map_kv, c * 64, row + G * PAGE, &kv_full[s]);
             }
         }
         __syncwarp();
@@ -187,7 +214,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PAGE >> 3) << 17) |
                                          ((uint32_t)(ROWS >> 4) << 24);
             constexpr uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |      // B is MN-major
-                                          ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
+                                          ((uint32_t)(VD >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
             bool ok = mbar_wait(q_full, 0);
             if (!ok) { atomicExch(status, 12); *failed = 1; }
             const uint32_t q_addr = smem_u32(q_tile);
@@ -213,12 +240,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (!mbar_wait(&p_ready[i & 1], (i >> 1) & 1)) { atomicExch(status, 14); *failed = 1; ok = false; break; }
                 tcgen05_fence_after();
                 const int s = i % STAGES;
-                const uint32_t v_addr = smem_u32(ring + s * STAGE_BYTES + KV_BYTES);
-                const uint64_t dp = smem_desc(smem_u32(p_tile + (i & 1) * P_BYTES));
+                const uint32_t v_addr = smem_u32(ring + s * STAGE_BYTES + K_BYTES);
+                const uint64_t dp = smem_desc(smem_u32(p_tile + (i % PB) * P_PAGE));
 #pragma unroll
                 for (int k = 0; k < PAGE / 16; ++k)          // 16 keys = two groups of 8 rows of the V tile
-                    tcgen05_mma(tmem_base + O_COL, dp + (uint64_t)(k * 2),
-                                smem_desc_mn(v_addr + k * 2048, PAGE * 128), idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+                {
+                    const uint64_t dv = smem_desc_mn(v_addr + k * 2048, PAGE * 128);
+                    tcgen05_mma(tmem_base + O_COL, dp + (uint64_t)(k * 2), dv, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+                    if (SPLIT) tcgen05_mma(tmem_base + O_COL, dp + (uint64_t)((P_BYTES >> 4) + k * 2), dv, idesc_pv, 1u);
+                }
                 tcgen05_commit(&kv_empty[s]);                // the stage is free once both products have read it
                 tcgen05_commit(&o_ready[i & 1]);
             }
@@ -227,11 +257,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     } else if (has_work) {
         // ------------------------------------------------------------ softmax, two threads per row
         constexpr int HALF = PAGE / 2;                       // keys of a page per thread
-        constexpr int OHALF = HD / 2;                        // output features per thread
+        constexpr int OHALF = VD / 2;                        // output features per thread
         const int quarter = warp & 3;
         const int half = (warp - 2) >> 2;                    // warps 2-5: first half, warps 6-9: second half
         const int r = quarter * 32 + lane;                   // row of the tile = TMEM lane
         const int pos = first_pos + min(r, rows - 1);
+        const int low = first_seen(pos, window, chunk), last_low = first_seen(last_pos, window, chunk);
+        const bool capped = SPLIT && shaping.cap_log2 > 0.f;
+        const float to_log2 = capped ? 1.0f : scale_log2;        // capped scores are formed in log2 units
         const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const uint32_t o_addr = lane_addr + O_COL + half * OHALF;
         float m = -1.0e30f, l = 0.f;                         // m: the reference maximum the exponentials are taken against
@@ -247,13 +280,21 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
                 for (int j = 0; j < HALF; ++j) sreg[j] = 0;
             }
-            const int key_base = (page_lo + i) * PAGE + half * HALF;
-            const bool edge = key_base + HALF - 1 > first_pos || (window > 0 && key_base <= last_pos - window);
+            if (capped) {                                    // cap * tanh(score / cap) from one exp2 and one fast division
+                const float in = shaping.scale_over_cap * 2.885390081777927f, cap = shaping.cap_log2;
+#pragma unroll
+                for (int j = 0; j < HALF; ++j) {
+                    const float e = ex2(__uint_as_float(sreg[j]) * in);
+                    sreg[j] = __float_as_uint(fmaf(__fdividef(2.0f, e + 1.0f), -cap, cap));
+                }
+            }
+            const int key_base = page_of(i) * PAGE + half * HALF;
+            const bool edge = key_base + HALF - 1 > first_pos || key_base < last_low;
             if (edge) {
 #pragma unroll
                 for (int j = 0; j < HALF; ++j) {
                     const int key = key_base + j;
-                    if (key > pos || (window > 0 && key <= pos - window)) sreg[j] = 0xff800000u;      // -inf
+                    if (key > pos || (key < low && key >= keep)) sreg[j] = 0xff800000u;      // -inf
                 }
             }
             // independent chains for the maximum (and below for the sum): one chain of dependent
@@ -272,7 +313,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mine[r] = mx;
             // the two warps that share these 32 rows (each has half of the keys) meet; the other six go on
             asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
-            mx = fmaxf(mx, other[r]) * scale_log2;
+            mx = fmaxf(mx, other[r]) * to_log2;
             // The reference maximum follows only when the row's maximum has outgrown it by more than a factor of
             // 2^8. Then the sum so far and this thread's half of the output in tensor memory come down to the new
             // reference; the product of the previous page must have arrived there first, and the product of this
@@ -302,7 +343,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 m = mx;
             }
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-            uint8_t* p_row = p_tile + (i & 1) * P_BYTES + r * 128;
+            if (PB == 1 && i > 0) {                          // the previous page's product has read the weights' only buffer
+                const int pi = i - 1;
+                if (ok && !mbar_wait(&o_ready[pi & 1], (pi >> 1) & 1)) { if (lane == 0) atomicExch(status, 16); *failed = 1; ok = false; }
+            }
+            uint8_t* p_row = p_tile + (i % PB) * P_PAGE + r * 128;
 #pragma unroll
             for (int c = 0; c < HALF / 8; ++c) {
                 float e[8];
@@ -310,7 +355,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 for (int j = 0; j < 8; j += 2) {
                     e[j] = __uint_as_float(sreg[c * 8 + j]);
                     e[j + 1] = __uint_as_float(sreg[c * 8 + j + 1]);
-                    fma2(e[j], e[j + 1], scale_log2, -m);
+                    fma2(e[j], e[j + 1], to_log2, -m);
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) e[j] = ex2(e[j]);
@@ -323,7 +368,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 __nv_bfloat162 t2 = __floats2bfloat162_rn(e[4], e[5]), t3 = __floats2bfloat162_rn(e[6], e[7]);
                 packed.x = *reinterpret_cast<uint32_t*>(&t0); packed.y = *reinterpret_cast<uint32_t*>(&t1);
                 packed.z = *reinterpret_cast<uint32_t*>(&t2); packed.w = *reinterpret_cast<uint32_t*>(&t3);
-                *reinterpret_cast<uint4*>(p_row + (((half * (HALF / 8) + c) ^ (r & 7)) << 4)) = packed;
+                uint8_t* at = p_row + (((half * (HALF / 8) + c) ^ (r & 7)) << 4);
+                *reinterpret_cast<uint4*>(at) = packed;
+                if (SPLIT) {                                 // what the rounding left over
+                    const __nv_bfloat162 hi[4] = {t0, t1, t2, t3};
+                    uint32_t rest[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = __bfloat1622float2(hi[j]);
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(e[2 * j] - f.x, e[2 * j + 1] - f.y);
+                        rest[j] = *reinterpret_cast<const uint32_t*>(&lo);
+                    }
+                    *reinterpret_cast<uint4*>(at + P_BYTES) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
+                }
             }
             l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
             // the probabilities were written through the generic proxy; the MMA reads through the async proxy
@@ -339,12 +396,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         mine[r] = l;
         asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
         l += other[r];
+        if (SPLIT && shaping.sinks) l += ex2(shaping.sinks[h] * 1.4426950408889634f - m);
         if (npages > 0) {
             const int pi = npages - 1;
             if (ok && !mbar_wait(&o_ready[pi & 1], (pi >> 1) & 1)) { if (lane == 0) atomicExch(status, 16); *failed = 1; ok = false; }
             tcgen05_fence_after();
             const bool store = ok && *failed == 0 && r < rows;
-            const float inv = 1.0f / l;
+            float inv = 1.0f / l;
+            if (SPLIT && shaping.gate)
+                inv *= 1.0f / (1.0f + __expf(-__ldcg(shaping.gate + (size_t)(t_begin + row0 + min(r, rows - 1)) * shaping.gate_ld + h)));
             __nv_bfloat16* dst = out + ((size_t)(t_begin + row0 + min(r, rows - 1)) * H + h) * HD + half * OHALF;
 #pragma unroll
             for (int c0 = 0; c0 < OHALF; c0 += 32) {
@@ -378,28 +438,27 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
 }
 
-template <int HD>
+template <int HD, int VD, bool SPLIT>
 int launch_prefill_tc(const void* q, void* out, const void* pages, long long num_pages, const int* page_table,
                       int pt_stride, const int* q_start, const int* kv_len, int B, int T, int max_new, int H, int G,
-                      float scale, int window, int* status, cudaStream_t stream) {
-    using SH = Shape<HD>;
+                      float scale, int window, const Shaping& shaping, int* status, cudaStream_t stream) {
+    using SH = Shape<HD, VD, SPLIT>;
     CUtensorMap mq, mkv;
     int rc = make_map(&mq, q, T, (long long)H * HD, (long long)H * HD, ROWS);
     if (rc) return rc;
     rc = make_map(&mkv, pages, num_pages * 2 * G * PAGE, HD, HD, PAGE);
     if (rc) return rc;
+    auto kernel = attention_prefill_tc_kernel<HD, VD, SPLIT>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             SH::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::SMEM_BYTES);
         if (e != cudaSuccess) LP_REFUSE("attention_prefill_tc: cannot reserve %d bytes of shared memory: %s", SH::SMEM_BYTES,
                                         cudaGetErrorString(e));
         configured = true;
     }
     dim3 grid((max_new + ROWS - 1) / ROWS, H, B);
-    cudaError_t err = lp_launch(attention_prefill_tc_kernel<HD>, grid, THREADS, SH::SMEM_BYTES, stream, mq, mkv,
-                                (__nv_bfloat16*)out, page_table, pt_stride, q_start, kv_len, H, G,
-                                scale * 1.4426950408889634f, window, status);
+    cudaError_t err = lp_launch(kernel, grid, THREADS, SH::SMEM_BYTES, stream, mq, mkv, (__nv_bfloat16*)out, page_table,
+                                pt_stride, q_start, kv_len, H, G, scale * 1.4426950408889634f, window, shaping, status);
     if (err != cudaSuccess) {
         snprintf(lp_error_text, sizeof(lp_error_text), "attention_prefill_tc: %s", cudaGetErrorString(err));
         return (int)err;
@@ -409,21 +468,47 @@ int launch_prefill_tc(const void* q, void* out, const void* pages, long long num
 
 }  // namespace
 
-// q, out: [T, H, hd] bf16 (T = all new tokens of the step), hd 64 or 128; pages: [num_pages, 2, G, 64, hd] bf16;
-// q_start: [B+1]; kv_len: [B] (after the step). status: one int in device memory.
+// q, out: [T, H, hd] bf16 (T = all new tokens of the step); pages: [num_pages, 2, G, 64, hd] bf16;
+// q_start: [B+1]; kv_len: [B] (after the step). status: one int in device memory. Heads of 64 and 128 with values of the same
+// size (value_dim = hd), and heads of 192 of which the first value_dim <= 128 value features count: the others are zero in
+// `pages` or not wanted, and the rest of each head of `out` is left as it is. split_weights, softcap, sinks, keep, chunk, gate: as
+// in lp_attention_prefill; the last five come with split_weights.
 extern "C" int lp_attention_prefill_tc(const void* q, void* out, const void* pages, long long num_pages,
                                        const int* page_table, int pt_stride, const int* q_start, const int* kv_len,
-                                       int B, int T, int max_new, int H, int G, int hd, int page_size, float scale,
-                                       int window, int* status, cudaStream_t stream) {
+                                       int B, int T, int max_new, int H, int G, int hd, int value_dim, int page_size, float scale,
+                                       int window, int split_weights, float softcap, const float* sinks, int keep, int chunk,
+                                       const float* gate, int gate_ld, int* status, cudaStream_t stream) {
     if (B <= 0 || max_new <= 0) return 0;
-    if (hd != 64 && hd != 128) LP_REFUSE("attention_prefill_tc: head size %d (this kernel is built for 64 and 128)", hd);
+    if (!((hd == 64 || hd == 128) && value_dim == hd) && !(hd == 192 && value_dim > 0 && value_dim <= 128))
+        LP_REFUSE("attention_prefill_tc: heads of %d with values of %d (built for 64, 128, and 192 with at most 128)", hd, value_dim);
     if (page_size != PAGE) LP_REFUSE("attention_prefill_tc: pages of %d positions (built for %d)", page_size, PAGE);
     if (H <= 0 || G <= 0 || H % G) LP_REFUSE("attention_prefill_tc: %d query heads over %d key heads", H, G);
     if (H > 65535 || B > 65535) LP_REFUSE("attention_prefill_tc: %d heads x %d sequences exceed the grid", H, B);
     if (((uintptr_t)q | (uintptr_t)pages) & 15) LP_REFUSE("attention_prefill_tc: operands must be 16-byte aligned");
-    if (hd == 64)
-        return launch_prefill_tc<64>(q, out, pages, num_pages, page_table, pt_stride, q_start, kv_len, B, T, max_new, H, G,
-                                     scale, window, status, stream);
-    return launch_prefill_tc<128>(q, out, pages, num_pages, page_table, pt_stride, q_start, kv_len, B, T, max_new, H, G,
-                                  scale, window, status, stream);
+    if (!split_weights && (softcap > 0.f || sinks || (keep > 0 && window > 0) || chunk > 0 || gate))
+        LP_REFUSE("attention_prefill_tc: shaped scores come with split weights");
+    if (gate && gate_ld < H) LP_REFUSE("attention_prefill_tc: rows of %d gates for %d heads", gate_ld, H);
+    if (keep > 0 && window > 0 && chunk > 0) LP_REFUSE("attention_prefill_tc: kept first tokens (%d) and chunks (%d) exclude each other", keep, chunk);
+    Shaping x{};
+    if (softcap > 0.f) {
+        x.cap_log2 = softcap * 1.4426950408889634f;
+        x.scale_over_cap = scale / softcap;
+    }
+    x.sinks = sinks;
+    x.keep = window > 0 && keep > 0 ? keep : 0;
+    x.chunk = chunk > 0 ? chunk : 0;
+    x.gate = gate;
+    x.gate_ld = gate_ld;
+#define LP_LAUNCH_TC(HD, VD, SPLIT)                                                                                                  \
+    return launch_prefill_tc<HD, VD, SPLIT>(q, out, pages, num_pages, page_table, pt_stride, q_start, kv_len, B, T, max_new, H, G,   \
+                                            scale, window, x, status, stream)
+    if (split_weights) {
+        if (hd == 64) LP_LAUNCH_TC(64, 64, true);
+        if (hd == 128) LP_LAUNCH_TC(128, 128, true);
+        LP_LAUNCH_TC(192, 128, true);
+    }
+    if (hd == 64) LP_LAUNCH_TC(64, 64, false);
+    if (hd == 128) LP_LAUNCH_TC(128, 128, false);
+    LP_LAUNCH_TC(192, 128, false);
+#undef LP_LAUNCH_TC
 }

@@ -72,8 +72,8 @@ _SIGNATURES = {
                                       _I, _I, _I, _P, _F, _I, ctypes.c_longlong, _P, _P],
     },
     "attention_tcgen05": {
-        "lp_attention_prefill_tc": [_P, _P, _P, ctypes.c_longlong, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I,
-                                    _P, _P],
+        "lp_attention_prefill_tc": [_P, _P, _P, ctypes.c_longlong, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _F, _P,
+                                    _I, _I, _P, _I, _P, _P],
     },
     "latent_attention": {
         "lp_latent_prepare": [_P, _I, _I, _I, _P, _F, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P,
@@ -1000,13 +1000,15 @@ def attention_prefill(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, p
                       q_start: torch.Tensor, kv_len: torch.Tensor, max_new: int, *, num_heads: int,
                       num_kv_heads: int, head_dim: int, scale: float, window: Optional[int],
                       softcap: Optional[float] = None, sinks: Optional[torch.Tensor] = None,
-                      exact_weights: bool = False, keep_first: int = 0, chunk: int = 0, distance=None, gate=None) -> torch.Tensor:
+                      exact_weights: bool = False, keep_first: int = 0, chunk: int = 0, distance=None, gate=None,
+                      value_dim: Optional[int] = None) -> torch.Tensor:
     """Tensor-core attention for a step that brings several tokens per sequence. ``keep_first`` (with a window): the
     sequence's first ``keep_first`` tokens stay visible to every later query.
     ``q_start`` [B+1]: offsets of each sequence's new tokens; ``kv_len`` [B]: lengths after the step.
     ``exact_weights``: the softmax weights enter the product with the values at float32 precision (as a bfloat16
     value plus a bfloat16 rest, two products) instead of rounded to bfloat16. ``chunk``, ``distance`` (with
-    ``exact_weights``), ``gate``: see :func:`attention_plain`."""
+    ``exact_weights``), ``gate``: see :func:`attention_plain`. ``value_dim``: only the first so many features of every
+    value head matter; what lies beyond them in each head of ``out`` is then undefined."""
     dist_scale, dist_rate = _distance_args(distance, num_heads, "attention_prefill")
     gate_ptr, gate_ld = _gate_args(gate, q.shape[0], num_heads, "attention_prefill")
     _check_attention(q, out, pages, page_table, num_heads, num_kv_heads, head_dim, "attention_prefill")
@@ -1017,15 +1019,18 @@ def attention_prefill(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, p
         raise KernelError(f"attention_prefill: {B} sequences, {q_start.numel()} offsets, table {tuple(page_table.shape)}")
     _check_sinks(sinks, num_heads, "attention_prefill")
     keep_first = int(keep_first) if window else 0
-    if (head_dim in (64, 128) and max_new > 64 and tcgen05_attention and not softcap and sinks is None and not exact_weights
-            and not keep_first and not chunk and distance is None and gate is None):
-        # long runs of new tokens with heads of 64 or 128: scores and P V on the tcgen05 tensor cores
+    # runs of more than 64 new tokens: the tcgen05 kernel where it is built for the heads (64, 128, and 192 with values of at most
+    # 128) and nothing shapes the scores, or what does comes with weights at float32 precision; a distance bias stays with mma.sync
+    built = head_dim in (64, 128) or (head_dim == 192 and value_dim is not None and value_dim <= 128)
+    plain = not softcap and sinks is None and not keep_first and not chunk and gate is None
+    if tcgen05_attention and max_new > 64 and built and distance is None and (plain or exact_weights):
         lib = library("attention_tcgen05")
         _check(lib, lib.lp_attention_prefill_tc(
             q.data_ptr(), out.data_ptr(), pages.data_ptr(), pages.shape[0], page_table.data_ptr(),
             page_table.shape[1], q_start.data_ptr(), kv_len.data_ptr(), B, q.shape[0], int(max_new), num_heads,
-            num_kv_heads, head_dim, pages.shape[3], float(scale), int(window) if window else 0,
-            kernel_status().data_ptr(), _stream()))
+            num_kv_heads, head_dim, int(value_dim) if head_dim == 192 else head_dim, pages.shape[3], float(scale),
+            int(window) if window else 0, 1 if exact_weights else 0, float(softcap or 0.0), _ptr(sinks), keep_first, int(chunk or 0),
+            gate_ptr, gate_ld, kernel_status().data_ptr(), _stream()))
         return out
     lib = library("attention_mma")
     _check(lib, lib.lp_attention_prefill(

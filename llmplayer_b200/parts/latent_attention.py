@@ -209,7 +209,7 @@ class LatentAttention(Part):
         with ops.section("attention.scores"):
             ops.attention_prefill(q_half, heads, step_pages, step_table, ctx.q_start, ctx.kv_len, ctx.max_new, num_heads=H,
                                   num_kv_heads=H, head_dim=hd, scale=s.scale, window=s.window,
-                                  exact_weights=s.exact_weights)
+                                  exact_weights=s.exact_weights, value_dim=dv)
         o = ctx.buffer("attn_out", (T, H * dv), torch.bfloat16)
         gate = proj[:, gate_off:gate_off + H] if s.out_gate is not None else None
         clear = None if add else self._out_to_clear(ctx, T, out)

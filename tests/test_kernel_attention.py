@@ -5,6 +5,8 @@ import math
 import pytest
 import torch
 
+from helpers import check_error
+
 pytestmark = pytest.mark.gpu
 
 PAGE = 64
@@ -432,3 +434,68 @@ def test_float32_attention_in_blocks(form, H, G, hd):
             ops.attention_plain(d(q[at]), out, d(pages), d(gone if late else table), d(seq[at]), d(pos[at]), **kw, **sk, scratch=use,
                                 longest=int(pos[at].max()) + 1)
             assert torch.equal(out, whole[at.to(dev)]), (rows, use is None)
+
+
+SHAPED = [dict(exact_weights=True), dict(exact_weights=True, softcap=15.0, sinks=True), dict(exact_weights=True, window=100, keep_first=5),
+          dict(exact_weights=True, window=150, keep_first=70, sinks=True, gate=True), dict(exact_weights=True, chunk=96, gate=True),
+          dict(exact_weights=True, chunk=200, softcap=20.0)]
+
+
+@pytest.mark.parametrize("hd,vd,H,G", [(64, 64, 4, 2), (128, 128, 4, 1), (192, 128, 3, 3), (192, 72, 2, 1)])
+@pytest.mark.parametrize("shape", [{}, dict(window=130)] + SHAPED, ids=lambda s: "-".join(s) or "plain")
+def test_tcgen05_prompt_attention_with_everything_that_shapes_it(hd, vd, H, G, shape):
+    """Long runs of new tokens against float64: sequences that start at their first token and ones that continue, at the edges of
+    tiles of 128 rows and pages; pages that no query reaches are gone."""
+    from llmplayer_b200.kernels import ops
+    dev, P = "cuda:0", 64
+    g = torch.Generator(device=dev).manual_seed(hd + len(shape))
+    before, new = [0, 0, 300, 129, 64], [257, 128, 65, 200, 1]
+    lengths = [a + b for a, b in zip(before, new)]
+    width = -(-max(lengths) // P)
+    order = torch.randperm(len(new) * width, generator=torch.Generator().manual_seed(3)).reshape(len(new), width)
+    pages = torch.randn(len(new) * width, 2, G, P, hd, generator=g, device=dev).to(torch.bfloat16)
+    pages[:, 1, :, :, vd:] = 0
+    T = sum(new)
+    q = (1.5 * torch.randn(T, H * hd, generator=g, device=dev)).to(torch.bfloat16)
+    shape = dict(shape)
+    window, keep, chunk, cap = shape.get("window"), shape.get("keep_first", 0), shape.get("chunk", 0), shape.get("softcap")
+    table = order.clone().to(torch.int32)
+    for i, b in enumerate(before):
+        first = max(b - window + 1 if window else 0, b // chunk * chunk if chunk else 0)
+        table[i, -(-keep // P):max(0, first) // P] = -1
+    if shape.pop("sinks", False):
+        shape["sinks"] = 2 * torch.randn(H, generator=g, device=dev)
+    if shape.pop("gate", False):
+        shape["gate"] = torch.randn(T, H + 3, generator=g, device=dev)[:, 2:2 + H]
+    out = torch.full((T, H * hd), 7.0, device=dev, dtype=torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)  # noqa: E731
+    starts = [sum(new[:i]) for i in range(len(new) + 1)]
+    scale = hd ** -0.5
+    kw = dict({"window": None}, **shape)
+    ops.attention_prefill(q, out, pages, table.to(dev), i32(starts), i32(lengths), max(new), num_heads=H, num_kv_heads=G, head_dim=hd,
+                          scale=scale, value_dim=vd, **kw)
+    torch.cuda.synchronize()
+    ops.check_kernel_status()
+    worst, top = 0.0, 0.0
+    for i, n in enumerate(new):
+        kv = torch.cat([pages[int(p)] for p in order[i, :-(-lengths[i] // P)]], dim=2)[:, :, :lengths[i]].double()      # [2, G, len, hd]
+        pos = before[i] + torch.arange(n, device=dev)[:, None]
+        key = torch.arange(lengths[i], device=dev)[None, :]
+        seen = key <= pos
+        if window:
+            seen &= (key > pos - window) | (key < keep)
+        if chunk:
+            seen &= key // chunk == pos // chunk
+        for h in range(H):
+            s = q[starts[i]:starts[i] + n].reshape(n, H, hd)[:, h].double() @ kv[0, h * G // H].T * scale
+            s = (cap * torch.tanh(s / cap) if cap else s).masked_fill(~seen, float("-inf"))
+            if "sinks" in shape:
+                s = torch.cat([s, shape["sinks"][h].double().expand(n, 1)], dim=1)
+            ref = torch.softmax(s, -1)[:, :lengths[i]] @ kv[1, h * G // H]
+            if "gate" in shape:
+                ref = ref * torch.sigmoid(shape["gate"][starts[i]:starts[i] + n, h].double())[:, None]
+            got = out[starts[i]:starts[i] + n].reshape(n, H, hd)[:, h, :vd].double()
+            worst, top = max(worst, float((got - ref[:, :vd]).abs().max())), max(top, float(ref.abs().max()))
+    # the result's own rounding to bfloat16 is 2^-9 of a value; weights rounded to bfloat16 add as much again and more in short rows
+    check_error("attention kernel (tcgen05, " + ("float32 weights)" if "exact_weights" in shape else "bfloat16 weights)"), f"{H}/{G} x {hd}",
+                worst / top, 4e-3 if "exact_weights" in shape else 2e-2)
