@@ -771,11 +771,17 @@ PERSISTENT_MIN_TOKENS = 512
 
 def _persistent_pays(tokens: int, features: int, k: int, mode: int) -> bool:
     """Whether the persistent form (one CTA per SM walking 128 x 256 tiles, 128 x 128 x 2 when gated)
-    fills the SMs at least as well as separate CTAs of 128 x 128 tiles, two to an SM."""
+    beats separate CTAs of 128 x 128 tiles, two to an SM. For the gated product: where it fills the SMs at least as well. The
+    others: always, but for long K loops over so few tiles that separate CTAs with K shared out use more of the chip (us on a B200,
+    persistent / separate: storing 1943 x 3664 x 2048 29 / 34, 2048 x 3072 x 2048 29 / 32, 1024 x 1024 x 2048 16 / 17, but
+    520 x 1024 x 4096 25 / 17, 1024 x 1024 x 4096 26 / 21, 1300 x 1024 x 4096 25 / 26; adding, where no output has to be cleared
+    first, 520 x 1024 x 2048 16 / 11, 1024 x 1024 x 2048 16 / 13, 1300 x 1024 x 2048 16 / 17, 520 x 1024 x 1024 12 / 12)."""
     feat_tiles = -(-features // 128)
     persistent_tiles = feat_tiles * -(-tokens // (128 if mode == SWIGLU else 256))
-    separate_ctas = feat_tiles * -(-tokens // 128)
     sms = num_sms()
+    if mode != SWIGLU:
+        return persistent_tiles * 4 > sms or k < (4096 if mode == STORE else 2048)
+    separate_ctas = feat_tiles * -(-tokens // 128)
     fill_p = persistent_tiles / (-(-persistent_tiles // sms) * sms)
     fill_s = separate_ctas / (-(-separate_ctas // (2 * sms)) * 2 * sms)
     # at equal fill the persistent form wins when the SMs are well filled (its tiles are twice as large and one
