@@ -750,6 +750,125 @@ qkv_prepare_kernel(const float* __restrict__ qkv, int ld, const float* __restric
     }
 }
 
+// The same for heads of HD = 64 or 128 features throughout (dk = dv = hdp), rows and buffers on 16-byte boundaries and rotary
+// halves of a multiple of four: a lane holds four neighbouring features, so a head is half a warp or a warp, a rotation's
+// partner is a shuffle away and every access is 16 bytes (8 of bfloat16). Bound by its bytes and the latency of one head's
+// steps: 2048 tokens, 16 + 2 x 4 heads of 128, B200: 27 us value by value (above) -> 17.
+__device__ __forceinline__ void prep_store4(float* to, const float* v) { *(float4*)to = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void prep_store4(__nv_bfloat16* to, const float* v) {
+    __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *(uint2*)to = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+template <int HD, typename TQ, typename TKV>
+__global__ void __launch_bounds__(256)
+qkv_prepare_vec4_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ bias, const float* __restrict__ inv_freq,
+                        const float2* __restrict__ angles, const int* __restrict__ positions, const int* __restrict__ seq_ids,
+                        const int* __restrict__ page_table, int pt_stride, TQ* __restrict__ q_out, TKV* __restrict__ pages, int T,
+                        int H, int G, int rd, int interleaved, int unit, float unit_eps, int page_size,
+                        float* __restrict__ zero, long long zero_count, const float* __restrict__ qgain,
+                        const float* __restrict__ kgain, float gain_eps, int vnorm, float vnorm_eps, float* __restrict__ vkeep,
+                        const float* __restrict__ vfirst, const float* __restrict__ vmix) {
+    constexpr int LANES = HD / 4, SUB = 32 / LANES;
+    lp_grid_release();
+    lp_grid_wait();
+    clear_on_the_side(zero, zero_count);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int li = lane % LANES, e0 = li * 4;
+    const int heads = H + 2 * G;
+    const long long work_all = (long long)T * heads, asked = ((long long)blockIdx.x * 8 + warp) * SUB + lane / LANES;
+    const bool live = asked < work_all;
+    const long long work = live ? asked : work_all - 1;      // (a half warp without a head follows along: shuffles need it)
+    const int t = (int)(work / heads), item = (int)(work - (long long)t * heads);
+    const int pos = positions[t];
+    const int half = rd >> 1;
+    const bool rotated = item < H + G;
+    const int g = item - H - G;
+    const int src = item * HD;                               // heads of one size lie one after another
+    const float4 x = *(const float4*)(qkv + (long long)t * ld + src + e0);
+    float v[4] = {x.x, x.y, x.z, x.w};
+    if (bias) {
+        const float4 b = *(const float4*)(bias + src + e0);
+        v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w;
+    }
+    const bool turns = rotated && e0 < rd;
+    // the lane's pairs: (e0, e0 + 1) and (e0 + 2, e0 + 3), or e0 .. e0 + 3 with the features half a rotary width away
+    const bool first = e0 < half;
+    const int pair = interleaved ? e0 >> 1 : (first ? e0 : e0 - half);
+    float c[4], s[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { c[i] = 1.f; s[i] = 0.f; }
+    if (turns) {
+        if (angles) {
+            const float4* a = (const float4*)(angles + (long long)t * half + pair);
+            const float4 a0 = a[0], a1 = interleaved ? a0 : a[1];
+            c[0] = a0.x; s[0] = a0.y; c[1] = a0.z; s[1] = a0.w;
+            c[2] = a1.x; s[2] = a1.y; c[3] = a1.z; s[3] = a1.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < 2 || !interleaved) sincosf((float)pos * inv_freq[pair + i], &s[i], &c[i]);
+        }
+    }
+    auto squares = [&] {
+        float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        return ss;
+    };
+    const float* gain = item < H ? qgain : kgain;
+    if (qgain || kgain) {
+        const float pre = 1.0f / sqrtf(squares() / (float)HD + gain_eps);
+        if (rotated && gain) {
+            const float4 w = *(const float4*)(gain + e0);
+            v[0] = v[0] * pre * w.x; v[1] = v[1] * pre * w.y; v[2] = v[2] * pre * w.z; v[3] = v[3] * pre * w.w;
+        }
+    }
+    if (rd > 0) {
+        float other[4];
+        const int partner = interleaved ? li : (e0 >= rd ? li : first ? li + (half >> 2) : li - (half >> 2));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) other[i] = __shfl_sync(0xffffffffu, v[i], partner, LANES);
+        if (turns) {
+            if (interleaved) {
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    const float a = v[i], b = v[i + 1], cc = c[i >> 1], sn = s[i >> 1];
+                    v[i] = a * cc - b * sn;
+                    v[i + 1] = b * cc + a * sn;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = first ? v[i] * c[i] - other[i] * s[i] : v[i] * c[i] + other[i] * s[i];
+            }
+        }
+    }
+    float factor = 1.0f;
+    if (unit || vnorm) {
+        const float ss = squares();
+        if (rotated) { if (unit) factor = 1.0f / sqrtf(ss / (float)HD + unit_eps); }
+        else if (vnorm) factor = 1.0f / sqrtf(ss / (float)HD + vnorm_eps);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] *= factor;
+    if (!live) return;
+    if (item < H) {
+        prep_store4(q_out + ((long long)t * H + item) * HD + e0, v);
+        return;
+    }
+    if (!rotated && (vkeep || vfirst)) {
+        const long long at = ((long long)t * G + g) * HD + e0;
+        if (vkeep) prep_store4(vkeep + at, v);
+        if (vfirst) {
+            const float lambda = *vmix;
+            const float4 f = *(const float4*)(vfirst + at);
+            v[0] = (1.0f - lambda) * v[0] + lambda * f.x; v[1] = (1.0f - lambda) * v[1] + lambda * f.y;
+            v[2] = (1.0f - lambda) * v[2] + lambda * f.z; v[3] = (1.0f - lambda) * v[3] + lambda * f.w;
+        }
+    }
+    const long long page = page_table[(long long)seq_ids[t] * pt_stride + pos / page_size];
+    prep_store4(pages + (((page * 2 + (rotated ? 0 : 1)) * G + (rotated ? item - H : g)) * page_size + pos % page_size) * HD + e0, v);
+}
+
 extern "C" int lp_qkv_prepare(const float* qkv, int ld, const float* bias, const float* inv_freq, const float* angles,
                               const int* positions, const int* seq_ids, const int* page_table, int pt_stride, void* q_out, int q_dtype,
                               void* pages, int kv_dtype, int T, int H, int G, int dk, int dv, int hdp, int rd,
@@ -767,6 +886,23 @@ extern "C" int lp_qkv_prepare(const float* qkv, int ld, const float* bias, const
     if (G == 0) page_size = 1;
     const long long blocks = ((long long)T * (H + 2 * G) + 7) / 8;
     if (blocks > 0x7fffffffLL) LP_REFUSE("qkv_prepare: %d tokens of %d heads exceed the grid", T, H + 2 * G);
+    const bool wide = dk == hdp && dv == hdp && (hdp == 64 || hdp == 128) && ld % 4 == 0 && rd % (interleaved ? 4 : 8) == 0 &&
+                      (((uintptr_t)qkv | (uintptr_t)bias | (uintptr_t)angles | (uintptr_t)q_out | (uintptr_t)pages | (uintptr_t)qgain |
+                        (uintptr_t)kgain | (uintptr_t)vkeep | (uintptr_t)vfirst) & 15) == 0;
+    if (wide) {
+        const unsigned grid = (unsigned)(((long long)T * (H + 2 * G) + (8 * 128 / hdp) - 1) / (8 * 128 / hdp));
+#define LP_LAUNCH_WIDE(HD, TQ, TKV)                                                                                               \
+        lp_launch(qkv_prepare_vec4_kernel<HD, TQ, TKV>, grid, 256, 0, stream, qkv, ld, bias, inv_freq, (const float2*)angles,     \
+                  positions, seq_ids, page_table, pt_stride, (TQ*)q_out, (TKV*)pages, T, H, G, rd, interleaved, unit, unit_eps,   \
+                  page_size, zero, zero_count, qgain, kgain, gain_eps, vnorm, vnorm_eps, vkeep, vfirst, vmix)
+        if (q_dtype == LP_F32 && kv_dtype == LP_F32) {
+            if (hdp == 64) LP_LAUNCH_WIDE(64, float, float); else LP_LAUNCH_WIDE(128, float, float);
+        } else if (q_dtype == LP_BF16 && kv_dtype == LP_BF16) {
+            if (hdp == 64) LP_LAUNCH_WIDE(64, __nv_bfloat16, __nv_bfloat16); else LP_LAUNCH_WIDE(128, __nv_bfloat16, __nv_bfloat16);
+        } else LP_REFUSE("qkv_prepare: dtype codes q=%d kv=%d", q_dtype, kv_dtype);
+#undef LP_LAUNCH_WIDE
+        return lp_check_launch("qkv_prepare");
+    }
 #define LP_LAUNCH_PREP(PER, TQ, TKV)                                                                                     \
     lp_launch(qkv_prepare_kernel<PER, TQ, TKV>, (unsigned)blocks, 256, 0, stream, qkv, ld, bias, inv_freq,                \
               (const float2*)angles, positions, seq_ids, page_table, pt_stride, (TQ*)q_out, (TKV*)pages, T, H, G, dk, dv,  \
