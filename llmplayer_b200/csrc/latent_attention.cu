@@ -107,7 +107,8 @@ latent_prepare_kernel(const float* __restrict__ proj, int ld, int q_off, int kv_
 }
 
 // The same four values at a time (sizes, offsets and row lengths of a multiple of four, rotary halves as well; 16-byte
-// aligned rows): a warp per head instead of a division per value. Bound by its bytes and the latency of one token's steps: 1925 tokens, 16 heads of 192, rank 512, B200: 29 us value by
+// aligned rows): a warp per head instead of a division per value, in steps of few tokens with CTAs of their own for the heads
+// (8 tokens: 8.7 -> 6.8 us). Bound by its bytes and the latency of one token's steps: 1925 tokens, 16 heads of 192, rank 512, B200: 29 us value by
 // value with the float32 queries -> 19 without them.
 __device__ __forceinline__ void store4(float* to, const float* v) { *(float4*)to = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void store4(__nv_bfloat16* to, const float* v) {
@@ -165,7 +166,9 @@ latent_prepare_vec4_kernel(const float* __restrict__ proj, int ld, int q_off, in
     const float* row = proj + (long long)t * ld;
     const float* kv = row + kv_off;
     float ss = 0.f;
-    for (int i = tid * 4; i < rank; i += blockDim.x * 4) {
+    // a grid of several CTAs per token: the first takes the latent and the shared key part, the others eight heads each
+    const bool whole = gridDim.y == 1, takes_row = blockIdx.y == 0;
+    for (int i = tid * 4; i < rank && takes_row; i += blockDim.x * 4) {
         const float4 v = *(const float4*)(kv + i);
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
@@ -174,21 +177,22 @@ latent_prepare_vec4_kernel(const float* __restrict__ proj, int ld, int q_off, in
     const int page = page_table[(long long)seq_ids[t] * pt_stride + pos / page_size];
     const int Dk = rank + dr;
     TKV* dst = pages + ((long long)page * page_size + pos % page_size) * Dk;
-    for (int i = tid * 4; i < rank; i += blockDim.x * 4) {
+    for (int i = tid * 4; i < rank && takes_row; i += blockDim.x * 4) {
         const float4 x = *(const float4*)(kv + i), g = *(const float4*)(gain + i);
         const float v[4] = {x.x * factor * g.x, x.y * factor * g.y, x.z * factor * g.z, x.w * factor * g.w};
         store4(dst + i, v);
         if (latent_out) store4(latent_out + (long long)t * rank + i, v);
     }
-    for (int i = tid * 4; i < dr; i += blockDim.x * 4) {
+    for (int i = tid * 4; i < dr && takes_row; i += blockDim.x * 4) {
         float v[4];
         rotate4(kv + rank, i, rot, interleaved, cs, sn, v);
         store4(dst + rank + i, v);
         if (shared_out) store4(shared_out + (long long)t * dr + i, v);
     }
+    if (takes_row && !whole) return;
     const int hd = dn + dr;
     const float* q = q_sep ? q_sep + (long long)t * ldq : row + q_off;
-    for (int h = warp; h < H; h += 8) {
+    for (int h = (whole ? 0 : ((int)blockIdx.y - 1) * 8) + warp; h < H; h += whole ? 8 : H) {
         const float* qh = q + h * hd;
         for (int i = lane * 4; i < max(hd, q_half ? q_half_hd : 0); i += 128) {
             float v[4] = {0.f, 0.f, 0.f, 0.f};            // heads padded with zeros to a size the attention kernels take
@@ -1134,8 +1138,9 @@ extern "C" int lp_latent_prepare(const float* proj, int ld, int q_off, int kv_of
                      (((uintptr_t)proj | (uintptr_t)gain | (uintptr_t)q_out | (uintptr_t)pages | (uintptr_t)latent_out | (uintptr_t)shared_out |
                        (uintptr_t)q_half | (uintptr_t)q_sep) & 15) == 0;
     if (!q_out && !q_half) LP_REFUSE("latent_prepare: nowhere to write the queries");
+    const int shares = vec && T * (1 + (H + 7) / 8) <= 2 * lp_sm_count() ? 1 + (H + 7) / 8 : 1;
 #define LP_LAUNCH_PREP(TKV)                                                                                       \
-    lp_launch(vec ? latent_prepare_vec4_kernel<TKV> : latent_prepare_kernel<TKV>, T, 256, 0, stream, proj, ld, q_off, kv_off, gain, eps, inv_freq, rot,    \
+    lp_launch(vec ? latent_prepare_vec4_kernel<TKV> : latent_prepare_kernel<TKV>, dim3(T, shares), 256, 0, stream, proj, ld, q_off, kv_off, gain, eps, inv_freq, rot,    \
               positions, seq_ids, page_table, pt_stride, q_out, (TKV*)pages, H, dn, dr, rank, page_size,                   \
               (__nv_bfloat16*)latent_out, (__nv_bfloat16*)shared_out, (__nv_bfloat16*)q_half, q_half_hd, q_sep, ldq,    \
               interleaved, magnitude)
