@@ -20,9 +20,9 @@
 //             thread per column, all in float32 arithmetic; the results go to a record per chunk and head, laid out as the
 //             operand fragments of the second kernel's products.
 //   carry     one CTA per (16 value columns, head, sequence) walks the sequence's chunks in order; the state's columns stay in
-//             shared memory. The products run on the tensor cores (mma.sync m16n8k8) at float32 precision: every
-//             operand is split into two TF32 parts, x = hi + lo with 22 bits of mantissa together, and hi hi + hi lo + lo hi
-//             are summed in float32. Records come by cp.async, one chunk ahead.
+//             registers, 16 key channels per warp. The products run on the tensor cores (mma.sync m16n8k8) at float32
+//             precision: every operand is split into two TF32 parts, x = hi + lo with 22 bits of mantissa together, and
+//             hi hi + hi lo + lo hi are summed in float32. Records come by cp.async, up to two chunks ahead.
 #include "common.cuh"
 
 namespace {
@@ -31,21 +31,24 @@ constexpr int CT = 32;                  // tokens per chunk
 constexpr int HB = 16;                  // tokens per block inside a chunk
 constexpr int NC = 16;                  // value columns per CTA of the second kernel
 constexpr int THREADS = 256;            // of the first kernel
-constexpr int CARRY_THREADS = 512;      // of the second: 16 warps, one per 16 key channels
+constexpr int JOINERS = CT / 8;         // warps of the second kernel beside one per 16 key channels: one per 8 tokens
 constexpr int MAX_DK = 256;
+constexpr int CARRY_THREADS = 32 * (MAX_DK / 16 + JOINERS);      // at most
 constexpr size_t MAX_SMEM = 227 * 1024;
 
 constexpr int DECAY_CHANNEL = 0, DECAY_HEAD = 1, DECAY_FIXED = 2;
 
-// Floats of a record: [W][Q][K^T][B][P_32], fragments of 16 x 8 values each (128 floats: a lane's four values together).
+// Floats of a record: [W][Q][K^T][B][P_32], fragments of 8 x 16 values each (128 floats: a lane's four values together).
 __host__ __device__ __forceinline__ int padded(int dk) { return (dk + 15) / 16 * 16; }
 __host__ __device__ __forceinline__ int record_floats(int dkp, bool delta) { return CT * dkp * (delta ? 3 : 2) + CT * CT + dkp; }
 __host__ __device__ __forceinline__ int value_floats(int dv) { return (dv + NC - 1) / NC * NC * CT; }
 
-// where element (r, c) of a matrix with `ksteps` = columns / 8 lies in its fragment order (m16n8k8, row operand)
+// Where element (r, c) of a matrix with `ksteps` = columns / 8 lies as the column operand of m16n8k8, two steps together. The
+// columns of a step are taken in the order 0, 2, 4, 6, 1, 3, 5, 7: a lane holds two neighbouring ones, as it does of a product's
+// results, which so are the other operand of the next product as they lie.
 __device__ __forceinline__ int fragment_at(int r, int c, int ksteps) {
-    const int lane = (r & 7) * 4 + (c & 3), reg = ((r >> 3) & 1) + ((c >> 2) & 1) * 2;
-    return (((r >> 4) * ksteps + (c >> 3)) * 32 + lane) * 4 + reg;
+    const int lane = (r & 7) * 4 + ((c & 7) >> 1), reg = (c & 1) + ((c >> 3) & 1) * 2;
+    return (((r >> 3) * (ksteps >> 1) + (c >> 4)) * 32 + lane) * 4 + reg;
 }
 
 __device__ __forceinline__ float rotated_channel(const float* head, int c, int rd, int interleaved, const float2* cs) {
@@ -300,30 +303,19 @@ __device__ __forceinline__ void cp16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-constexpr int SROW = 24;                // floats per row of S and U in shared memory: 16 columns, operand reads without conflicts
-
-// acc[two tiles of 16 x 8] += A[16 x 8 (s1 - s0)] X[8 (s1 - s0) x 16] for the steps s0 .. s1 - 1 of 8 columns of A (in fragment
-// order), X split into `xh` + `xl` (rows of SROW); three chains of sums per tile
-__device__ __forceinline__ void product(float (*acc)[3][4], const float* frag, const uint32_t* xh, const uint32_t* xl, int s0, int s1,
-                                        int lane) {
-    const float4* a = reinterpret_cast<const float4*>(frag) + lane;
-    const int at = (lane & 3) * SROW + (lane >> 2);
-#pragma unroll 4
-    for (int s = s0; s < s1; ++s) {
-        const float4 av = a[s * 32];
-        uint32_t ah[4], al[4];
-        split_tf32(av.x, ah[0], al[0]);
-        split_tf32(av.y, ah[1], al[1]);
-        split_tf32(av.z, ah[2], al[2]);
-        split_tf32(av.w, ah[3], al[3]);
+// acc += X Y over two steps of 8, X [16 x 16] split as row operands (xh, xl), Y [16 x 8] as one fragment of a record; three
+// chains of sums
+__device__ __forceinline__ void product(float (*acc)[4], const uint32_t (*xh)[4], const uint32_t (*xl)[4], float4 y) {
+    uint32_t h[4], l[4];
+    split_tf32(y.x, h[0], l[0]);
+    split_tf32(y.y, h[1], l[1]);
+    split_tf32(y.z, h[2], l[2]);
+    split_tf32(y.w, h[3], l[3]);
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
-            const int e = at + s * 8 * SROW + w * 8;
-            const uint32_t bh[2] = {xh[e], xh[e + 4 * SROW]}, bl[2] = {xl[e], xl[e + 4 * SROW]};
-            mma_tf32(acc[w][0], ah, bh);
-            mma_tf32(acc[w][1], ah, bl);
-            mma_tf32(acc[w][2], al, bh);
-        }
+    for (int w = 0; w < 2; ++w) {
+        mma_tf32(acc[0], xh[w], h + 2 * w);
+        mma_tf32(acc[1], xh[w], l + 2 * w);
+        mma_tf32(acc[2], xl[w], h + 2 * w);
     }
 }
 __device__ __forceinline__ float4 chains(const float (*acc)[4]) {
@@ -331,15 +323,13 @@ __device__ __forceinline__ float4 chains(const float (*acc)[4]) {
                        acc[0][3] + (acc[1][3] + acc[2][3]));
 }
 
-// 16 warps. W S and Q S (32 x 16 each) share the warps, four per 16 rows with a quarter of the key channels each (without W,
-// eight per 16 rows of Q S); their parts meet in shared memory. Then warp m owns the state's key channels 16 m .. 16 m + 15:
-// its threads hold those entries in registers, shared memory holds them split for the products; the last two warps add up
-// Q S for their rows, add B U and write the outputs.
-// Bound by the instructions of a chunk's steps (366 per warp, 48 % of the issue slots) and the barriers between them, one
-// chunk after another. With three records in flight a stage is free as soon as the next chunk begins, and the parts of Q S are read by the warps
-// that use them: three barriers per chunk for the delta rule, two without it (U is V then and is split beside the first
-// products), where four were. 2048 tokens, 8 heads of 128 x 256, B200: 117 -> 114 us; 3 sequences of 518 to 777, 8 heads of
-// 128 x 128, delta rule: 91 -> 88.
+// All products are taken transposed (value columns are their 16 rows). Worker m holds S^T for the key channels 16 m .. 16 m + 15
+// in registers, which are the row operand of its share of (W S)^T and (Q S)^T as they lie; the shares meet in shared memory.
+// Joiner n has the tokens 8 n .. 8 n + 7: it requests the records, makes U^T = (U0 - W S)^T (split, as the row operand of what
+// follows) while the workers multiply with Q, and adds (B U)^T to the shares of (Q S)^T and writes the outputs while they
+// update the state. Bound by the chain of a chunk's steps, with three barriers for the delta rule and two without it (U is V
+// then). With the state split in shared memory, read as column operands and stored again in every chunk, 2048 tokens of 8 heads
+// of 128 x 256 took 114 us on a B200, and take 97.
 // STAGES: records in flight (three, or fewer where they do not fit shared memory; then a barrier frees the stage).
 template <int STAGES>
 __global__ void __launch_bounds__(CARRY_THREADS)
@@ -347,13 +337,13 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
              const float* __restrict__ records, const float* __restrict__ values, float* __restrict__ out, int H, int dk, int dv,
              int delta) {
     extern __shared__ float sm[];
-    const int dkp = padded(dk), rec_n = record_floats(dkp, delta != 0);
-    uint32_t* Sh = reinterpret_cast<uint32_t*>(sm);      // [dkp][SROW] twice: the two parts of S
-    uint32_t* Sl = Sh + dkp * SROW;
-    uint32_t* Uh = Sl + dkp * SROW;                      // [CT][SROW] twice
-    uint32_t* Ul = Uh + CT * SROW;
-    float4* parts = reinterpret_cast<float4*>(Ul + CT * SROW);           // [16 warps][2 tiles][32 lanes]
-    float* ring = reinterpret_cast<float*>(parts + 16 * 64);             // STAGES records, each followed by the chunk's 32 x 16 values
+    const int dkp = padded(dk), rec_n = record_floats(dkp, delta != 0), kt = dkp >> 4;
+    uint4* Uh = reinterpret_cast<uint4*>(sm);            // [JOINERS][32 lanes] twice: U^T as row operands, its two parts
+    uint4* Ul = Uh + JOINERS * 32;
+    float4* parts_q = reinterpret_cast<float4*>(Ul + JOINERS * 32);      // [kt][JOINERS][32 lanes], and again for W
+    float4* parts_w = parts_q + kt * JOINERS * 32;
+    float* ring = reinterpret_cast<float*>(parts_w + (delta ? kt * JOINERS * 32 : 0));      // STAGES records, each followed by
+                                                         // the chunk's 32 x 16 values
     const int stage = rec_n + CT * NC;
     lp_grid_release();
     lp_grid_wait();
@@ -364,122 +354,143 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
     const int used = min(chunks, (t1 - begin + CT - 1) / CT);
     float* row = state + ((size_t)slots[b] * H + h) * dv * dk;
 
-    auto request = [&](int p) {                     // chunk p's record and values into stage p % STAGES
+    const bool joins = warp >= kt;
+    const int n = warp - kt;                        // of a joiner
+    auto request = [&](int p) {                     // joiners: chunk p's record and values into stage p % STAGES
         if (p < used) {
             const size_t slot = ((size_t)b * chunks + p) * H + h;
             const float* src = records + slot * rec_n;
             const float* val = values + slot * value_floats(dv) + blockIdx.x * (CT * NC);
             float* dst = ring + (p % STAGES) * stage;
-            for (int e = tid; e < rec_n / 4; e += CARRY_THREADS) cp16(dst + 4 * e, src + 4 * e);
-            for (int e = tid; e < CT * NC / 4; e += CARRY_THREADS) cp16(dst + rec_n + 4 * e, val + 4 * e);
+            for (int e = tid - 32 * kt; e < rec_n / 4; e += 32 * JOINERS) cp16(dst + 4 * e, src + 4 * e);
+            for (int e = tid - 32 * kt; e < CT * NC / 4; e += 32 * JOINERS) cp16(dst + rec_n + 4 * e, val + 4 * e);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     // a stage that the previous chunk has left takes the next record when a chunk begins; with fewer than three stages a
     // chunk's own stage does when it ends
     constexpr bool EARLY = STAGES >= 3;
+    if (joins) {
 #pragma unroll
-    for (int p = 0; p < (EARLY ? STAGES - 1 : STAGES); ++p) request(p);
+        for (int p = 0; p < (EARLY ? STAGES - 1 : STAGES); ++p) request(p);
+    }
     const int g8 = lane >> 2, t4 = lane & 3;
-    const int kt = dkp >> 4, ks = dkp >> 3;
-    const bool owns = warp < kt;
+    // s[w]: value columns g8 and g8 + 8 (entries 0, 1 and 2, 3) of two neighbouring channels
+    auto channel = [&](int w, int e) { return warp * 16 + w * 8 + t4 * 2 + (e & 1); };
+    auto column = [&](int e) { return j0 + g8 + (e >> 1) * 8; };
     float s[2][4];
 #pragma unroll
     for (int w = 0; w < 2; ++w)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = warp * 16 + g8 + (e >> 1) * 8, c = w * 8 + t4 * 2 + (e & 1);
-            s[w][e] = (owns && j0 + c < dv && r < dk) ? row[(size_t)(j0 + c) * dk + r] : 0.f;
-            if (owns) split_tf32(s[w][e], Sh[r * SROW + c], Sl[r * SROW + c]);
-        }
-    // this warp's share of the first products: rows 16 mt of W (role 0) or Q (role 1), steps s0 .. s1 over the key channels
-    const int nk = delta ? 4 : 8, per = (ks + nk - 1) / nk;
-    const int role = delta ? warp >> 3 : 1, mt = delta ? (warp >> 2) & 1 : warp >> 3;
-    const int s0 = (warp & (nk - 1)) * per, s1 = min(ks, s0 + per);
-    // the parts of 16 rows of a product, added in order: the same lane of every part
-    auto gather = [&](int first, int w) {
+        for (int e = 0; e < 4; ++e)
+            s[w][e] = (!joins && column(e) < dv && channel(w, e) < dk) ? row[(size_t)column(e) * dk + channel(w, e)] : 0.f;
+    // the shares of 8 tokens, added in order
+    auto gather = [&](const float4* parts) {
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4* at = parts + first * 64 + w * 32 + lane;
+        const float4* at = parts + n * 32 + lane;
 #pragma unroll 8
-        for (int k = 0; k < nk; ++k) {
-            const float4 v = at[k * 64];
+        for (int m = 0; m < kt; ++m) {
+            const float4 v = at[m * JOINERS * 32];
             sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
         }
         return sum;
     };
     for (int p = 0; p < used; ++p) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(EARLY ? STAGES - 2 : STAGES - 1) : "memory");
-        __syncthreads();                            // the record is there, S as the previous chunk left it, the chunk before done
-        if (EARLY) request(p + STAGES - 1);
+        if (joins) asm volatile("cp.async.wait_group %0;" ::"n"(EARLY ? STAGES - 2 : STAGES - 1) : "memory");
+        __syncthreads();                            // the record is there, the chunk before done
         const float* rec = ring + (p % STAGES) * stage;
         const float* rec_q = rec + (delta ? CT * dkp : 0);
         const float* rec_k = rec_q + CT * dkp;
         const float* rec_b = rec_k + CT * dkp;
         const float* rec_p = rec_b + CT * CT;
         const float* val = rec + rec_n;
-        if (!delta) split_tf32(val[tid], Uh[(tid >> 4) * SROW + (tid & 15)], Ul[(tid >> 4) * SROW + (tid & 15)]);
-        {
-            float acc[2][3][4] = {};
-            product(acc, (role == 1 ? rec_q : rec) + mt * ks * 128, Sh, Sl, s0, s1, lane);
-            parts[warp * 64 + lane] = chains(acc[0]);
-            parts[warp * 64 + 32 + lane] = chains(acc[1]);
-        }
-        __syncthreads();                            // S has been read
-        if (delta) {
-            if (warp < 4) {                         // warp (row half, tile): U = U0 - W S
-                const int half = warp >> 1, w = warp & 1;
-                const float4 sum = gather(half * 4, w);
-                const float x[4] = {sum.x, sum.y, sum.z, sum.w};
+        uint32_t sh[2][4], sl[2][4];
+        // a worker's share of (X S)^T for the matrix X of a record
+        auto share = [&](const float* x, float4* parts) {
+            const float4* at = reinterpret_cast<const float4*>(x) + warp * 32 + lane;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = half * 16 + g8 + (e >> 1) * 8, c = w * 8 + t4 * 2 + (e & 1);
-                    split_tf32(val[r * NC + c] - x[e], Uh[r * SROW + c], Ul[r * SROW + c]);
-                }
+            for (int i = 0; i < JOINERS; ++i) {
+                float acc[3][4] = {};
+                product(acc, sh, sl, at[i * kt * 32]);
+                parts[(warp * JOINERS + i) * 32 + lane] = chains(acc);
             }
-            __syncthreads();                        // U is there
-        }
-        if (owns) {
-            float up[2][3][4] = {};
-            product(up, rec_k + warp * (CT >> 3) * 128, Uh, Ul, 0, CT >> 3, lane);
-            const float p0 = rec_p[warp * 16 + g8], p1 = rec_p[warp * 16 + g8 + 8];
-#pragma unroll
-            for (int w = 0; w < 2; ++w)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = warp * 16 + g8 + (e >> 1) * 8, c = w * 8 + t4 * 2 + (e & 1);
-                    s[w][e] = fmaf(e < 2 ? p0 : p1, s[w][e], up[w][0][e] + (up[w][1][e] + up[w][2][e]));
-                    split_tf32(s[w][e], Sh[r * SROW + c], Sl[r * SROW + c]);
-                }
-        }
-        if (warp >= 14) {                           // the chunk's outputs: B U joins Q S
-            const int half = warp - 14;
-            float acc[2][3][4] = {};
-            product(acc, rec_b + half * (CT >> 3) * 128, Uh, Ul, 0, CT >> 3, lane);
-            const int t = begin + p * CT;
+        };
+        // a joiner's 8 tokens of U^T: the values less `sum`
+        auto join = [&](float4 sum) {
+            const float* at = val + (n * 8 + t4 * 2) * NC + g8;
+            uint4 hi, lo;
+            split_tf32(at[0] - sum.x, hi.x, lo.x);
+            split_tf32(at[NC] - sum.y, hi.z, lo.z);
+            split_tf32(at[8] - sum.z, hi.y, lo.y);
+            split_tf32(at[NC + 8] - sum.w, hi.w, lo.w);
+            Uh[n * 32 + lane] = hi;
+            Ul[n * 32 + lane] = lo;
+        };
+        if (!joins) {
 #pragma unroll
             for (int w = 0; w < 2; ++w) {
-                const float4 o = gather(delta ? 8 + half * 4 : half * 8, w), u = chains(acc[w]);
-                const float x[4] = {o.x + u.x, o.y + u.y, o.z + u.z, o.w + u.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = half * 16 + g8 + (e >> 1) * 8, c = j0 + w * 8 + t4 * 2 + (e & 1);
-                    if (t + r < t1 && c < dv) out[((size_t)(t + r) * H + h) * dv + c] = x[e];
-                }
+                split_tf32(s[w][0], sh[w][0], sl[w][0]);
+                split_tf32(s[w][2], sh[w][1], sl[w][1]);
+                split_tf32(s[w][1], sh[w][2], sl[w][2]);
+                split_tf32(s[w][3], sh[w][3], sl[w][3]);
             }
+            if (delta) share(rec, parts_w);
+        } else if (delta && EARLY) {
+            request(p + STAGES - 1);
+        }
+        if (delta) __syncthreads();                 // the shares of W S are there
+        if (!joins) {
+            share(rec_q, parts_q);
+        } else {
+            join(delta ? gather(parts_w) : make_float4(0.f, 0.f, 0.f, 0.f));
+            if (!delta && EARLY) request(p + STAGES - 1);
+        }
+        __syncthreads();                            // U and the shares of Q S are there
+        auto times_u = [&](float (*acc)[4], const float* frag, int q) {      // acc += U^T Y over the tokens 16 q .. 16 q + 15
+            uint32_t uh[2][4], ul[2][4];
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const uint4 hi = Uh[(2 * q + w) * 32 + lane], lo = Ul[(2 * q + w) * 32 + lane];
+                uh[w][0] = hi.x; uh[w][1] = hi.y; uh[w][2] = hi.z; uh[w][3] = hi.w;
+                ul[w][0] = lo.x; ul[w][1] = lo.y; ul[w][2] = lo.z; ul[w][3] = lo.w;
+            }
+            product(acc, uh, ul, reinterpret_cast<const float4*>(frag)[q * 32 + lane]);
+        };
+        if (!joins) {
+            float up[2][3][4] = {};
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int w = 0; w < 2; ++w) times_u(up[w], rec_k + (warp * 2 + w) * 2 * 128, q);
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const float2 decay = *reinterpret_cast<const float2*>(rec_p + channel(w, 0));
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    s[w][e] = fmaf(e & 1 ? decay.y : decay.x, s[w][e], up[w][0][e] + (up[w][1][e] + up[w][2][e]));
+            }
+        } else {                                    // the outputs of 8 tokens: B U joins Q S
+            float acc[3][4] = {};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) times_u(acc, rec_b + n * 2 * 128, q);
+            const float4 o = gather(parts_q), u = chains(acc);
+            const float x[4] = {o.x + u.x, o.y + u.y, o.z + u.z, o.w + u.w};
+            const int t = begin + p * CT + n * 8 + t4 * 2;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (t + (e & 1) < t1 && column(e) < dv) out[((size_t)(t + (e & 1)) * H + h) * dv + column(e)] = x[e];
         }
         if (!EARLY) {
             __syncthreads();                        // the stage is free
-            request(p + STAGES);
+            if (joins) request(p + STAGES);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
     for (int w = 0; w < 2; ++w)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = warp * 16 + g8 + (e >> 1) * 8, c = w * 8 + t4 * 2 + (e & 1);
-            if (owns && j0 + c < dv && r < dk) row[(size_t)(j0 + c) * dk + r] = s[w][e];
-        }
+        for (int e = 0; e < 4; ++e)
+            if (!joins && column(e) < dv && channel(w, e) < dk) row[(size_t)column(e) * dk + channel(w, e)] = s[w][e];
 }
 
 template <typename K> int reserve(K kernel, size_t bytes, size_t& granted) {
@@ -520,7 +531,8 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
     const int dkp = padded(dk), delta = beta ? 1 : 0;
     const size_t smem_p = ((size_t)(3 * CT + 3 * HB) * (dkp + 4) + 2 * CT * CT + CT) * sizeof(float);
     const size_t stage = (size_t)(record_floats(dkp, delta) + CT * NC) * sizeof(float);
-    const size_t kept = (size_t)(dkp + CT) * SROW * 2 * sizeof(float) + 16 * 64 * sizeof(float4);
+    const int kt = dkp / 16;
+    const size_t kept = (size_t)(2 + kt * (delta ? 2 : 1)) * JOINERS * 32 * sizeof(float4);
     const int stages = kept + 3 * stage <= MAX_SMEM ? 3 : kept + 2 * stage <= MAX_SMEM ? 2 : 1;
     const size_t smem_c = kept + stages * stage;
     auto prepare = dk <= 64 ? prepare_kernel<4> : dk <= 128 ? prepare_kernel<8> : prepare_kernel<16>;
@@ -537,7 +549,7 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
         lp_launch(prepare, dim3(here, H, B), THREADS, smem_p, stream, in, q_start, first, chunks, records, values);
         rc = lp_check_launch("chunked_recurrence (prepare)");
         if (rc) return rc;
-        lp_launch(carry, dim3((dv + NC - 1) / NC, H, B), CARRY_THREADS, smem_c, stream, state, slots, q_start, first, chunks,
+        lp_launch(carry, dim3((dv + NC - 1) / NC, H, B), 32 * (kt + JOINERS), smem_c, stream, state, slots, q_start, first, chunks,
                   (const float*)records, (const float*)values, out, H, dk, dv, delta);
         rc = lp_check_launch("chunked_recurrence (carry)");
         if (rc) return rc;
