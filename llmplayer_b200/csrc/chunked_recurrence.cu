@@ -22,8 +22,8 @@
 //   carry     one CTA per (16 value columns, head, sequence) walks the sequence's chunks in order; the state's columns stay in
 //             registers, 16 key channels per warp. The products run on the tensor cores (mma.sync m16n8k8) at float32
 //             precision: every operand is split into two TF32 parts, x = hi + lo with 22 bits of mantissa together, and
-//             hi hi + hi lo + lo hi are summed in float32. Records come by cp.async, up to two chunks ahead.
-#include "common.cuh"
+//             hi hi + hi lo + lo hi are summed in float32. Records come by bulk copies, up to two chunks ahead.
+#include "tcgen05_utils.cuh"
 
 namespace {
 
@@ -34,7 +34,7 @@ constexpr int THREADS = 256;            // of the first kernel
 constexpr int JOINERS = CT / 8;         // warps of the second kernel beside one per 16 key channels: one per 8 tokens
 constexpr int MAX_DK = 256;
 constexpr int CARRY_THREADS = 32 * (MAX_DK / 16 + JOINERS);      // at most
-constexpr size_t MAX_SMEM = 227 * 1024;
+constexpr size_t MAX_SMEM = 227 * 1024 - 64;      // beside the barriers
 
 constexpr int DECAY_CHANNEL = 0, DECAY_HEAD = 1, DECAY_FIXED = 2;
 
@@ -299,10 +299,6 @@ __device__ __forceinline__ void mma_tf32(float* c, const uint32_t* a, const uint
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-
 // acc += X Y over two steps of 8, X [16 x 16] split as row operands (xh, xl), Y [16 x 8] as one fragment of a record; three
 // chains of sums
 __device__ __forceinline__ void product(float (*acc)[4], const uint32_t (*xh)[4], const uint32_t (*xl)[4], float4 y) {
@@ -329,14 +325,18 @@ __device__ __forceinline__ float4 chains(const float (*acc)[4]) {
 // follows) while the workers multiply with Q, and adds (B U)^T to the shares of (Q S)^T and writes the outputs while they
 // update the state. Bound by the chain of a chunk's steps, with three barriers for the delta rule and two without it (U is V
 // then). With the state split in shared memory, read as column operands and stored again in every chunk, 2048 tokens of 8 heads
-// of 128 x 256 took 114 us on a B200, and take 97.
+// of 128 x 256 took 114 us on a B200, and 97 so; with bulk copies in place of 16 bytes per thread and request, which went through
+// the load unit that the fragments come through, 90 (three prompts of 518 to 777 tokens, 8 heads of 128 x 128, delta rule: 88 ->
+// 71). What is left are the shares' and the state's products, 8 cycles of a quarter SM for each of 432 (delta rule: 624) per
+// chunk, one behind the other.
 // STAGES: records in flight (three, or fewer where they do not fit shared memory; then a barrier frees the stage).
 template <int STAGES>
 __global__ void __launch_bounds__(CARRY_THREADS)
 carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ q_start, int first_chunk, int chunks,
              const float* __restrict__ records, const float* __restrict__ values, float* __restrict__ out, int H, int dk, int dv,
-             int delta) {
+             int delta, int* __restrict__ status) {
     extern __shared__ float sm[];
+    __shared__ uint64_t full[STAGES];                   // a stage's record is there
     const int dkp = padded(dk), rec_n = record_floats(dkp, delta != 0), kt = dkp >> 4;
     uint4* Uh = reinterpret_cast<uint4*>(sm);            // [JOINERS][32 lanes] twice: U^T as row operands, its two parts
     uint4* Ul = Uh + JOINERS * 32;
@@ -356,17 +356,21 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
 
     const bool joins = warp >= kt;
     const int n = warp - kt;                        // of a joiner
-    auto request = [&](int p) {                     // joiners: chunk p's record and values into stage p % STAGES
-        if (p < used) {
-            const size_t slot = ((size_t)b * chunks + p) * H + h;
-            const float* src = records + slot * rec_n;
-            const float* val = values + slot * value_floats(dv) + blockIdx.x * (CT * NC);
-            float* dst = ring + (p % STAGES) * stage;
-            for (int e = tid - 32 * kt; e < rec_n / 4; e += 32 * JOINERS) cp16(dst + 4 * e, src + 4 * e);
-            for (int e = tid - 32 * kt; e < CT * NC / 4; e += 32 * JOINERS) cp16(dst + rec_n + 4 * e, val + 4 * e);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    auto request = [&](int p) {                     // one thread: chunk p's record and values into stage p % STAGES
+        if (tid != 32 * kt || p >= used) return;
+        const size_t slot = ((size_t)b * chunks + p) * H + h;
+        float* dst = ring + (p % STAGES) * stage;
+        uint64_t* bar = &full[p % STAGES];
+        mbar_expect_tx(bar, stage * 4);
+        bulk_load(dst, records + slot * rec_n, rec_n * 4, bar);
+        bulk_load(dst + rec_n, values + slot * value_floats(dv) + blockIdx.x * (CT * NC), CT * NC * 4, bar);
     };
+    if (tid == 32 * kt) {
+#pragma unroll
+        for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
     // a stage that the previous chunk has left takes the next record when a chunk begins; with fewer than three stages a
     // chunk's own stage does when it ends
     constexpr bool EARLY = STAGES >= 3;
@@ -396,8 +400,14 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
         return sum;
     };
     for (int p = 0; p < used; ++p) {
-        if (joins) asm volatile("cp.async.wait_group %0;" ::"n"(EARLY ? STAGES - 2 : STAGES - 1) : "memory");
-        __syncthreads();                            // the record is there, the chunk before done
+        const bool there = mbar_wait(&full[p % STAGES], (p / STAGES) & 1);
+        if (!__syncthreads_and(there)) {            // the chunk before is done; a wait that ran out ends the block
+            if (tid == 32 * kt) {
+                atomicExch(status, 61);
+                for (int i = p + 1; i < min(used, p + (EARLY ? STAGES - 1 : STAGES)); ++i) mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
+            }
+            return;
+        }
         const float* rec = ring + (p % STAGES) * stage;
         const float* rec_q = rec + (delta ? CT * dkp : 0);
         const float* rec_k = rec_q + CT * dkp;
@@ -485,7 +495,6 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
             if (joins) request(p + STAGES);
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
     for (int w = 0; w < 2; ++w)
 #pragma unroll
@@ -514,7 +523,7 @@ extern "C" int lp_chunked_value_floats(int dv) { return value_floats(dv); }
 extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k_off, int v_off, const float* decay, int decay_form,
                                      const float* key_gain, const float* beta, const float* angles, int rd, int interleaved,
                                      float q_scale, float* state, const int* slots, const int* q_start, float* out, int B, int H,
-                                     int dk, int dv, int qk_heads, int max_new, int chunks, float* records, float* values,
+                                     int dk, int dv, int qk_heads, int max_new, int chunks, float* records, float* values, int* status,
                                      cudaStream_t stream) {
     if (B <= 0 || max_new <= 0) return 0;
     if (H <= 0 || H > 65535 || B > 65535 || dk <= 0 || dk > MAX_DK || dv <= 0) LP_REFUSE("chunked_recurrence: %d sequences, %d heads of %d x %d (at most %d key channels)", B, H, dk, dv, MAX_DK);
@@ -524,7 +533,7 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
         LP_REFUSE("chunked_recurrence: slices at %d, %d, %d do not fit rows of %d", q_off, k_off, v_off, ld);
     if (decay_form < DECAY_CHANNEL || decay_form > DECAY_FIXED) LP_REFUSE("chunked_recurrence: decay form %d", decay_form);
     if (rd < 0 || rd > dk || (rd & 1) || (rd > 0 && !angles)) LP_REFUSE("chunked_recurrence: a rotation over %d of %d channels", rd, dk);
-    if (chunks <= 0 || !records || !values) LP_REFUSE("chunked_recurrence: room for %d chunks", chunks);
+    if (chunks <= 0 || !records || !values || !status) LP_REFUSE("chunked_recurrence: room for %d chunks", chunks);
     if ((((uintptr_t)records | (uintptr_t)values) & 15) != 0) LP_REFUSE("chunked_recurrence: buffers must be aligned to 16 bytes");
     const Inputs in{proj, ld, q_off, k_off, v_off, decay, decay_form, key_gain, beta, (const float2*)angles, rd, interleaved, q_scale,
                     H, dk, dv, H / qk_heads};
@@ -550,7 +559,7 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
         rc = lp_check_launch("chunked_recurrence (prepare)");
         if (rc) return rc;
         lp_launch(carry, dim3((dv + NC - 1) / NC, H, B), 32 * (kt + JOINERS), smem_c, stream, state, slots, q_start, first, chunks,
-                  (const float*)records, (const float*)values, out, H, dk, dv, delta);
+                  (const float*)records, (const float*)values, out, H, dk, dv, delta, status);
         rc = lp_check_launch("chunked_recurrence (carry)");
         if (rc) return rc;
     }

@@ -106,7 +106,7 @@ _SIGNATURES = {
         "lp_chunked_record_floats": [_I, _I],
         "lp_chunked_value_floats": [_I],
         "lp_chunked_recurrence": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I,
-                                  _P, _P, _P],
+                                  _P, _P, _P, _P],
     },
     "recurrent_step": {
         "lp_retention_step": [_P, _I, _I, _I, _I, _I, _P, _I, _I, _P, _P, _F, _F, _P, _P, _P, _I, _I, _I, _I, _I, _P,
@@ -726,7 +726,7 @@ def check_kernel_status() -> None:
         raise KernelError(f"a tensor-core kernel gave up waiting on a barrier (code {code}: "
                           "1 = loader, 2 = MMA issuer, 3 = epilogue, 4-5 = operand maker; 2x the same in the "
                           "persistent product, 5x in the experts' (55: more choices than announced); "
-                          "6 = a page of the decode attention)")
+                          "6 = a page of the decode attention; 61 = a record of the chunked recurrence)")
 
 
 def _token_tile(tokens: int, gated: bool) -> int:
@@ -1512,7 +1512,7 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay: torc
             proj.data_ptr(), proj.shape[1], int(q_off), int(k_off), int(v_off), decay.data_ptr(), form, _ptr(key_gain),
             _ptr(delta_strength), _ptr(angles) if rd else None, rd, interleaved, float(q_scale), state.data_ptr(),
             slots.data_ptr(), q_start.data_ptr(), out.data_ptr(), B, H, dk, dv, int(qk_heads or H), int(max_new), room,
-            records.data_ptr(), values.data_ptr(), _stream()))
+            records.data_ptr(), values.data_ptr(), kernel_status().data_ptr(), _stream()))
         count_launches(2 * -(-total // room) - 1)
         return out
     chunks, chunk_state, chunk_decay = 1, None, None
