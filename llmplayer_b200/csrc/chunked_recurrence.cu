@@ -73,9 +73,27 @@ struct Inputs {
     int rd, interleaved;
     float q_scale;
     int H, dk, dv, qk_group;
+    int wide;                     // no rotation, and rows of queries, keys and decays that take reads of four channels
 };
 
 // ---------------------------------------------------------------- prepare
+// two float32 sums in one register pair
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float both(uint64_t a) { return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32)); }
+__device__ __forceinline__ float4 four(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+
+// Bound by its instructions and the latencies between its barriers (two blocks per SM, 41 % of the issue slots): rows read four
+// channels at a time, and the sums inside and between blocks as pairs of channels in one instruction, took 2048 tokens of 8
+// heads of 128 x 256 from 54 to 44 us on a B200 (three prompts of 518 to 777 tokens, 128 x 128, delta rule: 57 -> 47).
 // PER: key channels per lane of a sum over a head's channels (16 lanes): dk <= 16 PER.
 template <int PER>
 __global__ void __launch_bounds__(THREADS, PER <= 8 ? 2 : 1)
@@ -108,42 +126,83 @@ prepare_kernel(Inputs in, const int* __restrict__ q_start, int first_chunk, int 
     float* rec_b = rec_k + CT * dkp;
     float* rec_p = rec_b + CT * CT;
     const int hq = h / in.qk_group;
-    // four elements per thread and turn, so that their loads are in flight together
-    for (int e0 = tid; e0 < CT * dkp; e0 += 4 * THREADS) {
-        float q[4], k[4], g[4];
-        int at[4];
+    // four elements per thread and turn (four times four channels where the rows allow it), so that their loads are in flight
+    // together
+    if (in.wide) {
+        const int groups = dkp >> 2;
+        for (int e0 = tid; e0 < CT * groups; e0 += 4 * THREADS) {
+            float4 q[4], k[4], g[4];
+            int at[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int e = e0 + u * THREADS;
-            const int i = e / dkp, c = e - i * dkp;
-            at[u] = e < CT * dkp ? i * ks + c : -1;
-            q[u] = k[u] = 0.f;
-            g[u] = 1.f;
-            if (i < n && c < dk) {
-                const float* row = in.proj + (size_t)(t0 + i) * in.ld;
-                const float* qh = row + in.q_off + hq * dk;
-                const float* kh = row + in.k_off + hq * dk;
-                if (in.rd > 0) {
-                    const float2* cs = in.angles + (size_t)(t0 + i) * (in.rd >> 1);
-                    q[u] = rotated_channel(qh, c, in.rd, in.interleaved, cs);
-                    k[u] = rotated_channel(kh, c, in.rd, in.interleaved, cs);
-                } else {
-                    q[u] = __ldg(qh + c);
-                    k[u] = __ldg(kh + c);
+            for (int u = 0; u < 4; ++u) {
+                const int e = e0 + u * THREADS;
+                const int i = e / groups, c = (e - i * groups) * 4;
+                at[u] = e < CT * groups ? i * ks + c : -1;
+                q[u] = k[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                g[u] = make_float4(1.f, 1.f, 1.f, 1.f);
+                if (i < n && c < dk) {
+                    const size_t t = t0 + i;
+                    const float* row = in.proj + t * in.ld;
+                    q[u] = four(row + in.q_off + hq * dk + c);
+                    k[u] = four(row + in.k_off + hq * dk + c);
+                    if (in.decay_form == DECAY_CHANNEL) {
+                        g[u] = four(in.decay + (t * H + h) * dk + c);
+                    } else {
+                        const float one = __ldg(in.decay + (in.decay_form == DECAY_FIXED ? (size_t)h : t * H + h));
+                        g[u] = make_float4(one, one, one, one);
+                    }
+                    if (in.key_gain) {
+                        const float gain = __ldg(in.key_gain + t * H + h);
+                        k[u].x *= gain; k[u].y *= gain; k[u].z *= gain; k[u].w *= gain;
+                    }
                 }
-                g[u] = in.decay_form == DECAY_FIXED ? __ldg(in.decay + h)
-                       : in.decay_form == DECAY_HEAD ? __ldg(in.decay + (size_t)(t0 + i) * H + h)
-                                                     : __ldg(in.decay + ((size_t)(t0 + i) * H + h) * dk + c);
-                if (in.key_gain) k[u] *= __ldg(in.key_gain + (size_t)(t0 + i) * H + h);
             }
-        }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (at[u] >= 0) {
-                qs[at[u]] = q[u] * in.q_scale;
-                kk[at[u]] = k[u];
-                gs[at[u]] = g[u];
+            for (int u = 0; u < 4; ++u)
+                if (at[u] >= 0) {
+                    *reinterpret_cast<float4*>(qs + at[u]) =
+                        make_float4(q[u].x * in.q_scale, q[u].y * in.q_scale, q[u].z * in.q_scale, q[u].w * in.q_scale);
+                    *reinterpret_cast<float4*>(kk + at[u]) = k[u];
+                    *reinterpret_cast<float4*>(gs + at[u]) = g[u];
+                }
+        }
+    } else {
+        for (int e0 = tid; e0 < CT * dkp; e0 += 4 * THREADS) {
+            float q[4], k[4], g[4];
+            int at[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = e0 + u * THREADS;
+                const int i = e / dkp, c = e - i * dkp;
+                at[u] = e < CT * dkp ? i * ks + c : -1;
+                q[u] = k[u] = 0.f;
+                g[u] = 1.f;
+                if (i < n && c < dk) {
+                    const float* row = in.proj + (size_t)(t0 + i) * in.ld;
+                    const float* qh = row + in.q_off + hq * dk;
+                    const float* kh = row + in.k_off + hq * dk;
+                    if (in.rd > 0) {
+                        const float2* cs = in.angles + (size_t)(t0 + i) * (in.rd >> 1);
+                        q[u] = rotated_channel(qh, c, in.rd, in.interleaved, cs);
+                        k[u] = rotated_channel(kh, c, in.rd, in.interleaved, cs);
+                    } else {
+                        q[u] = __ldg(qh + c);
+                        k[u] = __ldg(kh + c);
+                    }
+                    g[u] = in.decay_form == DECAY_FIXED ? __ldg(in.decay + h)
+                           : in.decay_form == DECAY_HEAD ? __ldg(in.decay + (size_t)(t0 + i) * H + h)
+                                                         : __ldg(in.decay + ((size_t)(t0 + i) * H + h) * dk + c);
+                    if (in.key_gain) k[u] *= __ldg(in.key_gain + (size_t)(t0 + i) * H + h);
+                }
             }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (at[u] >= 0) {
+                    qs[at[u]] = q[u] * in.q_scale;
+                    kk[at[u]] = k[u];
+                    gs[at[u]] = g[u];
+                }
+        }
     }
     for (int i = tid; i < CT; i += THREADS) bs[i] = delta && i < n ? in.beta[(size_t)(t0 + i) * H + h] : 0.f;
     for (int e = tid; e < CT * CT; e += THREADS) L[e] = Bm[e] = 0.f;
@@ -191,28 +250,32 @@ prepare_kernel(Inputs in, const int* __restrict__ q_start, int first_chunk, int 
     {
         const int block = tid >> 7, jg = (tid >> 4) & 7, lane = tid & 15;
         const int base = block * HB, j0 = jg * 2;
-        float m0[PER], m1[PER];
+        constexpr int PAIRS = PER / 2;             // of neighbouring channels
+        auto pair = [&](const float* x, int row, int u) {
+            return *reinterpret_cast<const uint64_t*>(x + row * ks + 2 * lane + 32 * u);
+        };
+        uint64_t m0[PAIRS], m1[PAIRS];
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int c = lane + 16 * u;
-            m0[u] = c < dkp ? kk[(base + j0) * ks + c] : 0.f;
-            m1[u] = c < dkp ? kk[(base + j0 + 1) * ks + c] : 0.f;
+        for (int u = 0; u < PAIRS; ++u) {
+            const bool in_row = 2 * lane + 32 * u < dkp;
+            m0[u] = in_row ? pair(kk, base + j0, u) : 0;
+            m1[u] = in_row ? pair(kk, base + j0 + 1, u) : 0;
         }
         const int from = (jg & ~1) * 2;            // the two key groups of a warp walk the same rows (shuffles need both)
         for (int i = from; i < HB; ++i) {
-            float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+            uint64_t sa0 = 0, sa1 = 0, sb0 = 0, sb1 = 0;
             const bool on0 = i > j0, on1 = i > j0 + 1;
 #pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const int c = lane + 16 * u;
-                if (16 * u < dkp) {
-                    const float g = gs[(base + i) * ks + c], k = kk[(base + i) * ks + c], q = qs[(base + i) * ks + c];
-                    if (on0) m0[u] *= g;
-                    if (on1) m1[u] *= g;
-                    a0 = fmaf(k, m0[u], a0); b0 = fmaf(q, m0[u], b0);
-                    a1 = fmaf(k, m1[u], a1); b1 = fmaf(q, m1[u], b1);
+            for (int u = 0; u < PAIRS; ++u) {
+                if (2 * lane + 32 * u < dkp) {
+                    const uint64_t g = pair(gs, base + i, u), k = pair(kk, base + i, u), q = pair(qs, base + i, u);
+                    if (on0) m0[u] = mul2(m0[u], g);
+                    if (on1) m1[u] = mul2(m1[u], g);
+                    sa0 = fma2(k, m0[u], sa0); sb0 = fma2(q, m0[u], sb0);
+                    sa1 = fma2(k, m1[u], sa1); sb1 = fma2(q, m1[u], sb1);
                 }
             }
+            const float a0 = both(sa0), a1 = both(sa1), b0 = both(sb0), b1 = both(sb1);
             // lanes 0-7 keep (a0, b0), lanes 8-15 (a1, b1); then each half of those keeps one of the two
             const bool hi8 = lane & 8, hi4 = lane & 4;
             float x = hi8 ? a1 : a0, y = hi8 ? b1 : b0;
@@ -232,15 +295,16 @@ prepare_kernel(Inputs in, const int* __restrict__ q_start, int first_chunk, int 
     // between the blocks: thread (row of the second, key of the first)
     {
         const int i = tid >> 4, j = tid & 15;
-        float a = 0.f, bsum = 0.f;
-        const float4* kr = reinterpret_cast<const float4*>(kf + i * ks);
-        const float4* qr = reinterpret_cast<const float4*>(qf + i * ks);
-        const float4* er = reinterpret_cast<const float4*>(ke + j * ks);
+        uint64_t sa = 0, sb = 0;
+        const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(kf + i * ks);
+        const ulonglong2* qr = reinterpret_cast<const ulonglong2*>(qf + i * ks);
+        const ulonglong2* er = reinterpret_cast<const ulonglong2*>(ke + j * ks);
         for (int c = 0; c < dkp >> 2; ++c) {
-            const float4 k = kr[c], q = qr[c], e = er[c];
-            a = fmaf(k.x, e.x, fmaf(k.y, e.y, fmaf(k.z, e.z, fmaf(k.w, e.w, a))));
-            bsum = fmaf(q.x, e.x, fmaf(q.y, e.y, fmaf(q.z, e.z, fmaf(q.w, e.w, bsum))));
+            const ulonglong2 k = kr[c], q = qr[c], e = er[c];
+            sa = fma2(k.x, e.x, fma2(k.y, e.y, sa));
+            sb = fma2(q.x, e.x, fma2(q.y, e.y, sb));
         }
+        const float a = both(sa), bsum = both(sb);
         L[(HB + i) * CT + j] = bs[HB + i] * a;
         Bm[(HB + i) * CT + j] = bsum;
     }
@@ -536,7 +600,9 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
     if (chunks <= 0 || !records || !values || !status) LP_REFUSE("chunked_recurrence: room for %d chunks", chunks);
     if ((((uintptr_t)records | (uintptr_t)values) & 15) != 0) LP_REFUSE("chunked_recurrence: buffers must be aligned to 16 bytes");
     const Inputs in{proj, ld, q_off, k_off, v_off, decay, decay_form, key_gain, beta, (const float2*)angles, rd, interleaved, q_scale,
-                    H, dk, dv, H / qk_heads};
+                    H, dk, dv, H / qk_heads,
+                    rd == 0 && (dk & 3) == 0 && (ld & 3) == 0 && (q_off & 3) == 0 && (k_off & 3) == 0 && ((uintptr_t)proj & 15) == 0 &&
+                        (decay_form != DECAY_CHANNEL || ((uintptr_t)decay & 15) == 0)};
     const int dkp = padded(dk), delta = beta ? 1 : 0;
     const size_t smem_p = ((size_t)(3 * CT + 3 * HB) * (dkp + 4) + 2 * CT * CT + CT) * sizeof(float);
     const size_t stage = (size_t)(record_floats(dkp, delta) + CT * NC) * sizeof(float);

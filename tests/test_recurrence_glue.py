@@ -103,3 +103,31 @@ def test_chunked_recurrence(dk, dv, delta):
             assert float((out[t].double().reshape(H, dv) - o).abs().max()) < 2e-5 * float(o.abs().max() + 1), (i, t)
         assert rel(state[slot], S) < 1e-5
     assert torch.equal(state[2], start[2])
+
+
+@pytest.mark.parametrize("dk", [20, 64, 100, 128, 160])
+@pytest.mark.parametrize("form", ["channel", "head", "fixed"])
+def test_chunked_recurrence_reads(dk, form):
+    """Rows read four channels at a time and rows whose slices start at an odd column: the same arithmetic, bit for bit."""
+    from llmplayer_b200.kernels import ops
+    H, dv, lengths = 2, 24, [70, 33, 3]
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    T = sum(lengths)
+    wide = torch.randn(T, H * (2 * dk + dv), generator=g, device=DEV) * dk ** -0.5
+    odd = torch.cat([torch.full((T, 1), float("nan"), device=DEV), wide], dim=1).contiguous()
+    shape = {"channel": (T, H * dk), "head": (T, H), "fixed": (H,)}[form]
+    decay = 1.0 - 0.1 * torch.rand(*shape, generator=g, device=DEV)
+    gain, beta = torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
+    start = torch.randn(len(lengths), H, dv, dk, generator=g, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    at = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    scratch = lambda name, shape, dtype: torch.full(shape, float("nan"), dtype=dtype, device=DEV)  # noqa: E731
+    results = []
+    for proj, off in ((wide, 0), (odd, 1)):
+        state, out = start.clone(), torch.empty(T, H * dv, device=DEV)
+        ops.gla_scan(proj, off, off + H * dk, off + 2 * H * dk, decay, state, i32([2, 0, 1]), i32(at), out, num_heads=H, key_dim=dk,
+                     value_dim=dv, q_scale=0.5, max_new=max(lengths), scratch=scratch, delta_strength=beta, key_gain=gain,
+                     decay_per_head=form == "head", decay_fixed=form == "fixed", tensor_cores=True)
+        results.append((out, state))
+    assert torch.isfinite(results[0][0]).all()
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
