@@ -499,3 +499,32 @@ def test_tcgen05_prompt_attention_with_everything_that_shapes_it(hd, vd, H, G, s
     # the result's own rounding to bfloat16 is 2^-9 of a value; weights rounded to bfloat16 add as much again and more in short rows
     check_error("attention kernel (tcgen05, " + ("float32 weights)" if "exact_weights" in shape else "bfloat16 weights)"), f"{H}/{G} x {hd}",
                 worst / top, 4e-3 if "exact_weights" in shape else 2e-2)
+
+
+@pytest.mark.parametrize("vd", [128, 72])
+def test_a_rows_largest_weight_is_not_rounded_at_192(vd):
+    """Rows whose largest score stands in a later page, less than 2^8 above the first page's in weight: that weight is one and enters
+    the product exactly, so the only rounding left is the result's own. A value between 2^k and 2^(k + 1)
+    has 2^7 steps, so the error is uniform within 2^(k - 8); relative to mantissas spread evenly in the logarithm that is
+    2^-8 sqrt(3 / (8 ln 2) / 3) = 1.66e-3 in the root mean square, and sqrt(2) times as much if the weight were rounded as well. The
+    bound lies between the two."""
+    from llmplayer_b200.kernels import ops
+    dev, P, B, n, H, hd = "cuda:0", 64, 4, 256, 3, 192
+    pages = torch.zeros(B * (n // P), 2, 1, P, hd, device=dev, dtype=torch.bfloat16)
+    table = torch.arange(B * (n // P), device=dev, dtype=torch.int32).reshape(B, n // P)
+    at = 100                                              # the key that stands out, in the second page
+    pages[at // P::n // P, 0, :, at % P, 0] = 1.0
+    pages[at // P::n // P, 1, :, at % P, :vd] = 1.0
+    q = torch.zeros(B * n, H, hd, device=dev)
+    q[..., 0] = torch.linspace(1.0, 5.5, B * n * H, device=dev).reshape(B * n, H)       # in log2: 1.4 to 7.9
+    q = q.reshape(B * n, H * hd).to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)  # noqa: E731
+    out = torch.empty(B * n, H * hd, device=dev, dtype=torch.bfloat16)
+    ops.attention_prefill(q, out, pages, table, i32([n * i for i in range(B + 1)]), i32([n] * B), n, num_heads=H, num_kv_heads=1,
+                          head_dim=hd, scale=1.0, window=None, value_dim=vd)
+    ops.check_kernel_status()
+    e = torch.exp(q.reshape(B, n, H, hd)[..., 0].double())
+    ref = e / (e + torch.arange(n, device=dev)[None, :, None])                          # the other t keys have score zero
+    got = out.reshape(B, n, H, hd)[..., :vd].double()
+    error = ((got - ref[..., None]) / ref[..., None])[:, 128:]
+    check_error("attention kernel (tcgen05, a largest weight that is one)", f"{hd} x {vd}", float(error.square().mean().sqrt()), 1.95e-3)
