@@ -2,14 +2,18 @@
 //
 // The tokens of each expert are gathered into rows of their own (row tiles of 128, so that no tile holds two experts),
 // the gated product of a row tile with its expert's weights leaves the hidden activations, already multiplied by the
-// token's weight for that expert, and the down product adds each row's result to its token's row of the output. A
-// further expert may take every token with weight one (the shared expert); it is one more segment of rows.
+// token's weight for that expert, the down product stores each row's result, and a token's few results are added up in
+// the order of the experts and then to its row of the output: in one order, so that the same step gives the same bits.
+// A further expert may take every token with weight one (the shared expert); it is one more segment of rows, whose results
+// go to the output at once (one per element of it, before the others).
 // How many rows each expert has is known on the device only: the products walk a list of tiles that every CTA derives
 // from the counts, and the grids depend on the host's bounds alone, so a step with experts has no host decision.
 //
 //   expert_list_kernel    a block per expert: the tokens that chose it, in order, and their number
-//   expert_gather_kernel  rows of the input side by side, expert after expert; token and weight of every row
-//   expert_gemm_kernel    persistent tcgen05 product over the list of tiles, gated (up) or adding into tokens (down)
+//   expert_gather_kernel  rows of the input side by side, expert after expert; token and weight of every row, and the rows
+//                         of every token
+//   expert_gemm_kernel    persistent tcgen05 product over the list of tiles, gated (up) or storing float32 rows (down)
+//   expert_sum_kernel     a block per token: its rows into the output
 //
 // Before, every token passed through every expert: 2048 tokens, width 2048, 8 experts of 2048 and a shared one, 2 chosen,
 // B200: gated product 230 us, scaling of the hidden values about 25, down product 117; now list 6, gather 9, gated product
@@ -28,8 +32,10 @@ constexpr int MAX_EXPERTS = 256;
 
 // ---------------------------------------------------------------- which tokens chose which expert
 // weights [T, ldw]: a token's weight per expert, zero where it did not choose it. list[e * T ..]: the tokens of expert e.
+// place[e * T + t] becomes -1: no row yet.
 __global__ void __launch_bounds__(1024)
-expert_list_kernel(const float* __restrict__ weights, int ldw, int T, int* __restrict__ counts, int* __restrict__ list) {
+expert_list_kernel(const float* __restrict__ weights, int ldw, int T, int* __restrict__ counts, int* __restrict__ list,
+                   int* __restrict__ place) {
     __shared__ int warp_count[32];
     lp_grid_release();
     lp_grid_wait();
@@ -39,6 +45,7 @@ expert_list_kernel(const float* __restrict__ weights, int ldw, int T, int* __res
         const int t = t0 + threadIdx.x;
         const bool chosen = t < T && !(weights[(long long)t * ldw + e] == 0.f);     // a weight that is no number counts as chosen
         const unsigned votes = __ballot_sync(0xffffffffu, chosen);
+        if (t < T) place[(long long)e * T + t] = -1;
         __syncthreads();
         if (lane == 0) warp_count[warp] = __popc(votes);
         __syncthreads();
@@ -76,16 +83,15 @@ __device__ __forceinline__ int segment_starts(const int* counts, int E, int shar
     return end;
 }
 
-// x [T, d] -> rows [R, d] (16 bytes per thread and step), row_token (-1: padding) and row_weight. A block per four rows.
+// x [T, d] -> rows [R, d] (16 bytes per thread and step), row_token (-1: padding) and row_weight, and place [E, T]: the row
+// of every token and expert that belong together. A block per four rows.
 __global__ void __launch_bounds__(256)
 expert_gather_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ weights, int ldw, const int* __restrict__ counts,
                      const int* __restrict__ list, int T, int d, int E, int shared_rows, __nv_bfloat16* __restrict__ rows,
-                     int* __restrict__ row_token, float* __restrict__ row_weight, float* __restrict__ zero, long long zero_count,
-                     int* __restrict__ status) {
+                     int* __restrict__ row_token, float* __restrict__ row_weight, int* __restrict__ place, int* __restrict__ status) {
     __shared__ int start[MAX_EXPERTS + 2];
     lp_grid_release();
     lp_grid_wait();
-    clear_on_the_side(zero, zero_count);
     const int room = gridDim.x * 4;
     if (segment_starts(counts, E, shared_rows, room, start) > room && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(status, 55);
     const int r0 = blockIdx.x * 4;
@@ -104,6 +110,7 @@ expert_gather_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
         for (int i = 0; i < 4; ++i)
             if (threadIdx.x == i) mine = token[i];
         row_token[r0 + threadIdx.x] = mine;
+        if (mine >= 0 && e < E) place[(long long)e * T + mine] = r0 + threadIdx.x;
         row_weight[r0 + threadIdx.x] = mine < 0 ? 0.f : e < E ? weights[(long long)mine * ldw + e] : 1.f;
     }
     for (int c = threadIdx.x * 8; c < d; c += 256 * 8) {
@@ -129,21 +136,26 @@ struct Experts {
     int ff, shared_ff;           // hidden size of a routed expert and of the shared one, multiples of 128
     int d;                       // width of the stream
     int room;                    // rows that the buffers hold
+    int col0, cols;              // columns of the stream that the down product forms
 };
-
-__device__ __forceinline__ void add4(float* to, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+struct Stream {
+    float* at;                   // [T, ld]
+    int ld, overwrite;
+};
+__device__ __forceinline__ void add4(float4* to, const float4& v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // UP: hidden[row, f] = silu(gate) * up * weight of the row, bfloat16; W is the interleaved gate / up matrix of all experts.
-// Else: out[token of the row, f] += hidden[row] . W[f, columns of the row's expert], float32.
+// Else: out[row, f] = hidden[row] . W[col0 + f, columns of the row's expert], float32, f < cols; the shared expert's rows go to
+// stream[token of the row, col0 + f], added to it (the only addition to an element in this launch) or stored.
 // One CTA per SM walks the tiles (row tile first within an expert, so that the CTAs at work share weight tiles in L2) with
 // two accumulators in tensor memory: one tile's epilogue runs under the next one's MMAs. Rows are the MMA's M, so a thread
 // of the epilogue holds one row: its weight and its token are read once.
 template <bool UP>
 __global__ void __launch_bounds__(THREADS, 1)
 expert_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, void* __restrict__ out,
-                   int ldo, Experts ex, int* __restrict__ status) {
+                   int ldo, Experts ex, Stream stream, int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ int start[MAX_EXPERTS + 2];           // first row of a segment
     __shared__ int first_tile[MAX_EXPERTS + 2];      // first tile of a segment
@@ -176,7 +188,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         int at = 0;
         for (int e = 0; e <= ex.E; ++e) {
             first_tile[e] = at;
-            const int cols = UP ? (e < ex.E ? ex.ff : ex.shared_ff) / 128 : (ex.d + COLS - 1) / COLS;
+            const int cols = UP ? (e < ex.E ? ex.ff : ex.shared_ff) / 128 : (ex.cols + COLS - 1) / COLS;
             at += (start[e + 1] - start[e]) / ROWS * cols;
         }
         first_tile[ex.E + 1] = at;
@@ -203,7 +215,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 int f, row0;
                 tile_at(tile, e, f, row0);
                 const int k_blocks = k_blocks_of(e);
-                const int w_row = UP ? 2 * e * ex.ff + f * COLS : f * COLS, w_col = UP ? 0 : e * ex.ff;
+                const int w_row = UP ? 2 * e * ex.ff + f * COLS : ex.col0 + f * COLS, w_col = UP ? 0 : e * ex.ff;
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1)) { atomicExch(status, 51); *failed = 1; ok = false; break; }
@@ -299,17 +311,16 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     tmem_ld32(lane_addr + c0, g);
                     tmem_ld_wait();
                     const int f0 = f * COLS + c0;
-                    if (token >= 0 && f0 < ex.d) {
-                        float* to = (float*)out + (size_t)token * ldo + f0;
-                        if (f0 + 32 <= ex.d) {
+                    if (token >= 0) {
+                        float4* to = e < ex.E ? (float4*)((float*)out + (size_t)row * ldo + f0)
+                                              : (float4*)(stream.at + (size_t)token * stream.ld + ex.col0 + f0);
+                        const bool adds = e == ex.E && !stream.overwrite;
 #pragma unroll
-                            for (int q = 0; q < 8; ++q)
-                                add4(to + 4 * q, __uint_as_float(g[4 * q]), __uint_as_float(g[4 * q + 1]), __uint_as_float(g[4 * q + 2]),
-                                     __uint_as_float(g[4 * q + 3]));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (f0 + i < ex.d) atomicAdd(to + i, __uint_as_float(g[i]));
+                        for (int q = 0; q < 8; ++q) {
+                            if (f0 + 4 * q >= ex.cols) break;          // (widths are multiples of 8)
+                            const float4 v = make_float4(__uint_as_float(g[4 * q]), __uint_as_float(g[4 * q + 1]), __uint_as_float(g[4 * q + 2]),
+                                                         __uint_as_float(g[4 * q + 3]));
+                            if (adds) add4(to + q, v); else to[q] = v;
                         }
                     }
                 }
@@ -327,19 +338,55 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 }
 
+// out[t, col0 + c] (+)= the rows of token t, added in the order of the experts, c < cols. Bound by its bytes (the rows come from L2
+// where they fit) and by the two reads that wait for one another.
+template <bool OVERWRITE>
+__global__ void __launch_bounds__(256)
+expert_sum_kernel(const float* __restrict__ results, const int* __restrict__ place, int T, int E, float* __restrict__ out, int ldo, int col0,
+                  int cols) {
+    __shared__ int rows[MAX_EXPERTS];
+    __shared__ int held;
+    lp_grid_release();
+    lp_grid_wait();
+    const int t = blockIdx.x, lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        int n = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int row = e0 + lane < E ? place[(long long)(e0 + lane) * T + t] : -1;
+            const unsigned votes = __ballot_sync(0xffffffffu, row >= 0);
+            if (row >= 0) rows[n + __popc(votes & ((1u << lane) - 1u))] = row;
+            n += __popc(votes);
+        }
+        if (lane == 0) held = n;
+    }
+    __syncthreads();
+    const int n = held;
+    for (int c = threadIdx.x * 4; c < cols; c += 256 * 4) {
+        float4* to = (float4*)(out + (size_t)t * ldo + col0 + c);
+        const float4 old = OVERWRITE ? make_float4(0.f, 0.f, 0.f, 0.f) : *to;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) {
+            const float4 v = *(const float4*)(results + (size_t)rows[i] * cols + c);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        *to = OVERWRITE ? sum : make_float4(old.x + sum.x, old.y + sum.y, old.z + sum.z, old.w + sum.w);
+    }
+}
+
 int failed_launch(cudaError_t err, const char* what) {
     snprintf(lp_error_text, sizeof(lp_error_text), "experts (%s): %s", what, cudaGetErrorString(err));
     return (int)err;
 }
 
 template <bool UP>
-int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo, const Experts& ex, long long most_tiles, int* status,
-                cudaStream_t stream) {
+int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo, const Experts& ex, const Stream& to, long long most_tiles,
+                int* status, cudaStream_t stream) {
     auto kernel = expert_gemm_kernel<UP>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (err != cudaSuccess) return failed_launch(err, "shared memory");
     const int grid = most_tiles < lp_sm_count() ? (int)most_tiles : lp_sm_count();
-    err = lp_launch(kernel, dim3(grid), THREADS, SMEM_BYTES, stream, mw, mx, out, ldo, ex, status);
+    err = lp_launch(kernel, dim3(grid), THREADS, SMEM_BYTES, stream, mw, mx, out, ldo, ex, to, status);
     return err == cudaSuccess ? lp_check_launch("experts (product)") : failed_launch(err, "product");
 }
 
@@ -348,15 +395,17 @@ int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo
 // rows: the host's bound on the rows of all segments together, a multiple of 128 (checked against T * top + ...: every
 // segment is rounded up to 128). x: bfloat16 [T, d]. weights: float32 [T, ldw], its first E columns. w_up: bfloat16
 // [2 * (E * ff + shared_ff), d], gate and up rows interleaved in blocks of 64. w_down: bfloat16 [d, E * ff + shared_ff]. Scratch: counts
-// [E], list [E * T], gathered [rows, d], hidden [rows, max(ff, shared_ff)], row_token, row_weight [rows]. out: float32 [T, ldo], added to;
-// zero_count > 0: its first so many values (all of it) are cleared beforehand.
+// [E], list [E * T], place [E * T], gathered: 16-byte aligned, room for [rows, d] bfloat16 and, once those have been used, for
+// [rows, slice] float32: the down product forms `slice` columns at a time (a multiple of 256, or d). hidden [rows, max(ff, shared_ff)],
+// row_token, row_weight [rows]. out: float32 [T, ldo], added to, or (overwrite) stored. Launches 3 + 2 ceil(d / slice) kernels.
 extern "C" int lp_experts(const void* x, const float* weights, int ldw, const void* w_up, const void* w_down, float* out, int ldo, int T,
-                          int d, int E, int top, int ff, int shared_ff, int rows, int* counts, int* list, void* gathered, void* hidden,
-                          int* row_token, float* row_weight, long long zero_count, int* status, cudaStream_t stream) {
+                          int d, int E, int top, int ff, int shared_ff, int rows, int* counts, int* list, int* place, void* gathered,
+                          int slice, void* hidden, int* row_token, float* row_weight, int overwrite, int* status, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (E <= 0 || E > MAX_EXPERTS || top <= 0 || ldw < E) LP_REFUSE("experts: %d experts (at most %d), %d chosen, weights of %d", E, MAX_EXPERTS, top, ldw);
     if (ff <= 0 || ff % 128 || shared_ff < 0 || shared_ff % 128) LP_REFUSE("experts: hidden sizes %d and %d must be multiples of 128", ff, shared_ff);
     if (d <= 0 || d % 8 || ldo < d || ldo % 4) LP_REFUSE("experts: width %d (a multiple of 8), rows of %d", d, ldo);
+    if (slice <= 0 || (slice < d && slice % COLS)) LP_REFUSE("experts: slices of %d columns (a multiple of %d)", slice, COLS);
     if (((uintptr_t)x | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)gathered | (uintptr_t)hidden | (uintptr_t)out) & 15)
         LP_REFUSE("experts: operands must be 16-byte aligned");
     const long long tiles = (T + ROWS - 1) / ROWS;
@@ -372,14 +421,24 @@ extern "C" int lp_experts(const void* x, const float* weights, int ldw, const vo
     if (!rc) rc = make_map(&m_down, w_down, d, (long long)E * ff + shared_ff, (long long)E * ff + shared_ff, COLS);
     if (!rc) rc = make_map(&m_h, hidden, rows, ldh, ldh, ROWS);
     if (rc) return rc;
-    cudaError_t err = lp_launch(expert_list_kernel, dim3(E), dim3(1024), 0, stream, weights, ldw, T, counts, list);
+    cudaError_t err = lp_launch(expert_list_kernel, dim3(E), dim3(1024), 0, stream, weights, ldw, T, counts, list, place);
     if (err != cudaSuccess) return failed_launch(err, "list");
     err = lp_launch(expert_gather_kernel, dim3(rows / 4), dim3(256), 0, stream, (const __nv_bfloat16*)x, weights, ldw, (const int*)counts,
-                    (const int*)list, T, d, E, shared_rows, (__nv_bfloat16*)gathered, row_token, row_weight, zero_count > 0 ? out : nullptr,
-                    zero_count, status);
+                    (const int*)list, T, d, E, shared_rows, (__nv_bfloat16*)gathered, row_token, row_weight, place, status);
     if (err != cudaSuccess) return failed_launch(err, "gather");
-    const Experts ex = {counts, row_token, row_weight, E, shared_rows, ff, shared_ff, d, rows};
-    rc = launch_gemm<true>(m_up, m_x, hidden, ldh, ex, (long long)rows / ROWS * (ldh / 128), status, stream);
-    if (rc) return rc;
-    return launch_gemm<false>(m_down, m_h, out, ldo, ex, (long long)rows / ROWS * ((d + COLS - 1) / COLS), status, stream);
+    Experts ex = {counts, row_token, row_weight, E, shared_rows, ff, shared_ff, d, rows, 0, d};
+    const Stream to = {out, ldo, overwrite};
+    const bool stores = overwrite && shared_ff == 0;          // (the shared expert's rows have been stored by then)
+    rc = launch_gemm<true>(m_up, m_x, hidden, ldh, ex, to, (long long)rows / ROWS * (ldh / 128), status, stream);
+    for (int c = 0; c < d && !rc; c += slice) {
+        ex.col0 = c;
+        ex.cols = d - c < slice ? d - c : slice;
+        rc = launch_gemm<false>(m_down, m_h, gathered, ex.cols, ex, to, (long long)rows / ROWS * ((ex.cols + COLS - 1) / COLS), status, stream);
+        if (rc) break;
+        err = lp_launch(stores ? expert_sum_kernel<true> : expert_sum_kernel<false>, dim3(T), dim3(256), 0, stream, (const float*)gathered,
+                        (const int*)place, T, E, out, ldo, c, ex.cols);
+        if (err != cudaSuccess) return failed_launch(err, "sum");
+        rc = lp_check_launch("experts (sum)");
+    }
+    return rc;
 }

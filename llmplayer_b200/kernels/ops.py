@@ -118,7 +118,7 @@ _SIGNATURES = {
         "lp_stream_bundle": [_P, _I, _P, _P, _P, _F, _P, _P, _P, _F, _P, _I, _P, _I, _I, _I, _P, ctypes.c_longlong, _P],
     },
     "gemm_experts": {
-        "lp_experts": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, ctypes.c_longlong, _P, _P],
+        "lp_experts": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _P, _P],
     },
     "host_loop": {
         "lp_decode_loop": [_P, _P, _P, _I, _I, _I, _P, _I, _I, _P, _P, _P, _P, _P],
@@ -2148,6 +2148,7 @@ def expert_rows(tokens: int, num_experts: int, top: int, shared: bool) -> int:
 # width 1024, 8 of 512 + 1024, 2 chosen: 384 tokens 63 / 68 (6), 512: 86 / 70 (8), 2048: 97 / 72.
 EXPERTS_GROUPED_MIN_TOKENS = 128
 EXPERTS_GROUPED_MIN_SAVED = 8e9
+EXPERTS_RESULT_BYTES = 256 << 20     # float32 results of all rows that are held at a time
 
 
 def experts_grouped_pays(tokens: int, width: int, num_experts: int, top: int, expert_size: int) -> bool:
@@ -2163,7 +2164,8 @@ def experts(x: torch.Tensor, weights: torch.Tensor, w_up: torch.Tensor, w_down: 
     shared expert's (behind the others in ``w_up`` and ``w_down``, weight one), each expert run for its own tokens only.
     ``x``: bfloat16 [T, d]; ``weights``: float32 [T, >= E], zero where a token did not choose an expert, at most ``top``
     others per token; ``w_up``: the interleaved gate and up rows of all experts (:func:`interleave_gate_up`); ``w_down``:
-    bfloat16 [d, all hidden columns]; ``out``: float32 [T, d]. Hidden sizes are multiples of 128.
+    bfloat16 [d, all hidden columns]; ``out``: float32 [T, d]. Hidden sizes are multiples of 128. A token's results are added
+    in the order of the experts: the same inputs give the same bits.
     ``scratch(name, shape, dtype)`` gives the buffers."""
     _want(x, "experts x", torch.bfloat16, 2)
     _want(weights, "experts weights", torch.float32, 2)
@@ -2180,14 +2182,17 @@ def experts(x: torch.Tensor, weights: torch.Tensor, w_up: torch.Tensor, w_down: 
     counts = scratch("expert_lists", (E * (T + 1),), torch.int32)
     row_token = scratch("expert_row_tokens", (rows,), torch.int32)
     row_weight = scratch("expert_row_weights", (rows,), torch.float32)
-    gathered = scratch("expert_rows", (rows, d), torch.bfloat16)
+    place = scratch("expert_places", (T * E,), torch.int32)
+    # the gathered rows, then in their place the rows' results, as many columns at a time as EXPERTS_RESULT_BYTES hold
+    slice_cols = d if rows * d * 4 <= EXPERTS_RESULT_BYTES else min(d, max(256, EXPERTS_RESULT_BYTES // (rows * 4) // 256 * 256))
+    gathered = scratch("expert_rows", (max(rows * d, 2 * rows * slice_cols),), torch.bfloat16)
     hidden = scratch("expert_hidden", (rows, max(int(expert_size), int(shared_size))), torch.bfloat16)
     lib = library("gemm_experts")
     _check(lib, lib.lp_experts(x.data_ptr(), weights.data_ptr(), weights.shape[1], w_up.data_ptr(), w_down.data_ptr(), out.data_ptr(), d,
                                T, d, E, int(top), int(expert_size), int(shared_size), rows, counts.data_ptr(),
-                               counts.data_ptr() + 4 * E, gathered.data_ptr(), hidden.data_ptr(), row_token.data_ptr(),
-                               row_weight.data_ptr(), out.numel() if overwrite else 0, kernel_status().data_ptr(), _stream()))
-    count_launches(3)
+                               counts.data_ptr() + 4 * E, place.data_ptr(), gathered.data_ptr(), slice_cols, hidden.data_ptr(),
+                               row_token.data_ptr(), row_weight.data_ptr(), 1 if overwrite else 0, kernel_status().data_ptr(), _stream()))
+    count_launches(2 + 2 * -(-d // slice_cols))
     return out
 
 

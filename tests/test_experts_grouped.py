@@ -120,3 +120,29 @@ def test_mixture_of_many_tokens(scoring, shared, identity, overwrite):
         # the float64 run shows to stay within 2e-2 of the largest output; a token whose choice is closer than float32 may differ
         off = ((out.double() - ref).abs().max(-1).values > 2e-2 * float(ref.abs().max()))
         assert int(off.sum()) <= 1, int(off.sum())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,E,top,ff,shared,d", [(1025, 16, 4, 128, 128, 1032), (2048, 8, 3, 256, 0, 264)])
+@pytest.mark.parametrize("overwrite", [False, True])
+def test_the_same_inputs_give_the_same_bits(T, E, top, ff, shared, d, overwrite, monkeypatch):
+    """However the tiles finish, and in however many slices of columns the results are held."""
+    from llmplayer_b200.kernels import ops
+    dev = "cuda:0"
+    g = torch.Generator(device=dev).manual_seed(T)
+    x = torch.randn(T, d, generator=g, device=dev).to(torch.bfloat16)
+    total = E * ff + shared
+    gate, up = ((torch.randn(total, d, generator=g, device=dev) / d ** 0.5).to(torch.bfloat16) for _ in range(2))
+    w_up, w_down = ops.interleave_gate_up(gate, up), torch.randn(d, total, generator=g, device=dev).to(torch.bfloat16)
+    weights = torch.zeros(T, E, device=dev)
+    weights.scatter_(1, torch.rand(T, E, generator=g, device=dev).topk(top, dim=1).indices, 0.1 + torch.rand(T, top, generator=g, device=dev))
+    out0 = torch.randn(T, d, generator=g, device=dev)
+    scratch = lambda name, shape, dtype: torch.full(shape, -1, dtype=dtype, device=dev)  # noqa: E731
+    first = None
+    for room in (ops.EXPERTS_RESULT_BYTES,) * 6 + (1, 4 * ops.expert_rows(T, E, top, shared > 0) * 512):      # slices of 256, of 512
+        monkeypatch.setattr(ops, "EXPERTS_RESULT_BYTES", room)
+        out = out0.clone()
+        ops.experts(x, weights, w_up, w_down, out, scratch, num_experts=E, top=top, expert_size=ff, shared_size=shared, overwrite=overwrite)
+        first = out if first is None else first
+        assert torch.equal(out, first), room
+    ops.check_kernel_status()
