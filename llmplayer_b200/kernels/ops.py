@@ -771,22 +771,36 @@ PERSISTENT_MIN_TOKENS = 512
 
 def _persistent_pays(tokens: int, features: int, k: int, mode: int) -> bool:
     """Whether the persistent form (one CTA per SM walking 128 x 256 tiles, 128 x 128 x 2 when gated)
-    beats separate CTAs of 128 x 128 tiles, two to an SM. For the gated product: where it fills the SMs at least as well. The
-    others: always, but for long K loops over so few tiles that separate CTAs with K shared out use more of the chip (us on a B200,
-    persistent / separate: storing 1943 x 3664 x 2048 29 / 34, 2048 x 3072 x 2048 29 / 32, 1024 x 1024 x 2048 16 / 17, but
-    520 x 1024 x 4096 25 / 17, 1024 x 1024 x 4096 26 / 21, 1300 x 1024 x 4096 25 / 26; adding, where no output has to be cleared
-    first, 520 x 1024 x 2048 16 / 11, 1024 x 1024 x 2048 16 / 13, 1300 x 1024 x 2048 16 / 17, 520 x 1024 x 1024 12 / 12)."""
+    beats separate CTAs of 128 x 128 tiles, two to an SM. For the gated product: where it fills the SMs at least as well.
+    The others: with tiles for at most a quarter of the SMs, separate CTAs with K shared out use more of the chip (us on a B200,
+    persistent / separate into an output that the kernel in front has cleared, 2048 tokens: 8 features, K of 1024 10.4 / 7.6, of 2048
+    15 / 8, of 8192 44 / 11; 128 features of 2048 15 / 8; 512 of 2048 16 / 12, of 8192 45 / 30; 1024 tokens, 1024 features of 2048 16 / 12).
+    With more tiles K is not shared out any more, and adding gains from the persistent form at once (1024 x 2048 x 2048 16 / 18,
+    520 x 2048 x 2048 16 / 17); storing does where the K loop is long (520 x 3072 x 4096 26 / 29, 1024 x 2048 x 4096 26 / 28) or half of
+    the SMs have a tile (1024 x 3072 x 2048 17 / 18, 2048 x 3072 x 2048 28 / 31; below, 1024 x 2048 x 2048 16.1 / 15.8 and
+    1024 x 2048 x 1024 11.0 / 10.6)."""
     feat_tiles = -(-features // 128)
     persistent_tiles = feat_tiles * -(-tokens // (128 if mode == SWIGLU else 256))
     sms = num_sms()
     if mode != SWIGLU:
-        return persistent_tiles * 4 > sms or k < (4096 if mode == STORE else 2048)
+        return persistent_tiles * 4 > sms and (mode == ACCUMULATE or k >= 4096 or persistent_tiles * 2 > sms)
     separate_ctas = feat_tiles * -(-tokens // 128)
     fill_p = persistent_tiles / (-(-persistent_tiles // sms) * sms)
     fill_s = separate_ctas / (-(-separate_ctas // (2 * sms)) * 2 * sms)
     # at equal fill the persistent form wins when the SMs are well filled (its tiles are twice as large and one
     # tile's epilogue hides under the next one's MMAs) or the K loop is long
     return fill_p > fill_s + 0.02 or (fill_p >= fill_s and (fill_p >= 0.8 or k >= 4096))
+
+
+def gemm_persistent(tokens: int, features: int, k: int, mode: int) -> bool:
+    """Whether :func:`gemm`, left to choose, takes the persistent form for these sizes."""
+    return tokens >= PERSISTENT_MIN_TOKENS and _persistent_pays(tokens, features, k, mode)
+
+
+def gemm_adds_parts(tokens: int, features: int, k: int) -> bool:
+    """Whether :func:`gemm`, left to choose, stores into a float32 output of these sizes by adding partial sums, so that the output must
+    be zero beforehand."""
+    return not gemm_persistent(tokens, features, k, STORE) and gemm_plan(tokens, features, k, STORE)[1] > 1
 
 
 def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE, *, block_tok: int = 0,
@@ -819,8 +833,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE,
         raise KernelError("gemm: a following norm needs an output of whole rows")
     lib = library("gemm_tcgen05")
     status = kernel_status()
-    if (M >= PERSISTENT_MIN_TOKENS and not block_tok and not splits and norm_after is None
-            and _persistent_pays(M, N, K, mode)):
+    if not block_tok and not splits and norm_after is None and gemm_persistent(M, N, K, mode):
         # many tokens: one CTA per SM walks over the tiles, epilogue and MMAs of neighbouring tiles overlap
         if mode == ACCUMULATE and out.dtype != torch.float32:
             raise KernelError("gemm: accumulation needs a float32 output")

@@ -75,8 +75,7 @@ class Linear:
         ``out_name``: the workspace name of its output."""
         if not self._fast() or mode != ops.STORE:
             return None
-        _, splits = ops.gemm_plan(tokens, self.out_features, self.in_features, mode)
-        if splits <= 1:
+        if not ops.gemm_adds_parts(tokens, self.out_features, self.in_features):
             return None
         return ctx.buffer(out_name, (tokens, self.out_features), torch.float32)
 
@@ -85,7 +84,7 @@ class Linear:
         therefore be zero beforehand (a kernel in front may clear it on the side and say so with ``ctx.note_cleared()``)."""
         if not self._fast() or mode != ops.STORE:
             return False
-        return ops.gemm_plan(tokens, self.out_features, self.in_features, mode)[1] > 1
+        return ops.gemm_adds_parts(tokens, self.out_features, self.in_features)
 
     def can_few(self, tokens: int, mode: int) -> bool:
         """Whether :meth:`few` serves this product for ``tokens`` rows."""
