@@ -797,6 +797,12 @@ def gemm_persistent(tokens: int, features: int, k: int, mode: int) -> bool:
     return tokens >= PERSISTENT_MIN_TOKENS and _persistent_pays(tokens, features, k, mode)
 
 
+# Tokens per tile of a narrow product whose K is not shared out: more CTAs than with 128, and more stages in flight. 8 to 512 features,
+# 520 to 2048 tokens, B200, tiles of 64 / of 128 / K shared out over tiles of 128 (us): K of 1024 7.2-8.0 / 9.1-10.0 / 7.2-9.6, of
+# 2048 11.9-12.9 / 13.8-15.0 / 7.3-12.3, of 4096 21-22 / 23-25 / 7.4-17.7; tiles of 32 are as fast for few features, slower for many.
+ORDERED_TOKEN_TILE = 64
+
+
 def gemm_adds_parts(tokens: int, features: int, k: int) -> bool:
     """Whether :func:`gemm`, left to choose, stores into a float32 output of these sizes by adding partial sums, so that the output must
     be zero beforehand."""
@@ -2155,11 +2161,13 @@ def expert_rows(tokens: int, num_experts: int, top: int, shared: bool) -> int:
 
 
 # What running experts for their own tokens only must save against running all tokens through all experts, and the
-# tokens below which the weights' bytes bound both. Measured on a B200 (us, all through all / own tokens; saved GFLOP):
-# width 2048, 8 experts of 2048 + a shared one, 2 chosen: 128 tokens 83 / 76 (6), 192: 95 / 87 (16), 512: 178 / 92, 2048: 374 / 173;
-# width 2048, 32 of 1024, 4 chosen: 96 tokens 111 / 113 (8), 128: 115 / 114 (19), 192: 178 / 112 (42), 2048: 653 / 211;
-# width 1024, 8 of 512 + 1024, 2 chosen: 384 tokens 63 / 68 (6), 512: 86 / 70 (8), 2048: 97 / 72.
-EXPERTS_GROUPED_MIN_TOKENS = 128
+# tokens below which the weights' bytes bound both (a second tile of 128 tokens changes that at once). Whole layers, measured on a
+# B200 (us, all through all / own tokens; saved GFLOP):
+# width 2048, 8 experts of 2048 + a shared one, 2 chosen: 160 tokens 90 / 88 (11), 192: 90 / 88, 512: 137 / 92, 2048: 384 / 185;
+# width 2048, 32 of 1024 + 1024, 4 chosen: 128 tokens 108 / 114 (19), 129: 166 / 119, 192: 172 / 119, 2048: 686 / 238;
+# width 1024, 8 of 512 + 1024, 2 chosen: 256 tokens 40 / 44 (3), 384: 46 / 44 (6), 512: 47 / 45 (8), 2048: 89 / 70;
+# width 1024, 8 of 512, 1 chosen: 384 tokens 44 / 37 (7), 512: 37 / 38 (10), 768: 49 / 41.
+EXPERTS_GROUPED_MIN_TOKENS = 129
 EXPERTS_GROUPED_MIN_SAVED = 8e9
 EXPERTS_RESULT_BYTES = 256 << 20     # float32 results of all rows that are held at a time
 

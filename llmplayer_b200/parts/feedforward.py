@@ -378,7 +378,12 @@ class Mixture(Part):
         from ..kernels import ops
         if self.stacked_router:
             return self.up.sums_into(ctx, tokens, "ffn_up", ops.STORE)
-        return self.router.sums_into(ctx, tokens, "router_logits", ops.STORE)
+        return None if self._runs_grouped(tokens) else self.router.sums_into(ctx, tokens, "router_logits", ops.STORE)
+
+    def _runs_grouped(self, tokens: int) -> bool:
+        from ..kernels import ops
+        s, r = self.spec, self.spec.routing
+        return self.grouped and ops.experts_grouped_pays(tokens, s.hidden_size, r.num_experts, r.top, s.expert_size)
 
     def _forward_stacked(self, ctx, x, residual: torch.Tensor, overwrite: bool) -> bool:
         """Squared-ReLU experts chosen by their largest logits: sums and logits in one product, choice, weights and
@@ -415,7 +420,10 @@ class Mixture(Part):
         columns = self.router.out_features              # the experts' logits (and the shared expert's gate)
         logits = ctx.buffer("router_logits", (T, columns), torch.float32)
         with ops.section("ffn.router"):
-            self.router.store(x, logits, ctx)
+            # experts run for their own tokens add up in one order; so do the logits that choose them (2048 x 8 x 2048: 12 us, where
+            # partial sums in atomics take 8), and the layer gives the same bits for the same input
+            grouped = self._runs_grouped(T)
+            self.router.store(x, logits, ctx, ordered=grouped)
             weights = ctx.buffer("router_weights", (T, columns), torch.float32)
             if r.scoring in ("softmax_top", "sigmoid_top"):
                 ops.route_top(logits, self.router_bias, weights, num_experts=r.num_experts, top=r.top,
@@ -425,8 +433,7 @@ class Mixture(Part):
                                   scale=r.weight_scale)
             else:
                 ops.route(logits, weights, groups=r.groups, keep=r.keep_groups, top=r.top)
-        if (self.grouped and x.dtype == torch.bfloat16 and residual.dtype == torch.float32 and residual.is_contiguous()
-                and ops.experts_grouped_pays(T, s.hidden_size, r.num_experts, r.top, s.expert_size)):
+        if grouped and x.dtype == torch.bfloat16 and residual.dtype == torch.float32 and residual.is_contiguous():
             with ops.section("ffn.experts"):
                 ops.experts(x, weights, self.gate_up.weight, self.down.weight, residual, ctx.buffer, num_experts=r.num_experts,
                             top=r.top, expert_size=s.expert_size, shared_size=s.shared_size, overwrite=overwrite)

@@ -46,7 +46,14 @@ class Linear:
         """Whether this map's products run on the tensor-core kernels (bfloat16 weights, rows of a multiple of 8)."""
         return self._fast()
 
-    def store(self, x: torch.Tensor, out: torch.Tensor, ctx=None) -> torch.Tensor:
+    def store(self, x: torch.Tensor, out: torch.Tensor, ctx=None, ordered: bool = False) -> torch.Tensor:
+        """``ordered``: every element's sum is taken in one order, so that the same input gives the same bits (no partial sums that
+        meet in atomics)."""
+        if (ordered and self._fast() and x.dtype == torch.bfloat16
+                and ops.gemm_adds_parts(x.shape[0], self.out_features, self.in_features)):
+            if ctx is not None:
+                ctx.take_cleared()
+            return ops.gemm(x, self.weight, out, ops.STORE, block_tok=ops.ORDERED_TOKEN_TILE, splits=1)
         return self._run(x, out, ops.STORE, ctx)
 
     def accumulate(self, x: torch.Tensor, out: torch.Tensor, ctx=None, then_norm=None) -> bool:

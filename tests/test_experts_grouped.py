@@ -146,3 +146,26 @@ def test_the_same_inputs_give_the_same_bits(T, E, top, ff, shared, d, overwrite,
         first = out if first is None else first
         assert torch.equal(out, first), room
     ops.check_kernel_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,d", [(520, 1024), (1300, 2048)])
+def test_a_routed_layer_gives_the_same_bits(T, d):
+    from llmplayer_b200.engine.step import StepContext, Workspace
+    from llmplayer_b200.kernels import ops
+    from llmplayer_b200.parts import FEED_FORWARDS
+    from llmplayer_b200.parts.base import Runtime
+    from llmplayer_b200.parts.specs import ExpertRoutingSpec, MixtureSpec
+    part = FEED_FORWARDS.build(MixtureSpec(d, 512, ExpertRoutingSpec(8, 2, 4, 2, "router"), "", shared_size=128, shared_prefix="s."))
+    g = torch.Generator().manual_seed(T)
+    part.load({n: (torch.randn(*s.shape, generator=g) * s.shape[-1] ** -0.5).to(torch.bfloat16) for n, s in part.tensor_specs().items()},
+              Runtime(torch.device("cuda:0")))
+    x = torch.randn(T, d, generator=g).to(torch.bfloat16).cuda()
+    out0 = torch.randn(T, d, generator=g).cuda()
+    ctx = StepContext(Workspace("cuda:0"), [], [0] * T, [], [])
+    assert ops.experts_grouped_pays(T, d, 8, 2, 512) and part.buffer_to_clear(ctx, T) is None
+    outs = []
+    for _ in range(8):
+        outs.append(out0.clone())
+        part.forward(ctx, x, outs[-1])
+        assert torch.equal(outs[-1], outs[0])
