@@ -2154,7 +2154,8 @@ def expert_scale(hidden: torch.Tensor, weights: torch.Tensor, expert_size: int, 
 
 
 def expert_rows(tokens: int, num_experts: int, top: int, shared: bool) -> int:
-    """Rows that :func:`experts` needs at most: every expert's tokens rounded up to tiles of 128, and the shared expert's."""
+    """Rows that :func:`experts` works on at most: every routed expert's tokens rounded up to tiles of 128, and (``shared``) the
+    shared expert's."""
     tiles = -(-tokens // 128)
     routed = min((tokens * min(top, num_experts) + 127 * num_experts) // 128, num_experts * tiles)
     return 128 * (routed + (tiles if shared else 0))
@@ -2199,7 +2200,7 @@ def experts(x: torch.Tensor, weights: torch.Tensor, w_up: torch.Tensor, w_down: 
             or out.shape != (T, d)):
         raise KernelError(f"experts: x {tuple(x.shape)}, weights {tuple(weights.shape)}, w_up {tuple(w_up.shape)}, w_down "
                           f"{tuple(w_down.shape)}, out {tuple(out.shape)} for {E} experts of {expert_size} and {shared_size}")
-    rows = expert_rows(T, E, top, shared_size > 0)
+    rows = expert_rows(T, E, top, False)
     counts = scratch("expert_lists", (E * (T + 1),), torch.int32)
     row_token = scratch("expert_row_tokens", (rows,), torch.int32)
     row_weight = scratch("expert_row_weights", (rows,), torch.float32)
@@ -2207,7 +2208,7 @@ def experts(x: torch.Tensor, weights: torch.Tensor, w_up: torch.Tensor, w_down: 
     # the gathered rows, then in their place the rows' results, as many columns at a time as EXPERTS_RESULT_BYTES hold
     slice_cols = d if rows * d * 4 <= EXPERTS_RESULT_BYTES else min(d, max(256, EXPERTS_RESULT_BYTES // (rows * 4) // 256 * 256))
     gathered = scratch("expert_rows", (max(rows * d, 2 * rows * slice_cols),), torch.bfloat16)
-    hidden = scratch("expert_hidden", (rows, max(int(expert_size), int(shared_size))), torch.bfloat16)
+    hidden = scratch("expert_hidden", (rows * int(expert_size) + T * int(shared_size),), torch.bfloat16)
     lib = library("gemm_experts")
     _check(lib, lib.lp_experts(x.data_ptr(), weights.data_ptr(), weights.shape[1], w_up.data_ptr(), w_down.data_ptr(), out.data_ptr(), d,
                                T, d, E, int(top), int(expert_size), int(shared_size), rows, counts.data_ptr(),

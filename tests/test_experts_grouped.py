@@ -139,7 +139,7 @@ def test_the_same_inputs_give_the_same_bits(T, E, top, ff, shared, d, overwrite,
     out0 = torch.randn(T, d, generator=g, device=dev)
     scratch = lambda name, shape, dtype: torch.full(shape, -1, dtype=dtype, device=dev)  # noqa: E731
     first = None
-    for room in (ops.EXPERTS_RESULT_BYTES,) * 6 + (1, 4 * ops.expert_rows(T, E, top, shared > 0) * 512):      # slices of 256, of 512
+    for room in (ops.EXPERTS_RESULT_BYTES,) * 6 + (1, 4 * ops.expert_rows(T, E, top, False) * 512):      # slices of 256, of 512
         monkeypatch.setattr(ops, "EXPERTS_RESULT_BYTES", room)
         out = out0.clone()
         ops.experts(x, weights, w_up, w_down, out, scratch, num_experts=E, top=top, expert_size=ff, shared_size=shared, overwrite=overwrite)
@@ -169,3 +169,35 @@ def test_a_routed_layer_gives_the_same_bits(T, d):
         outs.append(out0.clone())
         part.forward(ctx, x, outs[-1])
         assert torch.equal(outs[-1], outs[0])
+
+
+@pytest.mark.parametrize("T,E,top,ff,shared,d", [(2048, 32, 4, 512, 8192, 2048), (4096, 64, 8, 256, 0, 7168), (600, 8, 2, 2048, 128, 1024)])
+def test_scratch_follows_each_experts_own_size(T, E, top, ff, shared, d, monkeypatch):
+    """Hidden values of a routed row at the routed size and of a token at the shared one, the gathered rows and their results in one
+    place, results never beyond their room."""
+    from llmplayer_b200.kernels import ops
+    launched = []
+
+    class Library:                                        # records the launch instead of making it
+        def __getattr__(self, name):
+            return lambda *args: launched.append(args) or 0
+
+    monkeypatch.setattr(ops, "library", lambda name: Library())
+    monkeypatch.setattr(ops, "kernel_status", lambda: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(ops, "_want", lambda *args, **kw: None)
+    taken = {}
+
+    def scratch(name, shape, dtype):
+        taken[name] = torch.empty(shape, dtype=dtype, device="meta").numel() * dtype.itemsize
+        return torch.empty(1, dtype=dtype)
+
+    empty = lambda *shape, dtype=torch.bfloat16: torch.empty(shape, dtype=dtype, device="meta")  # noqa: E731
+    total = E * ff + shared
+    ops.experts(empty(T, d), empty(T, E, dtype=torch.float32), empty(2 * total, d), empty(d, total), empty(T, d, dtype=torch.float32), scratch,
+                num_experts=E, top=top, expert_size=ff, shared_size=shared)
+    rows = ops.expert_rows(T, E, top, False)
+    assert len(launched) == 1
+    assert taken["expert_hidden"] == 2 * (rows * ff + T * shared)
+    assert taken["expert_rows"] == max(2 * rows * d, min(4 * rows * d, 4 * rows * max(256, (256 << 20) // (4 * rows) // 256 * 256)))
+    assert sum(n for name, n in taken.items() if name not in ("expert_hidden", "expert_rows")) <= 8 * rows + 8 * T * E + 4 * E
