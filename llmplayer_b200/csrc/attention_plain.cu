@@ -135,6 +135,11 @@ struct Scoring {
         return sc;
     }
 };
+// Whether a block takes no part in a row's sum: none of its keys is seen, or all that are have a weight of zero. Scores that are no
+// number leave no maximum either, but a sum that is none: they join, and the row's result is no number.
+__device__ __forceinline__ bool block_empty(float mb, float lb) { return mb == -INFINITY && lb == lb; }
+// What a block's exponentials are taken against: scores of minus infinity weigh nothing also where there are no others.
+__device__ __forceinline__ float block_base(float mb) { return mb == -INFINITY ? 0.f : mb; }
 // the factors by which what is held and a further block enter their sum
 __device__ __forceinline__ void join(float& m, float& l, float mb, float lb, float& held, float& fresh) {
     const float m_new = fmaxf(m, mb);
@@ -285,10 +290,11 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
                         top = fmaxf(top, s[r][j]);
                     }
                     mb[r] = lp_warp_max(top);
+                    const float base = block_base(mb[r]);
                     float sum = 0.f;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const float p = seen[j] ? expf(s[r][j] - mb[r]) : 0.f;
+                        const float p = seen[j] ? expf(s[r][j] - base) : 0.f;
                         mine[(lane + 32 * j) * RW + r] = p;
                         sum += p;
                     }
@@ -323,7 +329,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
                 }
 #pragma unroll
                 for (int r = 0; r < RW; ++r) {
-                    if (mb[r] == -INFINITY) continue;       // the row sees no key of this block
+                    if (block_empty(mb[r], lb[r])) continue;
                     float held, fresh;
                     join(m[r], l[r], mb[r], lb[r], held, fresh);
 #pragma unroll
@@ -417,7 +423,7 @@ attention_f32_share_kernel(const float* __restrict__ q, float* __restrict__ part
 #pragma unroll
         for (int r = 0; r < SHARE_HEADS; ++r) {
             const float top = fmaxf(fmaxf(warp_max[r][0], warp_max[r][1]), fmaxf(warp_max[r][2], warp_max[r][3]));
-            probs[tid][r] = seen && r < heads ? expf(s[r] - top) : 0.f;
+            probs[tid][r] = seen && r < heads ? expf(s[r] - block_base(top)) : 0.f;
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
@@ -471,7 +477,7 @@ attention_f32_join_kernel(const float* __restrict__ parts, float* __restrict__ o
         }
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
-            if (mb[i] == -INFINITY) continue;
+            if (block_empty(mb[i], lb[i])) continue;
             float held, fresh;
             join(m, l, mb[i], lb[i], held, fresh);
             acc = join_value(acc, held, vb[i], fresh);

@@ -528,3 +528,37 @@ def test_a_rows_largest_weight_is_not_rounded_at_192(vd):
     got = out.reshape(B, n, H, hd)[..., :vd].double()
     error = ((got - ref[..., None]) / ref[..., None])[:, 128:]
     check_error("attention kernel (tcgen05, a largest weight that is one)", f"{hd} x {vd}", float(error.square().mean().sqrt()), 1.95e-3)
+
+
+@pytest.mark.parametrize("form", ["no number", "minus infinity"])
+@pytest.mark.parametrize("H,G,hd", [(4, 2, 64), (3, 3, 20)])
+def test_float32_scores_that_are_no_number_reach_the_result(H, G, hd, form):
+    """A block of 128 keys all of whose scores are no number makes the rows that see it no number, also where it holds a single key;
+    scores of minus infinity weigh nothing. Tiles of queries, and blocks side by side."""
+    from llmplayer_b200.kernels import ops
+    dev, P, lengths = "cuda:0", 64, [300, 129, 257]
+    g = torch.Generator().manual_seed(hd)
+    pages = torch.randn(15, 2, G, P, hd, generator=g).abs()
+    table = torch.arange(15, dtype=torch.int32).reshape(3, 5)
+    T = sum(lengths)
+    q = torch.randn(T, H * hd, generator=g).abs()
+    seq = torch.tensor([i for i, n in enumerate(lengths) for _ in range(n)], dtype=torch.int32)
+    pos = torch.tensor([p for n in lengths for p in range(n)], dtype=torch.int32)
+    bad = [(0, range(0, 128)), (1, range(128, 129)), (2, range(128, 256))]            # (sequence, keys)
+    for i, keys in bad:
+        for key in keys:
+            pages[int(table[i, key // P]), 0, :, key % P] = float("nan") if form == "no number" else -float("inf")
+    kw = dict(num_heads=H, num_kv_heads=G, head_dim=hd, scale=hd ** -0.5, window=None)
+    d = lambda t: t.to(dev)  # noqa: E731
+    whole = torch.empty(T, H * hd, device=dev)
+    ops.attention_plain(d(q), whole, d(pages), d(table), d(seq), d(pos), **kw)
+    parts = torch.empty(T, H * hd, device=dev)
+    scratch = lambda name, shape, dtype: torch.full(shape, 3.0, dtype=dtype, device=dev)  # noqa: E731
+    ops.attention_plain(d(q), parts, d(pages), d(table), d(seq), d(pos), **kw, scratch=scratch, longest=max(lengths))
+    for out in (whole, parts):
+        none = torch.isnan(out).reshape(T, -1).cpu()
+        for t in range(T):
+            first, count = next((keys[0], len(keys)) for i, keys in bad if i == int(seq[t]))
+            # a row of nothing but minus infinities has no weights either
+            want = int(pos[t]) >= first if form == "no number" else first == 0 and int(pos[t]) < count
+            assert bool((none[t] == want).all()), (form, t, int(seq[t]), int(pos[t]))
