@@ -464,12 +464,12 @@ attention_f32_join_kernel(const float* __restrict__ parts, float* __restrict__ o
     float m = -INFINITY, l = 0.f, acc = 0.f;
     const float* from = parts + ((long long)t * H + h) * blocks * (hd + 2);
     constexpr int AHEAD = 8;                       // blocks asked for before the first of them is used
-    for (int b0 = 0; b0 * KB <= pos; b0 += AHEAD) {
+    for (int b0 = 0; b0 < blocks && b0 * KB <= pos; b0 += AHEAD) {
         float mb[AHEAD], lb[AHEAD], vb[AHEAD];
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
             const int c0 = (b0 + i) * KB;
-            const bool seen = c0 <= pos && block_seen(c0, lo, keep_end, pos);
+            const bool seen = b0 + i < blocks && c0 <= pos && block_seen(c0, lo, keep_end, pos);
             const float* p = from + (long long)(b0 + i) * (hd + 2);
             mb[i] = seen ? p[0] : -INFINITY;
             lb[i] = seen ? p[1] : 0.f;

@@ -946,9 +946,10 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, pag
     window): the sequence's first ``keep_first`` tokens stay visible to every later query. ``chunk`` > 0: a query at
     position p sees keys of its own chunk only, from p // chunk * chunk on. ``distance`` = (scale, rate), float32 [H] each:
     the score of a key n positions back loses scale[h] * ln(1 + rate[h] * n). ``gate``: float32 [T, H] (may be a column
-    slice): head h's output of token t is multiplied by sigmoid(gate[t, h]). ``scratch(name, shape, dtype)`` and ``longest``
-    (no position reaches it): a step of a few tokens per sequence may then look at the blocks of its keys side by side
-    (float32; the result is the same, bit for bit)."""
+    slice): head h's output of token t is multiplied by sigmoid(gate[t, h]). ``scratch(name, shape, dtype)``: a step of
+    a few tokens per sequence may then look at the blocks of its keys side by side (float32; the result is the same, bit for bit):
+    as many as the page table has positions for, which no step over that table outgrows, not even a replayed one, or fewer if no
+    position reaches ``longest``."""
     dist_scale, dist_rate = _distance_args(distance, num_heads, "attention")
     gate_ptr, gate_ld = _gate_args(gate, q.shape[0], num_heads, "attention")
     _check_sinks(sinks, num_heads, "attention")
@@ -966,8 +967,9 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, pag
         raise KernelError(f"attention: pages {tuple(pages.shape)} do not fit {G} key heads of {hd}")
     lib = library("attention_plain")
     parts, blocks = None, 0
-    if scratch is not None and longest > 0 and q.dtype == torch.float32 and pages.dtype == torch.float32:
-        blocks = -(-int(longest) // PLAIN_KEY_BLOCK)
+    if scratch is not None and q.dtype == torch.float32 and pages.dtype == torch.float32:
+        room = page_table.shape[1] * pages.shape[3]
+        blocks = -(-(min(room, int(longest)) if longest > 0 else room) // PLAIN_KEY_BLOCK)
         if T * H * blocks * (hd + 2) <= PLAIN_PARTS_MOST:
             parts = scratch("attention_parts", (T * H * blocks * (hd + 2),), torch.float32)
     _check(lib, lib.lp_attention_plain(
@@ -1207,7 +1209,7 @@ def attention(ctx, q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, page
     return attention_plain(q, out, pages, page_table, ctx.seq_ids, ctx.positions, num_heads=num_heads,
                            num_kv_heads=num_kv_heads, head_dim=head_dim, scale=scale, window=window, softcap=softcap,
                            sinks=sinks, keep_first=keep_first, chunk=chunk, distance=distance, gate=gate,
-                           scratch=ctx.buffer if ctx.max_new <= PLAIN_PARTS_TOKENS else None, longest=ctx.max_kv_len)
+                           scratch=ctx.buffer if ctx.max_new <= PLAIN_PARTS_TOKENS else None)
 
 
 # --------------------------------------------------------------------------- latent attention
