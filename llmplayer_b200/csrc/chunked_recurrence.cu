@@ -99,7 +99,7 @@ template <int PER>
 __global__ void __launch_bounds__(THREADS, PER <= 8 ? 2 : 1)
 prepare_kernel(Inputs in, const int* __restrict__ q_start, int first_chunk, int chunks, float* __restrict__ records,
                float* __restrict__ values) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     const int dk = in.dk, dv = in.dv, H = in.H, dkp = padded(dk), ks = dkp + 4;      // rows padded against bank conflicts
     float* qs = sm;                        // [CT][ks]
     float* kk = qs + CT * ks;              // [CT][ks]
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(CARRY_THREADS)
 carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ q_start, int first_chunk, int chunks,
              const float* __restrict__ records, const float* __restrict__ values, float* __restrict__ out, int H, int dk, int dv,
              int delta, int* __restrict__ status) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     __shared__ uint64_t full[STAGES];                   // a stage's record is there
     const int dkp = padded(dk), rec_n = record_floats(dkp, delta != 0), kt = dkp >> 4;
     uint4* Uh = reinterpret_cast<uint4*>(sm);            // [JOINERS][32 lanes] twice: U^T as row operands, its two parts

@@ -1251,7 +1251,7 @@ pair_norm_add_kernel(const float* __restrict__ a, const float* __restrict__ wa, 
                      const float* __restrict__ b, const float* __restrict__ wb, float sb, float eps_b, float* __restrict__ x,
                      const float* __restrict__ w2, float eps2, int parts, int cuts, TOut* __restrict__ out2, int d,
                      float* __restrict__ zero, long long zero_count) {
-    extern __shared__ float sum_row[];
+    extern __shared__ __align__(16) float sum_row[];
     __shared__ float scratch[32];
     __shared__ float slice[PAIR_NORM_MAX_SLICES];
     lp_grid_release();

@@ -385,7 +385,7 @@ latent_attend_kernel(const float* __restrict__ qa, const TKV* __restrict__ pages
                      int pt_stride, const int* __restrict__ q_start, const int* __restrict__ kv_len,
                      float* __restrict__ part, int H, int rank, int dr, int page_size, float scale, int shares,
                      int window) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     constexpr int ROWS = WARPS * RW;
     // rows of a multiple of 4 values are read four at a time (a key row's stride of Dk + 4 floats keeps the lanes'
     // 16-byte reads on distinct banks); other widths one value at a time with a stride of Dk + 1

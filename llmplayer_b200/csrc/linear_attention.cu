@@ -113,7 +113,7 @@ gla_scan_kernel(const float* __restrict__ proj, int ld, int q_off, int k_off, in
                 float* __restrict__ chunk_state, float* __restrict__ chunk_decay, int decay_form,
                 const float* __restrict__ key_gain, int ones, const float* __restrict__ bonus, int qk_group,
                 const float* __restrict__ beta, int state_cols, const float2* __restrict__ angles, int rd, int interleaved) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     float* qs = sm;                         // [TB][dk]
     float* ks = qs + TB * dk;
     float* as = ks + TB * dk;

@@ -18,7 +18,7 @@ namespace {
 __global__ void __launch_bounds__(128)
 route_kernel(const float* __restrict__ z, int ldz, float* __restrict__ weights, int ldw, int T, int E, int groups,
              int keep, int top) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     lp_grid_release();
     lp_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -177,7 +177,7 @@ __device__ __forceinline__ void choose_top(const float* __restrict__ z, const fl
 __global__ void __launch_bounds__(128)
 route_top_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ bias, float* __restrict__ weights, int ldw,
                  int T, int E, int top, int extra, int form) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     lp_grid_release();
     lp_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -205,7 +205,7 @@ template <typename TH, int VEC>
 __global__ void __launch_bounds__(256)
 expert_relu2_kernel(const float* __restrict__ z, int ldz, TH* __restrict__ hidden, const float* __restrict__ weights, int ldw,
                     int T, int E, int ff, int on_input, int top, int form, float* __restrict__ zero, long long zero_count) {
-    extern __shared__ float sm[];            // scores [E], weights [E]
+    extern __shared__ __align__(16) float sm[];            // scores [E], weights [E]
     lp_grid_release();
     lp_grid_wait();
     clear_on_the_side(zero, zero_count);
@@ -325,7 +325,7 @@ expert_act_vec4_kernel(const float* __restrict__ z, int ldz, int total, __nv_bfl
 __global__ void __launch_bounds__(128)
 route_softmax_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ correction, float* __restrict__ weights,
                      int ldw, int T, int E, int groups, int keep, int top, float scale) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     lp_grid_release();
     lp_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
