@@ -384,7 +384,7 @@ def test_fused_decode_over_more_than_32_pages_in_one_share(H, G, hd):
 
 
 @pytest.mark.parametrize("H,G,hd", [(4, 2, 64), (9, 1, 48), (3, 3, 128), (2, 1, 256), (2, 2, 20)])
-@pytest.mark.parametrize("form", ["all", "window", "kept", "chunk"])
+@pytest.mark.parametrize("form", ["all", "window", "kept", "chunk", "distance", "gate"])
 def test_float32_attention_in_blocks(form, H, G, hd):
     """Tiles of queries over blocks of keys, and blocks of keys side by side: against float64, and the same bits from both
     however the sequences are cut into calls. Lengths at the edges of blocks (128), tiles (32, 64) and pages."""
@@ -405,6 +405,8 @@ def test_float32_attention_in_blocks(form, H, G, hd):
     kw = dict(num_heads=H, num_kv_heads=G, head_dim=hd, scale=hd ** -0.5, window=window, keep_first=keep, chunk=chunk,
               softcap=20.0 if form == "kept" else None)
     sinks = torch.randn(H, generator=g) if form != "all" else None
+    distance = (torch.rand(H, generator=g), 0.05 * torch.rand(H, generator=g)) if form in ("distance", "gate") else None
+    gate = torch.randn(T, H + 3, generator=g) if form == "gate" else None
     ref = torch.empty(T, H, hd, dtype=torch.float64)
     for t in range(T):
         p, i = int(pos[t]), int(seq[t])
@@ -414,16 +416,19 @@ def test_float32_attention_in_blocks(form, H, G, hd):
             s = kv[:, 0] @ q[t].reshape(H, hd)[h].double() * hd ** -0.5
             if kw["softcap"]:
                 s = 20.0 * torch.tanh(s / 20.0)
+            if distance is not None:
+                s = s - distance[0][h].double() * torch.log1p(distance[1][h].double() * torch.arange(p, -1, -1, dtype=torch.float64))
             w = torch.softmax(s if sinks is None else torch.cat([s, sinks[h:h + 1].double()]), 0)[:len(keys)]
-            ref[t, h] = w @ kv[:, 1]
+            ref[t, h] = w @ kv[:, 1] * (1.0 if gate is None else torch.sigmoid(gate[t, 2 + h].double()))
     if window is not None:          # pages that no query of the last call below reaches are gone
         gone = table.clone()
         gone[0, 1 if keep else 0:2] = -1
     d = lambda t: t.to(dev)  # noqa: E731
     whole = torch.empty(T, H * hd, device=dev)
     scratch = lambda name, shape, dtype: torch.full(shape, float("nan"), dtype=dtype, device=dev)  # noqa: E731
-    sk = {"sinks": None if sinks is None else d(sinks)}
-    ops.attention_plain(d(q), whole, d(pages), d(table), d(seq), d(pos), **kw, **sk)
+    sk = {"sinks": None if sinks is None else d(sinks), "distance": None if distance is None else tuple(map(d, distance))}
+    gated = lambda rows: None if gate is None else d(gate[rows])[:, 2:2 + H]  # noqa: E731
+    ops.attention_plain(d(q), whole, d(pages), d(table), d(seq), d(pos), **kw, **sk, gate=gated(slice(None)))
     # scores carry hd products, exponentials and sums of up to 300 weights: a few hundred units of 2^-24 times scores of up to 20
     assert float((whole.double().cpu().reshape(T, H, hd) - ref).abs().max()) < 2e-5 * float(ref.abs().max())
     for rows in ([299, 300, 428, 429, 493], [0, 63, 64, 127, 128], list(range(250, 300))):
@@ -432,7 +437,7 @@ def test_float32_attention_in_blocks(form, H, G, hd):
         for use in (None, scratch):
             out = torch.empty(len(rows), H * hd, device=dev)
             ops.attention_plain(d(q[at]), out, d(pages), d(gone if late else table), d(seq[at]), d(pos[at]), **kw, **sk, scratch=use,
-                                longest=int(pos[at].max()) + 1)
+                                gate=gated(at), longest=int(pos[at].max()) + 1)
             assert torch.equal(out, whole[at.to(dev)]), (rows, use is None)
 
 

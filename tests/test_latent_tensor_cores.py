@@ -138,3 +138,45 @@ def test_prompt_layouts_four_and_eight_at_a_time(dn, dr, rot, rank, dv, interlea
     ops.latent_gate_heads(heads, gate, out, num_heads=H, head_dim=hd, value_dim=dv)
     ref = heads.reshape(T, H, hd)[..., :dv].double() * torch.sigmoid(gate.double())[..., None]
     assert rel(out.reshape(T, H, dv), ref) < 5e-3
+
+
+@pytest.mark.parametrize("lengths", [[400, 200], [70, 1, 64], [1, 1]])
+@pytest.mark.parametrize("H", [3, 16])
+def test_prepared_rows_and_queries(lengths, H):
+    """What is written to the cache and as queries against float64, in steps where the heads have CTAs of their own and in steps where
+    a CTA takes a whole token: normed latents and the rotated shared part at every token's page and place, nothing anywhere else."""
+    from llmplayer_b200.kernels import ops
+    dn, dr, rank, P = 64, 32, 256, 64
+    g = torch.Generator(device=DEV).manual_seed(len(lengths) + H)
+    T = sum(lengths)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    positions = [5 + p for n in lengths for p in range(n)]
+    seq = [i for i, n in enumerate(lengths) for _ in range(n)]
+    width = -(-(max(lengths) + 5) // P)
+    table = torch.randperm(len(lengths) * width + 1, generator=torch.Generator().manual_seed(2))[1:].reshape(len(lengths), width)
+    proj = torch.randn(T, H * (dn + dr) + rank + dr, generator=g, device=DEV)
+    freq, gain = torch.rand(dr // 2, generator=g, device=DEV), torch.randn(rank, generator=g, device=DEV)
+    pages = torch.full((len(lengths) * width + 1, P, rank + dr), 7.0, device=DEV, dtype=torch.bfloat16)
+    q = torch.zeros(T, H, dn + dr, device=DEV)
+    ops.latent_prepare(proj, 0, H * (dn + dr), gain, 1e-5, ops.Rotation(freq, dr, False), i32(positions), i32(seq), table.to(torch.int32).to(DEV),
+                       q, pages, num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank)
+    angle = (torch.tensor(positions, device=DEV, dtype=torch.float32)[:, None] * freq).double()        # as float32 forms them
+
+    def rotated(x):
+        a, b = x[..., :dr // 2].double(), x[..., dr // 2:].double()
+        shape = (T,) + (1,) * (x.dim() - 2) + (dr // 2,)
+        c, s = torch.cos(angle).reshape(shape), torch.sin(angle).reshape(shape)
+        return torch.cat([a * c - b * s, b * c + a * s], -1)
+
+    heads, kv = proj[:, :H * (dn + dr)].reshape(T, H, dn + dr), proj[:, H * (dn + dr):].double()
+    assert torch.equal(q[..., :dn], heads[..., :dn]) and rel(q[..., dn:], rotated(heads[..., dn:])) < 1e-6
+    latent = kv[:, :rank] / torch.sqrt((kv[:, :rank] ** 2).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    want = torch.cat([latent, rotated(proj[:, H * (dn + dr) + rank:])], -1)
+    page = table[torch.tensor(seq), torch.tensor(positions) // P].to(DEV)
+    place = torch.tensor(positions, device=DEV) % P
+    got = pages[page, place].double()
+    # one rounding to bfloat16 of a float32 value: 2^-8 of its power of two at most, and a bit for the value itself
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all())
+    touched = torch.zeros(pages.shape[:2], dtype=torch.bool, device=DEV)
+    touched[page, place] = True
+    assert bool((pages[~touched] == 7.0).all())
