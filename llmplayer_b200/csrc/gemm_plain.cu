@@ -133,7 +133,8 @@ constexpr int ROW_FEATURES = 8;          // output features of a CTA (in the gat
 constexpr int ROW_CHUNK = 32;            // products of a chain per stage
 constexpr int ROW_STRIDE = ROW_CHUNK + 4;   // 144 bytes from one chain's chunk to the next: eight lanes' 16-byte reads hit all banks
 
-// DEEP: a ring of up to eight stages, two CTAs per SM (for grids that have no more); else four stages and more CTAs
+// DEEP: a ring of up to eight stages, two CTAs per SM (for grids that have no more); else four stages, of which two (16 rows) to five (one
+// row) CTAs fit an SM, in the gated form two, and one at 16 rows (147 KB)
 template <int MR, int MODE, bool DEEP> struct RowsShape {
     static constexpr int WROWS = MODE == LP_GEMM_SWIGLU ? 2 * ROW_FEATURES : ROW_FEATURES;
     static constexpr int THREADS = WROWS * PARTS;

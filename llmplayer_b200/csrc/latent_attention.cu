@@ -548,7 +548,7 @@ __host__ __device__ constexpr size_t tc_smem(int Dk) {
 // their way while a block is worked on. Scores: a warp takes 32 keys and a quarter of the row's width, the quarters meet in
 // shared memory; softmax: two rows per warp; sums: a warp takes an eighth of the latent's columns (NT tiles of 8). Row strides of
 // an odd multiple of 16 bytes keep ldmatrix free of bank conflicts.
-// Bound by the tensor instructions (3 x 36 + 3 x 32 per 16 keys and CTA at rank 512) and the latency of a block's steps:
+// Bound by the tensor instructions (3 x 72 + 3 x 64 per 16 keys and CTA at rank 512, rows of 576) and the latency of a block's steps:
 // 32 sequences of 750 to 1500 rows of 576, 16 heads, B200: 210 us with a lane per key (above) -> 39 (cold
 // caches); with three chains of products one behind the other and a division per 16 bytes copied it was 41.
 template <int NT>

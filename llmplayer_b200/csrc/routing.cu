@@ -8,7 +8,8 @@
 //
 // The experts themselves are run as one stacked gated product over all experts (every token through every expert)
 // whose hidden activations are multiplied by the token's weight for that expert (zero for experts it did not choose)
-// before one stacked down product sums them; `lp_expert_scale` is that multiplication.
+// before one stacked down product sums them; `lp_expert_scale` is that multiplication. Many tokens run each expert for the
+// tokens that chose it instead (gemm_experts.cu).
 // Among equal scores the expert (group) with the lower index wins. Everything is float32.
 #include "common.cuh"
 
