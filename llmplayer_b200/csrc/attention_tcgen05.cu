@@ -26,7 +26,7 @@
 // tiles and two products per page; the sums use the float32 weights. It comes with everything else that may shape a score or an
 // output (a cap, sinks, kept first tokens, chunks, a gate per head) except a distance bias, which stays with the mma.sync kernel.
 // B200, one prompt of 2048 tokens, 16 heads of 128 on 4, capped scores and sinks: 174 us with mma.sync -> 89; 16 heads of
-// 192 with values of 128, sequences of 1100 and 825 tokens: 95 -> 39 (which also leaves out the values' 64 columns of zeros).
+// 192 with values of 128, sequences of 1100 and 825 tokens: 95 -> 41 (which also leaves out the values' 64 columns of zeros).
 //
 // Reference counterpart: src/main/resources/kernels/cuda/attention.cu:10-108 (one query at a
 // time, SIMT); the online-softmax recurrence is that of inference/Attention.java:161-207.
