@@ -762,11 +762,20 @@ def gemm_plan(tokens: int, features: int, k: int, mode: int):
     sms = num_sms()
     if ctas >= sms // 2 or k_blocks < 8:
         return tile, 1
+    if mode == STORE and tokens >= PERSISTENT_MIN_TOKENS and k <= ORDERED_MAX_K:
+        return ORDERED_TOKEN_TILE, 1
     return tile, max(1, min(sms // ctas, k_blocks // 4))
 
 
 FUSED_NORM_MAX_TOKENS = 4
 PERSISTENT_MIN_TOKENS = 512
+# Tokens per tile of a narrow product of many tokens whose K is not shared out: more CTAs than with 128, and more stages in flight. 8 to
+# 512 features, 520 to 2048 tokens, B200, storing, tiles of 64 / K shared out over tiles of 128 into a cleared output / the same with
+# a launch that clears it (us): K of 512 4.9-5.6 / 7.1-8.2 / 10-12, of 1024 7.2-7.9 / 7.2-9.5 / 10-12, of 1536 9.5-10.3 / 7.3-10.8 / 10-14,
+# of 2048 11.8-12.7 / 7.4-12.1 / 10-15, of 4096 21-22 / 7.4-17.7 / 10-21; without sharing, tiles of 128 take 2 us more.
+ORDERED_TOKEN_TILE = 64
+ORDERED_MAX_K = 1024                # up to here for every storing product of few tiles
+ORDERED_MAX_K_UNCLEARED = 2048      # and up to here where nobody has cleared the output
 
 
 def _persistent_pays(tokens: int, features: int, k: int, mode: int) -> bool:
@@ -797,15 +806,9 @@ def gemm_persistent(tokens: int, features: int, k: int, mode: int) -> bool:
     return tokens >= PERSISTENT_MIN_TOKENS and _persistent_pays(tokens, features, k, mode)
 
 
-# Tokens per tile of a narrow product whose K is not shared out: more CTAs than with 128, and more stages in flight. 8 to 512 features,
-# 520 to 2048 tokens, B200, tiles of 64 / of 128 / K shared out over tiles of 128 (us): K of 1024 7.2-8.0 / 9.1-10.0 / 7.2-9.6, of
-# 2048 11.9-12.9 / 13.8-15.0 / 7.3-12.3, of 4096 21-22 / 23-25 / 7.4-17.7; tiles of 32 are as fast for few features, slower for many.
-ORDERED_TOKEN_TILE = 64
-
-
 def gemm_adds_parts(tokens: int, features: int, k: int) -> bool:
-    """Whether :func:`gemm`, left to choose, stores into a float32 output of these sizes by adding partial sums, so that the output must
-    be zero beforehand."""
+    """Whether :func:`gemm`, left to choose, stores into a float32 output of these sizes by adding partial sums if somebody has cleared it
+    (it does so itself, or stores in another form, where nobody has)."""
     return not gemm_persistent(tokens, features, k, STORE) and gemm_plan(tokens, features, k, STORE)[1] > 1
 
 
@@ -815,7 +818,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE,
 
     ``a`` [tokens, K] and ``w`` [features, K] are bfloat16; for ``SWIGLU``, ``w`` is the
     interleaved gate/up matrix of :func:`interleave_gate_up` and ``out`` [tokens, features] gets
-    silu(gate) * up. When few CTAs would cover the output, the K range is split over more of
+    silu(gate) * up. When few CTAs would cover the output, a long K range is split over more of
     them and the partial sums meet in float32 atomics; ``cleared`` says that ``out`` is already
     zero for that. ``block_tok`` / ``splits`` override the plan (tests).
 
@@ -856,7 +859,10 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE,
         if out.dtype != torch.float32:
             n_splits = 1
         elif not cleared:
-            out.zero_()
+            if M >= PERSISTENT_MIN_TOKENS and K <= ORDERED_MAX_K_UNCLEARED and not block_tok and not splits:
+                tile, n_splits = ORDERED_TOKEN_TILE, 1
+            else:
+                out.zero_()
     norm_args = (None, 0.0, None, None, 0, None)
     if norm_after is not None:
         gain, eps, normed, clear, counter = norm_after

@@ -32,9 +32,13 @@ def test_few_tiles_share_k_out_and_callers_know(monkeypatch):
                 persistent = name == "lp_gemm_persistent"
                 tiles = -(-N // 128) * -(-T // 256)
                 assert not (persistent and tiles * 4 <= 148), (T, N, K)
-                adds = not persistent and args[12] > 1                # the splits
-                assert bool((out == 0).all()) == adds, (T, N, K)      # (an output that nobody cleared)
+                # an output that nobody cleared: cleared here if partial sums (more than one split) are added into it
+                assert bool((out == 0).all()) == (not persistent and args[12] > 1), (T, N, K)
+                ops.gemm(a, w, out, ops.STORE, cleared=True)
+                name, args = launched.pop()
+                adds = name != "lp_gemm_persistent" and args[12] > 1
                 assert linear.needs_zero(T) == adds, (T, N, K)
+                assert not adds or T < 512 or K > ops.ORDERED_MAX_K, (T, N, K)
                 forms.add((persistent, adds))
                 ops.gemm(a, w, out, ops.ACCUMULATE)
                 assert not (launched.pop()[0] == "lp_gemm_persistent" and tiles * 4 <= 148), (T, N, K)
