@@ -19,7 +19,7 @@
 // Before, every token passed through every expert: 2048 tokens, width 2048, 8 experts of 2048 and a shared one, 2 chosen,
 // B200: gated product 230 us, scaling of the hidden values about 25, down product 117; now list 6, gather 9, gated product
 // 79 (1.3 PFLOP/s, bound by the tensor cores with their last wave), down product 54 (0.96 PFLOP/s; its epilogue writes 50 MB of
-// float32 in 16-byte pieces), sums 12. The whole feed-forward: 443 -> 213 us. Adding into the tokens' rows with atomics instead
+// float32 in 16-byte pieces), sums 12. The whole feed-forward: 443 -> 217 us. Adding into the tokens' rows with atomics instead
 // takes 11 us less, in an order that changes from run to run.
 //
 // Every wait on an mbarrier is bounded, as in gemm_tcgen05.cu.
@@ -390,13 +390,17 @@ template <bool UP>
 int launch_gemm(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& ms, void* out, int ldo, const Experts& ex,
                 const Shared& shared, int* status, cudaStream_t stream) {
     auto kernel = expert_gemm_kernel<UP>;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (err != cudaSuccess) return failed_launch(err, "shared memory");
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (e != cudaSuccess) return failed_launch(e, "shared memory");
+        configured = true;
+    }
     const long long shared_tiles = (ex.shared_rows + ROWS - 1) / ROWS, cols = (ex.cols + COLS - 1) / COLS;
     const long long most_tiles = UP ? (long long)ex.room / ROWS * (ex.ff / 128) + shared_tiles * (ex.shared_ff / 128)
                                     : ((long long)ex.room / ROWS + shared_tiles) * cols;
     const int grid = most_tiles < lp_sm_count() ? (int)most_tiles : lp_sm_count();
-    err = lp_launch(kernel, dim3(grid), THREADS, SMEM_BYTES, stream, mw, mx, ms, out, ldo, ex, shared, status);
+    const cudaError_t err = lp_launch(kernel, dim3(grid), THREADS, SMEM_BYTES, stream, mw, mx, ms, out, ldo, ex, shared, status);
     return err == cudaSuccess ? lp_check_launch("experts (product)") : failed_launch(err, "product");
 }
 
@@ -428,10 +432,11 @@ extern "C" int lp_experts(const void* x, const float* weights, int ldw, const vo
     CUtensorMap m_up, m_x, m_xs, m_down, m_h, m_hs;
     int rc = make_map(&m_up, w_up, 2LL * ((long long)E * ff + shared_ff), d, d, COLS);
     if (!rc) rc = make_map(&m_x, gathered, rows, d, d, ROWS);
-    if (!rc) rc = make_map(&m_xs, x, T, d, d, ROWS);
     if (!rc) rc = make_map(&m_down, w_down, d, (long long)E * ff + shared_ff, (long long)E * ff + shared_ff, COLS);
     if (!rc) rc = make_map(&m_h, hidden, rows, ff, ff, ROWS);
+    m_xs = m_x;                                               // (not read without a shared expert)
     m_hs = m_h;
+    if (!rc && shared_ff > 0) rc = make_map(&m_xs, x, T, d, d, ROWS);
     if (!rc && shared_ff > 0) rc = make_map(&m_hs, hidden_s, T, shared_ff, shared_ff, ROWS);
     if (rc) return rc;
     cudaError_t err = lp_launch(expert_list_kernel, dim3(E), dim3(1024), 0, stream, weights, ldw, T, counts, list, place);

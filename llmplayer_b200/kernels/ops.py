@@ -2209,19 +2209,20 @@ def experts(x: torch.Tensor, weights: torch.Tensor, w_up: torch.Tensor, w_down: 
         raise KernelError(f"experts: x {tuple(x.shape)}, weights {tuple(weights.shape)}, w_up {tuple(w_up.shape)}, w_down "
                           f"{tuple(w_down.shape)}, out {tuple(out.shape)} for {E} experts of {expert_size} and {shared_size}")
     rows = expert_rows(T, E, top, False)
-    counts = scratch("expert_lists", (E * (T + 1),), torch.int32)
-    row_token = scratch("expert_row_tokens", (rows,), torch.int32)
-    row_weight = scratch("expert_row_weights", (rows,), torch.float32)
-    place = scratch("expert_places", (T * E,), torch.int32)
+    integers = scratch("expert_lists", (E * (2 * T + 1) + 2 * rows,), torch.int32)
+    counts = integers.data_ptr()
+    places = counts + 4 * E * (T + 1)                 # behind the counts and the lists
+    row_token = places + 4 * E * T
+    row_weight = row_token + 4 * rows                 # float32
     # the gathered rows, then in their place the rows' results, as many columns at a time as EXPERTS_RESULT_BYTES hold
     slice_cols = d if rows * d * 4 <= EXPERTS_RESULT_BYTES else min(d, max(256, EXPERTS_RESULT_BYTES // (rows * 4) // 256 * 256))
     gathered = scratch("expert_rows", (max(rows * d, 2 * rows * slice_cols),), torch.bfloat16)
     hidden = scratch("expert_hidden", (rows * int(expert_size) + T * int(shared_size),), torch.bfloat16)
     lib = library("gemm_experts")
     _check(lib, lib.lp_experts(x.data_ptr(), weights.data_ptr(), weights.shape[1], w_up.data_ptr(), w_down.data_ptr(), out.data_ptr(), d,
-                               T, d, E, int(top), int(expert_size), int(shared_size), rows, counts.data_ptr(),
-                               counts.data_ptr() + 4 * E, place.data_ptr(), gathered.data_ptr(), slice_cols, hidden.data_ptr(),
-                               row_token.data_ptr(), row_weight.data_ptr(), 1 if overwrite else 0, kernel_status().data_ptr(), _stream()))
+                               T, d, E, int(top), int(expert_size), int(shared_size), rows, counts,
+                               counts + 4 * E, places, gathered.data_ptr(), slice_cols, hidden.data_ptr(), row_token, row_weight,
+                               1 if overwrite else 0, kernel_status().data_ptr(), _stream()))
     count_launches(2 + 2 * -(-d // slice_cols))
     return out
 
