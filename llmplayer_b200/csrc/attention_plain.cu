@@ -170,13 +170,42 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool real) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(gmem), "r"(bytes) : "memory");
 }
 
+// Where the 128 keys of a block begin (keys of key head g; values lie G * page_size * hd further), -1 for those that nobody sees: worked out
+// once per block, so that the copies need neither the page table nor a division.
+template <typename Seen>
+__device__ __forceinline__ void find_rows(long long* rows, int c0, const int* pt, int page_size, int G, int g, int hd, Seen seen) {
+    if ((int)threadIdx.x < KB) {
+        const int key = c0 + threadIdx.x;
+        long long at = -1;
+        if (seen(key)) {
+            const int page = pt[key / page_size];
+            if (page >= 0) at = (((long long)page * 2 * G + g) * page_size + key % page_size) * hd;
+        }
+        rows[threadIdx.x] = at;
+    }
+}
+// rows of hd values (hd a multiple of 4) to shared memory, `stride` floats apart, by all THREADS threads
+template <int THREADS>
+__device__ __forceinline__ void copy_rows(float* to, int stride, const float* from, const long long* rows, int hd) {
+    const int n4 = hd / 4, step_row = THREADS / n4, step_piece = THREADS % n4;
+    int j = threadIdx.x / n4, c = threadIdx.x % n4;
+    while (j < KB) {
+        const long long at = rows[j];
+        copy16(to + j * stride + c * 4, at >= 0 ? from + at + c * 4 : from, at >= 0);
+        j += step_row;
+        c += step_piece;
+        if (c >= n4) { c -= n4; ++j; }
+    }
+}
+
 constexpr int TILE_WARPS = 8;
 
 // Prompts: a tile of 8 * RW consecutive tokens and one head per CTA; a warp owns RW of its rows, a lane four keys of a
 // block for the scores and features lane, lane + 32, ... for the values. Bound by the multiply-adds and the reads of shared
 // memory that feed them (RW x 4 scores per lane: RW + 4 reads of 16 bytes for 16 RW multiply-adds). Four rows per warp and
 // two CTAs per SM: 509 tokens, 32 heads of 64, B200: 1143 us with a block per query (above) -> 220 us with eight rows per
-// warp and one CTA per SM -> about 100 us.
+// warp and one CTA per SM -> 107 us -> 90 us with the keys' places worked out once per block and, for heads of up to 64, the values
+// asked for together with the keys.
 template <int NI, int RW>
 __global__ void __launch_bounds__(TILE_WARPS * 32, NI <= 4 ? 2 : 1)
 attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, const float* __restrict__ pages,
@@ -187,9 +216,12 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
     extern __shared__ __align__(16) float smem[];
     const int stride = hd + 4;                    // a multiple of 4 floats that walks through the banks
     float* qs = smem;                             // [ROWS][stride]
-    float* kv = qs + ROWS * stride;               // [KB][stride]: keys, then values
-    float* probs = kv + KB * stride;              // [warp][KB][RW]
+    float* kv = qs + ROWS * stride;               // [KB][stride]: keys, then values unless these have room of their own
+    constexpr bool BOTH = NI <= 2;                // there is room for the values beside the keys: asked for together
+    float* vals = BOTH ? kv + KB * stride : kv;
+    float* probs = vals + KB * stride;            // [warp][KB][RW]
     __shared__ int row_seq[ROWS], row_pos[ROWS];
+    __shared__ long long key_rows[KB];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // the last tiles of a sequence have the most keys: they start first
@@ -230,19 +262,18 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
         const int* pt = page_table + (long long)seq * pt_stride;
         for (int c0 = 0; c0 <= seg_pos; c0 += KB) {
             if (!block_seen(c0, seg_lo, seg_kept, seg_pos)) continue;
-            auto load = [&](long long shift) {
-                for (int i = tid; i < KB * n4; i += TILE_WARPS * 32) {
-                    const int j = i / n4, c = i % n4 * 4, key = c0 + j;
-                    const bool real = key <= seg_pos && (key >= seg_lo || key < seg_kept);      // other pages may be gone
-                    const int page = real ? pt[key / page_size] : -1;
-                    const float* from = pages;
-                    if (page >= 0) from = pages + (((long long)page * 2 * G + g) * page_size + key % page_size) * hd + shift + c;
-                    copy16(kv + j * stride + c, from, page >= 0);
-                }
-                asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-                __syncthreads();
-            };
-            load(0);
+            find_rows(key_rows, c0, pt, page_size, G, g, hd,
+                      [&](int key) { return key <= seg_pos && (key >= seg_lo || key < seg_kept); });      // other pages may be gone
+            __syncthreads();
+            copy_rows<TILE_WARPS * 32>(kv, stride, pages, key_rows, hd);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (BOTH) {
+                copy_rows<TILE_WARPS * 32>(vals, stride, pages + (long long)G * page_size * hd, key_rows, hd);
+                asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
             bool active = false;
 #pragma unroll
             for (int r = 0; r < RW; ++r) {
@@ -301,8 +332,13 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
                     lb[r] = lp_warp_sum(sum);
                 }
             }
-            __syncthreads();                       // all warps are through with the keys
-            load((long long)G * page_size * hd);
+            if (!BOTH) {
+                __syncthreads();                   // all warps are through with the keys
+                copy_rows<TILE_WARPS * 32>(vals, stride, pages + (long long)G * page_size * hd, key_rows, hd);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
             if (active) {
                 float part[RW][NI];
 #pragma unroll
@@ -319,7 +355,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
                         p[r] = four.x; p[r + 1] = four.y; p[r + 2] = four.z; p[r + 3] = four.w;
                     }
 #pragma unroll
-                    for (int i = 0; i < NI; ++i) v[i] = lane + 32 * i < hd ? kv[j * stride + lane + 32 * i] : 0.f;
+                    for (int i = 0; i < NI; ++i) v[i] = lane + 32 * i < hd ? vals[j * stride + lane + 32 * i] : 0.f;
 #pragma unroll
                     for (int r = 0; r < RW; ++r)
                         if (p[r] > 0.f) {          // a weight of zero takes nothing from a row, whatever it holds
@@ -354,7 +390,8 @@ attention_f32_tile_kernel(const float* __restrict__ q, float* __restrict__ out, 
 
 // Steps of a few tokens per sequence: a CTA per (block of keys, key head, token) serves all query heads that share the key
 // head (SHARE_HEADS at a time) and leaves maximum, sum and weighted values of its block; the blocks of long sequences lie side by
-// side on the chip instead of one behind the other. Bound by the latency of one block's reads.
+// side on the chip instead of one behind the other. Bound by the latency of one block's reads. 4 sequences of up to 700, 32 heads of 64 on
+// 8, B200: 19.1 us with a division and a look into the page table per 16 bytes and a chain per head, now 10.4.
 template <int SHARE_HEADS>
 __global__ void __launch_bounds__(KB)
 attention_f32_share_kernel(const float* __restrict__ q, float* __restrict__ parts, const float* __restrict__ pages,
@@ -366,7 +403,8 @@ attention_f32_share_kernel(const float* __restrict__ q, float* __restrict__ part
     float* ks = smem;                             // [KB][stride]
     float* vs = ks + KB * stride;                 // [KB][hd]
     float* qs = vs + KB * hd;                     // [SHARE_HEADS][hd]
-    __shared__ float probs[KB][SHARE_HEADS];
+    __shared__ __align__(16) float probs[KB][SHARE_HEADS];
+    __shared__ long long key_rows[KB];
     __shared__ float warp_max[SHARE_HEADS][KB / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = blockIdx.x, g = blockIdx.y, t = blockIdx.z;
@@ -376,20 +414,13 @@ attention_f32_share_kernel(const float* __restrict__ q, float* __restrict__ part
     const int lo = mask.first(pos), keep_end = mask.kept(lo);
     if (!block_seen(c0, lo, keep_end, pos)) return;
     const int* pt = page_table + (long long)seq_ids[t] * pt_stride;
-    const int n4 = hd / 4, rep = H / G;
-    for (int which = 0; which < 2; ++which) {
-        float* to = which ? vs : ks;
-        const int ld = which ? hd : stride;
-        for (int i = tid; i < KB * n4; i += KB) {
-            const int j = i / n4, c = i % n4 * 4, key = c0 + j;
-            const bool real = key <= pos && (key >= lo || key < keep_end);               // other pages may be gone
-            const float* from = pages;
-            if (real)
-                from = pages + (((long long)pt[key / page_size] * 2 * G + (which ? G : 0) + g) * page_size + key % page_size) * hd + c;
-            copy16(to + j * ld + c, from, real);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
+    const int rep = H / G;
+    find_rows(key_rows, c0, pt, page_size, G, g, hd, [&](int key) { return key <= pos && (key >= lo || key < keep_end); });
+    __syncthreads();
+    copy_rows<KB>(ks, stride, pages, key_rows, hd);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    copy_rows<KB>(vs, hd, pages + (long long)G * page_size * hd, key_rows, hd);
+    asm volatile("cp.async.commit_group;" ::: "memory");
     const int key = c0 + tid;
     const bool seen = key <= pos && (key >= lo || key < keep_end);
     for (int h0 = 0; h0 < rep; h0 += SHARE_HEADS) {
@@ -428,15 +459,26 @@ attention_f32_share_kernel(const float* __restrict__ q, float* __restrict__ part
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         const int count = min(KB, pos - c0 + 1);
-        for (int i = tid; i < hd * heads; i += KB) {        // neighbouring threads: neighbouring features of one head
-            const int r = i / hd, d = i % hd;
-            float part = 0.f;
+        // neighbouring threads: neighbouring features; two heads' chains at a time where there are two
+        constexpr int PAIR = SHARE_HEADS > 1 ? 2 : 1;
+        for (int i = tid; i < hd * (SHARE_HEADS / PAIR); i += KB) {
+            const int r = i / hd * PAIR, d = i % hd;
+            if (r >= heads) break;
+            float part[PAIR];
+#pragma unroll
+            for (int k = 0; k < PAIR; ++k) part[k] = 0.f;
 #pragma unroll 16
             for (int j = 0; j < count; ++j) {
-                const float p = probs[j][r], v = vs[j * hd + d];
-                part = p > 0.f ? fmaf(p, v, part) : part;
+                const float v = vs[j * hd + d];
+#pragma unroll
+                for (int k = 0; k < PAIR; ++k) {
+                    const float p = probs[j][r + k];
+                    part[k] = p > 0.f ? fmaf(p, v, part[k]) : part[k];
+                }
             }
-            parts[(((long long)t * H + g * rep + h0 + r) * blocks + b) * (hd + 2) + 2 + d] = part;
+#pragma unroll
+            for (int k = 0; k < PAIR; ++k)
+                if (r + k < heads) parts[(((long long)t * H + g * rep + h0 + r + k) * blocks + b) * (hd + 2) + 2 + d] = part[k];
         }
         for (int r = warp; r < heads; r += KB / 32) {
             float sum = 0.f;
@@ -498,7 +540,7 @@ int launch_tile(const float* q, float* out, const float* pages, const int* page_
                 const int* positions, int T, int H, int G, int hd, int page_size, Scoring scoring, Mask mask, const float* sinks,
                 const float* gate, int gate_ld, cudaStream_t stream) {
     constexpr int ROWS = TILE_WARPS * RW;
-    const size_t smem = ((size_t)(ROWS + KB) * (hd + 4) + (size_t)KB * ROWS) * sizeof(float);
+    const size_t smem = ((size_t)(ROWS + (NI <= 2 ? 2 : 1) * KB) * (hd + 4) + (size_t)KB * ROWS) * sizeof(float);
     auto kernel = attention_f32_tile_kernel<NI, RW>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err == cudaSuccess)
