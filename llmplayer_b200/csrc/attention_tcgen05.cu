@@ -114,9 +114,6 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 template <int HD, int VD, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, Shape<HD, VD, SPLIT>::CTAS_PER_SM)

@@ -1,11 +1,12 @@
 // Plain matrix product for weights stored [out, in]:  C[M, N] = A[M, K] * W[N, K]^T.
-// No tensor cores, float32 multiply-add only. Every output element is summed in one fixed way whatever M is and
-// whichever kernel below forms it: K is cut into eighths (rounded up to 32 products), each eighth is a chain of
-// multiply-adds in increasing k that starts at zero, and the eighths' sums are added in increasing order. So a
-// row's result does not depend on which other rows share the launch, the eighths can be formed side by side where
-// a launch would otherwise leave the chip idle, and the chains are an eighth as long as one over all of K would
-// be (which makes the rounding error smaller, not larger). It is the product of the float32 path and the
-// comparison twin of the tensor-core kernels.
+// Every output element is summed in one fixed way whatever M is, so a row's result does not depend on which other rows share the
+// launch: K is cut into eighths (rounded up to 32 products), each eighth is a sum of its own, the eighths of each half are
+// added in increasing order, then the halves. Two ways of forming an eighth:
+//   * rows of float32 that can be read 16 bytes at a time: on the tensor cores, float32 numbers as three bfloat16 parts, with
+//     errors below those of a chain of multiply-adds (gemm_f32_rows_kernel up to 16 rows, gemm_f32_split_kernel from 17 on: the same bits);
+//   * any other types, sizes and alignments: a chain of multiply-adds in increasing k that starts at zero (gemm_plain_kernel, which
+//     adds all eighths in order).
+// It is the product of the float32 path and the comparison twin of the bfloat16 kernels.
 //
 // Counterparts in the reference (src/main/resources/kernels/cuda/): matmul_f32.cu:6-39,
 // matmul_bf16.cu:6-37 (one warp per output row, one input vector), silu_mul.cu:6-15,
@@ -13,7 +14,7 @@
 // (java21 inference/CudaForwardPass.java:1012-1017).
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "tcgen05_utils.cuh"
 
 #define LP_GEMM_STORE 0      // C = A W^T
 #define LP_GEMM_ACCUMULATE 1 // C += A W^T         (C float32: the residual stream)
@@ -120,7 +121,476 @@ gemm_plain_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __rest
     }
 }
 
+// ---------------------------------------------------------------- float32 on the tensor cores
+// A float32 number is the sum of three bfloat16 ones (3 x 8 bits), and a product of two such parts is exact in float32. So a
+// product of float32 numbers is six products on the tensor cores: all pairs of parts but the three smallest (2^-24 of the
+// whole and below). What would lose bits is their sum: the tensor cores cut every partial sum off instead of rounding it. So
+// the sums in tensor memory are short: 32 products of K, the small pairs first, the two steps of the leading parts last
+// (a step is 16 products); such a block's sum is added to those before it in registers, rounded to nearest, as fmaf would.
+//
+// Per CTA: 128 weight rows (in the gated form 64 gate and the 64 up rows of the same features) x TOK tokens.
+//   warp 0       TMA: float32 boxes of 32 columns of the weights into a ring of stages
+//   warp 2       the tokens' parts, made beforehand by split_rows_kernel, into a ring of their own
+//   warps 1, 3   issue the MMAs of every second block: 12 of 128 x TOK x 16
+//   warps 4-     a weight row per thread: its 32 values in three parts, into tensor memory (the row operand of the MMAs); two groups
+//                of four warps, for every second block each, or one
+//   the last 4 or 8   a block's sums from tensor memory into registers, chains of an eighth of K, the output
+// Two buffers of operands and two of sums, so that all of these work at the same time on neighbouring blocks. Bound by the way round one
+// buffer (sums fetched, weights split, MMAs of about 80 cycles each beside the traffic to tensor memory): about 1,100 cycles per block
+// against 790 for its MMAs alone. B200, 509 rows, against register tiles of paired multiply-adds: 16384 x 2048 (gated) 831 -> 232 us,
+// 2048 x 8192 414 -> 120, 3072 x 2048 167 -> 58, 2048 x 2048 120 -> 50; error against 64 bits 2.9e-7 .. 5.8e-7 -> 1.3e-7 .. 1.6e-7.
+// 64 tokens: 133 -> 64 us, 139 -> 60, 43 -> 28, 43 -> 34.
+constexpr int SPLIT_K = 32;                     // products of a block
+
+template <int TOK> struct SplitTile {
+    static constexpr int ADDERS = TOK == 128 ? 8 : 4;             // warps that add blocks up
+    static constexpr int GROUPS = TOK == 128 ? 1 : 2;             // of four warps that split weights (registers allow 16 warps in all)
+    static constexpr int FIRST_ADDER = 4 + 4 * GROUPS;
+    static constexpr int THREADS = (FIRST_ADDER + ADDERS) * 32;
+    static constexpr int COLS = 64;                               // columns (tokens) of an adding thread
+    static constexpr int PART = TOK * 64;                         // bytes of one part of the tokens' block: rows of 32 bfloat16
+    static constexpr int W_BYTES = 128 * 128, STAGES = TOK == 128 ? 4 : 5;
+    static constexpr int X_STAGE = 3 * PART, X_STAGES = TOK == 128 ? 4 : 6;
+    static constexpr int RING = STAGES * W_BYTES + X_STAGES * X_STAGE;
+    static constexpr int TMEM_COLS = 512;
+    static constexpr int SUMS = 0, WEIGHTS = 2 * TOK, HELD = WEIGHTS + 2 * 48;      // columns of tensor memory
+    static constexpr int SLOTS = TOK == 128 ? 1 : 2;              // sums of chains that tensor memory has room for
+    static constexpr int HALF = TOK == 128 ? TOK * 128 * 4 : 0;   // bytes for the sums of the first half of K, where that room is one slot
+    static constexpr size_t SMEM = 1024 + (size_t)RING + HALF + 256;
+    static_assert(HELD + SLOTS * TOK <= TMEM_COLS, "tensor memory");
+    static_assert(RING >= SLOTS * TOK * 128 * 4, "the ring also holds the sums that a cluster adds up");
+    static_assert(X_STAGE % 1024 == 0 && PART % 512 == 0, "swizzled boxes");
+};
+
+__device__ __forceinline__ void split_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// K-major tile of rows of 64 bytes, swizzled in groups of 8 rows (512 bytes): 16-byte piece c of row r lies at piece c ^ (r / 2 % 4)
+__device__ __forceinline__ uint64_t smem_desc_rows64(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
+// Two neighbouring values in three parts each, cut off and not rounded (byte moves and masks; the conversion to bfloat16 issues at a
+// quarter of their rate): 8 + 8 + 8 bits are all 24. An infinity or a NaN makes sums that are no numbers, which the epilogue
+// forms again one by one.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
+    auto rest = [&]() {
+        asm("{\n\t.reg .b64 v, h;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 h, {%2, %3};\n\tsub.rn.f32x2 v, v, h;\n\tmov.b64 {%0, %1}, v;\n\t}"
+            : "+f"(x), "+f"(y) : "r"(__float_as_uint(x) & 0xffff0000u), "r"(__float_as_uint(y) & 0xffff0000u));
+    };
+    a = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    rest();
+    b = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    rest();
+    c = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+}
+
+// The values are formed here and not where they are used, behind a wait: the time from the end of a block's MMAs to the buffer's next
+// ones is what bounds the kernel.
+__device__ __forceinline__ void keep_here(uint32_t* v, int n) {
+#pragma unroll
+    for (int j = 0; j < n; ++j) asm volatile("" : "+r"(v[j]));
+}
+
+// The rows of A in three parts [3][M][K rounded up to 8] of bfloat16, once for all the tiles that read them.
+__global__ void __launch_bounds__(256)
+split_rows_kernel(const float* __restrict__ A, uint16_t* __restrict__ parts, int M, int K, int lda, int ldp) {
+    lp_grid_wait();
+    lp_grid_release();
+    const long long pieces = (long long)M * (K / 4);
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < pieces; i += (long long)gridDim.x * 256) {
+        const int m = (int)(i / (K / 4)), k = (int)(i % (K / 4)) * 4;
+        const float4 v = *(const float4*)(A + (long long)m * lda + k);
+        uint2 p[3];
+        split_pair(v.x, v.y, p[0].x, p[1].x, p[2].x);
+        split_pair(v.z, v.w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *(uint2*)(parts + ((long long)q * M + m) * ldp + k) = p[q];
+    }
+}
+
+// The product of two rows by multiply-adds, in the order of gemm_plain_kernel: for outputs that are no finite numbers in parts.
+__device__ __noinline__ float row_product(const float* a, const float* w, int K) {
+    const int part = part_length(K);
+    float total = 0.f;
+    for (int k0 = 0; k0 < K; k0 += part) {
+        float s = 0.f;
+        for (int k = k0; k < min(K, k0 + part); ++k) s = fmaf(a[k], w[k], s);
+        total += s;
+    }
+    return total;
+}
+
+// SPLIT: the gridDim.z CTAs of a cluster form PARTS / gridDim.z chains each and add them up through distributed shared memory: two
+// CTAs a half's sum each, four or eight CTAs the single chains.
+template <int TOK, int MODE, bool SPLIT>
+__global__ void __launch_bounds__(SplitTile<TOK>::THREADS, 1)
+gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const float* __restrict__ A,
+                      const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
+                      int* __restrict__ status) {
+    using T = SplitTile<TOK>;
+    constexpr bool GATED = MODE == LP_GEMM_SWIGLU;
+    constexpr int FEATURES = GATED ? 64 : 128;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* token_ring = smem + T::STAGES * T::W_BYTES;
+    float* first_half = (float*)(smem + T::RING);
+    uint64_t* full = (uint64_t*)(smem + T::RING + T::HALF);
+    uint64_t* empty = full + T::STAGES;
+    uint64_t* x_full = empty + T::STAGES;          // the tokens' ring
+    uint64_t* x_empty = x_full + T::X_STAGES;
+    uint64_t* ready = x_empty + T::X_STAGES;       // [2] a block's operands are made, and the sums before it are fetched
+    uint64_t* formed = ready + 2;                  // [2] its MMAs have ended: the operands may go, the sums are there
+    uint64_t* turn = formed + 2;                   // [2] whose MMAs are issued next
+    uint32_t* tmem_slot = (uint32_t*)(turn + 2);
+    volatile uint32_t* failed = tmem_slot + 1;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int token_tiles = (M + TOK - 1) / TOK;                 // token tile first: a weight tile's readers run together
+    const int m0 = (int)(blockIdx.x % token_tiles) * TOK, n0 = (int)(blockIdx.x / token_tiles) * FEATURES;
+    const int part = part_length(K);
+    const int share = SPLIT ? PARTS / (int)gridDim.z : PARTS;    // chains of this CTA
+    const int k_begin = SPLIT ? min(K, (int)blockIdx.z * share * part) : 0;
+    const int k_end = SPLIT ? min(K, k_begin + share * part) : K;
+    const int blocks = (k_end - k_begin + SPLIT_K - 1) / SPLIT_K;
+    const int chain_blocks = part / SPLIT_K;
+
+    lp_grid_release();
+    if (tid == 0) {
+        *failed = 0;
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+        for (int s = 0; s < T::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+        for (int s = 0; s < T::X_STAGES; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&ready[i], 4 + T::ADDERS); mbar_init(&formed[i], 1); mbar_init(&turn[i], 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)T::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    if (warp != 0) lp_grid_wait();
+    bool done = false;                               // this adding thread's sums are whole
+    float sum[T::COLS];                              // of the chain that is being formed, at the end (of one chain, or not SPLIT) the whole
+
+    auto all_wait = [&](uint64_t* bar, int parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
+    auto give_up = [&](int code) {
+        if (lane == 0) atomicExch(status, code);
+        *failed = 1;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            auto weights = [&](int b) {
+                const int s = b % T::STAGES;
+                mbar_expect_tx(&full[s], T::W_BYTES);
+                uint8_t* to = smem + s * T::W_BYTES;
+                tma_load_2d(to, &map_w, k_begin + b * SPLIT_K, n0, &full[s]);
+                if (GATED) tma_load_2d(to + T::W_BYTES / 2, &map_w, k_begin + b * SPLIT_K, N + n0, &full[s]);
+            };
+            // no kernel of a step writes weights, and this thread touches nothing else: it does not wait for the kernel before
+            int b = 0;
+            for (; b < blocks; ++b) {
+                if (!mbar_wait(&empty[b % T::STAGES], ((b / T::STAGES) & 1) ^ 1)) { atomicExch(status, 71); *failed = 1; break; }
+                weights(b);
+            }
+            if (b < blocks)                          // gave up: no copy may be in flight when the CTA ends
+                for (int i = max(0, b - T::STAGES); i < b; ++i) mbar_wait(&full[i % T::STAGES], (i / T::STAGES) & 1);
+        }
+        __syncwarp();
+    } else if (warp == 2) {
+        if (lane == 0) {
+            constexpr int RING = T::X_STAGES;
+            int b = 0;
+            for (; b < blocks; ++b) {
+                const int s = b % RING;
+                if (!mbar_wait(&x_empty[s], ((b / RING) & 1) ^ 1)) { atomicExch(status, 70); *failed = 1; break; }
+                mbar_expect_tx(&x_full[s], T::X_STAGE);
+                uint8_t* to = token_ring + s * T::X_STAGE;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) tma_load_2d(to + q * T::PART, &map_x, k_begin + b * SPLIT_K, q * M + m0, &x_full[s]);
+            }
+            if (b < blocks)
+                for (int i = max(0, b - RING); i < b; ++i) mbar_wait(&x_full[i % RING], (i / RING) & 1);
+        }
+        __syncwarp();
+    } else if (warp == 1 || warp == 3) {
+        // Two warps issue, one block each in turn: behind its MMAs a warp's next wait takes some 400 cycles to return. They take turns,
+        // or the MMAs of two blocks would mix and both blocks end late.
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        constexpr int RING = T::X_STAGES;
+        const int i = warp >> 1;
+        const uint32_t d = tmem + T::SUMS + i * TOK, a = tmem + T::WEIGHTS + i * 48;
+        for (int b = i; b < blocks; b += 2) {
+            const int s = b % RING;
+            bool ok = true;
+            if (lane == 0) {
+                ok = mbar_wait(&x_full[s], (b / RING) & 1);
+                if (ok) ok = mbar_wait(&ready[i], (b >> 1) & 1);
+                if (ok && b > 0) ok = mbar_wait(&turn[i], ((b - 1) >> 1) & 1);
+                if (ok) {
+                    tcgen05_fence_after();
+                    const uint64_t x = smem_desc_rows64(smem_u32(token_ring + s * T::X_STAGE));
+                    constexpr uint64_t P = T::PART >> 4;
+                    uint32_t more = 0;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {    // parts 0 (leading) to 2 of 16 products: 8 columns of weights, 32 bytes of tokens
+                        const uint32_t w = a + k * 8;
+                        const uint64_t t = x + k * 2;
+                        split_mma(d, w + 16, t + P, idesc, more);
+                        more = 1;
+                        split_mma(d, w, t + 2 * P, idesc, 1);
+                        split_mma(d, w + 32, t, idesc, 1);
+                        if (k == 1) mbar_arrive(&turn[i ^ 1]);       // it arrives behind the MMAs issued so far
+                        split_mma(d, w, t + P, idesc, 1);
+                        split_mma(d, w + 16, t, idesc, 1);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) split_mma(d, a + k * 8, x + k * 2, idesc, 1);
+                    tcgen05_commit(&formed[i]);
+                    tcgen05_commit(&x_empty[s]);
+                }
+            }
+            if (!ok) { give_up(72); break; }
+        }
+        __syncwarp();
+    } else if (warp >= 4 && warp < T::FIRST_ADDER) {
+        const uint32_t row_addr = (uint32_t)((warp & 3) * 32) << 16;
+        const int row = (warp & 3) * 32 + lane;
+        const int begin = T::GROUPS == 2 ? (warp - 4) >> 2 : 0;
+        constexpr bool AHEAD = T::GROUPS == 1;       // the next block's values are asked for before the wait for the last one's MMAs
+        float4 v[8];
+        auto fetch = [&](int b) {
+            const int s = b % T::STAGES;
+            if (!all_wait(&full[s], (b / T::STAGES) & 1)) return false;
+            const uint8_t* from = smem + s * T::W_BYTES;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = *(const float4*)(from + row * 128 + ((c ^ (row & 7)) << 4));
+            return true;
+        };
+        if (AHEAD && begin < blocks && !fetch(begin)) give_up(74);
+        for (int b = begin; b < blocks; b += T::GROUPS) {
+            const int s = b % T::STAGES, i = b & 1;
+            if (!AHEAD && !fetch(b)) { give_up(74); break; }
+            uint32_t p[3][16];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                split_pair(v[c].x, v[c].y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
+                split_pair(v[c].z, v[c].w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
+            }
+            keep_here(&p[0][0], 48);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
+            if (AHEAD && b + 1 < blocks && !fetch(b + 1)) { give_up(74); break; }
+            if (!all_wait(&formed[i], ((b >> 1) & 1) ^ 1)) { give_up(75); break; }
+            tcgen05_fence_after();
+#pragma unroll
+            for (int q = 0; q < 3; ++q) tmem_st16(tmem + T::WEIGHTS + i * 48 + q * 16 + row_addr, p[q]);
+            tmem_st_wait();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[i]);
+        }
+    } else if (warp >= T::FIRST_ADDER) {
+        // a thread: one weight row (its lane of tensor memory), COLS tokens
+        const int half = (warp - T::FIRST_ADDER) >> 2;
+        const uint32_t lane_addr = ((uint32_t)((warp & 3) * 32) << 16) + half * T::COLS;
+        if (lane == 0) { mbar_arrive(&ready[0]); mbar_arrive(&ready[1]); }         // nothing to fetch before the first two blocks
+        int in_chain = 0, chain = 0;
+        bool ok = true;
+        for (int b = 0; b < blocks; ++b) {
+            const int i = b & 1;
+            if (!all_wait(&formed[i], (b >> 1) & 1)) { give_up(78); ok = false; break; }
+            tcgen05_fence_after();
+#pragma unroll
+            for (int c = 0; c < T::COLS; c += 32) {
+                uint32_t r[32];
+                tmem_ld32(tmem + T::SUMS + i * TOK + lane_addr + c, r);
+                tmem_ld_wait();
+                if (in_chain == 0) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[c + j] = __uint_as_float(r[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[c + j] += __uint_as_float(r[j]);
+                }
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0 && b + 2 < blocks) mbar_arrive(&ready[i]);
+            if (++in_chain < chain_blocks && b + 1 < blocks) continue;
+            in_chain = 0;                            // a chain ends
+            const bool apart = SPLIT && share < PARTS / 2, again = !SPLIT && chain == PARTS / 2 - 1;
+            if (!apart && chain % (PARTS / 2) > 0) { // it joins those of its half
+#pragma unroll
+                for (int c = 0; c < T::COLS; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(tmem + T::HELD + lane_addr + c, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[c + j] = __uint_as_float(r[j]) + sum[c + j];
+                }
+            }
+            const bool last = b + 1 == blocks;
+            if (T::HALF && again && !last) {         // the first half is whole
+#pragma unroll
+                for (int j = 0; j < T::COLS; ++j) first_half[(half * T::COLS + j) * 128 + (warp & 3) * 32 + lane] = sum[j];
+            } else if (!last || (apart && T::SLOTS > 1)) {
+                const int slot = apart ? chain : again ? 1 : 0;
+#pragma unroll
+                for (int c = 0; c < T::COLS; c += 16) {
+                    uint32_t r[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(sum[c + j]);
+                    tmem_st16(tmem + T::HELD + slot * TOK + lane_addr + c, r);
+                }
+                tmem_st_wait();
+            }
+            ++chain;
+        }
+        if (!SPLIT && chain > PARTS / 2) {           // both halves
+#pragma unroll
+            for (int c = 0; c < T::COLS; c += 16) {
+                uint32_t r[16];
+                if (T::HALF) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(first_half[(half * T::COLS + c + j) * 128 + (warp & 3) * 32 + lane]);
+                } else {
+                    tmem_ld16(tmem + T::HELD + TOK + lane_addr + c, r);
+                    tmem_ld_wait();
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum[c + j] = __uint_as_float(r[j]) + sum[c + j];
+            }
+        }
+        done = ok;
+    }
+
+    const int quarter = warp & 3, column0 = (warp - T::FIRST_ADDER) / 4 * T::COLS;      // of an adding warp
+    const bool adder = warp >= T::FIRST_ADDER;
+    auto weight_row = [&](int f) { return W + (long long)f * ldw; };
+    auto whole = [&](float v, int m, int f) {       // a sum that is no finite number is formed again
+        return fabsf(v) < INFINITY ? v : row_product(A + (long long)m * lda, weight_row(f), K);
+    };
+    auto store = [&](int m, int f, float v) {
+        float* c = C + (long long)m * ldc + f;
+        *c = MODE == LP_GEMM_ACCUMULATE ? *c + v : v;
+    };
+    if constexpr (SPLIT) {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        const int chains = (K + part - 1) / part;    // of the whole
+        const bool apart = share < PARTS / 2;
+        float* sums = (float*)smem;                  // [slot][token][weight row]; every copy and MMA that used this memory has ended
+        if (adder && done && blocks > 0) {
+            if (apart && T::SLOTS > 1) {
+                const int here = min(share, chains - (int)blockIdx.z * share);
+                for (int q = 0; q < here; ++q) {
+#pragma unroll
+                    for (int c = 0; c < T::COLS; c += 16) {
+                        uint32_t r[16];
+                        tmem_ld16(tmem + T::HELD + q * TOK + ((uint32_t)(quarter * 32) << 16) + column0 + c, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sums[((size_t)q * TOK + column0 + c + j) * 128 + quarter * 32 + lane] = __uint_as_float(r[j]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < T::COLS; ++j) sums[(column0 + j) * 128 + quarter * 32 + lane] = sum[j];
+            }
+        }
+        __syncthreads();
+        cluster.sync();
+        const int tokens = TOK / (int)gridDim.z;     // of the tile, finished by this CTA
+        uint32_t bad = 0;
+        for (int c = 0; c < (int)gridDim.z; ++c) bad |= *(volatile uint32_t*)cluster.map_shared_rank((uint32_t*)failed, c);
+        if (!bad) {
+            for (int e = tid; e < tokens * FEATURES; e += T::THREADS) {
+                const int t = (int)blockIdx.z * tokens + e / FEATURES, f = e % FEATURES;
+                const int m = m0 + t, n = n0 + f;
+                if (m >= M || n >= N) continue;
+                float g = 0.f, u = 0.f, g0 = 0.f, u0 = 0.f;
+                const int step = apart ? 1 : share;  // chains per sum
+                for (int c = 0; c < chains; c += step) {
+                    const float* from = cluster.map_shared_rank(sums, c / share) + ((apart ? c % share : 0) * TOK + t) * 128 + f;
+                    const bool starts = c % (PARTS / 2) == 0;
+                    if (starts) { g0 = g; u0 = u; }
+                    g = starts ? from[0] : g + from[0];
+                    if (GATED) u = starts ? from[64] : u + from[64];
+                }
+                if (chains > PARTS / 2) { g = g0 + g; u = u0 + u; }
+                if (GATED) C[(long long)m * ldc + n] = silu_mul(whole(g, m, n), whole(u, m, N + n));
+                else store(m, n, whole(g, m, n));
+            }
+        }
+        cluster.sync();                              // nobody leaves while its sums are still read
+    } else if constexpr (GATED) {
+        float* up = (float*)smem;                    // [token][feature]
+        if (adder && quarter >= 2) {
+#pragma unroll
+            for (int j = 0; j < T::COLS; ++j) up[(column0 + j) * 64 + (quarter - 2) * 32 + lane] = sum[j];
+        }
+        __syncthreads();
+        const int f = quarter * 32 + lane, n = n0 + f;
+        if (adder && quarter < 2 && n < N && !*failed) {
+#pragma unroll
+            for (int j = 0; j < T::COLS; ++j) {
+                const int m = m0 + column0 + j;
+                if (m < M) C[(long long)m * ldc + n] = silu_mul(whole(sum[j], m, n), whole(up[(column0 + j) * 64 + f], m, N + n));
+            }
+        }
+    } else {
+        __syncthreads();
+        const int n = n0 + quarter * 32 + lane;
+        if (adder && n < N && !*failed) {
+#pragma unroll
+            for (int j = 0; j < T::COLS; ++j) {
+                const int m = m0 + column0 + j;
+                if (m < M) store(m, n, whole(sum[j], m, n));
+            }
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)T::TMEM_COLS));
+    }
+}
+
 // ---------------------------------------------------------------- float32, a handful of rows
+// A step of a few sequences reads every weight once and is bound by that: 16 weight rows (in the gated form 8 gate and 8 up rows) x
+// TOK tokens per CTA, a warp per chain of K. A warp copies its own stages (its rows' next 32 values, and the tokens'), splits them in
+// registers and multiplies them with mma.sync, whose sums of 16 products are those of tcgen05.mma bit for bit: same steps, same
+// order, so a row's result is the same as in the tiles above. Nothing but the chains' sums crosses warps. Bound by the copies in flight
+// and the chain of twelve MMAs per block. B200, the four products of a layer of width 2048 one behind the other (243 MB), against a
+// thread per chain and weight row: 16 rows 169 -> 78 us, 8 rows 91 -> 62, 4 rows 64 -> 59, 1 row 53 -> 58 (4.2 TB/s).
+constexpr int ROW_FEATURES = 16;
+
+template <int TOK, bool DEEP> struct RowsShape {
+    static constexpr int THREADS = PARTS * 32;
+    static constexpr int STAGE = (ROW_FEATURES + TOK) * 128;      // bytes of a warp's stage: rows of 32 values
+    // two CTAs per SM; DEEP: one, for grids that have no more (four products of 4 rows: 73 us with the short ring everywhere, 59)
+    static constexpr int STAGES = (DEEP ? 200 : 96) * 1024 / (PARTS * STAGE);
+    static constexpr int TOGETHER = DEEP && TOK == 8 ? 2 : 1;     // blocks whose MMAs (a chain of twelve) run side by side
+    static constexpr size_t SMEM = (size_t)PARTS * STAGES * STAGE;
+};
+
 __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool real) {
     const unsigned to = (unsigned)__cvta_generic_to_shared(smem);
     const int bytes = real ? 16 : 0;       // the rest of the 16 bytes is zero
@@ -128,341 +598,164 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool real) 
 }
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void mma_16x8(float* c, const uint32_t* a, const uint32_t* b) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
 
-constexpr int ROW_FEATURES = 8;          // output features of a CTA (in the gated form as many gate and up rows)
-constexpr int ROW_CHUNK = 32;            // products of a chain per stage
-constexpr int ROW_STRIDE = ROW_CHUNK + 4;   // 144 bytes from one chain's chunk to the next: eight lanes' 16-byte reads hit all banks
-
-// DEEP: a ring of up to eight stages, two CTAs per SM (for grids that have no more); else four stages, of which two (16 rows) to five (one
-// row) CTAs fit an SM, in the gated form two, and one at 16 rows (147 KB)
-template <int MR, int MODE, bool DEEP> struct RowsShape {
-    static constexpr int WROWS = MODE == LP_GEMM_SWIGLU ? 2 * ROW_FEATURES : ROW_FEATURES;
-    static constexpr int THREADS = WROWS * PARTS;
-    static constexpr int STAGE = (WROWS + MR) * PARTS * ROW_STRIDE;       // floats
-    static constexpr int ROOM = 113 * 1024 / 4 / STAGE;
-    static constexpr int STAGES = !DEEP || ROOM < 4 ? 4 : ROOM < 8 ? ROOM : 8;
-    static constexpr size_t SMEM = (size_t)STAGE * STAGES * sizeof(float);
-};
-
-template <int MR, int MODE, bool DEEP>
-__global__ void __launch_bounds__(RowsShape<MR, MODE, DEEP>::THREADS, 1)
+template <int TOK, int MODE, bool DEEP>
+__global__ void __launch_bounds__(PARTS * 32, DEEP ? 1 : 2)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
                      int lda, int ldw, int ldc) {
-    // A step of a few sequences reads every weight once and is bound by that. A thread owns one chain of one weight row
-    // for all MR rows of A: the chains of a CTA's rows run side by side, so N / 8 CTAs of 64 threads are enough to keep
-    // the memory busy, and the order of every sum stays the one named above. 4 rows, B200: 16384 x 2048 (gated) 229 -> 30 us
-    // (4.5 TB/s), 2048 x 8192 about 700 -> 19 us (3.5 TB/s) against the 64 x 64 tiles of the kernel above, which left most of
-    // the chip idle. What is left is issue: about 60 instructions per warp and 4 KB of weights, and the launch itself.
-    using S = RowsShape<MR, MODE, DEEP>;
-    extern __shared__ __align__(16) float ring[];
-    const int tid = threadIdx.x;
-    const int n0 = blockIdx.x * ROW_FEATURES, m0 = blockIdx.y * MR;
-    const int row = tid % S::WROWS, chain = tid / S::WROWS;
+    using S = RowsShape<TOK, DEEP>;
+    constexpr bool GATED = MODE == LP_GEMM_SWIGLU;
+    constexpr int FEATURES = GATED ? ROW_FEATURES / 2 : ROW_FEATURES, TILES = TOK / 8;
+    extern __shared__ __align__(128) uint8_t rows_smem[];
+    __shared__ float sums[PARTS][TOK][ROW_FEATURES];
+    const int tid = threadIdx.x, chain = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int n0 = blockIdx.x * FEATURES;
     const int part = part_length(K);
-    const int steps = part / ROW_CHUNK;
+    const int k_begin = min(K, chain * part), k_end = min(K, k_begin + part);
+    const int blocks = (k_end - k_begin + SPLIT_K - 1) / SPLIT_K;
+    uint8_t* ring = rows_smem + chain * S::STAGES * S::STAGE;
 
-    // Copies go in pieces of 16 bytes, eight to a chunk, chunks ordered [chain][row]: thread tid always copies piece
-    // tid % 8 of weight row tid / 8, for every chain, so only the step moves its addresses.
-    const int piece = (tid & 7) * 4, copy_row = tid >> 3;
-    const int feature = n0 + (copy_row % ROW_FEATURES);
-    const bool feature_ok = feature < N;
-    const float* from_w = W + (feature_ok ? (long long)(copy_row < ROW_FEATURES ? feature : N + feature) * ldw + piece : 0);
-    float* to_w = ring + copy_row * ROW_STRIDE + piece;
-    auto fetch_w = [&](int step, int slot) {
-        if (step >= steps) return;
-        float* to = to_w + slot * S::STAGE;
-        const float* from = from_w + step * ROW_CHUNK;
-        const int limit = feature_ok ? K - piece - step * ROW_CHUNK : 0;
+    // 16-byte piece c of row r lies at piece c ^ 4 (r % 2): the eight lanes that are served together read two rows
+    const int piece = lane & 7, copy_row = lane >> 3;             // rows copy_row, + 4, + 8, ...
+    auto weight_row = [&](int r) { return GATED ? (r < FEATURES ? n0 + r : N + n0 + r - FEATURES) : n0 + r; };
+    auto feature_real = [&](int r) { return n0 + (GATED ? r % FEATURES : r) < N; };
+    const float* from_w[4];
+    bool real_w[4];
 #pragma unroll
-        for (int c = 0; c < PARTS; ++c) copy16(to + c * S::WROWS * ROW_STRIDE, c * part < limit ? from + c * part : W, c * part < limit);
+    for (int i = 0; i < 4; ++i) {
+        const int r = copy_row + i * 4;
+        real_w[i] = feature_real(r);
+        from_w[i] = W + (real_w[i] ? (long long)weight_row(r) * ldw : 0) + k_begin + piece * 4;
+    }
+    const uint32_t to = copy_row * 128 + ((piece ^ ((copy_row & 1) * 4)) << 4);
+    auto fetch_w = [&](int b) {
+        if (b >= blocks) return;
+        uint8_t* stage = ring + b % S::STAGES * S::STAGE + to;
+        const bool inside = k_begin + b * SPLIT_K + piece * 4 < k_end;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) copy16(stage + i * 512, real_w[i] && inside ? from_w[i] + b * SPLIT_K : W, real_w[i] && inside);
     };
-    constexpr int A_COPIES = MR * PARTS * 8 / S::THREADS > 0 ? MR * PARTS * 8 / S::THREADS : 1;     // per thread
-    auto fetch_a = [&](int step, int slot) {
-        if (step >= steps) return;
-        float* base = ring + slot * S::STAGE + PARTS * S::WROWS * ROW_STRIDE;
+    auto fetch_x = [&](int b) {
+        if (b >= blocks) return;
+        uint8_t* stage = ring + b % S::STAGES * S::STAGE + ROW_FEATURES * 128 + to;
+        const int k = k_begin + b * SPLIT_K + piece * 4;
 #pragma unroll
-        for (int i = 0; i < A_COPIES; ++i) {
-            const int p = (i * S::THREADS + tid) >> 3, r = p % MR, c = p / MR;
-            if (c >= PARTS) break;
-            const int k = c * part + step * ROW_CHUNK + piece;
-            const bool real = k < K && m0 + r < M;
-            copy16(base + (c * MR + r) * ROW_STRIDE + piece, real ? A + (long long)(m0 + r) * lda + k : A, real);
+        for (int i = 0; i < TOK / 4; ++i) {
+            const int m = copy_row + i * 4;
+            const bool real = m < M && k < k_end;
+            copy16(stage + i * 512, real ? A + (long long)m * lda + k : A, real);
         }
     };
 
-    // weights are written by no kernel of a step: the first stages of them are asked for before the wait
+    // no kernel of a step writes weights: the first stages of them are asked for before the wait
 #pragma unroll
-    for (int s = 0; s < S::STAGES - 1; ++s) fetch_w(s, s);
+    for (int b = 0; b < S::STAGES - S::TOGETHER; ++b) fetch_w(b);
     lp_grid_wait();
     lp_grid_release();
 #pragma unroll
-    for (int s = 0; s < S::STAGES - 1; ++s) {
-        fetch_a(s, s);
+    for (int b = 0; b < S::STAGES - S::TOGETHER; ++b) {
+        fetch_x(b);
         copies_commit();       // the first group also holds all weights asked for above
     }
-    float acc[MR];
+    float sum[TILES][4];
 #pragma unroll
-    for (int m = 0; m < MR; ++m) acc[m] = 0.f;
-    int slot = 0;
-    for (int step = 0; step < steps; ++step) {
-        copies_wait<S::STAGES - 2>();
-        __syncthreads();
-        {
-            const int next = step + S::STAGES - 1, to = slot == 0 ? S::STAGES - 1 : slot - 1;
-            fetch_w(next, to);
-            fetch_a(next, to);
+    for (int n = 0; n < TILES; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[n][i] = 0.f;
+    constexpr int U = S::TOGETHER;
+    for (int b = 0; b < blocks; b += U) {
+        copies_wait<S::STAGES - 2 * U>();
+        __syncwarp();
+        // parts [part][register]: a lane's four neighbouring values of 16 are its two pairs of an operand, so products 4 t .. 4 t + 3 of a
+        // step stand where the instruction counts 2 t, 2 t + 1, 2 t + 8, 2 t + 9; which of the 16 comes where does not matter to their sum
+        uint32_t w[U][2][3][4], x[U][TILES][2][3][2];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint8_t* stage = ring + (b + u) % S::STAGES * S::STAGE;
+            auto at = [&](int row, int step) { return *(const float4*)(stage + row * 128 + (((step * 4 + t) ^ ((row & 1) * 4)) << 4)); };
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 v = at(g + h * 8, s);
+                    split_pair(v.x, v.y, w[u][s][0][h], w[u][s][1][h], w[u][s][2][h]);
+                    split_pair(v.z, v.w, w[u][s][0][h + 2], w[u][s][1][h + 2], w[u][s][2][h + 2]);
+                }
+#pragma unroll
+                for (int n = 0; n < TILES; ++n) {
+                    const float4 v = at(ROW_FEATURES + n * 8 + g, s);
+                    split_pair(v.x, v.y, x[u][n][s][0][0], x[u][n][s][1][0], x[u][n][s][2][0]);
+                    split_pair(v.z, v.w, x[u][n][s][0][1], x[u][n][s][1][1], x[u][n][s][2][1]);
+                }
+            }
+        }
+        __syncwarp();                                // the stages before these are free
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            fetch_w(b + u + S::STAGES - U);
+            fetch_x(b + u + S::STAGES - U);
             copies_commit();
         }
-        const float* w = ring + slot * S::STAGE + (chain * S::WROWS + row) * ROW_STRIDE;
-        const float* a = ring + slot * S::STAGE + PARTS * S::WROWS * ROW_STRIDE + chain * MR * ROW_STRIDE;
+        float d[U][TILES][4];
 #pragma unroll
-        for (int c = 0; c < ROW_CHUNK / 4; ++c) {
-            const float4 wv = *(const float4*)(w + c * 4);
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int m = 0; m < MR; ++m) {
-                const float4 av = *(const float4*)(a + m * ROW_STRIDE + c * 4);
-                acc[m] = fmaf(av.x, wv.x, acc[m]);
-                acc[m] = fmaf(av.y, wv.y, acc[m]);
-                acc[m] = fmaf(av.z, wv.z, acc[m]);
-                acc[m] = fmaf(av.w, wv.w, acc[m]);
-            }
+            for (int n = 0; n < TILES; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) d[u][n][i] = 0.f;
+        auto product = [&](int s, int p, int q) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int n = 0; n < TILES; ++n) mma_16x8(d[u][n], w[u][s][p], x[u][n][s][q]);
+        };
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            product(s, 1, 1);
+            product(s, 0, 2);
+            product(s, 2, 0);
+            product(s, 0, 1);
+            product(s, 1, 0);
         }
-        slot = slot + 1 == S::STAGES ? 0 : slot + 1;
+        product(0, 0, 0);
+        product(1, 0, 0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (b + u >= blocks) break;
+#pragma unroll
+            for (int n = 0; n < TILES; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[n][i] = b + u == 0 ? d[u][n][i] : sum[n][i] + d[u][n][i];
+        }
     }
     copies_wait<0>();
-    __syncthreads();
-    float* sums = ring;                                   // [chain][m][weight row]
 #pragma unroll
-    for (int m = 0; m < MR; ++m) sums[(chain * MR + m) * S::WROWS + row] = acc[m];
+    for (int n = 0; n < TILES; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sums[chain][n * 8 + t * 2 + (i & 1)][g + (i >> 1) * 8] = sum[n][i];
     __syncthreads();
     const int chains = (K + part - 1) / part;
-    for (int i = tid; i < MR * ROW_FEATURES; i += S::THREADS) {
-        const int m = i / ROW_FEATURES, f = i % ROW_FEATURES;
-        if (m0 + m >= M || n0 + f >= N) continue;
-        float s = 0.f, u = 0.f;
-        for (int c = 0; c < chains; ++c) {
-            s += sums[(c * MR + m) * S::WROWS + f];
-            if (MODE == LP_GEMM_SWIGLU) u += sums[(c * MR + m) * S::WROWS + ROW_FEATURES + f];
-        }
-        float* out = C + (long long)(m0 + m) * ldc + n0 + f;
-        if (MODE == LP_GEMM_STORE) *out = s;
-        else if (MODE == LP_GEMM_ACCUMULATE) *out += s;
-        else *out = silu_mul(s, u);
-    }
-}
-
-// ---------------------------------------------------------------- float32, many rows
-// Two multiply-adds in one instruction, each rounded like fmaf: a plain fmaf per product leaves half of the units idle.
-typedef unsigned long long pair_t;
-__device__ __forceinline__ pair_t make_pair(float lo, float hi) {
-    pair_t p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
-    return p;
-}
-__device__ __forceinline__ float2 from_pair(pair_t p) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ pair_t fma_pair(pair_t a, pair_t b, pair_t c) {
-    pair_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
-constexpr int TILE_N = 128, TILE_K = 16;
-
-template <int ROWS> struct TileShape {
-    static constexpr int THREADS = ROWS * 2;              // 8 x 8 outputs each
-    static constexpr int LDA = ROWS + 4, LDW = TILE_N + 4;
-    static constexpr int STAGE = TILE_K * (LDA + LDW);    // floats; two stages
-    static constexpr int HELD = 64 * THREADS;             // floats: every thread's outputs, [16 groups of 4][thread]
-    static constexpr size_t SMEM = (size_t)(2 * STAGE + HELD) * sizeof(float);
-};
-
-// A thread forms rows {ty*4.., ROWS/2 + ty*4..} x columns {tx*4.., 64 + tx*4..} of a ROWS x 128 tile; in the gated form
-// the first 64 columns are gate rows of W and the last 64 the up rows of the same features, so a thread holds both.
-// SPLIT: the eight CTAs of a cluster form one chain each and add them up through distributed shared memory.
-// Bound by the multiply-add units (71 TFLOP/s measured for multiply-adds alone). B200, 509 rows: 16384 x 2048 (gated) 1272 ->
-// 821 us, 2048 x 8192 about 900 -> 407 us, 3072 x 2048 307 -> 164 us (42 TFLOP/s; 50 at 2048 rows, where the last wave is
-// fuller). The kernel above reads shared memory four bytes at a time and reaches 27.
-template <int ROWS, int MODE, bool SPLIT>
-__global__ void __launch_bounds__(ROWS * 2, ROWS == 128 ? 2 : 4)
-gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
-                     int lda, int ldw, int ldc) {
-    using S = TileShape<ROWS>;
-    extern __shared__ __align__(16) float smem[];
-    float* held = smem + 2 * S::STAGE;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
-    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? TILE_N / 2 : TILE_N;
-    const int n0 = blockIdx.x * FEATURES, m0 = blockIdx.y * ROWS;
-    const int part = part_length(K);
-    const int k_begin = SPLIT ? (int)blockIdx.z * part : 0;
-    const int k_end = SPLIT ? min(K, k_begin + part) : K;
-
-    // loads: 4 values along k of one row; lanes cover 8 rows x 16 k, so a row's 64 bytes are read together
-    constexpr int PASS = S::THREADS / 4;                  // rows per pass
-    constexpr int PA = ROWS / PASS, PW = TILE_N / PASS;
-    const int lr = tid >> 2, lk = (tid & 3) * 4;
-    const float* wrow[PW];
-    bool wok[PW];
-#pragma unroll
-    for (int i = 0; i < PW; ++i) {
-        const int c = lr + i * PASS;
-        const int f = MODE == LP_GEMM_SWIGLU ? n0 + (c & 63) : n0 + c;
-        wok[i] = f < N;
-        wrow[i] = W + (long long)(MODE == LP_GEMM_SWIGLU && c >= 64 ? N + f : f) * ldw;
-    }
-    float4 ra[PA], rw[PW];
-    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto fetch = [&](int k0) {
-        const int k = k0 + lk;
-#pragma unroll
-        for (int i = 0; i < PW; ++i) rw[i] = wok[i] && k < k_end ? *(const float4*)(wrow[i] + k) : none;
-#pragma unroll
-        for (int i = 0; i < PA; ++i) {
-            const int m = m0 + lr + i * PASS;
-            ra[i] = m < M && k < k_end ? *(const float4*)(A + (long long)m * lda + k) : none;
-        }
-    };
-    auto put = [&](int stage) {
-        float* as = smem + stage * S::STAGE;
-        float* ws = as + TILE_K * S::LDA;
-#pragma unroll
-        for (int i = 0; i < PA; ++i) {
-            const int r = lr + i * PASS;
-            as[(lk + 0) * S::LDA + r] = ra[i].x;
-            as[(lk + 1) * S::LDA + r] = ra[i].y;
-            as[(lk + 2) * S::LDA + r] = ra[i].z;
-            as[(lk + 3) * S::LDA + r] = ra[i].w;
-        }
-#pragma unroll
-        for (int i = 0; i < PW; ++i) {
-            const int c = lr + i * PASS;
-            ws[(lk + 0) * S::LDW + c] = rw[i].x;
-            ws[(lk + 1) * S::LDW + c] = rw[i].y;
-            ws[(lk + 2) * S::LDW + c] = rw[i].z;
-            ws[(lk + 3) * S::LDW + c] = rw[i].w;
-        }
-    };
-
-    pair_t acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-
-    lp_grid_wait();
-    lp_grid_release();
-    fetch(k_begin);
-    put(0);
-    __syncthreads();
-    int stage = 0;
-    bool first_part = true;
-    for (int k0 = k_begin; k0 < k_end; k0 += TILE_K) {
-        const bool more = k0 + TILE_K < k_end;
-        if (more) fetch(k0 + TILE_K);
-        const float* as = smem + stage * S::STAGE + ty * 4;
-        const float* ws = smem + stage * S::STAGE + TILE_K * S::LDA + tx * 4;
-#pragma unroll
-        for (int k = 0; k < TILE_K; ++k) {
-            const float4 a0 = *(const float4*)(as + k * S::LDA), a1 = *(const float4*)(as + k * S::LDA + ROWS / 2);
-            const ulonglong2 w0 = *(const ulonglong2*)(ws + k * S::LDW), w1 = *(const ulonglong2*)(ws + k * S::LDW + 64);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const pair_t a = make_pair(av[i], av[i]);
-                acc[i][0] = fma_pair(a, w0.x, acc[i][0]);
-                acc[i][1] = fma_pair(a, w0.y, acc[i][1]);
-                acc[i][2] = fma_pair(a, w1.x, acc[i][2]);
-                acc[i][3] = fma_pair(a, w1.y, acc[i][3]);
+    for (int e = tid; e < TOK * FEATURES; e += S::THREADS) {
+        const int m = e / FEATURES, f = e % FEATURES;
+        if (m >= M || n0 + f >= N) continue;
+        auto whole = [&](int r) {
+            float v = 0.f, first = 0.f;
+            for (int c = 0; c < chains; ++c) {
+                if (c == PARTS / 2) first = v;
+                v = c % (PARTS / 2) == 0 ? sums[c][m][r] : v + sums[c][m][r];
             }
-        }
-        if (!SPLIT && more && (k0 + TILE_K) % part == 0) {        // a chain ends: its sums join those held
-            float4* h = (float4*)held + tid;
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const float2 lo = from_pair(acc[i][2 * j]), hi = from_pair(acc[i][2 * j + 1]);
-                    float4 v = first_part ? none : h[(i * 2 + j) * S::THREADS];
-                    v.x += lo.x; v.y += lo.y; v.z += hi.x; v.w += hi.y;
-                    h[(i * 2 + j) * S::THREADS] = v;
-                    acc[i][2 * j] = acc[i][2 * j + 1] = 0ull;
-                }
-            first_part = false;
-        }
-        if (more) {
-            put(stage ^ 1);
-            __syncthreads();
-            stage ^= 1;
-        }
-    }
-
-    auto finish = [&](int i, float4 s0, float4 s1) {
-        const int m = m0 + (i < 4 ? ty * 4 + i : ROWS / 2 + ty * 4 + i - 4);
-        if (m >= M) return;
-        float* c = C + (long long)m * ldc;
-        auto store4 = [&](int n, const float4& v) {
-            const float x[4] = {v.x, v.y, v.z, v.w};
-            if (n + 3 < N && (ldc & 3) == 0 && ((size_t)C & 15) == 0) {
-                float4* to = (float4*)(c + n);
-                if (MODE == LP_GEMM_ACCUMULATE) {
-                    const float4 old = *to;
-                    *to = make_float4(old.x + x[0], old.y + x[1], old.z + x[2], old.w + x[3]);
-                } else {
-                    *to = v;
-                }
-                return;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (n + j < N) c[n + j] = MODE == LP_GEMM_ACCUMULATE ? c[n + j] + x[j] : x[j];
+            if (chains > PARTS / 2) v = first + v;
+            // a sum that is no finite number is formed again
+            return fabsf(v) < INFINITY ? v : row_product(A + (long long)m * lda, W + (long long)weight_row(r) * ldw, K);
         };
-        if (MODE == LP_GEMM_SWIGLU) {
-            store4(n0 + tx * 4, make_float4(silu_mul(s0.x, s1.x), silu_mul(s0.y, s1.y), silu_mul(s0.z, s1.z), silu_mul(s0.w, s1.w)));
-        } else {
-            store4(n0 + tx * 4, s0);
-            store4(n0 + 64 + tx * 4, s1);
-        }
-    };
-    float4* h = (float4*)held + tid;
-    if (SPLIT) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const float2 lo = from_pair(acc[i][2 * j]), hi = from_pair(acc[i][2 * j + 1]);
-                h[(i * 2 + j) * S::THREADS] = make_float4(lo.x, lo.y, hi.x, hi.y);
-            }
-        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-        cluster.sync();
-        const int i = blockIdx.z;                        // this CTA adds up one of the eight rows of every thread
-        float4 s[2] = {none, none};
-#pragma unroll
-        for (int c = 0; c < PARTS; ++c) {
-            const float4* from = (const float4*)cluster.map_shared_rank(held, c) + tid;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const float4 v = from[(i * 2 + j) * S::THREADS];
-                s[j].x += v.x; s[j].y += v.y; s[j].z += v.z; s[j].w += v.w;
-            }
-        }
-        finish(i, s[0], s[1]);
-        cluster.sync();                                  // nobody leaves while its sums are still read
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        float4 s[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const float2 lo = from_pair(acc[i][2 * j]), hi = from_pair(acc[i][2 * j + 1]);
-            s[j] = first_part ? none : h[(i * 2 + j) * S::THREADS];
-            s[j].x += lo.x; s[j].y += lo.y; s[j].z += hi.x; s[j].w += hi.y;
-        }
-        finish(i, s[0], s[1]);
+        float* out = C + (long long)m * ldc + n0 + f;
+        if (GATED) *out = silu_mul(whole(f), whole(FEATURES + f));
+        else if (MODE == LP_GEMM_ACCUMULATE) *out += whole(f);
+        else *out = whole(f);
     }
 }
 
@@ -472,37 +765,51 @@ int failed(cudaError_t err, const char* what) {
     return (int)err;
 }
 
-template <int MR, int MODE, bool DEEP>
-int launch_rows_as(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-    using S = RowsShape<MR, MODE, DEEP>;
-    auto kernel = gemm_f32_rows_kernel<MR, MODE, DEEP>;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    if (err != cudaSuccess) return failed(err, "rows");
-    dim3 grid((N + ROW_FEATURES - 1) / ROW_FEATURES, (M + MR - 1) / MR);
-    err = lp_launch(kernel, grid, dim3(S::THREADS), S::SMEM, stream, A, W, C, M, N, K, lda, ldw, ldc);
-    return err == cudaSuccess ? lp_check_launch("gemm_plain (rows)") : failed(err, "rows");
+// [rows, K] bfloat16, row stride ld, boxes of box_rows x 32 (64 bytes, swizzled)
+int make_map_rows64(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
+    EncodeTiled enc = encode_fn();
+    if (!enc) LP_REFUSE("gemm: the driver does not offer cuTensorMapEncodeTiled");
+    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    cuuint32_t box[2] = {(cuuint32_t)SPLIT_K, (cuuint32_t)box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) LP_REFUSE("gemm: cuTensorMapEncodeTiled failed with code %d for a [%lld, %lld] matrix of parts",
+                                     (int)r, rows, K);
+    return 0;
 }
 
-template <int MR, int MODE>
-int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-    const long long ctas = (long long)((N + ROW_FEATURES - 1) / ROW_FEATURES) * ((M + MR - 1) / MR);
-    if (MODE != LP_GEMM_SWIGLU && ctas <= 2 * lp_sm_count())
-        return launch_rows_as<MR, MODE, true>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    return launch_rows_as<MR, MODE, false>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-}
+struct F32Call {
+    const float *A, *W;
+    float* C;
+    int M, N, K, lda, ldw, ldc;
+    uint16_t* parts;           // room for the parts of A (lp_gemm_plain), or null
+    int* status;
+    cudaStream_t stream;
+};
 
-template <int ROWS, int MODE, bool SPLIT>
-int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-    using S = TileShape<ROWS>;
-    auto kernel = gemm_f32_tile_kernel<ROWS, MODE, SPLIT>;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    if (err != cudaSuccess) return failed(err, "tile");
-    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? TILE_N / 2 : TILE_N;
+template <int TOK, int MODE, bool SPLIT>
+int launch_split(const F32Call& c, int ctas) {
+    using T = SplitTile<TOK>;
+    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? 64 : 128;
+    CUtensorMap mw, mx;
+    int rc = make_map_f32(&mw, c.W, MODE == LP_GEMM_SWIGLU ? 2ll * c.N : c.N, c.K, c.ldw, FEATURES);
+    if (!rc) rc = make_map_rows64(&mx, c.parts, 3ll * c.M, c.K, (c.K + 7) / 8 * 8, TOK);
+    if (rc) return rc;
+    const long long pieces = (long long)c.M * (c.K / 4);
+    cudaError_t err = lp_launch(split_rows_kernel, (unsigned)min((pieces + 255) / 256, (long long)lp_sm_count() * 8), 256, 0, c.stream,
+                                c.A, c.parts, c.M, c.K, c.lda, (c.K + 7) / 8 * 8);
+    if (err != cudaSuccess) return failed(err, "parts");
+    auto kernel = gemm_f32_split_kernel<TOK, MODE, SPLIT>;
+    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
+    if (err != cudaSuccess) return failed(err, "float32");
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((N + FEATURES - 1) / FEATURES, (M + ROWS - 1) / ROWS, SPLIT ? PARTS : 1);
-    cfg.blockDim = dim3(S::THREADS);
-    cfg.dynamicSmemBytes = S::SMEM;
-    cfg.stream = stream;
+    cfg.gridDim = dim3((unsigned)((c.M + TOK - 1) / TOK) * ((c.N + FEATURES - 1) / FEATURES), 1, ctas);
+    cfg.blockDim = dim3(T::THREADS);
+    cfg.dynamicSmemBytes = T::SMEM;
+    cfg.stream = c.stream;
     cudaLaunchAttribute attr[2];
     int attrs = 0;
     if (lp_pdl_enabled()) {
@@ -513,33 +820,58 @@ int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, i
         attr[attrs].id = cudaLaunchAttributeClusterDimension;
         attr[attrs].val.clusterDim.x = 1;
         attr[attrs].val.clusterDim.y = 1;
-        attr[attrs++].val.clusterDim.z = PARTS;
+        attr[attrs++].val.clusterDim.z = ctas;
     }
     cfg.attrs = attr;
     cfg.numAttrs = attrs;
-    err = cudaLaunchKernelEx(&cfg, kernel, A, W, C, M, N, K, lda, ldw, ldc);
-    return err == cudaSuccess ? lp_check_launch("gemm_plain (tile)") : failed(err, "tile");
+    err = cudaLaunchKernelEx(&cfg, kernel, mw, mx, c.A, c.W, c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc, c.status);
+    return err == cudaSuccess ? lp_check_launch("gemm_plain (float32)") : failed(err, "float32");
+}
+
+template <int TOK, int MODE>
+int launch_tokens(const F32Call& c) {
+    using T = SplitTile<TOK>;
+    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? 64 : 128;
+    const long long tiles = (long long)((c.N + FEATURES - 1) / FEATURES) * ((c.M + TOK - 1) / TOK);
+    const long long blocks = (c.K + SPLIT_K - 1) / SPLIT_K;
+    // how many CTAs share a tile's chains: the number whose busiest SM has least to do, a CTA's beginning and end counted as eight blocks
+    int best = 1;
+    long long least = 0;
+    for (int ctas = 1; ctas <= PARTS; ctas *= 2) {
+        if (ctas > 1 && (c.K <= SPLIT_K * PARTS || (ctas > 2 && PARTS / ctas > T::SLOTS))) continue;
+        const long long each = (tiles * ctas + lp_sm_count() - 1) / lp_sm_count();            // CTAs of the busiest SM
+        const long long cost = each * ((blocks + ctas - 1) / ctas + 8);
+        if (ctas == 1 || cost < least) { best = ctas; least = cost; }
+    }
+    return best > 1 ? launch_split<TOK, MODE, true>(c, best) : launch_split<TOK, MODE, false>(c, 1);
+}
+
+template <int TOK, int MODE, bool DEEP>
+int launch_rows_as(const F32Call& c) {
+    using S = RowsShape<TOK, DEEP>;
+    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? ROW_FEATURES / 2 : ROW_FEATURES;
+    auto kernel = gemm_f32_rows_kernel<TOK, MODE, DEEP>;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (err == cudaSuccess)
+        err = lp_launch(kernel, dim3((c.N + FEATURES - 1) / FEATURES), dim3(S::THREADS), S::SMEM, c.stream, c.A, c.W, c.C, c.M, c.N, c.K,
+                        c.lda, c.ldw, c.ldc);
+    return err == cudaSuccess ? lp_check_launch("gemm_plain (rows)") : failed(err, "rows");
+}
+
+template <int TOK, int MODE>
+int launch_rows(const F32Call& c) {
+    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? ROW_FEATURES / 2 : ROW_FEATURES;
+    return (c.N + FEATURES - 1) / FEATURES <= lp_sm_count() ? launch_rows_as<TOK, MODE, true>(c) : launch_rows_as<TOK, MODE, false>(c);
 }
 
 template <int MODE>
-int launch_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    // up to 32 rows the weights' bytes bound the product (16 rows at a time; from 33 rows on the tile of 64 is faster:
-    // 16384 x 2048 gated, 32 / 48 rows: 130 / 129 us)
-    if (M <= 1) return launch_rows<1, MODE>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    if (M <= 2) return launch_rows<2, MODE>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    if (M <= 4) return launch_rows<4, MODE>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    if (M <= 8) return launch_rows<8, MODE>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    if (M <= 32) return launch_rows<16, MODE>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? TILE_N / 2 : TILE_N;
-    const bool tall = (M + 127) / 128 * 2 == (M + 63) / 64;       // the 128-row tile wastes no more rows than the 64-row one
-    const long long tiles = (long long)((N + FEATURES - 1) / FEATURES) * ((M + (tall ? 127 : 63)) / (tall ? 128 : 64));
-    // fewer tiles than two per SM: the chains side by side (64 tiles, 2048 x 2048 at 509 rows: 111 us in clusters)
-    const bool split = K > 32 * PARTS && tiles < 2 * lp_sm_count();
-    if (tall)
-        return split ? launch_tile<128, MODE, true>(A, W, C, M, N, K, lda, ldw, ldc, s)
-                     : launch_tile<128, MODE, false>(A, W, C, M, N, K, lda, ldw, ldc, s);
-    return split ? launch_tile<64, MODE, true>(A, W, C, M, N, K, lda, ldw, ldc, s)
-                 : launch_tile<64, MODE, false>(A, W, C, M, N, K, lda, ldw, ldc, s);
+int launch_f32(const F32Call& c) {
+    // up to 16 rows the weights' bytes bound the product; the tiles start at 34 us for 2048 x 2048 where 16 rows take 14
+    if (c.M <= 8) return launch_rows<8, MODE>(c);
+    if (c.M <= 16) return launch_rows<16, MODE>(c);
+    // from 65 rows on a tile of 128 splits the weights half as often (509 rows, gated: 232 us, 315 in tiles of 64)
+    if (c.M <= 64) return launch_tokens<64, MODE>(c);
+    return launch_tokens<128, MODE>(c);
 }
 
 template <typename TA, typename TW, typename TC>
@@ -565,11 +897,19 @@ int launch_out(const void* A, const void* W, void* C, int c_dtype, int M, int N,
     return launch_mode<TA, TW, __nv_bfloat16>(A, W, C, M, N, K, lda, ldw, ldc, mode, stream);
 }
 
+// rows of float32 that can be read 16 bytes at a time go to the tensor cores, everything else to the kernel for any types
+bool wide_f32(const void* A, int a_dtype, const void* W, int w_dtype, int c_dtype, int K, int lda, int ldw) {
+    return a_dtype == LP_F32 && w_dtype == LP_F32 && c_dtype == LP_F32 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0
+           && (size_t)A % 16 == 0 && (size_t)W % 16 == 0;
+}
+
 }  // namespace
 
+// scratch: room for 3 x M x (K rounded up to 8) bfloat16, 16-byte aligned, for float32 products of more than 16 rows on the tensor
+// cores (may be null: they then run on the kernel for any types).
 // A: [M, K] row stride lda; W: [N, K] (or [2N, K] in SWIGLU mode) row stride ldw; C: [M, N] row stride ldc.
 extern "C" int lp_gemm_plain(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int M,
-                             int N, int K, int lda, int ldw, int ldc, int mode, cudaStream_t stream) {
+                             int N, int K, int lda, int ldw, int ldc, int mode, void* scratch, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) LP_REFUSE("gemm_plain: inner size %d", K);
     if (mode < 0 || mode > 2) LP_REFUSE("gemm_plain: mode %d", mode);
@@ -578,14 +918,11 @@ extern "C" int lp_gemm_plain(const void* A, int a_dtype, const void* W, int w_dt
         LP_REFUSE("gemm_plain: accumulation needs a float32 output");
     if ((N + BN - 1) / BN > 2147483647 || (M + BM - 1) / BM > 65535)
         LP_REFUSE("gemm_plain: %d rows exceed the grid", M);
-    // rows of float32 that can be read 16 bytes at a time: the kernels made for that, others: the one for everything
-    const bool wide = a_dtype == LP_F32 && w_dtype == LP_F32 && c_dtype == LP_F32 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0
-                      && (size_t)A % 16 == 0 && (size_t)W % 16 == 0;
-    if (wide) {
-        const float *a = (const float*)A, *w = (const float*)W;
-        if (mode == LP_GEMM_STORE) return launch_f32<LP_GEMM_STORE>(a, w, (float*)C, M, N, K, lda, ldw, ldc, stream);
-        if (mode == LP_GEMM_ACCUMULATE) return launch_f32<LP_GEMM_ACCUMULATE>(a, w, (float*)C, M, N, K, lda, ldw, ldc, stream);
-        return launch_f32<LP_GEMM_SWIGLU>(a, w, (float*)C, M, N, K, lda, ldw, ldc, stream);
+    if (wide_f32(A, a_dtype, W, w_dtype, c_dtype, K, lda, ldw) && (M <= 16 || scratch)) {
+        const F32Call c{(const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc, (uint16_t*)scratch, status, stream};
+        if (mode == LP_GEMM_STORE) return launch_f32<LP_GEMM_STORE>(c);
+        if (mode == LP_GEMM_ACCUMULATE) return launch_f32<LP_GEMM_ACCUMULATE>(c);
+        return launch_f32<LP_GEMM_SWIGLU>(c);
     }
     if (a_dtype == LP_F32 && w_dtype == LP_F32)
         return launch_out<float, float>(A, W, C, c_dtype, M, N, K, lda, ldw, ldc, mode, stream);

@@ -51,7 +51,7 @@ _SIGNATURES = {
         "lp_identity_experts": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _P],
     },
     "gemm_plain": {
-        "lp_gemm_plain": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "lp_gemm_plain": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P],
     },
     "attention_plain": {
         "lp_attention_plain": [_P, _P, _I, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _F, _P, _I, _I, _P, _P, _P, _I, _P, _I, _P],
@@ -677,7 +677,7 @@ def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, angles: Optional[torch.Tenso
 
 # --------------------------------------------------------------------------- matrix products
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE) -> torch.Tensor:
-    """out (=|+=) a @ w.T with float32 multiply-adds, each element in one fixed order whatever the number of rows.
+    """out (=|+=) a @ w.T at float32 precision, each element in one fixed order whatever the number of rows.
 
     ``SWIGLU``: ``w`` is [2N, K], gate rows then up rows; out = silu(a gate^T) * (a up^T).
     """
@@ -690,8 +690,11 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = 
     if w.shape != (rows, K) or out.shape[0] != M:
         raise KernelError(f"gemm: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, mode {mode}")
     lib = library("gemm_plain")
+    scratch = None
+    if M > 16 and a.dtype == w.dtype == out.dtype == torch.float32:      # the rows' parts: three bfloat16 per value, rows of 16 bytes
+        scratch = torch.empty(3, M, (K + 7) // 8 * 8, dtype=torch.bfloat16, device=a.device)
     _check(lib, lib.lp_gemm_plain(a.data_ptr(), _code(a, "gemm a"), w.data_ptr(), _code(w, "gemm w"), out_ptr,
-                                  _code(out, "gemm out"), M, N, K, K, K, ldc, mode, _stream()))
+                                  _code(out, "gemm out"), M, N, K, K, K, ldc, mode, _ptr(scratch), kernel_status().data_ptr(), _stream()))
     return out
 
 
@@ -726,7 +729,7 @@ def check_kernel_status() -> None:
         raise KernelError(f"a tensor-core kernel gave up waiting on a barrier (code {code}: "
                           "1 = loader, 2 = MMA issuer, 3 = epilogue, 4-5 = operand maker; 2x the same in the "
                           "persistent product, 5x in the experts' (55: more choices than announced); "
-                          "6 = a page of the decode attention; 61 = a record of the chunked recurrence)")
+                          "6 = a page of the decode attention; 61 = a record of the chunked recurrence; 7x = the float32 product)")
 
 
 def _token_tile(tokens: int, gated: bool) -> int:

@@ -135,6 +135,36 @@ def test_float32_gemm_at_the_edges_of_its_kernels(mode, N, K):
             assert torch.equal(out[:M], whole[:M]) and bool((out[M] == 7.0).all()), M
 
 
+@pytest.mark.parametrize("M", [3, 12, 40, 200])
+@pytest.mark.parametrize("mode", ["store", "swiglu"])
+def test_float32_gemm_with_values_that_are_not_finite_in_parts(mode, M):
+    """Infinities, NaN, values at the end of the range and rows of very different sizes: infinite, not a number and finite exactly where
+    float64 rounded to float32 is; finite ones within the bound of sums of K products."""
+    from llmplayer_b200.kernels import ops
+    torch.manual_seed(M)
+    K, N = 520, 72
+    code = ops.SWIGLU if mode == "swiglu" else ops.STORE
+    a = torch.randn(M, K, device="cuda:0") * torch.exp2(torch.randint(-30, 30, (M, 1), device="cuda:0").float())
+    w = torch.randn(N * (2 if mode == "swiglu" else 1), K, device="cuda:0") * 1e-3
+    a[0, 7], a[1, 9], w[5, 8] = float("inf"), float("nan"), -float("inf")
+    a[2, 11] = 3.4e38
+    w[:, 11] *= 1e-3
+    out = torch.full((M, N), 7.0, device="cuda:0")
+    ops.gemm_plain(a, w, out, code)
+    sums = (a.double() @ w.double().T)
+    if mode == "swiglu":
+        g, u = sums[:, :N].float(), sums[:, N:].float()          # what is infinite as a float32 sum
+        ref = (g / (1 + torch.exp(-g)) * u).double()
+    else:
+        ref = sums
+    ref32 = ref.float()
+    assert torch.equal(torch.isnan(out), torch.isnan(ref32))
+    assert torch.equal(torch.isinf(out), torch.isinf(ref32))
+    if mode == "store":
+        fine = torch.isfinite(ref32)
+        bound = (K + 9) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+        assert bool(((out.double() - ref).abs() <= bound)[fine].all())
+
 def test_refusals():
     from llmplayer_b200.errors import KernelError
     from llmplayer_b200.kernels import ops
