@@ -34,6 +34,7 @@ constexpr int THREADS = 256;            // of the first kernel
 constexpr int JOINERS = CT / 8;         // warps of the second kernel beside one per 16 key channels: one per 8 tokens
 constexpr int MAX_DK = 256;
 constexpr int CARRY_THREADS = 32 * (MAX_DK / 16 + JOINERS);      // at most
+constexpr int NARROW_DK = 128, CARRY_THREADS_NARROW = 32 * (NARROW_DK / 16 + JOINERS);
 constexpr size_t MAX_SMEM = 227 * 1024 - 64;      // beside the barriers
 
 constexpr int DECAY_CHANNEL = 0, DECAY_HEAD = 1, DECAY_FIXED = 2;
@@ -358,25 +359,26 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
     lo = (__float_as_uint(x - __uint_as_float(hi)) + 0x1000u) & 0xffffe000u;
 }
 __device__ __forceinline__ void mma_tf32(float* c, const uint32_t* a, const uint32_t* b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// acc += X Y over two steps of 8, X [16 x 16] split as row operands (xh, xl), Y [16 x 8] as one fragment of a record; three
-// chains of sums
-__device__ __forceinline__ void product(float (*acc)[4], const uint32_t (*xh)[4], const uint32_t (*xl)[4], float4 y) {
-    uint32_t h[4], l[4];
-    split_tf32(y.x, h[0], l[0]);
-    split_tf32(y.y, h[1], l[1]);
-    split_tf32(y.z, h[2], l[2]);
-    split_tf32(y.w, h[3], l[3]);
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        mma_tf32(acc[0], xh[w], h + 2 * w);
-        mma_tf32(acc[1], xh[w], l + 2 * w);
-        mma_tf32(acc[2], xl[w], h + 2 * w);
+// A fragment of a record, split as the column operand of two steps of 8
+struct Columns {
+    uint32_t hi[4], lo[4];
+    __device__ __forceinline__ explicit Columns(float4 y) {
+        split_tf32(y.x, hi[0], lo[0]);
+        split_tf32(y.y, hi[1], lo[1]);
+        split_tf32(y.z, hi[2], lo[2]);
+        split_tf32(y.w, hi[3], lo[3]);
     }
+};
+template <int N> struct Count { static constexpr int value = N; };
+// acc += step w of X Y, X [16 x 16] split as row operands (xh, xl), Y [16 x 8]; three chains of sums
+__device__ __forceinline__ void product(float (*acc)[4], const uint32_t (*xh)[4], const uint32_t (*xl)[4], const Columns& y, int w) {
+    mma_tf32(acc[0], xh[w], y.hi + 2 * w);
+    mma_tf32(acc[1], xh[w], y.lo + 2 * w);
+    mma_tf32(acc[2], xl[w], y.hi + 2 * w);
 }
 __device__ __forceinline__ float4 chains(const float (*acc)[4]) {
     return make_float4(acc[0][0] + (acc[1][0] + acc[2][0]), acc[0][1] + (acc[1][1] + acc[2][1]), acc[0][2] + (acc[1][2] + acc[2][2]),
@@ -386,28 +388,36 @@ __device__ __forceinline__ float4 chains(const float (*acc)[4]) {
 // All products are taken transposed (value columns are their 16 rows). Worker m holds S^T for the key channels 16 m .. 16 m + 15
 // in registers, which are the row operand of its share of (W S)^T and (Q S)^T as they lie; the shares meet in shared memory.
 // Joiner n has the tokens 8 n .. 8 n + 7: it requests the records, makes U^T = (U0 - W S)^T (split, as the row operand of what
-// follows) while the workers multiply with Q, and adds (B U)^T to the shares of (Q S)^T and writes the outputs while they
-// update the state. Bound by the chain of a chunk's steps, with three barriers for the delta rule and two without it (U is V
-// then). With the state split in shared memory, read as column operands and stored again in every chunk, 2048 tokens of 8 heads
-// of 128 x 256 took 114 us on a B200, and 97 so; with bulk copies in place of 16 bytes per thread and request, which went through
-// the load unit that the fragments come through, 90 (three prompts of 518 to 777 tokens, 8 heads of 128 x 128, delta rule: 88 ->
-// 71). What is left are the shares' and the state's products, 8 cycles of a quarter SM for each of 432 (delta rule: 624) per
-// chunk, one behind the other.
-// STAGES: records in flight (three, or fewer where they do not fit shared memory; then a barrier frees the stage).
-template <int STAGES>
-__global__ void __launch_bounds__(CARRY_THREADS)
+// follows) and the outputs of its tokens from the shares of (Q S)^T and (B U)^T.
+// The plain recurrence's chain is the state alone (U is V), with one barrier per chunk: behind it the workers take their shares
+// of Q S and go on to the next state, while the joiners write the chunk before (its shares lie in the other half of a double
+// buffer), form B U and split the next chunk's values (likewise). The delta rule's chain goes through U, with two barriers: the
+// workers' shares of W S; U^T from them, while the workers take their shares of Q S; the next state, while the outputs are
+// written, which may last into the next chunk's shares of W S.
+// 2048 tokens of 8 heads of 128 x 256, B200: 114 us with the state split in shared memory, read as column operands and stored again
+// in every chunk; 97 with it in registers; 90 with bulk copies in place of 16 bytes per thread and request, which went through the
+// load unit that the fragments come through; 82 with one barrier in place of two and a warp's reads, splits and products of a
+// chunk side by side (three prompts of 518 to 777 tokens, 8 heads of 128 x 128, delta rule: 88, -, 71, 68 with two barriers in
+// place of three). What is left, per chunk of 1.28 us: 864 cycles of the tensor cores (8 per product and quarter SM), some 1,180
+// of shared memory and 780 issue slots, partly one behind the other in the two workers of a quarter SM; with the records not
+// copied at all it takes 74 us, so neither L2 nor the copies bound it.
+// STAGES: records in flight (three, or fewer where they do not fit shared memory; with fewer the delta rule frees a stage by a
+// barrier at a chunk's end).
+// WIDE: more than 128 key channels, and more warps with fewer registers each.
+template <int STAGES, bool DELTA, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? CARRY_THREADS : CARRY_THREADS_NARROW)
 carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ q_start, int first_chunk, int chunks,
              const float* __restrict__ records, const float* __restrict__ values, float* __restrict__ out, int H, int dk, int dv,
-             int delta, int* __restrict__ status) {
+             int* __restrict__ status) {
+    static_assert(DELTA || STAGES >= 2, "the plain recurrence reads the next chunk's values during a chunk");
     extern __shared__ __align__(16) float sm[];
     __shared__ uint64_t full[STAGES];                   // a stage's record is there
-    const int dkp = padded(dk), rec_n = record_floats(dkp, delta != 0), kt = dkp >> 4;
-    uint4* Uh = reinterpret_cast<uint4*>(sm);            // [JOINERS][32 lanes] twice: U^T as row operands, its two parts
-    uint4* Ul = Uh + JOINERS * 32;
-    float4* parts_q = reinterpret_cast<float4*>(Ul + JOINERS * 32);      // [kt][JOINERS][32 lanes], and again for W
-    float4* parts_w = parts_q + kt * JOINERS * 32;
-    float* ring = reinterpret_cast<float*>(parts_w + (delta ? kt * JOINERS * 32 : 0));      // STAGES records, each followed by
-                                                         // the chunk's 32 x 16 values
+    const int dkp = padded(dk), rec_n = record_floats(dkp, DELTA), kt = dkp >> 4;
+    uint4* Us = reinterpret_cast<uint4*>(sm);            // [2 unless DELTA][JOINERS][32 lanes] twice: U^T as row operands, its two parts
+    float4* parts_q = reinterpret_cast<float4*>(Us + (DELTA ? 2 : 4) * JOINERS * 32);      // [kt][JOINERS][32 lanes], and again
+    float4* parts_w = parts_q + kt * JOINERS * 32;       // for W, or for the odd chunks
+    float* ring = reinterpret_cast<float*>(parts_w + kt * JOINERS * 32);      // STAGES records, each followed by the chunk's
+                                                         // 32 x 16 values
     const int stage = rec_n + CT * NC;
     lp_grid_release();
     lp_grid_wait();
@@ -435,9 +445,9 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // a stage that the previous chunk has left takes the next record when a chunk begins; with fewer than three stages a
-    // chunk's own stage does when it ends
-    constexpr bool EARLY = STAGES >= 3;
+    // a stage that every warp has left takes the next record during a chunk; with fewer than three stages the delta rule's own
+    // stage does when the chunk ends
+    constexpr bool EARLY = !DELTA || STAGES >= 3;
     if (joins) {
 #pragma unroll
         for (int p = 0; p < (EARLY ? STAGES - 1 : STAGES); ++p) request(p);
@@ -452,6 +462,34 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             s[w][e] = (!joins && column(e) < dv && channel(w, e) < dk) ? row[(size_t)column(e) * dk + channel(w, e)] : 0.f;
+    uint32_t sh[2][4], sl[2][4];
+    auto split_state = [&] {
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            split_tf32(s[w][0], sh[w][0], sl[w][0]);
+            split_tf32(s[w][2], sh[w][1], sl[w][1]);
+            split_tf32(s[w][1], sh[w][2], sl[w][2]);
+            split_tf32(s[w][3], sh[w][3], sl[w][3]);
+        }
+    };
+    constexpr int TOGETHER = WIDE ? 1 : JOINERS;     // of a worker's products: their reads, splits and sums overlap
+    // a worker's share of (X S)^T for the matrix X of a record
+    auto share = [&](const float* x, float4* parts) {
+        const float4* at = reinterpret_cast<const float4*>(x) + warp * 32 + lane;
+#pragma unroll
+        for (int i0 = 0; i0 < JOINERS; i0 += TOGETHER) {
+            float4 y[TOGETHER];
+#pragma unroll
+            for (int i = 0; i < TOGETHER; ++i) y[i] = at[(i0 + i) * kt * 32];
+            float acc[TOGETHER][3][4] = {};
+#pragma unroll
+            for (int w = 0; w < 2; ++w)
+#pragma unroll
+                for (int i = 0; i < TOGETHER; ++i) product(acc[i], sh, sl, Columns(y[i]), w);
+#pragma unroll
+            for (int i = 0; i < TOGETHER; ++i) parts[(warp * JOINERS + i0 + i) * 32 + lane] = chains(acc[i]);
+        }
+    };
     // the shares of 8 tokens, added in order
     auto gather = [&](const float4* parts) {
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -463,100 +501,133 @@ carry_kernel(float* __restrict__ state, const int* __restrict__ slots, const int
         }
         return sum;
     };
-    for (int p = 0; p < used; ++p) {
-        const bool there = mbar_wait(&full[p % STAGES], (p / STAGES) & 1);
-        if (!__syncthreads_and(there)) {            // the chunk before is done; a wait that ran out ends the block
-            if (tid == 32 * kt) {
-                atomicExch(status, 61);
-                for (int i = p + 1; i < min(used, p + (EARLY ? STAGES - 1 : STAGES)); ++i) mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
-            }
-            return;
+    // a joiner's 8 tokens of U^T: the values less `sum`
+    auto join = [&](const float* val, float4 sum, uint4* u) {
+        const float* at = val + (n * 8 + t4 * 2) * NC + g8;
+        uint4 hi, lo;
+        split_tf32(at[0] - sum.x, hi.x, lo.x);
+        split_tf32(at[NC] - sum.y, hi.z, lo.z);
+        split_tf32(at[8] - sum.z, hi.y, lo.y);
+        split_tf32(at[NC + 8] - sum.w, hi.w, lo.w);
+        u[n * 32 + lane] = hi;
+        u[(JOINERS + n) * 32 + lane] = lo;
+    };
+    // acc[i] += U^T Y_i over the tokens 16 q .. 16 q + 15, for `count` fragment columns Y_i
+    auto times_u = [&](auto count, float (*acc)[3][4], const uint4* u, const float* frag, int q) {
+        constexpr int COUNT = decltype(count)::value;
+        uint32_t uh[2][4], ul[2][4];
+        float4 y[COUNT];
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) y[i] = reinterpret_cast<const float4*>(frag)[(2 * i + q) * 32 + lane];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const uint4 hi = u[(2 * q + w) * 32 + lane], lo = u[(JOINERS + 2 * q + w) * 32 + lane];
+            uh[w][0] = hi.x; uh[w][1] = hi.y; uh[w][2] = hi.z; uh[w][3] = hi.w;
+            ul[w][0] = lo.x; ul[w][1] = lo.y; ul[w][2] = lo.z; ul[w][3] = lo.w;
         }
-        const float* rec = ring + (p % STAGES) * stage;
-        const float* rec_q = rec + (delta ? CT * dkp : 0);
-        const float* rec_k = rec_q + CT * dkp;
-        const float* rec_b = rec_k + CT * dkp;
-        const float* rec_p = rec_b + CT * CT;
-        const float* val = rec + rec_n;
-        uint32_t sh[2][4], sl[2][4];
-        // a worker's share of (X S)^T for the matrix X of a record
-        auto share = [&](const float* x, float4* parts) {
-            const float4* at = reinterpret_cast<const float4*>(x) + warp * 32 + lane;
 #pragma unroll
-            for (int i = 0; i < JOINERS; ++i) {
-                float acc[3][4] = {};
-                product(acc, sh, sl, at[i * kt * 32]);
-                parts[(warp * JOINERS + i) * 32 + lane] = chains(acc);
-            }
-        };
-        // a joiner's 8 tokens of U^T: the values less `sum`
-        auto join = [&](float4 sum) {
-            const float* at = val + (n * 8 + t4 * 2) * NC + g8;
-            uint4 hi, lo;
-            split_tf32(at[0] - sum.x, hi.x, lo.x);
-            split_tf32(at[NC] - sum.y, hi.z, lo.z);
-            split_tf32(at[8] - sum.z, hi.y, lo.y);
-            split_tf32(at[NC + 8] - sum.w, hi.w, lo.w);
-            Uh[n * 32 + lane] = hi;
-            Ul[n * 32 + lane] = lo;
-        };
-        if (!joins) {
+        for (int w = 0; w < 2; ++w)
 #pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                split_tf32(s[w][0], sh[w][0], sl[w][0]);
-                split_tf32(s[w][2], sh[w][1], sl[w][1]);
-                split_tf32(s[w][1], sh[w][2], sl[w][2]);
-                split_tf32(s[w][3], sh[w][3], sl[w][3]);
-            }
-            if (delta) share(rec, parts_w);
-        } else if (delta && EARLY) {
-            request(p + STAGES - 1);
-        }
-        if (delta) __syncthreads();                 // the shares of W S are there
-        if (!joins) {
-            share(rec_q, parts_q);
-        } else {
-            join(delta ? gather(parts_w) : make_float4(0.f, 0.f, 0.f, 0.f));
-            if (!delta && EARLY) request(p + STAGES - 1);
-        }
-        __syncthreads();                            // U and the shares of Q S are there
-        auto times_u = [&](float (*acc)[4], const float* frag, int q) {      // acc += U^T Y over the tokens 16 q .. 16 q + 15
-            uint32_t uh[2][4], ul[2][4];
+            for (int i = 0; i < COUNT; ++i) product(acc[i], uh, ul, Columns(y[i]), w);
+    };
+    auto move_state = [&](const uint4* u, const float* rec_k, const float* rec_p) {
+        float up[2][3][4] = {};
 #pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const uint4 hi = Uh[(2 * q + w) * 32 + lane], lo = Ul[(2 * q + w) * 32 + lane];
-                uh[w][0] = hi.x; uh[w][1] = hi.y; uh[w][2] = hi.z; uh[w][3] = hi.w;
-                ul[w][0] = lo.x; ul[w][1] = lo.y; ul[w][2] = lo.z; ul[w][3] = lo.w;
-            }
-            product(acc, uh, ul, reinterpret_cast<const float4*>(frag)[q * 32 + lane]);
-        };
-        if (!joins) {
-            float up[2][3][4] = {};
+        for (int q = 0; q < 2; ++q) times_u(Count<2>{}, up, u, rec_k + warp * 4 * 128, q);
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
-#pragma unroll
-                for (int w = 0; w < 2; ++w) times_u(up[w], rec_k + (warp * 2 + w) * 2 * 128, q);
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const float2 decay = *reinterpret_cast<const float2*>(rec_p + channel(w, 0));
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    s[w][e] = fmaf(e & 1 ? decay.y : decay.x, s[w][e], up[w][0][e] + (up[w][1][e] + up[w][2][e]));
-            }
-        } else {                                    // the outputs of 8 tokens: B U joins Q S
-            float acc[3][4] = {};
-#pragma unroll
-            for (int q = 0; q < 2; ++q) times_u(acc, rec_b + n * 2 * 128, q);
-            const float4 o = gather(parts_q), u = chains(acc);
-            const float x[4] = {o.x + u.x, o.y + u.y, o.z + u.z, o.w + u.w};
-            const int t = begin + p * CT + n * 8 + t4 * 2;
+        for (int w = 0; w < 2; ++w) {
+            const float2 decay = *reinterpret_cast<const float2*>(rec_p + channel(w, 0));
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (t + (e & 1) < t1 && column(e) < dv) out[((size_t)(t + (e & 1)) * H + h) * dv + column(e)] = x[e];
+                s[w][e] = fmaf(e & 1 ? decay.y : decay.x, s[w][e], up[w][0][e] + (up[w][1][e] + up[w][2][e]));
         }
-        if (!EARLY) {
-            __syncthreads();                        // the stage is free
-            if (joins) request(p + STAGES);
+    };
+    // a joiner's 8 tokens of chunk p's outputs: the shares of Q S and B U
+    auto write_out = [&](int p, float4 o, float4 u) {
+        const float x[4] = {o.x + u.x, o.y + u.y, o.z + u.z, o.w + u.w};
+        const int t = begin + p * CT + n * 8 + t4 * 2;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (t + (e & 1) < t1 && column(e) < dv) out[((size_t)(t + (e & 1)) * H + h) * dv + column(e)] = x[e];
+    };
+    // a wait that ran out ends the block: its own copies in flight are waited for first
+    auto give_up = [&](int p) {
+        if (tid != 32 * kt) return;
+        atomicExch(status, 61);
+        for (int i = p + 1; i < min(used, p + (EARLY ? STAGES - 1 : STAGES)); ++i) mbar_wait(&full[i % STAGES], (i / STAGES) & 1);
+    };
+    auto wait = [&](int p) { return mbar_wait(&full[p % STAGES], (p / STAGES) & 1); };
+    auto record = [&](int p) { return ring + (p % STAGES) * stage; };
+    constexpr int U_CHUNK = 2 * JOINERS * 32;
+    if constexpr (!DELTA) {
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool there = true;
+        float4 held = none;                          // a joiner's share of B U until the chunk's shares of Q S are there
+        if (joins) {
+            there = wait(0);
+            join(record(0) + rec_n, none, Us);
+        }
+        for (int p = 0; p < used; ++p) {
+            there = wait(p) && there;
+            if (!__syncthreads_and(there)) {         // the chunk before is done, this one's values are split
+                give_up(p);
+                return;
+            }
+            const float* rec_k = record(p) + CT * dkp;
+            const float* rec_b = rec_k + CT * dkp;
+            const uint4* u = Us + (p & 1) * U_CHUNK;
+            if (!joins) {
+                split_state();
+                share(record(p), p & 1 ? parts_w : parts_q);
+                move_state(u, rec_k, rec_b + CT * CT);
+            } else {
+                request(p + STAGES - 1);
+                if (p > 0) write_out(p - 1, gather(p & 1 ? parts_q : parts_w), held);
+                float acc[1][3][4] = {};
+#pragma unroll
+                for (int q = 0; q < 2; ++q) times_u(Count<1>{}, acc, u, rec_b + n * 2 * 128, q);
+                held = chains(acc[0]);
+                if (p + 1 < used) {
+                    there = wait(p + 1);
+                    join(record(p + 1) + rec_n, none, Us + ((p + 1) & 1) * U_CHUNK);
+                }
+            }
+        }
+        __syncthreads();
+        if (joins) write_out(used - 1, gather((used - 1) & 1 ? parts_w : parts_q), held);
+    } else {
+        for (int p = 0; p < used; ++p) {
+            const bool there = wait(p);
+            const float* rec_q = record(p) + CT * dkp;
+            const float* rec_k = rec_q + CT * dkp;
+            const float* rec_b = rec_k + CT * dkp;
+            if (!joins) {
+                split_state();
+                if (there) share(record(p), parts_w);
+            }
+            if (!__syncthreads_and(there)) {         // the shares of W S are there, and the chunk before is done
+                give_up(p);
+                return;
+            }
+            if (!joins) {
+                share(rec_q, parts_q);
+            } else {
+                join(record(p) + rec_n, gather(parts_w), Us);
+                if (EARLY) request(p + STAGES - 1);
+            }
+            __syncthreads();                         // U and the shares of Q S are there
+            if (!joins) {
+                move_state(Us, rec_k, rec_b + CT * CT);
+            } else {
+                float acc[1][3][4] = {};
+#pragma unroll
+                for (int q = 0; q < 2; ++q) times_u(Count<1>{}, acc, Us, rec_b + n * 2 * 128, q);
+                write_out(p, gather(parts_q), chains(acc[0]));
+            }
+            if (!EARLY) {
+                __syncthreads();                     // the stage is free
+                if (joins) request(p + STAGES);
+            }
         }
     }
 #pragma unroll
@@ -607,16 +678,20 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
     const size_t smem_p = ((size_t)(3 * CT + 3 * HB) * (dkp + 4) + 2 * CT * CT + CT) * sizeof(float);
     const size_t stage = (size_t)(record_floats(dkp, delta) + CT * NC) * sizeof(float);
     const int kt = dkp / 16;
-    const size_t kept = (size_t)(2 + kt * (delta ? 2 : 1)) * JOINERS * 32 * sizeof(float4);
-    const int stages = kept + 3 * stage <= MAX_SMEM ? 3 : kept + 2 * stage <= MAX_SMEM ? 2 : 1;
+    const size_t kept = (size_t)((delta ? 2 : 4) + kt * 2) * JOINERS * 32 * sizeof(float4);
+    const int stages = kept + 3 * stage <= MAX_SMEM ? 3 : kept + 2 * stage <= MAX_SMEM ? 2 : 1;      // (plain: two at least)
     const size_t smem_c = kept + stages * stage;
     auto prepare = dk <= 64 ? prepare_kernel<4> : dk <= 128 ? prepare_kernel<8> : prepare_kernel<16>;
     const int size = dk <= 64 ? 0 : dk <= 128 ? 1 : 2;
-    auto carry = stages == 3 ? carry_kernel<3> : stages == 2 ? carry_kernel<2> : carry_kernel<1>;
-    static size_t granted_p[3] = {}, granted_c[3] = {};       // what each kernel has been allowed so far
+    const bool wide = dkp > NARROW_DK;                        // (narrow: three stages always fit)
+    auto carry = delta ? (!wide ? carry_kernel<3, true, false> : stages == 3 ? carry_kernel<3, true, true>
+                          : stages == 2 ? carry_kernel<2, true, true> : carry_kernel<1, true, true>)
+                       : (!wide ? carry_kernel<3, false, false> : stages == 3 ? carry_kernel<3, false, true>
+                                                                              : carry_kernel<2, false, true>);
+    static size_t granted_p[3] = {}, granted_c[2][4] = {};       // what each kernel has been allowed so far
     int rc = reserve(prepare, smem_p, granted_p[size]);
     if (rc) return rc;
-    rc = reserve(carry, smem_c, granted_c[stages - 1]);
+    rc = reserve(carry, smem_c, granted_c[delta][wide ? stages : 0]);
     if (rc) return rc;
     const int total = (max_new + CT - 1) / CT;
     for (int first = 0; first < total; first += chunks) {
@@ -625,7 +700,7 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
         rc = lp_check_launch("chunked_recurrence (prepare)");
         if (rc) return rc;
         lp_launch(carry, dim3((dv + NC - 1) / NC, H, B), 32 * (kt + JOINERS), smem_c, stream, state, slots, q_start, first, chunks,
-                  (const float*)records, (const float*)values, out, H, dk, dv, delta, status);
+                  (const float*)records, (const float*)values, out, H, dk, dv, status);
         rc = lp_check_launch("chunked_recurrence (carry)");
         if (rc) return rc;
     }
