@@ -7,6 +7,7 @@ behind them: without a GPU and the compiled library they raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_void_p
 from dataclasses import dataclass
 from typing import Dict, Optional
@@ -383,6 +384,9 @@ def _code(t: torch.Tensor, what: str) -> int:
 
 
 def _want(t: torch.Tensor, what: str, dtype=None, ndim: Optional[int] = None) -> torch.Tensor:
+    if (isinstance(t, torch.Tensor) and t.is_cuda and (dtype is None or t.dtype is dtype) and (ndim is None or t.dim() == ndim)
+            and t.is_contiguous()):
+        return t
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{what}: expected a CUDA tensor")
     if dtype is not None and t.dtype != dtype:
@@ -757,12 +761,17 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 def gemm_plan(tokens: int, features: int, k: int, mode: int):
     """(token tile, splits) that :func:`gemm` uses for these sizes."""
+    return _gemm_plan(tokens, features, k, mode, num_sms())
+
+
+# (the two rules are asked several times for each product: working them out again took 3 us of the 14 that a product's call costs)
+@functools.lru_cache(maxsize=1024)
+def _gemm_plan(tokens: int, features: int, k: int, mode: int, sms: int):
     k_blocks = -(-k // 64)
     tile = _token_tile(tokens, mode == SWIGLU)
     if mode == SWIGLU:
         return tile, 1
     ctas = -(-features // 128) * -(-tokens // tile)
-    sms = num_sms()
     if ctas >= sms // 2 or k_blocks < 8:
         return tile, 1
     if mode == STORE and tokens >= PERSISTENT_MIN_TOKENS and k <= ORDERED_MAX_K:
@@ -781,7 +790,8 @@ ORDERED_MAX_K = 1024                # up to here for every storing product of fe
 ORDERED_MAX_K_UNCLEARED = 2048      # and up to here where nobody has cleared the output
 
 
-def _persistent_pays(tokens: int, features: int, k: int, mode: int) -> bool:
+@functools.lru_cache(maxsize=1024)
+def _persistent_pays(tokens: int, features: int, k: int, mode: int, sms: int) -> bool:
     """Whether the persistent form (one CTA per SM walking 128 x 256 tiles, 128 x 128 x 2 when gated)
     beats separate CTAs of 128 x 128 tiles, two to an SM. For the gated product: where it fills the SMs at least as well.
     The others: with tiles for at most a quarter of the SMs, separate CTAs with K shared out use more of the chip (us on a B200,
@@ -793,7 +803,6 @@ def _persistent_pays(tokens: int, features: int, k: int, mode: int) -> bool:
     1024 x 2048 x 1024 11.0 / 10.6)."""
     feat_tiles = -(-features // 128)
     persistent_tiles = feat_tiles * -(-tokens // (128 if mode == SWIGLU else 256))
-    sms = num_sms()
     if mode != SWIGLU:
         return persistent_tiles * 4 > sms and (mode == ACCUMULATE or k >= 4096 or persistent_tiles * 2 > sms)
     separate_ctas = feat_tiles * -(-tokens // 128)
@@ -806,7 +815,7 @@ def _persistent_pays(tokens: int, features: int, k: int, mode: int) -> bool:
 
 def gemm_persistent(tokens: int, features: int, k: int, mode: int) -> bool:
     """Whether :func:`gemm`, left to choose, takes the persistent form for these sizes."""
-    return tokens >= PERSISTENT_MIN_TOKENS and _persistent_pays(tokens, features, k, mode)
+    return tokens >= PERSISTENT_MIN_TOKENS and _persistent_pays(tokens, features, k, mode, num_sms())
 
 
 def gemm_adds_parts(tokens: int, features: int, k: int) -> bool:
@@ -1349,6 +1358,14 @@ def latent_absorb(q: torch.Tensor, k_up: torch.Tensor, out: torch.Tensor, *, nop
     return out
 
 
+@functools.lru_cache(maxsize=64)
+def _latent_attend_tile(kv_code: int, rank: int, rope_dim: int, page_size: int):
+    """(rows per CTA, keys per block) of the kernel that :func:`latent_attend` runs."""
+    lib = library("latent_attention")
+    sizes = (kv_code, rank, rope_dim, page_size)
+    return lib.lp_latent_attend_rows(*sizes), lib.lp_latent_attend_keys(*sizes)
+
+
 def latent_shares(batch: int, max_new: int, num_heads: int, table_width: int, page_size: int, pages: Optional[torch.Tensor] = None,
                   kv_rank: int = 0, window: Optional[int] = None) -> int:
     """Into how many shares :func:`latent_attend` cuts a sequence's keys: one while the (token, head) rows
@@ -1356,9 +1373,7 @@ def latent_shares(batch: int, max_new: int, num_heads: int, table_width: int, pa
     ``kv_rank`` say which kernel will run (its rows per CTA and keys per block); ``window``: no row sees more keys."""
     rows, keys = 32, 32
     if pages is not None:
-        sizes = (_code(pages, "latent_attend pages"), kv_rank, pages.shape[2] - kv_rank, page_size)
-        lib = library("latent_attention")
-        rows, keys = lib.lp_latent_attend_rows(*sizes), lib.lp_latent_attend_keys(*sizes)
+        rows, keys = _latent_attend_tile(_code(pages, "latent_attend pages"), kv_rank, pages.shape[2] - kv_rank, page_size)
     ctas = batch * -(-max_new * num_heads // rows)
     blocks = table_width * (page_size // keys)
     if window is not None:
