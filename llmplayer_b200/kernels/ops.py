@@ -19,6 +19,7 @@ from . import build
 
 F32, BF16 = 0, 1
 STORE, ACCUMULATE, SWIGLU = 0, 1, 2
+NOT_SERVED = 1          # what an entry of fused work returns for sizes that go through the separate kernels (nothing was launched)
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
 
 _P, _I, _F = c_void_p, c_int, c_float
@@ -28,6 +29,7 @@ _SIGNATURES = {
         "lp_layernorm": [_P, _P, _P, _P, _I, _I, _I, _F, _P, ctypes.c_longlong, _P],
         "lp_scaled_sum": [_P, _P, _P, _F, _P, _P, _F, _I, _I, _P],
         "lp_xielu": [_P, _I, _P, _P, _I, _I, _I, _P, ctypes.c_longlong, _P],
+        "lp_gated_sum_norm": [_P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _F, _P, _I, _P],
         "lp_gated_sum": [_P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
         "lp_rmsnorm": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _F, _P, ctypes.c_longlong, _I, _P],
         "lp_rope_cache_write": [_P, _I, _P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
@@ -522,11 +524,12 @@ def xielu(z: torch.Tensor, pq: torch.Tensor, out: torch.Tensor, clear: Optional[
 
 def gated_sum(x: torch.Tensor, a: Optional[torch.Tensor], a_gate=None, b: Optional[torch.Tensor] = None, b_gate=None, *,
               streams: Optional[torch.Tensor] = None, mix: Optional[torch.Tensor] = None, count: int = 0,
-              keep_input: bool = False) -> torch.Tensor:
+              keep_input: bool = False, norm_after=None) -> torch.Tensor:
     """x <- x + a * sigmoid(ga + ba) + b * sigmoid(gb + bb), float32, in place. ``a_gate`` / ``b_gate``:
     ``(logits [T, d], may be a column slice; bias [d] or None)`` or None for an ungated branch; ``b`` may be None.
     ``streams`` [>= count, T, d] with ``mix`` [count]: the sum is kept as stream ``count - 1`` and x becomes
-    sum_j mix[j] * streams[j]; ``keep_input`` first stores the incoming x as stream ``count - 2``."""
+    sum_j mix[j] * streams[j]; ``keep_input`` first stores the incoming x as stream ``count - 2``. ``norm_after`` =
+    (gain, eps, out): the layer norm of the new x is written to ``out`` [T, d] on the way."""
     _want(x, "gated_sum x", torch.float32, 2)
     T, d = x.shape
 
@@ -556,8 +559,21 @@ def gated_sum(x: torch.Tensor, a: Optional[torch.Tensor], a_gate=None, b: Option
         if streams.shape[1:] != x.shape or streams.shape[0] < count or mix.numel() != count or count < 1:
             raise KernelError(f"gated_sum: streams {tuple(streams.shape)}, {mix.numel()} weights, count {count}")
     lib = library("elementwise")
-    _check(lib, lib.lp_gated_sum(x.data_ptr(), ap, agp, ald, abp, bp, bgp, bld, bbp, _ptr(streams), _ptr(mix), int(count),
-                                 1 if keep_input else 0, T, d, _stream()))
+    operands = (x.data_ptr(), ap, agp, ald, abp, bp, bgp, bld, bbp, _ptr(streams), _ptr(mix), int(count), 1 if keep_input else 0, T, d)
+    if norm_after is None:
+        _check(lib, lib.lp_gated_sum(*operands, _stream()))
+        return x
+    gain, eps, out = norm_after
+    _want(gain, "gated_sum norm gain", torch.float32, 1)
+    _want(out, "gated_sum norm out", ndim=2)
+    if gain.numel() != d or out.shape != x.shape:
+        raise KernelError(f"gated_sum: norm gain {tuple(gain.shape)}, normed out {tuple(out.shape)} for x {tuple(x.shape)}")
+    code = lib.lp_gated_sum_norm(*operands, gain.data_ptr(), float(eps), out.data_ptr(), _code(out, "gated_sum norm out"), _stream())
+    if code == NOT_SERVED:
+        _check(lib, lib.lp_gated_sum(*operands, _stream()))
+        layernorm(x, gain, eps, out)
+        return x
+    _check(lib, code)
     return x
 
 

@@ -205,12 +205,19 @@ class ParallelBlock(Part):
     def cache_request(self):
         return self.mixer.cache_request()
 
-    def forward(self, ctx, cache, residual: torch.Tensor) -> bool:
+    kind_parallel = True
+
+    def forward(self, ctx, cache, residual: torch.Tensor, normed_ready: bool = False, next_block=None) -> bool:
+        """Run the layer on the residual stream in place. ``normed_ready``: the previous block already left this
+        block's norm of the stream in the shared "normed" buffer. ``next_block``: the block that runs next on the stream
+        as this one leaves it; if it is of this kind and its norm is a layer norm, the kernel that forms the stream also
+        writes that norm. Returns whether it did."""
         s, act = self.spec, self.runtime.act_dtype
         T, d = residual.shape
         h = ctx.buffer("normed", (T, d), act)
-        with ops.section("norm"):
-            self.norm.apply(residual, h)
+        if not normed_ready:
+            with ops.section("norm"):
+                self.norm.apply(residual, h)
         proj = None
         if self.proj is not None:
             proj = ctx.buffer("layer_proj", (T, self.proj.out_features), torch.float32)
@@ -236,14 +243,18 @@ class ParallelBlock(Part):
             m_gate = (proj[:, self._mixer_gate_at:self._mixer_gate_at + d], self.mixer_gate_bias)
         if self._ffn_gate_at is not None:
             f_gate = (proj[:, self._ffn_gate_at:self._ffn_gate_at + d], self.ffn_gate_bias)
+        following = next_block.norm if getattr(next_block, "kind_parallel", False) else None
+        if not getattr(following, "fusable_layernorm", False):
+            following = None
+        norm_after = None if following is None else (following.weight, following.spec.eps, h)
         with ops.section("layer.sum"):
             if s.depth_mix is not None:
                 streams = ctx.buffer("depth_streams", (s.depth_mix.total, T, d), torch.float32)
                 ops.gated_sum(residual, m, m_gate, f, f_gate, streams=streams, mix=self.depth_weights,
-                              count=s.depth_mix.count, keep_input=s.depth_mix.count == 2)
+                              count=s.depth_mix.count, keep_input=s.depth_mix.count == 2, norm_after=norm_after)
             else:
-                ops.gated_sum(residual, m, m_gate, f, f_gate)
-        return False
+                ops.gated_sum(residual, m, m_gate, f, f_gate, norm_after=norm_after)
+        return following is not None
 
 
 class SandwichBlock(Part):

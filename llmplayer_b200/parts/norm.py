@@ -45,6 +45,7 @@ class RMSNorm(Part):
 class LayerNorm(Part):
     """out = (x - mean(x)) / sqrt(mean((x - mean(x))^2) + eps) * gain, in float32; no bias."""
     capture_safe = True
+    fusable_layernorm = True        # the kernel that forms the stream may write this norm
 
     def __init__(self, spec: NormSpec):
         self.spec = spec
