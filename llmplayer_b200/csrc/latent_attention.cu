@@ -916,10 +916,47 @@ latent_expand_rows_kernel(const float* __restrict__ part, int shares, const TW* 
 
 // qa[t, h, r] = sum over d of uk[h, d, r] q[t, h, d]: 64 columns of the latent per CTA, 16 per warp. Bound by latency: 32
 // tokens, 16 heads of 128, rank 512, B200: 28 us with a thread per column (above) -> 12 (cold caches).
+// With `k.pages` the same launch does what latent_prepare does in front of it: the queries come as the projection leaves them
+// (their rope parts are rotated on the way), and CTAs of their own (blockIdx.y == H) norm the tokens' latents, rotate the shared
+// key parts and write both into the cache. A decode step's chain loses
+// a kernel: a layer with 32 sequences, captured, B200: 59.6 -> 56.1 us; a request of 8 x 300 tokens and 16 steps to a hybrid of 4
+// layers 5330 -> 5174. Queries read four values at a time, all in flight, took the absorb alone from 5.9 to 5.0 us (8 tokens 4.5 -> 3.4).
+struct KeyRows {
+    const float* kv;                // [T, ld]: the latent and the shared key part of a token, rank + dr values
+    int ld;
+    const float* gain;
+    float eps;
+    const float* inv_freq;
+    int rot, interleaved;
+    float magnitude;
+    const int *positions, *seq_ids, *page_table;
+    int pt_stride, page_size;
+    __nv_bfloat16* pages;           // null: no keys, and queries whose rope parts are rotated already
+};
+// unit u of a part of dr values whose first `rot` turn: a pair of them, or one that passes
+template <typename F>
+__device__ __forceinline__ void rope_unit(const KeyRows& k, const float* x, int u, int pos, F store) {
+    const int half = k.rot >> 1;
+    if (u >= half) {
+        store(u + half, x[u + half]);
+        return;
+    }
+    float sn, cs;
+    sincosf((float)pos * k.inv_freq[u], &sn, &cs);
+    if (k.magnitude != 1.0f) {
+        sn *= k.magnitude;
+        cs *= k.magnitude;
+    }
+    const int i = k.interleaved ? 2 * u : u, j = k.interleaved ? 2 * u + 1 : u + half;
+    const float lo = x[i], hi = x[j];
+    store(i, __fsub_rn(__fmul_rn(lo, cs), __fmul_rn(hi, sn)));
+    store(j, __fadd_rn(__fmul_rn(hi, cs), __fmul_rn(lo, sn)));
+}
+
 constexpr int AB_COLS = 64, AB_WARPS = 4;
 __global__ void __launch_bounds__(AB_WARPS * 32)
-latent_absorb_tc_kernel(const float* __restrict__ q, const __nv_bfloat16* __restrict__ uk, float* __restrict__ qa, int T, int H, int dn,
-                        int dr, int rank) {
+latent_absorb_tc_kernel(const float* __restrict__ q, int ldq, const __nv_bfloat16* __restrict__ uk, float* __restrict__ qa, int T, int H,
+                        int dn, int dr, int rank, const KeyRows k) {
     extern __shared__ __align__(16) uint8_t raw[];
     const int stride = dn + 8;
     constexpr int WSTRIDE = AB_COLS + 8;
@@ -927,7 +964,32 @@ latent_absorb_tc_kernel(const float* __restrict__ q, const __nv_bfloat16* __rest
     __nv_bfloat16* Ws = Qs + 3 * TC_ROWS * stride;            // [dn][WSTRIDE]
     const int t0 = blockIdx.x * TC_ROWS, h = blockIdx.y, c0 = blockIdx.z * AB_COLS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int hd = dn + dr, Dk = rank + dr, nt = min(TC_ROWS, T - t0);
+    const int hd = dn + dr, Dk = rank + dr, nt = min(TC_ROWS, T - t0), units = dr - (k.rot >> 1);
+    if (h == H) {                                             // the tokens' rows of the cache, shared out over blockIdx.z
+        __shared__ float scratch[32];
+        lp_grid_release();
+        lp_grid_wait();
+        for (int i = blockIdx.z; i < nt; i += gridDim.z) {
+            const int t = t0 + i, pos = k.positions[t];
+            const float* kv = k.kv + (long long)t * k.ld;
+            const int page = k.page_table[(long long)k.seq_ids[t] * k.pt_stride + pos / k.page_size];
+            __nv_bfloat16* dst = k.pages + ((long long)page * k.page_size + pos % k.page_size) * Dk;
+            for (int u = tid; u < units; u += AB_WARPS * 32)
+                rope_unit(k, kv + rank, u, pos, [&](int c, float v) { dst[rank + c] = __float2bfloat16_rn(v); });
+            float ss = 0.f;
+            for (int c = tid * 4; c < rank; c += AB_WARPS * 128) {
+                const float4 v = *(const float4*)(kv + c);
+                ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+            }
+            const float factor = 1.0f / sqrtf(lp_block_sum(ss, scratch) / (float)rank + k.eps);
+            for (int c = tid * 4; c < rank; c += AB_WARPS * 128) {
+                const float4 v = *(const float4*)(kv + c), g = *(const float4*)(k.gain + c);
+                const float normed[4] = {v.x * factor * g.x, v.y * factor * g.y, v.z * factor * g.z, v.w * factor * g.w};
+                store4(dst + c, normed);
+            }
+        }
+        return;
+    }
     // weights are written by no kernel of a step: asked for before the wait
     for (int i = tid; i < dn * (AB_COLS / 8); i += AB_WARPS * 32) {
         const int d = i / (AB_COLS / 8), c = i % (AB_COLS / 8) * 8;
@@ -937,17 +999,28 @@ latent_absorb_tc_kernel(const float* __restrict__ q, const __nv_bfloat16* __rest
     asm volatile("cp.async.commit_group;" ::: "memory");
     lp_grid_release();
     lp_grid_wait();
-    for (int e = tid; e < TC_ROWS * dn; e += AB_WARPS * 32) {
-        const int i = e / dn, d = e - i * dn;
-        __nv_bfloat16 p[3];
-        three_parts(i < nt ? q[((long long)(t0 + i) * H + h) * hd + d] : 0.f, p);
+    const float* first = q + (long long)t0 * ldq + h * hd;    // of the tile's first token
+    const int quads = dn >> 2;
+#pragma unroll 4
+    for (int e = tid; e < TC_ROWS * quads; e += AB_WARPS * 32) {
+        const int i = e / quads, d = (e - i * quads) * 4;
+        const float4 x = i < nt ? *(const float4*)(first + (long long)i * ldq + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float v[4] = {x.x, x.y, x.z, x.w};
+        __nv_bfloat16 p[4][3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) Qs[(k * TC_ROWS + i) * stride + d] = p[k];
+        for (int j = 0; j < 4; ++j) three_parts(v[j], p[j]);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            __nv_bfloat162* to = (__nv_bfloat162*)(Qs + (m * TC_ROWS + i) * stride + d);
+            to[0] = __halves2bfloat162(p[0][m], p[1][m]);
+            to[1] = __halves2bfloat162(p[2][m], p[3][m]);
+        }
     }
     if (blockIdx.z == 0)
-        for (int e = tid; e < nt * dr; e += AB_WARPS * 32) {
-            const int i = e / dr, d = e - i * dr;
-            qa[((long long)(t0 + i) * H + h) * Dk + rank + d] = q[((long long)(t0 + i) * H + h) * hd + dn + d];
+        for (int e = tid; e < nt * units; e += AB_WARPS * 32) {
+            const int i = e / units;
+            float* to = qa + ((long long)(t0 + i) * H + h) * Dk + rank;
+            rope_unit(k, first + (long long)i * ldq + dn, e - i * units, k.pages ? k.positions[t0 + i] : 0, [&](int c, float v) { to[c] = v; });
         }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -1151,18 +1224,48 @@ extern "C" int lp_latent_prepare(const float* proj, int ld, int q_off, int kv_of
     return lp_check_launch("latent_prepare");
 }
 
+namespace {
+size_t absorb_bytes(int dn) { return ((size_t)3 * TC_ROWS * (dn + 8) + (size_t)dn * (AB_COLS + 8)) * 2; }
+// Whether the tensor-core kernel serves the map: 16-bit weights whose tiles can be read 16 bytes at a time.
+bool absorb_on_tensor_cores(int w_dtype, int dn, int dr, int rank, const void* uk, const float* qa) {
+    return w_dtype == LP_BF16 && dn > 0 && dn % 16 == 0 && rank % AB_COLS == 0 && dr % 2 == 0 && (uintptr_t)uk % 16 == 0 &&
+           (uintptr_t)qa % 8 == 0 && absorb_bytes(dn) <= 200 * 1024;
+}
+}  // namespace
+
+// What lp_latent_prepare and lp_latent_absorb do one after the other, in one launch, for a 16-bit cache and 16-bit weights; see there for
+// the operands. Returns 1 (nothing was launched) for sizes and addresses that it does not take.
+extern "C" int lp_latent_queries(const float* proj, int ld, int q_off, int kv_off, const float* gain, float eps, const float* inv_freq,
+                                 int rot, const int* positions, const int* seq_ids, const int* page_table, int pt_stride, void* pages,
+                                 int kv_dtype, int T, int H, int dn, int dr, int rank, int page_size, const float* q_sep, int ldq,
+                                 int interleaved, float magnitude, const void* uk, int w_dtype, float* qa, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    const float* q = q_sep ? q_sep : proj + q_off;
+    if (!q_sep) ldq = ld;
+    if (H <= 0 || H >= 65535 || page_size <= 0 || kv_dtype != LP_BF16 || rot < 0 || (rot & 1) || rot > dr || (rot > 0 && !inv_freq) || q_off < 0 ||
+        kv_off < 0 || kv_off + rank + dr > ld || (q_sep ? 0 : q_off) + H * (dn + dr) > ldq || !absorb_on_tensor_cores(w_dtype, dn, dr, rank, uk, qa) ||
+        ld % 4 || ldq % 4 || kv_off % 4 || dr % 4 || (((uintptr_t)q | (uintptr_t)proj | (uintptr_t)gain | (uintptr_t)pages) & 15) != 0)
+        return 1;
+    const KeyRows k{proj + kv_off, ld, gain, eps, inv_freq, rot, interleaved, magnitude, positions, seq_ids, page_table, pt_stride, page_size,
+                    (__nv_bfloat16*)pages};
+    const size_t bytes = absorb_bytes(dn);
+    if (grant_shared(latent_absorb_tc_kernel, bytes, "latent_queries")) return -1;
+    lp_launch(latent_absorb_tc_kernel, dim3((T + TC_ROWS - 1) / TC_ROWS, H + 1, rank / AB_COLS), AB_WARPS * 32, bytes, stream, q, ldq,
+              (const __nv_bfloat16*)uk, qa, T, H, dn, dr, rank, k);
+    return lp_check_launch("latent_queries");
+}
+
 // q: float32 [T, H, dn + dr]; uk: [H * dn, rank]; qa: float32 [T, H, rank + dr].
 extern "C" int lp_latent_absorb(const float* q, const void* uk, int w_dtype, float* qa, int T, int H, int dn, int dr,
                                 int rank, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (H <= 0 || H > 65535 || dn < 0 || dr < 0 || rank <= 0) LP_REFUSE("latent_absorb: %d heads of %d + %d over rank %d", H, dn, dr, rank);
     // bfloat16 weights whose tiles can be read 16 bytes at a time go to the tensor cores
-    const size_t tc_bytes = ((size_t)3 * TC_ROWS * (dn + 8) + (size_t)dn * (AB_COLS + 8)) * 2;
-    if (w_dtype == LP_BF16 && dn > 0 && dn % 16 == 0 && rank % AB_COLS == 0 && dr % 2 == 0 && (uintptr_t)uk % 16 == 0 && (uintptr_t)qa % 8 == 0 &&
-        tc_bytes <= 200 * 1024) {
-        if (grant_shared(latent_absorb_tc_kernel, tc_bytes, "latent_absorb")) return -1;
-        lp_launch(latent_absorb_tc_kernel, dim3((T + TC_ROWS - 1) / TC_ROWS, H, rank / AB_COLS), AB_WARPS * 32, tc_bytes, stream, q,
-                  (const __nv_bfloat16*)uk, qa, T, H, dn, dr, rank);
+    if (absorb_on_tensor_cores(w_dtype, dn, dr, rank, uk, qa) && (dn + dr) % 4 == 0 && (uintptr_t)q % 16 == 0) {
+        const size_t bytes = absorb_bytes(dn);
+        if (grant_shared(latent_absorb_tc_kernel, bytes, "latent_absorb")) return -1;
+        lp_launch(latent_absorb_tc_kernel, dim3((T + TC_ROWS - 1) / TC_ROWS, H, rank / AB_COLS), AB_WARPS * 32, bytes, stream, q,
+                  H * (dn + dr), (const __nv_bfloat16*)uk, qa, T, H, dn, dr, rank, KeyRows{});
         return lp_check_launch("latent_absorb");
     }
     dim3 grid((T + TOK_TILE - 1) / TOK_TILE, H, (rank + 127) / 128);

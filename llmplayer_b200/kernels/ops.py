@@ -83,6 +83,7 @@ _SIGNATURES = {
                               _I, _P, _I, _I, _F, _P],
         "lp_latent_heads_to_pages": [_P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
         "lp_latent_gate_heads": [_P, _P, _I, _P, _I, _I, _I, _I, _P, ctypes.c_longlong, _P],
+        "lp_latent_queries": [_P, _I, _I, _I, _P, _F, _P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _F, _P, _I, _P, _P],
         "lp_latent_absorb": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _P],
         "lp_latent_attend_rows": [_I, _I, _I, _I],
         "lp_latent_attend_keys": [_I, _I, _I, _I],
@@ -1371,6 +1372,48 @@ def latent_absorb(q: torch.Tensor, k_up: torch.Tensor, out: torch.Tensor, *, nop
     lib = library("latent_attention")
     _check(lib, lib.lp_latent_absorb(q.data_ptr(), k_up.data_ptr(), _code(k_up, "latent_absorb k_up"), out.data_ptr(),
                                      T, H, nope_dim, rope_dim, rank, _stream()))
+    return out
+
+
+def latent_queries(proj: torch.Tensor, q_off: int, kv_off: int, gain: torch.Tensor, eps: float, rotation: Rotation,
+                   positions: torch.Tensor, seq_ids: torch.Tensor, page_table: torch.Tensor, pages: torch.Tensor, k_up: torch.Tensor,
+                   out: torch.Tensor, scratch, *, num_heads: int, nope_dim: int, rope_dim: int, kv_rank: int,
+                   q_from: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """:func:`latent_prepare` and :func:`latent_absorb` one after the other: the new tokens' rows into ``pages``, the absorbed
+    queries to ``out`` float32 [T, H, rank + rope], in one launch where the sizes allow it. ``scratch(name, shape, dtype)``: a buffer
+    for the queries between the two where they do not."""
+    _want(proj, "latent_queries proj", torch.float32, 2)
+    _want(gain, "latent_queries gain", torch.float32, 1)
+    _want(positions, "latent_queries positions", torch.int32, 1)
+    _want(seq_ids, "latent_queries seq_ids", torch.int32, 1)
+    _want(page_table, "latent_queries page_table", torch.int32, 2)
+    _want(pages, "latent_queries pages", ndim=3)
+    _want(k_up, "latent_queries k_up", ndim=2)
+    _want(out, "latent_queries out", torch.float32, 3)
+    T, ld = proj.shape
+    H, dn, dr, rank = num_heads, nope_dim, rope_dim, kv_rank
+    if (pages.shape[2] != rank + dr or gain.numel() != rank or positions.numel() != T or seq_ids.numel() != T
+            or k_up.shape != (H * dn, rank) or out.shape != (T, H, rank + dr)):
+        raise KernelError(f"latent_queries: proj {tuple(proj.shape)}, k_up {tuple(k_up.shape)}, out {tuple(out.shape)}, pages "
+                          f"{tuple(pages.shape)} for {H} heads of {dn} + {dr} over rank {rank}")
+    freq_ptr, rot, interleaved = rotation.checked("latent_queries", takes_magnitude=True)
+    q_ptr, ldq = None, 0
+    if q_from is not None:
+        q_ptr, ldq = _slice(q_from, "latent_queries q_from")
+        if q_from.shape != (T, H * (dn + dr)):
+            raise KernelError(f"latent_queries: queries {tuple(q_from.shape)} for {H} heads of {dn + dr}")
+    lib = library("latent_attention")
+    code = lib.lp_latent_queries(
+        proj.data_ptr(), ld, int(q_off), int(kv_off), gain.data_ptr(), float(eps), freq_ptr, rot, positions.data_ptr(),
+        seq_ids.data_ptr(), page_table.data_ptr(), page_table.shape[1], pages.data_ptr(), _code(pages, "latent_queries pages"),
+        T, H, dn, dr, rank, pages.shape[1], q_ptr, ldq, interleaved, float(rotation.magnitude), k_up.data_ptr(),
+        _code(k_up, "latent_queries k_up"), out.data_ptr(), _stream())
+    if code == NOT_SERVED:
+        q = scratch("latent_q", (T, H, dn + dr), torch.float32)
+        latent_prepare(proj, q_off, kv_off, gain, eps, rotation, positions, seq_ids, page_table, q, pages, num_heads=H, nope_dim=dn,
+                       rope_dim=dr, kv_rank=rank, q_from=q_from)
+        return latent_absorb(q, k_up, out, nope_dim=dn, rope_dim=dr)
+    _check(lib, code)
     return out
 
 

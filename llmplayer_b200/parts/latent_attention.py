@@ -118,13 +118,11 @@ class LatentAttention(Part):
                 self.q_up.store(q_latent, q_from, ctx)
         if self._forms_heads(ctx, cache):
             return self._forward_heads(ctx, cache, proj, q_off, kv_off, gate_off, rotation, table, out, q_from, add)
-        q = ctx.buffer("latent_q", (T, H, dn + dr), torch.float32)
-        with ops.section("attention.position"):
-            ops.latent_prepare(proj, q_off, kv_off, self.latent_gain, s.norm_eps, rotation, ctx.positions, ctx.seq_ids,
-                               table, q, cache.pages, num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank, q_from=q_from)
         q_abs = ctx.buffer("latent_q_absorbed", (T, H, rank + dr), torch.float32)
         with ops.section("attention.absorb"):
-            ops.latent_absorb(q, self.k_up, q_abs, nope_dim=dn, rope_dim=dr)
+            ops.latent_queries(proj, q_off, kv_off, self.latent_gain, s.norm_eps, rotation, ctx.positions, ctx.seq_ids, table,
+                               cache.pages, self.k_up, q_abs, ctx.buffer, num_heads=H, nope_dim=dn, rope_dim=dr, kv_rank=rank,
+                               q_from=q_from)
         shares = ops.latent_shares(ctx.num_sequences, ctx.max_new, H, table.shape[1], cache.pages.shape[1], cache.pages, rank,
                                    s.window)
         partials = ctx.buffer("latent_partials", (T, H, shares, rank + 2), torch.float32)
