@@ -20,6 +20,7 @@
 // are visited in blocks of 32 (64 on the tensor cores) aligned to absolute positions, so a position's result does not depend on how its
 // sequence was cut into steps or batched (the number of shares changes only the last merge).
 #include "bf16_parts.cuh"
+#include "tcgen05_utils.cuh"
 
 namespace {
 
@@ -540,34 +541,47 @@ constexpr int TC_ROWS = 16;          // (token, head) rows of a CTA = MMA M
 constexpr int TC_KEYS = 64;          // keys per block
 constexpr int TC_PSTRIDE = TC_KEYS + 8, TC_SSTRIDE = TC_KEYS + 4;
 
+constexpr int TC_BOX = TC_KEYS * 128;      // bytes of a block's 64 columns: rows of 128 bytes whose 16-byte pieces lie at piece ^ (row & 7)
+
+__host__ __device__ constexpr int tc_stage(int Dk) { return (Dk + 63) / 64 * TC_BOX; }
 __host__ __device__ constexpr size_t tc_smem(int Dk) {
-    return (size_t)(3 * TC_ROWS + 2 * TC_KEYS) * (Dk + 8) * 2 + (size_t)4 * TC_ROWS * TC_SSTRIDE * 4 + (size_t)3 * TC_ROWS * TC_PSTRIDE * 2;
+    return 1024 + 2 * (size_t)tc_stage(Dk) + (size_t)3 * TC_ROWS * (Dk + 8) * 2 + (size_t)4 * TC_ROWS * TC_SSTRIDE * 4 +
+           (size_t)3 * TC_ROWS * TC_PSTRIDE * 2;
 }
 
 // A CTA takes 16 (token, head) rows of one sequence and one share of its blocks of 64 keys; the next block's rows are on
-// their way while a block is worked on. Scores: a warp takes 32 keys and a quarter of the row's width, the quarters meet in
-// shared memory; softmax: two rows per warp; sums: a warp takes an eighth of the latent's columns (NT tiles of 8). Row strides of
-// an odd multiple of 16 bytes keep ldmatrix free of bank conflicts.
-// Bound by the tensor instructions (3 x 72 + 3 x 64 per 16 keys and CTA at rank 512, rows of 576) and the latency of a block's steps:
-// 32 sequences of 750 to 1500 rows of 576, 16 heads, B200: 210 us with a lane per key (above) -> 39 (cold
-// caches); with three chains of products one behind the other and a division per 16 bytes copied it was 41.
+// their way while a block is worked on, by TMA in boxes of 64 columns. Scores: a warp takes 32 keys and a quarter of the row's width, the
+// quarters meet in shared memory; softmax: half a warp per row; sums: a warp takes an eighth of the latent's columns (NT tiles of
+// 8). The boxes' swizzle, and row strides of an odd multiple of 16 bytes elsewhere, keep ldmatrix free of bank conflicts.
+// Bound by the tensor instructions (3 x 72 + 3 x 64 per 16 keys and CTA at rank 512, rows of 576; 3,260 cycles of a block's 5,100)
+// and the latency of a block's steps: 32 sequences of 750 to 1500 rows of 576, 16 heads, B200: 210 us with a lane per key
+// (above) -> 32 (39 with cold caches) -> 26. Of the 32, stamped inside, the threads' own copies of 16 bytes took 2,230 cycles per block
+// (a bulk copy per row is no better: 64 of them take one warp as long), the softmax with a warp per row and two rows behind one another 1,540, and reading the queries one
+// round trip at a time 6,000 per CTA.
 template <int NT>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__ pages, const int* __restrict__ page_table,
+latent_attend_tc_kernel(const __grid_constant__ CUtensorMap rows_map, const float* __restrict__ qa, const int* __restrict__ page_table,
                         int pt_stride, const int* __restrict__ q_start, const int* __restrict__ kv_len, float* __restrict__ part, int H,
-                        int dr, int page_size, float scale, int shares, int window) {
+                        int dr, int page_size, float scale, int shares, int window, int* __restrict__ status) {
     extern __shared__ __align__(16) uint8_t raw[];
     constexpr int rank = NT * 64;
     const int Dk = rank + dr, stride = Dk + 8;
-    __nv_bfloat16* Qs = (__nv_bfloat16*)raw;                                  // [3][TC_ROWS][stride]
-    __nv_bfloat16* Ks = Qs + 3 * TC_ROWS * stride;                            // [2][TC_KEYS][stride]
-    float* Ss = (float*)(Ks + 2 * TC_KEYS * stride);                          // [4][TC_ROWS][TC_SSTRIDE]
+    const uint32_t stage_bytes = tc_stage(Dk);
+    uint8_t* Ks = raw + (1024 - (smem_at(raw) & 1023) & 1023);               // two stages of boxes, each box at a multiple of 1024
+    __nv_bfloat16* Qs = (__nv_bfloat16*)(Ks + 2 * stage_bytes);               // [3][TC_ROWS][stride]
+    float* Ss = (float*)(Qs + 3 * TC_ROWS * stride);                          // [4][TC_ROWS][TC_SSTRIDE]
     __nv_bfloat16* Ps = (__nv_bfloat16*)(Ss + 4 * TC_ROWS * TC_SSTRIDE);      // [3][TC_ROWS][TC_PSTRIDE]
     __shared__ float alphas[TC_ROWS];
-    lp_grid_release();
-    lp_grid_wait();
+    __shared__ uint64_t full[2];                                              // a stage's rows are there
     const int b = blockIdx.y, share = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    lp_grid_release();
+    lp_grid_wait();
     const int first_tok = q_start[b], n_new = q_start[b + 1] - first_tok;
     const int rows_total = n_new * H, r0 = blockIdx.x * TC_ROWS;
     if (r0 >= rows_total) return;
@@ -579,43 +593,49 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
     const int per = (blk_end - blk_first + shares - 1) / shares;
     const int blk_lo = blk_first + share * per, blk_hi = min(blk_lo + per, blk_end);
     const int* pt = page_table + (long long)b * pt_stride;
-    // a warp brings rows warp, warp + 8, ..., a lane 16 bytes of a row at a time: the addresses only count up
+    // one lane of every warp asks for its share of a block's boxes (a box takes some 150 cycles to ask for)
+    int page = lane == 0 && blk_lo < blk_hi ? pt[blk_lo * TC_KEYS / page_size] : 0;      // of the block to fetch next
     auto fetch = [&](int blk) {
-        if (blk < blk_hi) {
-            const int k0 = blk * TC_KEYS;
-            const __nv_bfloat16* from = pages + ((long long)pt[k0 / page_size] * page_size + k0 % page_size + warp) * Dk + lane * 8;
-            uint32_t to = smem_at(Ks + ((blk & 1) * TC_KEYS + warp) * stride + lane * 8);
-#pragma unroll
-            for (int u = 0; u < TC_KEYS / WARPS; ++u) {
-                const int bytes = k0 + warp + u * WARPS <= last_pos ? 16 : 0;          // rows beyond the last position are zero
-                const __nv_bfloat16* src = bytes ? from : pages;
-                for (int c = lane * 8, d = 0; c < Dk; c += 256, d += 256)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + d * 2), "l"(src + (bytes ? d : 0)), "r"(bytes) : "memory");
-                from += (long long)WARPS * Dk;
-                to += WARPS * stride * 2;
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (lane != 0 || blk >= blk_hi) return;
+        const int k0 = blk * TC_KEYS, st = (blk - blk_lo) & 1;
+        if (warp == 0) mbar_expect_tx(&full[st], stage_bytes);
+        for (uint32_t c = warp; c * TC_BOX < stage_bytes; c += WARPS)
+            tma_load_2d(Ks + st * stage_bytes + c * TC_BOX, &rows_map, c * 64, page * page_size + k0 % page_size, &full[st]);
+        if (blk + 1 < blk_hi) page = pt[(k0 + TC_KEYS) / page_size];
     };
+    __syncthreads();                                      // the barriers are set up
     fetch(blk_lo);
-    for (int r = warp; r < TC_ROWS; r += WARPS) {
-        const float* src = qa + ((long long)first_tok * H + r0 + r) * Dk;
-#pragma unroll 5
-        for (int e = lane * 4; e < Dk; e += 128) {
-            const float4 x = r < n_rows ? *(const float4*)(src + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float v[4] = {x.x, x.y, x.z, x.w};
-            __nv_bfloat16 p[4][3];
+    constexpr int Q_LOADS = NT / 2 + 1;                   // float4s of a row per lane and turn
+    for (int e0 = lane * 4; e0 < Dk; e0 += Q_LOADS * 128) {
+        float4 x[2][Q_LOADS];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) three_parts(v[i], p[i]);
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                __nv_bfloat162* to = (__nv_bfloat162*)(Qs + (k * TC_ROWS + r) * stride + e);
-                to[0] = __halves2bfloat162(p[0][k], p[1][k]);
-                to[1] = __halves2bfloat162(p[2][k], p[3][k]);
+            for (int u = 0; u < Q_LOADS; ++u) {
+                const int r = warp + i * WARPS, e = e0 + u * 128;
+                x[i][u] = r < n_rows && e < Dk ? *(const float4*)(qa + ((long long)first_tok * H + r0 + r) * Dk + e) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int u = 0; u < Q_LOADS; ++u) {
+                const int r = warp + i * WARPS, e = e0 + u * 128;
+                if (e >= Dk) continue;
+                const float v[4] = {x[i][u].x, x[i][u].y, x[i][u].z, x[i][u].w};
+                __nv_bfloat16 p[4][3];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) three_parts(v[j], p[j]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    __nv_bfloat162* to = (__nv_bfloat162*)(Qs + (k * TC_ROWS + r) * stride + e);
+                    to[0] = __halves2bfloat162(p[0][k], p[1][k]);
+                    to[1] = __halves2bfloat162(p[2][k], p[3][k]);
+                }
+            }
     }
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};        // of rows 2 warp, 2 warp + 1
+    const int my_row = 2 * warp + (lane >> 4);            // of the softmax: half a warp per row
+    const int my_pos = my_row < n_rows ? first_pos + (r0 + my_row) / H : -1;
+    float m = -INFINITY, l = 0.f;
     float acc[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
@@ -625,9 +645,25 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
     const int k_steps = Dk / 16, step_lo = quarter * k_steps / 4, step_hi = (quarter + 1) * k_steps / 4;
     for (int blk = blk_lo; blk < blk_hi; ++blk) {
         fetch(blk + 1);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        const __nv_bfloat16* K = Ks + (blk & 1) * TC_KEYS * stride;
+        const int turn = blk - blk_lo;
+        const bool there = mbar_wait(&full[turn & 1], (turn >> 1) & 1);
+        if (!__syncthreads_and(there)) {                  // a wait that ran out ends the block; its other copies are waited for first
+            if (tid == 0) {
+                atomicExch(status, 62);
+                if (blk + 1 < blk_hi) mbar_wait(&full[(turn + 1) & 1], ((turn + 1) >> 1) & 1);
+            }
+            return;
+        }
+        uint8_t* K = Ks + (turn & 1) * stage_bytes;
+        const int held = last_pos + 1 - blk * TC_KEYS;
+        if (held < TC_KEYS) {                             // what lies behind the last position is no row: zeros
+            const int per_row = stage_bytes / (TC_KEYS * 16);
+            for (int e = tid; e < (TC_KEYS - held) * per_row; e += WARPS * 32) {
+                const int r = held + e / per_row, c = e % per_row;
+                *(uint4*)(K + (c >> 3) * TC_BOX + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
+            }
+            __syncthreads();
+        }
         {
             // a chain of products per part and tile of 8 keys: none waits for another
             float s[3][4][4];
@@ -638,12 +674,13 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
 #pragma unroll
                     for (int k = 0; k < 4; ++k) s[p][n][k] = 0.f;
             const uint32_t a_at = smem_at(Qs + (lane & 15) * stride + (lane >> 4) * 8);
-            const uint32_t b_at = smem_at(K + (key_group * 32 + (lane >> 4) * 8 + (lane & 7)) * stride + ((lane >> 3) & 1) * 8);
+            const uint32_t b_at = smem_at(K + (key_group * 32 + (lane >> 4) * 8 + (lane & 7)) * 128);
 #pragma unroll 3
             for (int step = step_lo; step < step_hi; ++step) {
                 uint32_t kf[2][4];
-                ldmatrix4(b_at + step * 32, kf[0]);
-                ldmatrix4(b_at + 16 * stride * 2 + step * 32, kf[1]);
+                const uint32_t at = b_at + (step >> 2) * TC_BOX + ((((step & 3) * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
+                ldmatrix4(at, kf[0]);
+                ldmatrix4(at + 16 * 128, kf[1]);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
                     uint32_t qf[4];
@@ -663,36 +700,47 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
             }
         }
         __syncthreads();
+        {
+            const int c = (lane & 15) * 4, key0 = blk * TC_KEYS + c;       // four neighbouring keys per lane
+            const float* from = Ss + my_row * TC_SSTRIDE + c;
+            float4 quarter4[4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = 2 * warp + i, pos = r < n_rows ? first_pos + (r0 + r) / H : -1;
-            float sc[2], p[2];
-            bool seen[2];
+            for (int k = 0; k < 4; ++k) quarter4[k] = *(const float4*)(from + k * TC_ROWS * TC_SSTRIDE);
+            const float dot[4] = {(quarter4[0].x + quarter4[1].x) + (quarter4[2].x + quarter4[3].x),
+                                  (quarter4[0].y + quarter4[1].y) + (quarter4[2].y + quarter4[3].y),
+                                  (quarter4[0].z + quarter4[1].z) + (quarter4[2].z + quarter4[3].z),
+                                  (quarter4[0].w + quarter4[1].w) + (quarter4[2].w + quarter4[3].w)};
+            float sc[4];
+            bool seen[4];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int key = blk * TC_KEYS + lane + 32 * k;
-                seen[k] = key <= pos && (window <= 0 || key > pos - window);
-                const float* from = Ss + r * TC_SSTRIDE + lane + 32 * k;
-                const float dot = (from[0] + from[TC_ROWS * TC_SSTRIDE]) + (from[2 * TC_ROWS * TC_SSTRIDE] + from[3 * TC_ROWS * TC_SSTRIDE]);
-                sc[k] = seen[k] ? dot * scale : -INFINITY;
+            for (int k = 0; k < 4; ++k) {
+                seen[k] = key0 + k <= my_pos && (window <= 0 || key0 + k > my_pos - window);
+                sc[k] = seen[k] ? dot[k] * scale : -INFINITY;
             }
-            const float m_new = fmaxf(m[i], lp_warp_max(fmaxf(sc[0], sc[1])));
-            float alpha = 1.f;
-            p[0] = p[1] = 0.f;
+            float top = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float m_new = fmaxf(m, top);
+            float alpha = 1.f, p[4] = {0.f, 0.f, 0.f, 0.f};
             if (m_new != -INFINITY) {
 #pragma unroll
-                for (int k = 0; k < 2; ++k) p[k] = seen[k] ? expf(sc[k] - m_new) : 0.f;
-                alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+                for (int k = 0; k < 4; ++k) p[k] = seen[k] ? expf(sc[k] - m_new) : 0.f;
+                alpha = m == -INFINITY ? 0.f : expf(m - m_new);
             }
-            l[i] = l[i] * alpha + lp_warp_sum(p[0] + p[1]);
-            m[i] = m_new;
-            if (lane == 0) alphas[r] = alpha;
+            float sum = (p[0] + p[1]) + (p[2] + p[3]);
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                __nv_bfloat16 parts[3];
-                three_parts(p[k], parts);
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            l = l * alpha + sum;
+            m = m_new;
+            if ((lane & 15) == 0) alphas[my_row] = alpha;
+            __nv_bfloat16 parts[4][3];
 #pragma unroll
-                for (int q = 0; q < 3; ++q) Ps[(q * TC_ROWS + r) * TC_PSTRIDE + lane + 32 * k] = parts[q];
+            for (int k = 0; k < 4; ++k) three_parts(p[k], parts[k]);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                __nv_bfloat162* to = (__nv_bfloat162*)(Ps + (q * TC_ROWS + my_row) * TC_PSTRIDE + c);
+                to[0] = __halves2bfloat162(parts[0][q], parts[1][q]);
+                to[1] = __halves2bfloat162(parts[2][q], parts[3][q]);
             }
         }
         __syncthreads();
@@ -705,7 +753,7 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
             acc[n][3] *= f1;
         }
         const uint32_t p_at = smem_at(Ps + (lane & 15) * TC_PSTRIDE + (lane >> 4) * 8);
-        const uint32_t c_at = smem_at(K + (lane & 15) * stride + warp * (NT * 8) + (lane >> 4) * 8);
+        const uint32_t c_at = smem_at(K + (lane & 15) * 128);
 #pragma unroll
         for (int step = 0; step < TC_KEYS / 16; ++step) {
             uint32_t pf[3][4];
@@ -715,7 +763,8 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
             for (int n = 0; n < NT; n += 2) {
                 uint32_t cf[4];
                 // (NT = 1: the second tile belongs to the next warp or to the key part; it is read and not used)
-                ldmatrix4_trans(c_at + step * 16 * stride * 2 + n * 16, cf);
+                const int piece = warp * NT + n + (lane >> 4);
+                ldmatrix4_trans(c_at + step * 16 * 128 + (piece >> 3) * TC_BOX + (((piece & 7) ^ (lane & 7)) << 4), cf);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
                     mma_bf16(acc[n], pf[p], cf[0], cf[1]);
@@ -734,15 +783,8 @@ latent_attend_tc_kernel(const float* __restrict__ qa, const __nv_bfloat16* __res
 #pragma unroll
         for (int n = 0; n < NT; ++n) *(float2*)(dst + n * 8) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
     }
-    if (lane == 0)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = 2 * warp + i;
-            if (r >= n_rows) continue;
-            float* dst = part + (((long long)first_tok * H + r0 + r) * shares + share) * (rank + 2) + rank;
-            dst[0] = m[i];
-            dst[1] = l[i];
-        }
+    if ((lane & 15) == 0 && my_row < n_rows)
+        *(float2*)(part + (((long long)first_tok * H + r0 + my_row) * shares + share) * (rank + 2) + rank) = make_float2(m, l);
 }
 
 // Whether the tensor-core kernel serves these sizes: a rank of 64, 128, 256 or 512, rows of a multiple of 16 values that
@@ -1294,9 +1336,10 @@ extern "C" int lp_latent_attend_keys(int kv_dtype, int rank, int dr, int page_si
 // weights); q_start [B + 1], kv_len [B] (lengths after the step); max_new: most new tokens of a sequence.
 extern "C" int lp_latent_attend(const float* qa, const void* pages, int kv_dtype, const int* page_table, int pt_stride,
                                 const int* q_start, const int* kv_len, float* part, int B, int max_new, int H,
-                                int rank, int dr, int page_size, float scale, int shares, int window,
+                                int rank, int dr, int page_size, long long num_pages, float scale, int shares, int window, int* status,
                                 cudaStream_t stream) {
     if (B <= 0 || max_new <= 0) return 0;
+    if (!status) LP_REFUSE("latent_attend: nowhere to report a wait that ran out%s", "");
     if (H <= 0 || rank <= 0 || dr < 0) LP_REFUSE("latent_attend: %d heads over rank %d + %d", H, rank, dr);
     if (rank > 512) LP_REFUSE("latent_attend: rank %d (supported: up to 512)", rank);
     if (page_size <= 0 || page_size % KEYS) LP_REFUSE("latent_attend: page size %d must be a multiple of %d", page_size, KEYS);
@@ -1304,12 +1347,14 @@ extern "C" int lp_latent_attend(const float* qa, const void* pages, int kv_dtype
     if (attend_on_tensor_cores(kv_dtype, rank, dr, page_size) && (uintptr_t)pages % 16 == 0 && (uintptr_t)qa % 16 == 0 &&
         (uintptr_t)part % 8 == 0) {
         const size_t bytes = tc_smem(rank + dr);
+        CUtensorMap rows_map;
+        if (make_map(&rows_map, pages, num_pages * page_size, rank + dr, rank + dr, TC_KEYS)) return -1;
         const dim3 tc_grid((unsigned)(((long long)max_new * H + TC_ROWS - 1) / TC_ROWS), B, shares);
 #define LP_LAUNCH_TC(NT)                                                                                                     \
     do {                                                                                                                     \
         if (grant_shared(latent_attend_tc_kernel<NT>, bytes, "latent_attend")) return -1;                                    \
-        lp_launch(latent_attend_tc_kernel<NT>, tc_grid, WARPS * 32, bytes, stream, qa, (const __nv_bfloat16*)pages,          \
-                  page_table, pt_stride, q_start, kv_len, part, H, dr, page_size, scale, shares, window);                    \
+        lp_launch(latent_attend_tc_kernel<NT>, tc_grid, WARPS * 32, bytes, stream, rows_map, qa, page_table, pt_stride,      \
+                  q_start, kv_len, part, H, dr, page_size, scale, shares, window, status);                    \
     } while (0)
         if (rank == 64) LP_LAUNCH_TC(1);
         else if (rank == 128) LP_LAUNCH_TC(2);

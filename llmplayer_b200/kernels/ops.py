@@ -87,7 +87,7 @@ _SIGNATURES = {
         "lp_latent_absorb": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _P],
         "lp_latent_attend_rows": [_I, _I, _I, _I],
         "lp_latent_attend_keys": [_I, _I, _I, _I],
-        "lp_latent_attend": [_P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P],
+        "lp_latent_attend": [_P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, ctypes.c_longlong, _F, _I, _I, _P, _P],
         "lp_latent_merge": [_P, _I, _P, _I, _I, _P],
         "lp_latent_query_norm": [_P, _I, _I, _I, _P, _F, _P, _I, _I, _P],
         "lp_latent_expand": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P],
@@ -750,7 +750,7 @@ def check_kernel_status() -> None:
         raise KernelError(f"a tensor-core kernel gave up waiting on a barrier (code {code}: "
                           "1 = loader, 2 = MMA issuer, 3 = epilogue, 4-5 = operand maker; 2x the same in the "
                           "persistent product, 5x in the experts' (55: more choices than announced); "
-                          "6 = a page of the decode attention; 61 = a record of the chunked recurrence; 7x = the float32 product)")
+                          "6 = a page of the decode attention; 61 = a record of the chunked recurrence; 62 = rows of the latent attention; 7x = the float32 product)")
 
 
 def _token_tile(tokens: int, gated: bool) -> int:
@@ -1463,8 +1463,8 @@ def latent_attend(q_abs: torch.Tensor, pages: torch.Tensor, page_table: torch.Te
     lib = library("latent_attention")
     _check(lib, lib.lp_latent_attend(q_abs.data_ptr(), pages.data_ptr(), _code(pages, "latent_attend pages"),
                                      page_table.data_ptr(), page_table.shape[1], q_start.data_ptr(), kv_len.data_ptr(),
-                                     partials.data_ptr(), B, int(max_new), H, kv_rank, Dk - kv_rank, pages.shape[1],
-                                     float(scale), shares, int(window) if window else 0, _stream()))
+                                     partials.data_ptr(), B, int(max_new), H, kv_rank, Dk - kv_rank, pages.shape[1], pages.shape[0],
+                                     float(scale), shares, int(window) if window else 0, kernel_status().data_ptr(), _stream()))
     return partials
 
 
