@@ -1091,13 +1091,14 @@ latent_absorb_tc_kernel(const float* __restrict__ q, int ldq, const __nv_bfloat1
 }
 
 // out[t, h * dv + v] = gate * sum over r of uv[h, v, r] latent[t, h, r], the latent being the merge of the shares: 32 value
-// features per CTA, 8 per pair of warps, each with half of the rank; the halves meet in shared memory. Every CTA merges the
-// shares of its 16 (token, head) rows itself. Bound by latency: 32 tokens, 16 heads of 128, rank 512, 4 shares, B200:
-// 26 us with a CTA per row (above) -> 19 (cold caches; 38 with
-// one row's shares asked for at a time).
+// features per CTA, 8 per pair of warps, each with half of the rank; the halves meet in shared memory. The CL CTAs of a cluster
+// have the same rows: each merges the shares of 1 / CL of the latent's columns and leaves them in all of them. Bound by latency: 32 tokens,
+// 16 heads of 128, rank 512, 4 shares, B200: 26 us with a CTA per row (above) -> 19 (cold caches; 38 with one row's shares asked for at a
+// time). Warm, one launch behind the other, every CTA merging all columns / clusters of 4: 64 tokens of 2 shares 14.4 / 9.7, 32 of 4 11.8 / 8.6,
+// 8 of 8 9.4 / 5.9, 4 of 16 9.2 / 6.7, 2 of 16 7.0 / 6.0, 1 of 16 5.9 / 6.3: one token goes without.
 constexpr int EX_FEATURES = 32, EX_WARPS = 8;
-template <typename TOut>
-__global__ void __launch_bounds__(EX_WARPS * 32, 2)
+template <typename TOut, int CL>
+__global__ void __cluster_dims__(1, 1, CL) __launch_bounds__(EX_WARPS * 32, 2)
 latent_expand_tc_kernel(const float* __restrict__ part, int shares, const __nv_bfloat16* __restrict__ uv, const float* __restrict__ gate,
                         int ldg, TOut* __restrict__ out, int T, int H, int rank, int dv, float* __restrict__ zero, long long zero_count) {
     extern __shared__ __align__(16) uint8_t raw[];
@@ -1110,6 +1111,8 @@ latent_expand_tc_kernel(const float* __restrict__ part, int shares, const __nv_b
     const int t0 = blockIdx.x * TC_ROWS, h = blockIdx.y, v0 = blockIdx.z * EX_FEATURES;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nt = min(TC_ROWS, T - t0), width = rank + 2, nv = min(EX_FEATURES, dv - v0);
+    // a CTA stores into the others' shared memory only when all have started
+    if (CL > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     for (int i = tid; i < EX_FEATURES * (rank / 8); i += EX_WARPS * 32) {
         const int v = i / (rank / 8), c = i % (rank / 8) * 8;
         const int bytes = v < nv ? 16 : 0;
@@ -1121,43 +1124,70 @@ latent_expand_tc_kernel(const float* __restrict__ part, int shares, const __nv_b
     lp_grid_wait();
     clear_on_the_side(zero, zero_count);
     for (int i = warp; i < nt; i += EX_WARPS) {
-        const float* p = part + ((long long)(t0 + i) * H + h) * shares * width;
-        float M = -INFINITY;
-        for (int s = lane; s < shares; s += 32) M = fmaxf(M, p[s * width + rank]);
+        const float* p = part + ((long long)(t0 + i) * H + h) * shares * width + rank;
+        const float g = gate ? gate[(long long)(t0 + i) * ldg + h] : 0.f;
+        const float2 own = lane < shares ? *(const float2*)(p + (long long)lane * width) : make_float2(-INFINITY, 0.f);      // maximum, sum
+        float M = own.x;
+        for (int s = lane + 32; s < shares; s += 32) M = fmaxf(M, p[(long long)s * width]);
         M = lp_warp_max(M);
-        float L = 0.f;
-        for (int s = lane; s < shares; s += 32) {
-            const float ms = p[s * width + rank];
-            const float e = ms == -INFINITY ? 0.f : expf(ms - M);
+        const float e_own = own.x == -INFINITY ? 0.f : expf(own.x - M);
+        float L = own.y * e_own;
+        for (int s = lane + 32; s < shares; s += 32) {
+            const float2 other = *(const float2*)(p + (long long)s * width);
+            const float e = other.x == -INFINITY ? 0.f : expf(other.x - M);
             ws[i * shares + s] = e;
-            L += p[s * width + rank + 1] * e;
+            L += other.y * e;
         }
         L = lp_warp_sum(L);
         const float inv = 1.0f / L;
-        for (int s = lane; s < shares; s += 32) ws[i * shares + s] *= inv;
-        if (lane == 0) gs[i] = gate ? 1.0f / (1.0f + expf(-gate[(long long)(t0 + i) * ldg + h])) : 1.0f;
+        if (lane < shares) ws[i * shares + lane] = e_own * inv;
+        for (int s = lane + 32; s < shares; s += 32) ws[i * shares + s] *= inv;
+        if (lane == 0) gs[i] = gate ? 1.0f / (1.0f + expf(-g)) : 1.0f;
     }
     __syncthreads();
-    for (int r = tid * 2; r < rank; r += EX_WARPS * 64)
+    if (CL > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int quads = rank / CL / 4, first = (blockIdx.z % CL) * (rank / CL);
+#pragma unroll 2
+    for (int e = tid; e < TC_ROWS * quads; e += EX_WARPS * 32) {
+        const int i = e / quads, r = first + (e - i * quads) * 4;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (i < nt) {
+            const float* p = part + ((long long)(t0 + i) * H + h) * shares * width + r;
+            const float* wi = ws + i * shares;
 #pragma unroll 4
-        for (int i = 0; i < TC_ROWS; ++i) {
-            float2 v = make_float2(0.f, 0.f);
-            if (i < nt) {
-                const float* p = part + ((long long)(t0 + i) * H + h) * shares * width + r;
-                const float* wi = ws + i * shares;
-#pragma unroll 4
-                for (int s = 0; s < shares; ++s) {
-                    const float2 x = *(const float2*)(p + (long long)s * width);
-                    v.x = fmaf(x.x, wi[s], v.x);
-                    v.y = fmaf(x.y, wi[s], v.y);
+            for (int s = 0; s < shares; ++s) {
+                const float2 x = *(const float2*)(p + (long long)s * width), y = *(const float2*)(p + (long long)s * width + 2);
+                v[0] = fmaf(x.x, wi[s], v[0]);
+                v[1] = fmaf(x.y, wi[s], v[1]);
+                v[2] = fmaf(y.x, wi[s], v[2]);
+                v[3] = fmaf(y.y, wi[s], v[3]);
+            }
+        }
+        __nv_bfloat16 parts[4][3];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) three_parts(v[j], parts[j]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const __nv_bfloat162 lo = __halves2bfloat162(parts[0][k], parts[1][k]), hi = __halves2bfloat162(parts[2][k], parts[3][k]);
+            __nv_bfloat162* to = (__nv_bfloat162*)(Ls + (k * TC_ROWS + i) * stride + r);
+            if (CL == 1) {
+                to[0] = lo;
+                to[1] = hi;
+            } else {
+#pragma unroll
+                for (int peer = 0; peer < CL; ++peer) {
+                    uint32_t at;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_at(to)), "r"(peer));
+                    asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};"
+                                 ::"r"(at), "r"(*reinterpret_cast<const uint32_t*>(&lo)), "r"(*reinterpret_cast<const uint32_t*>(&hi)) : "memory");
                 }
             }
-            __nv_bfloat16 a[3], b[3];
-            three_parts(v.x, a);
-            three_parts(v.y, b);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) *(__nv_bfloat162*)(Ls + (k * TC_ROWS + i) * stride + r) = __halves2bfloat162(a[k], b[k]);
         }
+    }
+    if (CL > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int group = warp & 3, half = warp >> 2;             // 8 features; half of the rank
@@ -1414,9 +1444,12 @@ extern "C" int lp_latent_expand(const float* part, int shares, const void* uv, i
         const dim3 tc_grid((T + TC_ROWS - 1) / TC_ROWS, H, (dv + EX_FEATURES - 1) / EX_FEATURES);
 #define LP_LAUNCH_TC(TOut)                                                                                           \
     do {                                                                                                             \
-        if (grant_shared(latent_expand_tc_kernel<TOut>, tc_bytes, "latent_expand")) return -1;                       \
-        lp_launch(latent_expand_tc_kernel<TOut>, tc_grid, EX_WARPS * 32, tc_bytes, stream, part, shares,             \
-                  (const __nv_bfloat16*)uv, gate, ldg, (TOut*)out, T, H, rank, dv, zero, zero_count);                \
+        auto kernel = T > 1 && tc_grid.z % 4 == 0 ? latent_expand_tc_kernel<TOut, 4>                                          \
+                      : T > 1 && tc_grid.z % 2 == 0 ? latent_expand_tc_kernel<TOut, 2>                               \
+                                                    : latent_expand_tc_kernel<TOut, 1>;                              \
+        if (grant_shared(kernel, tc_bytes, "latent_expand")) return -1;                                              \
+        lp_launch(kernel, tc_grid, EX_WARPS * 32, tc_bytes, stream, part, shares, (const __nv_bfloat16*)uv, gate,    \
+                  ldg, (TOut*)out, T, H, rank, dv, zero, zero_count);                                                \
     } while (0)
         if (out_dtype == LP_BF16) LP_LAUNCH_TC(__nv_bfloat16);
         else LP_LAUNCH_TC(float);
