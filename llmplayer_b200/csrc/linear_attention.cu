@@ -887,8 +887,8 @@ low_rank_gates_kernel(const float* __restrict__ proj, int ld, int T, int H, Rank
 // The same with bfloat16 maps whose ranks are multiples of 16, on the tensor cores: the factors' float32 values as three
 // bfloat16 parts, the map's rows as they are. 64 tokens x 128 channels per CTA over the whole rank; a warp takes 32 x 32.
 // Bound by splitting the factors (every column of CTAs does it again) and by its outputs: 1943 tokens, two maps of 1024
-// channels with rank 128, B200: 50 us with float32 multiply-adds (above) -> 36; half of
-// its instructions are the exponentials and logarithms of the decays.
+// channels with rank 128, B200: 50 us with float32 multiply-adds (above) -> 36 -> 31 with all rows of a warp asked for before the first is
+// split; half of its instructions are the exponentials and logarithms of the decays.
 constexpr int LR_TOKENS = 64, LR_CHANNELS = 128;
 inline size_t low_rank_smem(int rank) { return (size_t)(3 * LR_TOKENS + LR_CHANNELS) * (rank + 8) * 2; }
 
@@ -916,24 +916,26 @@ low_rank_gates_tc_kernel(const float* __restrict__ proj, int ld, int T, int H, R
     lp_grid_release();
     lp_grid_wait();
     const bool wide = ((m.off | ld) & 3) == 0;
-    for (int r = warp; r < LR_TOKENS; r += 8) {
-        const bool real = t0 + r < T;
-        const float* from = proj + (long long)(real ? t0 + r : 0) * ld + m.off;
-        for (int c = lane * 4; c < R; c += 128) {
-            float v[4];
-            if (wide) {
-                const float4 x = *(const float4*)(from + c);
-                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-            } else {
+    constexpr int LR_ROWS = LR_TOKENS / 8;                         // of a warp, all asked for before the first is split
+    for (int c = lane * 4; c < R; c += 128) {
+        float4 x[LR_ROWS];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] = from[c + i];
-            }
+        for (int u = 0; u < LR_ROWS; ++u) {
+            const int t = t0 + warp + u * 8;
+            const float* from = proj + (long long)t * ld + m.off + c;
+            if (t >= T) x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            else if (wide) x[u] = *(const float4*)from;
+            else x[u] = make_float4(from[0], from[1], from[2], from[3]);
+        }
+#pragma unroll
+        for (int u = 0; u < LR_ROWS; ++u) {
+            const float v[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
             __nv_bfloat16 p[4][3];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) three_parts(real ? v[i] : 0.f, p[i]);
+            for (int i = 0; i < 4; ++i) three_parts(v[i], p[i]);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                __nv_bfloat162* to = (__nv_bfloat162*)(Xs + (k * LR_TOKENS + r) * stride + c);
+                __nv_bfloat162* to = (__nv_bfloat162*)(Xs + (k * LR_TOKENS + warp + u * 8) * stride + c);
                 to[0] = __halves2bfloat162(p[0][k], p[1][k]);
                 to[1] = __halves2bfloat162(p[2][k], p[3][k]);
             }
