@@ -15,7 +15,7 @@
 // (the plain recurrence has U = V). Decays enter as running products only, forwards or backwards from a token or a block
 // border, so nothing is divided by a product of decays and no logarithm is taken: strong decays (down to zero) are exact.
 //
-//   prepare   one CTA per (chunk, head, sequence): products of decays, A and B (16 x 16 blocks: between two blocks as sums
+//   prepare   one CTA per (chunk, head, sequence): products of decays, A and B (blocks of 4 tokens: between two blocks as sums
 //             over factored decays, inside a block with the decays multiplied token by token), the triangular solve with a
 //             thread per column, all in float32 arithmetic; the results go to a record per chunk and head, laid out as the
 //             operand fragments of the second kernel's products.
@@ -28,7 +28,8 @@
 namespace {
 
 constexpr int CT = 32;                  // tokens per chunk
-constexpr int HB = 16;                  // tokens per block inside a chunk
+constexpr int HB = 4;                   // tokens per block inside a chunk
+constexpr int BLOCKS = CT / HB, BLOCK_PAIRS = BLOCKS * (BLOCKS - 1) / 2;
 constexpr int NC = 16;                  // value columns per CTA of the second kernel
 constexpr int THREADS = 256;            // of the first kernel
 constexpr int JOINERS = CT / 8;         // warps of the second kernel beside one per 16 key channels: one per 8 tokens
@@ -92,23 +93,27 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ float both(uint64_t a) { return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32)); }
 __device__ __forceinline__ float4 four(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 
-// Bound by its instructions and the latencies between its barriers (two blocks per SM, 41 % of the issue slots): rows read four
+// Bound by its instructions and the latencies between its barriers (two blocks per SM): rows read four
 // channels at a time, and the sums inside and between blocks as pairs of channels in one instruction, took 2048 tokens of 8
-// heads of 128 x 256 from 54 to 44 us on a B200 (three prompts of 518 to 777 tokens, 128 x 128, delta rule: 57 -> 47).
-// PER: key channels per lane of a sum over a head's channels (16 lanes): dk <= 16 PER.
-template <int PER>
-__global__ void __launch_bounds__(THREADS, PER <= 8 ? 2 : 1)
+// heads of 128 x 256 from 54 to 44 us on a B200 (three prompts of 518 to 777 tokens, 128 x 128, delta rule: 57 -> 47). Stamped inside,
+// 17,000 of a block's 38,000 cycles went into the sums inside blocks of 16 (a half-warp per pair of keys, whose sums met in
+// shuffles for every row), 9,900 into the products of decays (the keys' record stored four bytes at a time, 64 apart). Blocks of
+// 4 whose pairs are plain sums of a thread, a tile of 2 x 2 per thread between blocks, and a key's record stored 16 bytes at a
+// time: the layer of 2048 tokens 219.5 -> 209.5 us, the delta rule's 231.6 -> 222.1.
+// NARROW: at most 128 key channels (two blocks per SM).
+template <bool NARROW>
+__global__ void __launch_bounds__(THREADS, NARROW ? 2 : 1)
 prepare_kernel(Inputs in, const int* __restrict__ q_start, int first_chunk, int chunks, float* __restrict__ records,
                float* __restrict__ values) {
     extern __shared__ __align__(16) float sm[];
     const int dk = in.dk, dv = in.dv, H = in.H, dkp = padded(dk), ks = dkp + 4;      // rows padded against bank conflicts
-    float* qs = sm;                        // [CT][ks]
-    float* kk = qs + CT * ks;              // [CT][ks]
-    float* gs = kk + CT * ks;              // [CT][ks]
-    float* kf = gs + CT * ks;              // [HB][ks]: keys of the second block times the decays since its start
-    float* qf = kf + HB * ks;              // [HB][ks]: its queries likewise
-    float* ke = qf + HB * ks;              // [HB][ks]: keys of the first block times the decays up to its end
-    float* L = ke + HB * ks;               // [CT][CT]: b_i A_ij
+    float* qs = sm;                        // [CT][ks]: queries; later times the decays since their block's start
+    float* kk = qs + CT * ks;              // [CT][ks]: keys
+    float* gs = kk + CT * ks;              // [CT][ks]: decays
+    float* kf = gs + CT * ks;              // [CT][ks]: keys times the decays since their block's start (their own included)
+    float* ke = kf + CT * ks;              // [CT][ks]: keys times the decays up to their block's end
+    float* between = ke + CT * ks;         // [BLOCK_PAIRS][ks]: products of the decays of the blocks between two
+    float* L = between + BLOCK_PAIRS * ks; // [CT][CT]: b_i A_ij
     float* Bm = L + CT * CT;               // [CT][CT]
     float* bs = Bm + CT * CT;              // [CT]
     lp_grid_release();
@@ -209,114 +214,138 @@ prepare_kernel(Inputs in, const int* __restrict__ q_start, int first_chunk, int 
     for (int e = tid; e < CT * CT; e += THREADS) L[e] = Bm[e] = 0.f;
     __syncthreads();
 
+    // pairs (i, j) of one block: a pair, or a token with itself (B alone), per two threads, which take every other four channels
+    {
+        const int item = tid >> 1, half = tid & 1;
+        constexpr int INSIDE = HB * (HB - 1) / 2, PAIRS = BLOCKS * INSIDE;
+        int i = 0, j = 0;
+        if (item < PAIRS) {
+            const int pair = item % INSIDE;
+            const int r = pair < 1 ? 1 : pair < 3 ? 2 : 3;
+            i = item / INSIDE * HB + r;
+            j = item / INSIDE * HB + pair - r * (r - 1) / 2;
+        } else if (item < PAIRS + CT) i = j = item - PAIRS;
+        uint64_t sa = 0, sb = 0;
+        if (item < PAIRS + CT)
+            for (int c = half; c < dkp >> 2; c += 2) {
+                auto row = [&](const float* x, int r) { return reinterpret_cast<const ulonglong2*>(x + r * ks)[c]; };
+                const ulonglong2 k = row(kk, i), q = row(qs, i);
+                ulonglong2 m = row(kk, j);
+                for (int t = j + 1; t <= i; ++t) {
+                    const ulonglong2 g = row(gs, t);
+                    m.x = mul2(m.x, g.x);
+                    m.y = mul2(m.y, g.y);
+                }
+                sa = fma2(k.x, m.x, fma2(k.y, m.y, sa));
+                sb = fma2(q.x, m.x, fma2(q.y, m.y, sb));
+            }
+        float a = both(sa), bsum = both(sb);
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        bsum += __shfl_xor_sync(0xffffffffu, bsum, 1);
+        if (half == 0 && item < PAIRS + CT) {
+            Bm[i * CT + j] = bsum;
+            if (i > j) L[i * CT + j] = bs[i] * a;
+        }
+    }
+    __syncthreads();
+
     // products of decays, a thread per key channel (forwards; its column of diag(b) (P k) stays in registers for the solve) and
     // one backwards (other threads where there are enough)
     float col[CT];
     const int back = dkp <= THREADS / 2 ? THREADS / 2 : 0;
     if (tid < dkp) {
         const int c = tid;
-        float p = 1.f, pb = 1.f;
+        float p = 1.f, pb = 1.f, block[BLOCKS];
 #pragma unroll
         for (int i = 0; i < CT; ++i) {
             const float g = gs[i * ks + c], k = kk[i * ks + c], q = qs[i * ks + c];
             p *= g;
             rec_q[fragment_at(i, c, dkp >> 3)] = q * p;
             col[i] = bs[i] * k * p;
-            if (i >= HB) {
-                pb *= g;
-                kf[(i - HB) * ks + c] = k * pb;
-                qf[(i - HB) * ks + c] = q * pb;
-            }
+            pb = i % HB ? pb * g : g;
+            kf[i * ks + c] = k * pb;
+            qs[i * ks + c] = q * pb;
+            if (i % HB == HB - 1) block[i / HB] = pb;
         }
         rec_p[c] = p;
+#pragma unroll
+        for (int from = 0; from < BLOCKS - 1; ++from) {
+            float gap = 1.f;
+#pragma unroll
+            for (int to = from + 1; to < BLOCKS; ++to) {
+                between[(to * (to - 1) / 2 + from) * ks + c] = gap;
+                gap *= block[to];
+            }
+        }
     }
     if (tid >= back && tid - back < dkp) {
         const int c = tid - back;
         float p = 1.f, pb = 1.f;
 #pragma unroll
-        for (int i = CT - 1; i >= 0; --i) {
-            const float g = gs[i * ks + c], k = kk[i * ks + c];
-            rec_k[fragment_at(c, i, CT >> 3)] = k * p;
-            p *= g;
-            if (i < HB) {
+        for (int i0 = CT - 16; i0 >= 0; i0 -= 16) {
+            float x[16];
+#pragma unroll
+            for (int u = 15; u >= 0; --u) {
+                const int i = i0 + u;
+                const float g = gs[i * ks + c], k = kk[i * ks + c];
+                x[u] = k * p;
+                p *= g;
+                if (u % HB == HB - 1) pb = 1.f;
                 ke[i * ks + c] = k * pb;
                 pb *= g;
             }
+            float4* at = reinterpret_cast<float4*>(rec_k + fragment_at(c, i0, CT >> 3));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) at[u] = make_float4(x[2 * u], x[2 * u + 1], x[2 * u + 8], x[2 * u + 9]);
         }
     }
     __syncthreads();
 
-    // inside the two blocks: thread (block, two neighbouring keys j, 16 lanes over the channels); m = k_j times the decays
-    // of tokens j + 1 .. i moves on with i, and the four sums of a row meet in five shuffles
+    // between the blocks: a tile of two rows and two keys per two threads, which take every other four channels
     {
-        const int block = tid >> 7, jg = (tid >> 4) & 7, lane = tid & 15;
-        const int base = block * HB, j0 = jg * 2;
-        constexpr int PAIRS = PER / 2;             // of neighbouring channels
-        auto pair = [&](const float* x, int row, int u) {
-            return *reinterpret_cast<const uint64_t*>(x + row * ks + 2 * lane + 32 * u);
-        };
-        uint64_t m0[PAIRS], m1[PAIRS];
+        const int item = tid >> 1, half = tid & 1, pair = item >> 2;
+        int to = 1;
+        while (to * (to + 1) / 2 <= pair) ++to;
+        const int from = pair - to * (to - 1) / 2;
+        const bool real = pair < BLOCK_PAIRS;
+        const int i = real ? to * HB + (item >> 1 & 1) * 2 : 0, j = real ? from * HB + (item & 1) * 2 : 0;
+        uint64_t sa[2][2] = {}, sb[2][2] = {};
+        if (real)
+            for (int c = half; c < dkp >> 2; c += 2) {
+                auto row = [&](const float* x, int r) { return reinterpret_cast<const ulonglong2*>(x + r * ks)[c]; };
+                const ulonglong2 g = row(between, pair);
 #pragma unroll
-        for (int u = 0; u < PAIRS; ++u) {
-            const bool in_row = 2 * lane + 32 * u < dkp;
-            m0[u] = in_row ? pair(kk, base + j0, u) : 0;
-            m1[u] = in_row ? pair(kk, base + j0 + 1, u) : 0;
-        }
-        const int from = (jg & ~1) * 2;            // the two key groups of a warp walk the same rows (shuffles need both)
-        for (int i = from; i < HB; ++i) {
-            uint64_t sa0 = 0, sa1 = 0, sb0 = 0, sb1 = 0;
-            const bool on0 = i > j0, on1 = i > j0 + 1;
+                for (int v = 0; v < 2; ++v) {
+                    ulonglong2 e = row(ke, j + v);
+                    e.x = mul2(e.x, g.x);
+                    e.y = mul2(e.y, g.y);
 #pragma unroll
-            for (int u = 0; u < PAIRS; ++u) {
-                if (2 * lane + 32 * u < dkp) {
-                    const uint64_t g = pair(gs, base + i, u), k = pair(kk, base + i, u), q = pair(qs, base + i, u);
-                    if (on0) m0[u] = mul2(m0[u], g);
-                    if (on1) m1[u] = mul2(m1[u], g);
-                    sa0 = fma2(k, m0[u], sa0); sb0 = fma2(q, m0[u], sb0);
-                    sa1 = fma2(k, m1[u], sa1); sb1 = fma2(q, m1[u], sb1);
+                    for (int u = 0; u < 2; ++u) {
+                        const ulonglong2 k = row(kf, i + u), q = row(qs, i + u);
+                        sa[u][v] = fma2(k.x, e.x, fma2(k.y, e.y, sa[u][v]));
+                        sb[u][v] = fma2(q.x, e.x, fma2(q.y, e.y, sb[u][v]));
+                    }
                 }
             }
-            const float a0 = both(sa0), a1 = both(sa1), b0 = both(sb0), b1 = both(sb1);
-            // lanes 0-7 keep (a0, b0), lanes 8-15 (a1, b1); then each half of those keeps one of the two
-            const bool hi8 = lane & 8, hi4 = lane & 4;
-            float x = hi8 ? a1 : a0, y = hi8 ? b1 : b0;
-            x += __shfl_xor_sync(0xffffffffu, hi8 ? a0 : a1, 8);
-            y += __shfl_xor_sync(0xffffffffu, hi8 ? b0 : b1, 8);
-            float z = hi4 ? y : x;
-            z += __shfl_xor_sync(0xffffffffu, hi4 ? x : y, 4);
-            z += __shfl_xor_sync(0xffffffffu, z, 2);
-            z += __shfl_xor_sync(0xffffffffu, z, 1);
-            const int j = j0 + (hi8 ? 1 : 0);
-            if ((lane & 3) == 0) {
-                if (hi4) { if (i >= j) Bm[(base + i) * CT + base + j] = z; }
-                else if (i > j) L[(base + i) * CT + base + j] = bs[base + i] * z;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const float a = both(sa[u][v]), bsum = both(sb[u][v]);
+                // the first thread of the two finishes A, the other B
+                const float sum = (half ? bsum : a) + __shfl_xor_sync(0xffffffffu, half ? a : bsum, 1);
+                if (!real) continue;
+                if (half) Bm[(i + u) * CT + j + v] = sum;
+                else L[(i + u) * CT + j + v] = bs[i + u] * sum;
             }
-        }
-    }
-    // between the blocks: thread (row of the second, key of the first)
-    {
-        const int i = tid >> 4, j = tid & 15;
-        uint64_t sa = 0, sb = 0;
-        const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(kf + i * ks);
-        const ulonglong2* qr = reinterpret_cast<const ulonglong2*>(qf + i * ks);
-        const ulonglong2* er = reinterpret_cast<const ulonglong2*>(ke + j * ks);
-        for (int c = 0; c < dkp >> 2; ++c) {
-            const ulonglong2 k = kr[c], q = qr[c], e = er[c];
-            sa = fma2(k.x, e.x, fma2(k.y, e.y, sa));
-            sb = fma2(q.x, e.x, fma2(q.y, e.y, sb));
-        }
-        const float a = both(sa), bsum = both(sb);
-        L[(HB + i) * CT + j] = bs[HB + i] * a;
-        Bm[(HB + i) * CT + j] = bsum;
     }
     __syncthreads();
     for (int e = tid; e < CT * CT; e += THREADS) rec_b[fragment_at(e / CT, e % CT, CT >> 3)] = Bm[e];
 
     // the solve: x_i = r_i - sum_(j<i) L_ij x_j, a thread per column of [diag(b) (P k) | diag(b) V]
     const int columns = dkp + (dv + NC - 1) / NC * NC;
-    for (int item = tid; item < columns; item += THREADS) {
+    for (int item = delta ? tid : tid + dkp; item < columns; item += THREADS) {      // (the plain recurrence needs no keys here)
         const bool key = item < dkp;
-        if (key && !delta) continue;
         const int c = item - dkp;
         if (!key) {
 #pragma unroll
@@ -675,21 +704,20 @@ extern "C" int lp_chunked_recurrence(const float* proj, int ld, int q_off, int k
                     rd == 0 && (dk & 3) == 0 && (ld & 3) == 0 && (q_off & 3) == 0 && (k_off & 3) == 0 && ((uintptr_t)proj & 15) == 0 &&
                         (decay_form != DECAY_CHANNEL || ((uintptr_t)decay & 15) == 0)};
     const int dkp = padded(dk), delta = beta ? 1 : 0;
-    const size_t smem_p = ((size_t)(3 * CT + 3 * HB) * (dkp + 4) + 2 * CT * CT + CT) * sizeof(float);
+    const size_t smem_p = ((size_t)(5 * CT + BLOCK_PAIRS) * (dkp + 4) + 2 * CT * CT + CT) * sizeof(float);
     const size_t stage = (size_t)(record_floats(dkp, delta) + CT * NC) * sizeof(float);
     const int kt = dkp / 16;
     const size_t kept = (size_t)((delta ? 2 : 4) + kt * 2) * JOINERS * 32 * sizeof(float4);
     const int stages = kept + 3 * stage <= MAX_SMEM ? 3 : kept + 2 * stage <= MAX_SMEM ? 2 : 1;      // (plain: two at least)
     const size_t smem_c = kept + stages * stage;
-    auto prepare = dk <= 64 ? prepare_kernel<4> : dk <= 128 ? prepare_kernel<8> : prepare_kernel<16>;
-    const int size = dk <= 64 ? 0 : dk <= 128 ? 1 : 2;
+    auto prepare = dkp <= NARROW_DK ? prepare_kernel<true> : prepare_kernel<false>;
     const bool wide = dkp > NARROW_DK;                        // (narrow: three stages always fit)
     auto carry = delta ? (!wide ? carry_kernel<3, true, false> : stages == 3 ? carry_kernel<3, true, true>
                           : stages == 2 ? carry_kernel<2, true, true> : carry_kernel<1, true, true>)
                        : (!wide ? carry_kernel<3, false, false> : stages == 3 ? carry_kernel<3, false, true>
                                                                               : carry_kernel<2, false, true>);
-    static size_t granted_p[3] = {}, granted_c[2][4] = {};       // what each kernel has been allowed so far
-    int rc = reserve(prepare, smem_p, granted_p[size]);
+    static size_t granted_p[2] = {}, granted_c[2][4] = {};       // what each kernel has been allowed so far
+    int rc = reserve(prepare, smem_p, granted_p[dkp <= NARROW_DK]);
     if (rc) return rc;
     rc = reserve(carry, smem_c, granted_c[delta][wide ? stages : 0]);
     if (rc) return rc;
