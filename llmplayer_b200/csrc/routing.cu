@@ -11,9 +11,57 @@
 // before one stacked down product sums them; `lp_expert_scale` is that multiplication. Many tokens run each expert for the
 // tokens that chose it instead (gemm_experts.cu).
 // Among equal scores the expert (group) with the lower index wins. Everything is float32.
-#include "common.cuh"
+#include "bf16_parts.cuh"
 
 namespace {
+
+// out[t, e] = sum_k x[t, k] w[e, k] for a few rows of w (a router's): 16 tokens per CTA, a warp per eighth of K, the warps' sums added in
+// one order, so that a token's result does not depend on the tokens beside it. The products' operands are read as they lie: both take the
+// columns of 32 in the same order, a lane 8 neighbouring ones, which are the pairs of two steps of mma.sync. TILES: of 8 rows of w.
+// Bound by the latency of two round trips and its bytes, with more rows by reading w again for every 16 tokens. As a product in tiles of 128
+// x 64 (few CTAs, each with K in one chain) / so, B200, us: 2048 tokens, 8 rows of 2048 11.8 / 3.6, 32 rows 11.7 / 7.7, 64 rows 11.7 / 15.1;
+// 512 tokens, 16 rows of 1024 6.9 / 2.9; 300 tokens, 33 rows of 1024 6.9 / 6.2; 2048 tokens, 33 rows of 4096 20.9 / 20.4: up to 32 rows.
+constexpr int RL_TOKENS = 16, RL_WARPS = 8;
+template <int TILES>
+__global__ void __launch_bounds__(RL_WARPS * 32)
+router_logits_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, float* __restrict__ out, int ldo, int T, int E,
+                     int K) {
+    __shared__ float sums[RL_WARPS][RL_TOKENS][TILES * 8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+    const int t0 = blockIdx.x * RL_TOKENS, chunks = K / 32;
+    const int lo = warp * chunks / RL_WARPS, hi = (warp + 1) * chunks / RL_WARPS;
+    lp_grid_release();
+    lp_grid_wait();
+    const uint4 none = make_uint4(0, 0, 0, 0);
+    const bool real[2] = {t0 + g8 < T, t0 + g8 + 8 < T};
+    const uint4* rows[2] = {reinterpret_cast<const uint4*>(x + (long long)(real[0] ? t0 + g8 : 0) * K) + t4,
+                            reinterpret_cast<const uint4*>(x + (long long)(real[1] ? t0 + g8 + 8 : 0) * K) + t4};
+    float acc[TILES][4] = {};
+#pragma unroll 4
+    for (int c = lo; c < hi; ++c) {
+        const uint4 a = real[0] ? rows[0][c * 4] : none, b = real[1] ? rows[1][c * 4] : none;
+        const uint32_t first[4] = {a.x, b.x, a.y, b.y}, second[4] = {a.z, b.z, a.w, b.w};
+#pragma unroll
+        for (int n = 0; n < TILES; ++n) {
+            const int e = n * 8 + g8;
+            const uint4 v = e < E ? reinterpret_cast<const uint4*>(w + (long long)e * K)[c * 4 + t4] : none;
+            mma_bf16(acc[n], first, v.x, v.y);
+            mma_bf16(acc[n], second, v.z, v.w);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < TILES; ++n)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sums[warp][g8 + (k >> 1) * 8][n * 8 + t4 * 2 + (k & 1)] = acc[n][k];
+    __syncthreads();
+    for (int i = threadIdx.x; i < RL_TOKENS * TILES * 8; i += RL_WARPS * 32) {
+        const int r = i / (TILES * 8), e = i % (TILES * 8);
+        float sum = 0.f;
+#pragma unroll
+        for (int k = 0; k < RL_WARPS; ++k) sum += sums[k][r][e];
+        if (t0 + r < T && e < E) out[(long long)(t0 + r) * ldo + e] = sum;
+    }
+}
 
 // A warp per token. Shared memory per warp: s[E], allowed/chosen flags[E] (as float), group scores[groups].
 __global__ void __launch_bounds__(128)
@@ -407,6 +455,16 @@ identity_experts_kernel(float* __restrict__ x, const TH* __restrict__ h, const f
 }
 
 }  // namespace
+
+// x: bfloat16 [T, K], w: bfloat16 [E, K], out: float32 [T, ldo], E values per row written. At most 32 rows of w, K a multiple of 32.
+extern "C" int lp_router_logits(const void* x, const void* w, float* out, int ldo, int T, int E, int K, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (E <= 0 || E > 32 || ldo < E) LP_REFUSE("router_logits: %d rows (at most 32) into rows of %d", E, ldo);
+    if (K <= 0 || K % 32 || (((uintptr_t)x | (uintptr_t)w) & 15) != 0) LP_REFUSE("router_logits: rows of %d values (a multiple of 32, 16-byte aligned)", K);
+    auto kernel = E <= 8 ? router_logits_kernel<1> : E <= 16 ? router_logits_kernel<2> : router_logits_kernel<4>;
+    lp_launch(kernel, (T + RL_TOKENS - 1) / RL_TOKENS, RL_WARPS * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, ldo, T, E, K);
+    return lp_check_launch("router_logits");
+}
 
 // z: float32 [T, ldz] (E logits per row); weights: float32 [T, ldw], E values per row written.
 extern "C" int lp_route(const float* z, int ldz, float* weights, int ldw, int T, int E, int groups, int keep, int top,

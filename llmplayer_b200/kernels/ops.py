@@ -45,6 +45,7 @@ _SIGNATURES = {
         "lp_relu2": [_P, _I, _P, _I, _I, _I, _P, ctypes.c_longlong, _P],
     },
     "routing": {
+        "lp_router_logits": [_P, _P, _P, _I, _I, _I, _I, _P],
         "lp_route": [_P, _I, _P, _I, _I, _I, _I, _I, _I, _P],
         "lp_expert_scale": [_P, _I, _I, _P, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _P, _I, _I, _I, _I, _P],
         "lp_route_top": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P],
@@ -2160,6 +2161,28 @@ def relu2(z: torch.Tensor, out: torch.Tensor, clear: Optional[torch.Tensor] = No
 
 
 # --------------------------------------------------------------------------- routing of a mixture of experts
+ROUTER_ROWS = 32              # rows of a map that router_logits takes
+
+
+def router_logits_serves(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether :func:`router_logits` takes this product. Up to 32 rows of ``w`` a product in tiles of 128 features computes mostly padding,
+    and its K is one chain per tile of tokens (both sides measured: beside the kernel)."""
+    return w.shape[0] <= ROUTER_ROWS and w.shape[1] % 32 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0
+
+
+def router_logits(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out = x @ w.T with float32 sums in one order, for a map of few rows: ``x`` [T, K] and ``w`` [E, K] bfloat16, ``out``
+    float32 [T, E] (may be a column slice)."""
+    _want(x, "router_logits x", torch.bfloat16, 2)
+    _want(w, "router_logits w", torch.bfloat16, 2)
+    ptr, ldo = _slice(out, "router_logits out")
+    if w.shape[1] != x.shape[1] or out.shape != (x.shape[0], w.shape[0]):
+        raise KernelError(f"router_logits: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    lib = library("routing")
+    _check(lib, lib.lp_router_logits(x.data_ptr(), w.data_ptr(), ptr, ldo, x.shape[0], w.shape[0], x.shape[1], _stream()))
+    return out
+
+
 def route(logits: torch.Tensor, weights: torch.Tensor, *, groups: int, keep: int, top: int) -> torch.Tensor:
     """weights[t, e] = the weight of expert e for token t (zero if it was not chosen) from the router's float32
     ``logits`` [T, E] (may be a column slice): scores sigmoid(logit); a group of E / groups neighbours scores the sum

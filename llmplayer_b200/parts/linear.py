@@ -49,6 +49,11 @@ class Linear:
     def store(self, x: torch.Tensor, out: torch.Tensor, ctx=None, ordered: bool = False) -> torch.Tensor:
         """``ordered``: every element's sum is taken in one order, so that the same input gives the same bits (no partial sums that
         meet in atomics)."""
+        if (ordered and self._fast() and x.dtype == torch.bfloat16 and out.dtype == torch.float32
+                and ops.router_logits_serves(x, self.weight)):
+            if ctx is not None:
+                ctx.take_cleared()
+            return ops.router_logits(x, self.weight, out)
         if (ordered and self._fast() and x.dtype == torch.bfloat16
                 and ops.gemm_adds_parts(x.shape[0], self.out_features, self.in_features)):
             if ctx is not None:
