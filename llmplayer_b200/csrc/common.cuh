@@ -4,6 +4,8 @@
 // Every entry point is `extern "C" int lp_*(...)`: 0 on success, a positive
 // cudaError_t when a launch failed, -1 when the arguments were refused; the
 // text of the last refusal or failure is kept per library (lp_last_error).
+// Entry points of fused work return LP_NOT_SERVED, which is neither, for operands that
+// go through the separate kernels: nothing was launched then.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -13,6 +15,7 @@
 
 #define LP_F32 0
 #define LP_BF16 1
+#define LP_NOT_SERVED (-2)
 
 #ifndef LP_ERROR_DEFINED
 #define LP_ERROR_DEFINED

@@ -669,7 +669,7 @@ gated_sum_norm_kernel(float* __restrict__ x, const float* __restrict__ a, const 
 
 constexpr int SUM_NORM_MAX = 8192;      // values per row that the fused kernel takes
 
-// w, eps, out: the layer norm's; the other operands as for lp_gated_sum. 1: rows that this kernel does not take (nothing was launched).
+// w, eps, out: the layer norm's; the other operands as for lp_gated_sum. LP_NOT_SERVED: rows that this kernel does not take.
 extern "C" int lp_gated_sum_norm(float* x, const float* a, const float* ga, int ldga, const float* ba, const float* b,
                                  const float* gb, int ldgb, const float* bb, float* streams, const float* mix, int count,
                                  int keep_input, int T, int d, const float* w, float eps, void* out, int out_dtype,
@@ -681,7 +681,7 @@ extern "C" int lp_gated_sum_norm(float* x, const float* a, const float* ga, int 
     const bool whole = d % 4 == 0 && (!ga || ldga % 4 == 0) && (!gb || ldgb % 4 == 0) &&
                        (((uintptr_t)x | (uintptr_t)a | (uintptr_t)ga | (uintptr_t)ba | (uintptr_t)b | (uintptr_t)gb | (uintptr_t)bb |
                          (uintptr_t)streams | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
-    if (!whole || d > SUM_NORM_MAX) return 1;
+    if (!whole || d > SUM_NORM_MAX) return LP_NOT_SERVED;
 #define LP_LAUNCH_SUM(TOut, QUADS)                                                                                                 \
     lp_launch(gated_sum_norm_kernel<TOut, QUADS>, T, 512, 0, stream, x, a, ga, ldga, ba, b, gb, ldgb, bb, streams, mix, count, keep_input, \
               T, d, w, eps, (TOut*)out)

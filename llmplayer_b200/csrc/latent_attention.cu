@@ -1306,7 +1306,7 @@ bool absorb_on_tensor_cores(int w_dtype, int dn, int dr, int rank, const void* u
 }  // namespace
 
 // What lp_latent_prepare and lp_latent_absorb do one after the other, in one launch, for a 16-bit cache and 16-bit weights; see there for
-// the operands. Returns 1 (nothing was launched) for sizes and addresses that it does not take.
+// the operands. Returns LP_NOT_SERVED for sizes and addresses that it does not take.
 extern "C" int lp_latent_queries(const float* proj, int ld, int q_off, int kv_off, const float* gain, float eps, const float* inv_freq,
                                  int rot, const int* positions, const int* seq_ids, const int* page_table, int pt_stride, void* pages,
                                  int kv_dtype, int T, int H, int dn, int dr, int rank, int page_size, const float* q_sep, int ldq,
@@ -1317,7 +1317,7 @@ extern "C" int lp_latent_queries(const float* proj, int ld, int q_off, int kv_of
     if (H <= 0 || H >= 65535 || page_size <= 0 || kv_dtype != LP_BF16 || rot < 0 || (rot & 1) || rot > dr || (rot > 0 && !inv_freq) || q_off < 0 ||
         kv_off < 0 || kv_off + rank + dr > ld || (q_sep ? 0 : q_off) + H * (dn + dr) > ldq || !absorb_on_tensor_cores(w_dtype, dn, dr, rank, uk, qa) ||
         ld % 4 || ldq % 4 || kv_off % 4 || dr % 4 || (((uintptr_t)q | (uintptr_t)proj | (uintptr_t)gain | (uintptr_t)pages) & 15) != 0)
-        return 1;
+        return LP_NOT_SERVED;
     const KeyRows k{proj + kv_off, ld, gain, eps, inv_freq, rot, interleaved, magnitude, positions, seq_ids, page_table, pt_stride, page_size,
                     (__nv_bfloat16*)pages};
     const size_t bytes = absorb_bytes(dn);

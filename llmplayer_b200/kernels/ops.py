@@ -19,7 +19,7 @@ from . import build
 
 F32, BF16 = 0, 1
 STORE, ACCUMULATE, SWIGLU = 0, 1, 2
-NOT_SERVED = 1          # what an entry of fused work returns for sizes that go through the separate kernels (nothing was launched)
+NOT_SERVED = -2         # what an entry of fused work returns for operands that go through the separate kernels (nothing was launched)
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
 
 _P, _I, _F = c_void_p, c_int, c_float
