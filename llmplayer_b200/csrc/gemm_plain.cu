@@ -2,10 +2,15 @@
 // Every output element is summed in one fixed way whatever M is, so a row's result does not depend on which other rows share the
 // launch: K is cut into eighths (rounded up to 32 products), each eighth is a sum of its own, the eighths of each half are
 // added in increasing order, then the halves. Two ways of forming an eighth:
-//   * rows of float32 that can be read 16 bytes at a time: on the tensor cores, float32 numbers as three bfloat16 parts, with
-//     errors below those of a chain of multiply-adds (gemm_f32_rows_kernel up to 16 rows, gemm_f32_split_kernel from 17 on: the same bits);
+//   * rows of 64 float32 and more that can be read 16 bytes at a time: on the tensor cores, float32 numbers as three bfloat16 parts
+//     (gemm_f32_rows_kernel up to 16 rows, gemm_f32_split_kernel from 17 on: the same bits);
 //   * any other types, sizes and alignments: a chain of multiply-adds in increasing k that starts at zero (gemm_plain_kernel, which
 //     adds all eighths in order).
+// Errors against 64 bits, root mean square in units of 2^-24 of the sum of the products' magnitudes, in parts / by multiply-adds, at
+// K = 64, 256, 2048, 8192: normal numbers 0.17 / 0.35, 0.11 / 0.19, 0.05 / 0.17, 0.04 / 0.17; numbers in [1, 2) 0.82 / 1.21, 0.90 / 0.96,
+// 0.92 / 1.62, 1.02 / 2.94; numbers of very different sizes (normal times e^(2 normal)) 0.62 / 1.02, 0.62 / 0.92, 0.54 / 1.58, 0.55 / 2.30; mantissas
+// of ones 1.16 / 1.63, 1.22 / 2.22, 1.43 / 2.38, 1.64 / 115, but 1.17 / 0.87 at K = 16: hence the line at 64. A product that stands alone in its sum is off
+// by 0.63 (3.5 at most) where a rounded one is by 0.42 (1.0).
 // It is the product of the float32 path and the comparison twin of the bfloat16 kernels.
 //
 // Counterparts in the reference (src/main/resources/kernels/cuda/): matmul_f32.cu:6-39,
@@ -123,10 +128,13 @@ gemm_plain_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __rest
 
 // ---------------------------------------------------------------- float32 on the tensor cores
 // A float32 number is the sum of three bfloat16 ones (3 x 8 bits), and a product of two such parts is exact in float32. So a
-// product of float32 numbers is six products on the tensor cores: all pairs of parts but the three smallest (2^-24 of the
-// whole and below). What would lose bits is their sum: the tensor cores cut every partial sum off instead of rounding it. So
+// product of float32 numbers is six products on the tensor cores: all pairs of parts but the three smallest (together at most 3 x 2^-24 of
+// the whole, of either sign: split_tokens). What would lose bits is their sum: the tensor cores cut every partial sum off instead of rounding it. So
 // the sums in tensor memory are short: 32 products of K, the small pairs first, the two steps of the leading parts last
 // (a step is 16 products); such a block's sum is added to those before it in registers, rounded to nearest, as fmaf would.
+// The exponents of float32 and bfloat16 end at the same place, parts and products of parts do not: operands are taken times 2^24, so that
+// every part of every float32 number has room and no product that a float32 result could hold vanishes, and sums times 2^-48 at the end; sums beyond 2^80
+// are formed again one by one, like those that are not finite.
 //
 // Per CTA: 128 weight rows (in the gated form 64 gate and the 64 up rows of the same features) x TOK tokens.
 //   warp 0       TMA: float32 boxes of 32 columns of the weights into a ring of stages
@@ -137,10 +145,12 @@ gemm_plain_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __rest
 //   the last 4 or 8   a block's sums from tensor memory into registers, chains of an eighth of K, the output
 // Two buffers of operands and two of sums, so that all of these work at the same time on neighbouring blocks. Bound by the way round one
 // buffer (sums fetched, weights split, MMAs of about 80 cycles each beside the traffic to tensor memory): about 1,100 cycles per block
-// against 790 for its MMAs alone. B200, 509 rows, against register tiles of paired multiply-adds: 16384 x 2048 (gated) 831 -> 232 us,
-// 2048 x 8192 414 -> 120, 3072 x 2048 167 -> 58, 2048 x 2048 120 -> 50; error against 64 bits 2.9e-7 .. 5.8e-7 -> 1.3e-7 .. 1.6e-7.
-// 64 tokens: 133 -> 64 us, 139 -> 60, 43 -> 28, 43 -> 34.
+// against 790 for its MMAs alone. B200, each product back to back with itself (weights partly in L2), against register tiles of paired multiply-adds, 509
+// rows: 16384 x 2048 (gated) 820 -> 222 us, 2048 x 8192 407 -> 105, 3072 x 2048 163 -> 53, 2048 x 2048 111 -> 39; the four one behind the other
+// (243 MB of weights, cold) 1499 -> 420. 64 rows: 130 -> 60, 121 -> 53, 34 -> 22, 34 -> 26; together 359 -> 177. 17 rows: together 301 -> 170.
 constexpr int SPLIT_K = 32;                     // products of a block
+constexpr int SPLIT_MIN_K = 64;                 // shorter sums run on gemm_plain_kernel
+constexpr float SPLIT_SCALE = 16777216.f, SUM_SCALE = 1.f / (SPLIT_SCALE * SPLIT_SCALE);      // 2^24 of an operand, 2^-48 of a sum
 
 template <int TOK> struct SplitTile {
     static constexpr int ADDERS = TOK == 128 ? 8 : 4;             // warps that add blocks up
@@ -180,19 +190,50 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ uint64_t smem_desc_rows64(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
 }
-// Two neighbouring values in three parts each, cut off and not rounded (byte moves and masks; the conversion to bfloat16 issues at a
-// quarter of their rate): 8 + 8 + 8 bits are all 24. An infinity or a NaN makes sums that are no numbers, which the epilogue
-// forms again one by one.
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-    auto rest = [&]() {
-        asm("{\n\t.reg .b64 v, h;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 h, {%2, %3};\n\tsub.rn.f32x2 v, v, h;\n\tmov.b64 {%0, %1}, v;\n\t}"
-            : "+f"(x), "+f"(y) : "r"(__float_as_uint(x) & 0xffff0000u), "r"(__float_as_uint(y) & 0xffff0000u));
-    };
-    a = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
-    rest();
-    b = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
-    rest();
-    c = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+// Neighbouring values, times 2^24, in three parts each: leading eight bits, the next eight, the rest. An infinity or a NaN, or a value
+// that the factor or the rounding takes beyond the range, makes sums that are no numbers, which the epilogue forms again one by one.
+__device__ __forceinline__ void scale_pair(float& x, float& y) {
+    asm("{\n\t.reg .b64 v, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 f, {%2, %2};\n\tmul.rn.f32x2 v, v, f;\n\tmov.b64 {%0, %1}, v;\n\t}"
+        : "+f"(x), "+f"(y) : "f"(SPLIT_SCALE));
+}
+template <bool ROUND>
+__device__ __forceinline__ uint32_t leading_pair(float& x, float& y) {       // x and y keep what is behind their leading bits
+    const uint32_t p = __float_as_uint(x) + (ROUND ? 0x8000u : 0u), q = __float_as_uint(y) + (ROUND ? 0x8000u : 0u);
+    asm("{\n\t.reg .b64 v, h;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 h, {%2, %3};\n\tsub.rn.f32x2 v, v, h;\n\tmov.b64 {%0, %1}, v;\n\t}"
+        : "+f"(x), "+f"(y) : "r"(p & 0xffff0000u), "r"(q & 0xffff0000u));
+    return __byte_perm(p, q, 0x7632);
+}
+__device__ __forceinline__ uint32_t cut_pair(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+
+// Weights: cut off (byte moves and masks; the conversion to bfloat16 issues at a quarter of their rate).
+__device__ __forceinline__ void split_weights(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
+    scale_pair(x, y);
+    a = leading_pair<false>(x, y);
+    b = leading_pair<false>(x, y);
+    c = cut_pair(x, y);
+}
+// Tokens, four values of a row at a time (k, k + 1 in the first of two words): the first two parts rounded to nearest (a tie away from
+// zero), so that what is left out of a product has either sign. Where one of the four has a third part, 2^-25 of each is added to
+// it, against the two cuts of a block's leading sum, which take off some 0.9 x 2^-24 of numbers of one sign: as much as leaves sums that are
+// exact as they are (with 3/4 of 2^-24 numbers just below a power of two came back a last bit larger from a product with one).
+__device__ __forceinline__ void split_tokens(const float4& v, uint32_t* a, uint32_t* b, uint32_t* c) {
+    float x[4] = {v.x, v.y, v.z, v.w}, whole[4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        scale_pair(x[2 * i], x[2 * i + 1]);
+        whole[2 * i] = x[2 * i];
+        whole[2 * i + 1] = x[2 * i + 1];
+        a[i] = leading_pair<true>(x[2 * i], x[2 * i + 1]);
+        b[i] = leading_pair<true>(x[2 * i], x[2 * i + 1]);
+    }
+    const uint32_t any = (__float_as_uint(x[0]) | __float_as_uint(x[1])) | (__float_as_uint(x[2]) | __float_as_uint(x[3]));
+    const float share = any ? 0x1p-25f : 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        asm("{\n\t.reg .b64 v, h, f;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 h, {%2, %3};\n\tmov.b64 f, {%4, %4};\n\tfma.rn.f32x2 v, h, f, v;\n\t"
+            "mov.b64 {%0, %1}, v;\n\t}" : "+f"(x[2 * i]), "+f"(x[2 * i + 1]) : "f"(whole[2 * i]), "f"(whole[2 * i + 1]), "f"(share));
+        c[i] = cut_pair(x[2 * i], x[2 * i + 1]);
+    }
 }
 
 // The values are formed here and not where they are used, behind a wait: the time from the end of a block's MMAs to the buffer's next
@@ -211,11 +252,10 @@ split_rows_kernel(const float* __restrict__ A, uint16_t* __restrict__ parts, int
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < pieces; i += (long long)gridDim.x * 256) {
         const int m = (int)(i / (K / 4)), k = (int)(i % (K / 4)) * 4;
         const float4 v = *(const float4*)(A + (long long)m * lda + k);
-        uint2 p[3];
-        split_pair(v.x, v.y, p[0].x, p[1].x, p[2].x);
-        split_pair(v.z, v.w, p[0].y, p[1].y, p[2].y);
+        uint32_t p[3][2];
+        split_tokens(v, p[0], p[1], p[2]);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) *(uint2*)(parts + ((long long)q * M + m) * ldp + k) = p[q];
+        for (int q = 0; q < 3; ++q) *(uint2*)(parts + ((long long)q * M + m) * ldp + k) = make_uint2(p[q][0], p[q][1]);
     }
 }
 
@@ -303,7 +343,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 tma_load_2d(to, &map_w, k_begin + b * SPLIT_K, n0, &full[s]);
                 if (GATED) tma_load_2d(to + T::W_BYTES / 2, &map_w, k_begin + b * SPLIT_K, N + n0, &full[s]);
             };
-            // no kernel of a step writes weights, and this thread touches nothing else: it does not wait for the kernel before
+            // this thread reads nothing but weights, and split_rows_kernel lets this kernel start only when all before it has ended: no wait
             int b = 0;
             for (; b < blocks; ++b) {
                 if (!mbar_wait(&empty[b % T::STAGES], ((b / T::STAGES) & 1) ^ 1)) { atomicExch(status, 71); *failed = 1; break; }
@@ -390,8 +430,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             uint32_t p[3][16];
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                split_pair(v[c].x, v[c].y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
-                split_pair(v[c].z, v[c].w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
+                split_weights(v[c].x, v[c].y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
+                split_weights(v[c].z, v[c].w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
             }
             keep_here(&p[0][0], 48);
             __syncwarp();
@@ -485,7 +525,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const bool adder = warp >= T::FIRST_ADDER;
     auto weight_row = [&](int f) { return W + (long long)f * ldw; };
     auto whole = [&](float v, int m, int f) {       // a sum that is no finite number is formed again
-        return fabsf(v) < INFINITY ? v : row_product(A + (long long)m * lda, weight_row(f), K);
+        return fabsf(v) < INFINITY ? v * SUM_SCALE : row_product(A + (long long)m * lda, weight_row(f), K);
     };
     auto store = [&](int m, int f, float v) {
         float* c = C + (long long)m * ldc + f;
@@ -575,17 +615,17 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
 // ---------------------------------------------------------------- float32, a handful of rows
 // A step of a few sequences reads every weight once and is bound by that: 16 weight rows (in the gated form 8 gate and 8 up rows) x
-// TOK tokens per CTA, a warp per chain of K. A warp copies its own stages (its rows' next 32 values, and the tokens'), splits them in
+// 8 or 16 tokens per CTA, a warp per chain of K. A warp copies its own stages, splits them in
 // registers and multiplies them with mma.sync, whose sums of 16 products are those of tcgen05.mma bit for bit: same steps, same
-// order, so a row's result is the same as in the tiles above. Nothing but the chains' sums crosses warps. Bound by the copies in flight
-// and the chain of twelve MMAs per block. B200, the four products of a layer of width 2048 one behind the other (243 MB), against a
-// thread per chain and weight row: 16 rows 169 -> 78 us, 8 rows 91 -> 62, 4 rows 64 -> 59, 1 row 53 -> 58 (4.2 TB/s).
+// order, so a row's result is the same as in the tiles above. Nothing but the chains' sums crosses warps. Bound by the copies in flight,
+// the splitting (100 of some 170 instructions per warp and block of 2 KB) and the chain of twelve MMAs per block. B200, the four products of a layer of width
+// 2048 one behind the other (243 MB), by a thread per chain and weight row with multiply-adds / in parts, us: 1 row 53 / 61, 4 rows 62 / 62, 8 rows 93 / 62, 16 rows 165 / 85.
 constexpr int ROW_FEATURES = 16;
 
 template <int TOK, bool DEEP> struct RowsShape {
     static constexpr int THREADS = PARTS * 32;
     static constexpr int STAGE = (ROW_FEATURES + TOK) * 128;      // bytes of a warp's stage: rows of 32 values
-    // two CTAs per SM; DEEP: one, for grids that have no more (four products of 4 rows: 73 us with the short ring everywhere, 59)
+    // two CTAs per SM; DEEP: one, for grids that have no more (four products of 16 rows: 85 us, 106 with the short ring everywhere)
     static constexpr int STAGES = (DEEP ? 200 : 96) * 1024 / (PARTS * STAGE);
     static constexpr int TOGETHER = DEEP && TOK == 8 ? 2 : 1;     // blocks whose MMAs (a chain of twelve) run side by side
     static constexpr size_t SMEM = (size_t)PARTS * STAGES * STAGE;
@@ -623,25 +663,25 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     const int piece = lane & 7, copy_row = lane >> 3;             // rows copy_row, + 4, + 8, ...
     auto weight_row = [&](int r) { return GATED ? (r < FEATURES ? n0 + r : N + n0 + r - FEATURES) : n0 + r; };
     auto feature_real = [&](int r) { return n0 + (GATED ? r % FEATURES : r) < N; };
-    const float* from_w[4];
-    bool real_w[4];
+    const float* from_w[4];                          // (rows that there are not repeat the first: their sums go nowhere)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = copy_row + i * 4;
-        real_w[i] = feature_real(r);
-        from_w[i] = W + (real_w[i] ? (long long)weight_row(r) * ldw : 0) + k_begin + piece * 4;
+        from_w[i] = W + (feature_real(r) ? (long long)weight_row(r) * ldw : 0);
     }
     const uint32_t to = copy_row * 128 + ((piece ^ ((copy_row & 1) * 4)) << 4);
     auto fetch_w = [&](int b) {
         if (b >= blocks) return;
-        uint8_t* stage = ring + b % S::STAGES * S::STAGE + to;
-        const bool inside = k_begin + b * SPLIT_K + piece * 4 < k_end;
+        uint8_t* stage = ring + (unsigned)b % S::STAGES * S::STAGE + to;
+        const int k = k_begin + b * SPLIT_K + piece * 4;
+        const bool inside = k < k_end;
+        const int at = inside ? k : 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) copy16(stage + i * 512, real_w[i] && inside ? from_w[i] + b * SPLIT_K : W, real_w[i] && inside);
+        for (int i = 0; i < 4; ++i) copy16(stage + i * 512, from_w[i] + at, inside);
     };
     auto fetch_x = [&](int b) {
         if (b >= blocks) return;
-        uint8_t* stage = ring + b % S::STAGES * S::STAGE + ROW_FEATURES * 128 + to;
+        uint8_t* stage = ring + (unsigned)b % S::STAGES * S::STAGE + ROW_FEATURES * 128 + to;
         const int k = k_begin + b * SPLIT_K + piece * 4;
 #pragma unroll
         for (int i = 0; i < TOK / 4; ++i) {
@@ -675,21 +715,20 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         uint32_t w[U][2][3][4], x[U][TILES][2][3][2];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const uint8_t* stage = ring + (b + u) % S::STAGES * S::STAGE;
+            const uint8_t* stage = ring + (unsigned)(b + u) % S::STAGES * S::STAGE;
             auto at = [&](int row, int step) { return *(const float4*)(stage + row * 128 + (((step * 4 + t) ^ ((row & 1) * 4)) << 4)); };
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float4 v = at(g + h * 8, s);
-                    split_pair(v.x, v.y, w[u][s][0][h], w[u][s][1][h], w[u][s][2][h]);
-                    split_pair(v.z, v.w, w[u][s][0][h + 2], w[u][s][1][h + 2], w[u][s][2][h + 2]);
+                    split_weights(v.x, v.y, w[u][s][0][h], w[u][s][1][h], w[u][s][2][h]);
+                    split_weights(v.z, v.w, w[u][s][0][h + 2], w[u][s][1][h + 2], w[u][s][2][h + 2]);
                 }
 #pragma unroll
                 for (int n = 0; n < TILES; ++n) {
                     const float4 v = at(ROW_FEATURES + n * 8 + g, s);
-                    split_pair(v.x, v.y, x[u][n][s][0][0], x[u][n][s][1][0], x[u][n][s][2][0]);
-                    split_pair(v.z, v.w, x[u][n][s][0][1], x[u][n][s][1][1], x[u][n][s][2][1]);
+                    split_tokens(v, x[u][n][s][0], x[u][n][s][1], x[u][n][s][2]);
                 }
             }
         }
@@ -750,7 +789,7 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
             }
             if (chains > PARTS / 2) v = first + v;
             // a sum that is no finite number is formed again
-            return fabsf(v) < INFINITY ? v : row_product(A + (long long)m * lda, W + (long long)weight_row(r) * ldw, K);
+            return fabsf(v) < INFINITY ? v * SUM_SCALE : row_product(A + (long long)m * lda, W + (long long)weight_row(r) * ldw, K);
         };
         float* out = C + (long long)m * ldc + n0 + f;
         if (GATED) *out = silu_mul(whole(f), whole(FEATURES + f));
@@ -834,7 +873,8 @@ int launch_tokens(const F32Call& c) {
     constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? 64 : 128;
     const long long tiles = (long long)((c.N + FEATURES - 1) / FEATURES) * ((c.M + TOK - 1) / TOK);
     const long long blocks = (c.K + SPLIT_K - 1) / SPLIT_K;
-    // how many CTAs share a tile's chains: the number whose busiest SM has least to do, a CTA's beginning and end counted as eight blocks
+    // how many CTAs share a tile's chains: the number whose busiest SM has least to do, a CTA's beginning and end counted as eight blocks (as none, the
+    // four products take 480 us for 509 rows and 213 for 17, as four 420 and 170, as eight 420 and 170, as sixteen 441 and 169)
     int best = 1;
     long long least = 0;
     for (int ctas = 1; ctas <= PARTS; ctas *= 2) {
@@ -866,10 +906,12 @@ int launch_rows(const F32Call& c) {
 
 template <int MODE>
 int launch_f32(const F32Call& c) {
-    // up to 16 rows the weights' bytes bound the product; the tiles start at 34 us for 2048 x 2048 where 16 rows take 14
+    // up to 16 rows the weights' bytes bound the product; four products (above), us: 16 rows 85, 17 rows in a tile of 64 170, as two launches of 16
+    // would take, 32 rows 172
     if (c.M <= 8) return launch_rows<8, MODE>(c);
     if (c.M <= 16) return launch_rows<16, MODE>(c);
-    // from 65 rows on a tile of 128 splits the weights half as often (509 rows, gated: 232 us, 315 in tiles of 64)
+    // from 65 rows on a tile of 128 splits the weights half as often (the four, tiles of 64 / 128: 65 rows 221 / 206, 96 rows 225 / 210, 130 rows
+    // 323 / 293, 190 rows 339 / 311, 256 rows 373 / 322, 509 rows 630 / 420)
     if (c.M <= 64) return launch_tokens<64, MODE>(c);
     return launch_tokens<128, MODE>(c);
 }
@@ -897,9 +939,9 @@ int launch_out(const void* A, const void* W, void* C, int c_dtype, int M, int N,
     return launch_mode<TA, TW, __nv_bfloat16>(A, W, C, M, N, K, lda, ldw, ldc, mode, stream);
 }
 
-// rows of float32 that can be read 16 bytes at a time go to the tensor cores, everything else to the kernel for any types
+// rows of float32 that can be read 16 bytes at a time go to the tensor cores, everything else (and short sums) to the kernel for any types
 bool wide_f32(const void* A, int a_dtype, const void* W, int w_dtype, int c_dtype, int K, int lda, int ldw) {
-    return a_dtype == LP_F32 && w_dtype == LP_F32 && c_dtype == LP_F32 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0
+    return a_dtype == LP_F32 && w_dtype == LP_F32 && c_dtype == LP_F32 && K >= SPLIT_MIN_K && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0
            && (size_t)A % 16 == 0 && (size_t)W % 16 == 0;
 }
 

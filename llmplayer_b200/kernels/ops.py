@@ -701,7 +701,8 @@ def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, angles: Optional[torch.Tenso
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = STORE) -> torch.Tensor:
     """out (=|+=) a @ w.T at float32 precision, each element in one fixed order whatever the number of rows.
 
-    ``SWIGLU``: ``w`` is [2N, K], gate rows then up rows; out = silu(a gate^T) * (a up^T).
+    ``w`` is asked for before the kernel in front has ended where float32 rows are few (16 and less): as a step's weights it must not be what
+    the kernel launched just before, of this library, writes. ``SWIGLU``: ``w`` is [2N, K], gate rows then up rows; out = silu(a gate^T) * (a up^T).
     """
     _want(a, "gemm a", ndim=2)
     _want(w, "gemm w", ndim=2)
