@@ -3,7 +3,7 @@
 // launch: K is cut into eighths (rounded up to 32 products), each eighth is a sum of its own, the eighths of each half are
 // added in increasing order, then the halves. Two ways of forming an eighth:
 //   * rows of 64 float32 and more that can be read 16 bytes at a time: on the tensor cores, float32 numbers as three bfloat16 parts
-//     (gemm_f32_rows_kernel up to 16 rows, gemm_f32_split_kernel from 17 on: the same bits);
+//     (gemm_f32_few_kernel and gemm_f32_rows_kernel up to 16 rows, gemm_f32_split_kernel from 17 on: the same bits);
 //   * any other types, sizes and alignments: a chain of multiply-adds in increasing k that starts at zero (gemm_plain_kernel, which
 //     adds all eighths in order).
 // Errors against 64 bits, root mean square in units of 2^-24 of the sum of the products' magnitudes, in parts / by multiply-adds, at
@@ -615,11 +615,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
 // ---------------------------------------------------------------- float32, a handful of rows
 // A step of a few sequences reads every weight once and is bound by that: 16 weight rows (in the gated form 8 gate and 8 up rows) x
-// 8 or 16 tokens per CTA, a warp per chain of K. A warp copies its own stages, splits them in
+// 8 or 16 tokens per CTA and turn, a warp per chain of K. A warp copies its own stages, splits them in
 // registers and multiplies them with mma.sync, whose sums of 16 products are those of tcgen05.mma bit for bit: same steps, same
 // order, so a row's result is the same as in the tiles above. Nothing but the chains' sums crosses warps. Bound by the copies in flight,
 // the splitting (100 of some 170 instructions per warp and block of 2 KB) and the chain of twelve MMAs per block. B200, the four products of a layer of width
-// 2048 one behind the other (243 MB), by a thread per chain and weight row with multiply-adds / in parts, us: 1 row 53 / 61, 4 rows 62 / 62, 8 rows 93 / 62, 16 rows 165 / 85.
+// 2048 one behind the other (243 MB), by a thread per chain and weight row with multiply-adds / in parts, us: 1 row 53 / 54, 2 rows 55 / 56, 4 rows 62 / 56, 8 rows
+// 93 / 60, 16 rows 165 / 85.
 constexpr int ROW_FEATURES = 16;
 
 template <int TOK, bool DEEP> struct RowsShape {
@@ -798,6 +799,170 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     }
 }
 
+// Up to 8 tokens whose parts fit shared memory: a CTA per SM walks over the tiles of features and splits the tokens once, and its weights' ring
+// runs on from tile to tile. With a CTA per tile, which splits the tokens that it multiplies with again, the four products above take 61 us (1 row) to 62
+// (8 rows). GROUPS of eight warps walk over tiles of their own.
+template <int GROUPS_, int STAGES_, int TOGETHER_> struct FewShape {
+    static constexpr int GROUPS = GROUPS_, STAGES = STAGES_, TOGETHER = TOGETHER_, THREADS = GROUPS * PARTS * 32;
+    static constexpr int STAGE = ROW_FEATURES * 128;
+    static constexpr int RING = GROUPS * PARTS * STAGES * STAGE, SUMS = GROUPS * 2 * PARTS * 8 * ROW_FEATURES * 4;
+    static constexpr int ROOM = 225 * 1024 - RING - SUMS;            // for the tokens' parts
+};
+__host__ __device__ __forceinline__ int token_bytes(int K) { return part_length(K) * 6 + 32; }       // of one chain; tokens 32 bytes apart in the banks
+__host__ __device__ __forceinline__ int tokens_bytes(int M, int K) { return PARTS * M * token_bytes(K) + 64; }      // (a last pair of blocks reads on)
+
+template <int MODE, class S>
+__global__ void __launch_bounds__(S::THREADS, 1)
+gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, int lda, int ldw,
+                    int ldc) {
+    constexpr bool GATED = MODE == LP_GEMM_SWIGLU;
+    constexpr int FEATURES = GATED ? ROW_FEATURES / 2 : ROW_FEATURES, U = S::TOGETHER;
+    extern __shared__ __align__(128) uint8_t few_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int group = tid / (PARTS * 32), chain = (tid >> 5) % PARTS;
+    const int part = part_length(K);
+    const int k_begin = min(K, chain * part), k_end = min(K, k_begin + part);
+    const int blocks = (k_end - k_begin + SPLIT_K - 1) / SPLIT_K, steps = (blocks + U - 1) / U * U;
+    uint8_t* ring = few_smem + (group * PARTS + chain) * S::STAGES * S::STAGE;
+    float* sums = (float*)(few_smem + S::RING) + group * 2 * PARTS * 8 * ROW_FEATURES;       // [2][chain][token][weight row]
+    uint8_t* parts = few_smem + S::RING + S::SUMS;
+    const int x_row = token_bytes(K);
+    uint8_t* xs = parts + chain * M * x_row;                        // [token][part][value] of this chain
+    const int tiles = (N + FEATURES - 1) / FEATURES, stride = (int)gridDim.x * S::GROUPS;
+    const int first = (int)blockIdx.x + group * (int)gridDim.x;
+
+    // copies: 16-byte piece c of row r lies at piece c ^ 4 (r % 2): the eight lanes that are served together read two rows
+    const int piece = lane & 7, copy_row = lane >> 3;
+    const uint32_t to = copy_row * 128 + ((piece ^ ((copy_row & 1) * 4)) << 4);
+    auto weight_row = [&](int n0, int r) { return GATED ? (r < FEATURES ? n0 + r : N + n0 + r - FEATURES) : n0 + r; };
+    const float* from_w[4];
+    int next_tile = first, next_block = 0, next_slot = 0;
+    auto fetch = [&]() {                                            // the next block of this chain, of this tile or the one behind it
+        if (next_tile < tiles) {
+            if (next_block == 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int r = copy_row + i * 4, n0 = next_tile * FEATURES;      // (rows that there are not repeat the first: their sums go nowhere)
+                    from_w[i] = W + (n0 + (GATED ? r % FEATURES : r) < N ? (long long)weight_row(n0, r) * ldw : 0);
+                }
+            }
+            const int k = k_begin + next_block * SPLIT_K + piece * 4;
+            const bool inside = k < k_end;
+            const int at = inside ? k : 0;
+            uint8_t* stage = ring + next_slot * S::STAGE + to;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) copy16(stage + i * 512, from_w[i] + at, inside);
+            if (++next_block == steps) {
+                next_block = 0;
+                next_tile += stride;
+            }
+        }
+        next_slot = next_slot + 1 == S::STAGES ? 0 : next_slot + 1;
+        copies_commit();
+    };
+    // no kernel of a step writes weights: the first stages of them are asked for before the wait
+    if (steps > 0)
+#pragma unroll
+        for (int b = 0; b < S::STAGES - U; ++b) fetch();
+    lp_grid_wait();
+    lp_grid_release();
+    const int quads = part / 4;
+#pragma unroll 4
+    for (int e = lane + group * 32; e < M * quads; e += 32 * S::GROUPS) {
+        const int m = e / quads, k = (e - m * quads) * 4;
+        const float4 v = k_begin + k < k_end ? *(const float4*)(A + (long long)m * lda + k_begin + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t p[3][2];
+        split_tokens(v, p[0], p[1], p[2]);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *(uint2*)(xs + m * x_row + (q * part + k) * 2) = make_uint2(p[q][0], p[q][1]);
+    }
+    __syncthreads();
+    const bool x_real = g < M;                                      // columns of tokens that there are not go nowhere
+    const uint8_t* x_from = xs + (x_real ? g : 0) * x_row + t * 8;
+    const int chains = (K + part - 1) / part;
+    int slot = 0, turn = 0;
+    for (int tile = first; tile < tiles; tile += stride, turn ^= 1) {
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int b = 0; b < steps; b += U) {
+            copies_wait<S::STAGES - 2 * U>();
+            __syncwarp();
+            // parts [part][register]: a lane's four neighbouring values of 16 are its two pairs of an operand, so products 4 t .. 4 t + 3 of a
+            // step stand where the instruction counts 2 t, 2 t + 1, 2 t + 8, 2 t + 9; which of the 16 comes where does not matter to their sum
+            uint32_t w[U][2][3][4];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint8_t* stage = ring + slot * S::STAGE;
+                auto at = [&](int row, int step) { return *(const float4*)(stage + row * 128 + (((step * 4 + t) ^ ((row & 1) * 4)) << 4)); };
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float4 v = at(g + h * 8, s);
+                        split_weights(v.x, v.y, w[u][s][0][h], w[u][s][1][h], w[u][s][2][h]);
+                        split_weights(v.z, v.w, w[u][s][0][h + 2], w[u][s][1][h + 2], w[u][s][2][h + 2]);
+                    }
+                slot = slot + 1 == S::STAGES ? 0 : slot + 1;
+            }
+            __syncwarp();                                           // the stages are free
+#pragma unroll
+            for (int u = 0; u < U; ++u) fetch();
+            uint2 x[U][2][3];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+                        x[u][s][q] = x_real ? *(const uint2*)(x_from + (q * part + (b + u) * SPLIT_K + s * 16) * 2) : make_uint2(0, 0);
+            float d[U][4] = {};
+            auto product = [&](int s, int p, int q) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) mma_16x8(d[u], w[u][s][p], (const uint32_t*)&x[u][s][q]);
+            };
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                product(s, 1, 1);
+                product(s, 0, 2);
+                product(s, 2, 0);
+                product(s, 0, 1);
+                product(s, 1, 0);
+            }
+            product(0, 0, 0);
+            product(1, 0, 0);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (b + u >= blocks) break;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[i] = b + u == 0 ? d[u][i] : sum[i] + d[u][i];
+            }
+        }
+        float* mine = sums + turn * PARTS * 8 * ROW_FEATURES;       // the other half may still be read for the tile before
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mine[(chain * 8 + t * 2 + (i & 1)) * ROW_FEATURES + g + (i >> 1) * 8] = sum[i];
+        if (S::GROUPS == 1) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(PARTS * 32) : "memory");
+        const int e = tid % (PARTS * 32), m = e / FEATURES, f = e % FEATURES, n0 = tile * FEATURES;
+        if (m >= M || n0 + f >= N) continue;
+        auto whole = [&](int r) {
+            const float* from = mine + m * ROW_FEATURES + r;
+            float v = 0.f, half = 0.f;
+            for (int c = 0; c < chains; ++c) {
+                const float s = from[c * 8 * ROW_FEATURES];
+                if (c == PARTS / 2) half = v;
+                v = c % (PARTS / 2) == 0 ? s : v + s;
+            }
+            if (chains > PARTS / 2) v = half + v;
+            // a sum that is no finite number is formed again
+            return fabsf(v) < INFINITY ? v * SUM_SCALE : row_product(A + (long long)m * lda, W + (long long)weight_row(n0, r) * ldw, K);
+        };
+        float* out = C + (long long)m * ldc + n0 + f;
+        if (GATED) *out = silu_mul(whole(f), whole(FEATURES + f));
+        else if (MODE == LP_GEMM_ACCUMULATE) *out += whole(f);
+        else *out = whole(f);
+    }
+    copies_wait<0>();
+}
+
 // ---------------------------------------------------------------- choice and launch
 int failed(cudaError_t err, const char* what) {
     snprintf(lp_error_text, sizeof(lp_error_text), "gemm_plain (%s): %s", what, cudaGetErrorString(err));
@@ -904,11 +1069,38 @@ int launch_rows(const F32Call& c) {
     return (c.N + FEATURES - 1) / FEATURES <= lp_sm_count() ? launch_rows_as<TOK, MODE, true>(c) : launch_rows_as<TOK, MODE, false>(c);
 }
 
+template <int MODE, class S>
+int launch_few_as(const F32Call& c) {
+    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? ROW_FEATURES / 2 : ROW_FEATURES;
+    auto kernel = gemm_f32_few_kernel<MODE, S>;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::RING + S::SUMS + S::ROOM);
+    const int tiles = (c.N + FEATURES - 1) / FEATURES;
+    if (err == cudaSuccess)
+        err = lp_launch(kernel, dim3(min(tiles, lp_sm_count())), dim3(S::THREADS), S::RING + S::SUMS + tokens_bytes(c.M, c.K), c.stream, c.A,
+                        c.W, c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
+    return err == cudaSuccess ? lp_check_launch("gemm_plain (few)") : failed(err, "few");
+}
+
+template <int MODE>
+int launch_few(const F32Call& c) {
+    constexpr int FEATURES = MODE == LP_GEMM_SWIGLU ? ROW_FEATURES / 2 : ROW_FEATURES;
+    const int tokens = c.K <= 65536 ? tokens_bytes(c.M, c.K) : 1 << 30;
+    // with a tile per SM or fewer a second group would have nothing to do, and two blocks' MMAs run side by side instead (four products of one row
+    // with two groups everywhere: 55 us, so 54); the ring gives way to the tokens (8 rows of 2048: 60 us, 62 with gemm_f32_rows_kernel)
+    using Alone = FewShape<1, 6, 2>;
+    using Wide = FewShape<2, 4, 1>;
+    using Tight = FewShape<2, 3, 1>;
+    if ((c.N + FEATURES - 1) / FEATURES <= lp_sm_count() && tokens <= Alone::ROOM) return launch_few_as<MODE, Alone>(c);
+    if (tokens <= Wide::ROOM) return launch_few_as<MODE, Wide>(c);
+    if (tokens <= Tight::ROOM) return launch_few_as<MODE, Tight>(c);
+    return launch_rows<8, MODE>(c);
+}
+
 template <int MODE>
 int launch_f32(const F32Call& c) {
     // up to 16 rows the weights' bytes bound the product; four products (above), us: 16 rows 85, 17 rows in a tile of 64 170, as two launches of 16
     // would take, 32 rows 172
-    if (c.M <= 8) return launch_rows<8, MODE>(c);
+    if (c.M <= 8) return launch_few<MODE>(c);
     if (c.M <= 16) return launch_rows<16, MODE>(c);
     // from 65 rows on a tile of 128 splits the weights half as often (the four, tiles of 64 / 128: 65 rows 221 / 206, 96 rows 225 / 210, 130 rows
     // 323 / 293, 190 rows 339 / 311, 256 rows 373 / 322, 509 rows 630 / 420)

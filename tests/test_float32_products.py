@@ -92,3 +92,22 @@ def test_the_ends_of_the_range(of_a, of_w, M):
     want = a.double() @ w.double().T
     bound = 11 * UNIT * (a.double().abs() @ w.double().abs().T) + 2.0 ** -150
     assert bool(((product(a, w).double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("mode", ["store", "accumulate", "swiglu"])
+@pytest.mark.parametrize("N,K,M", [(7, 64, 1), (40, 8192, 2), (40, 8192, 5), (2391, 100, 1), (2391, 512, 3), (5000, 2048, 4), (2391, 2048, 8), (2391, 4096, 8)])
+def test_a_few_rows_in_every_form(N, K, M, mode):
+    """A tile of features per SM or fewer, several for each of two groups of warps, the short ring beside many tokens, tokens that fit no
+    shared memory; chains of odd numbers of blocks, ragged last tiles: the bits of the same rows in a tile of 64."""
+    from llmplayer_b200.kernels import ops
+    g = torch.Generator(device=DEV).manual_seed(N + K + M)
+    code = {"store": ops.STORE, "accumulate": ops.ACCUMULATE, "swiglu": ops.SWIGLU}[mode]
+    a = torch.randn(17, K, generator=g, device=DEV)
+    w = torch.randn(N * (2 if mode == "swiglu" else 1), K, generator=g, device=DEV)
+    first = torch.randn(17, N, generator=g, device=DEV)
+    whole, out = first.clone(), torch.cat([first[:M], torch.full((1, N), 7.0, device=DEV)])
+    ops.gemm_plain(a, w, whole, code)
+    ops.gemm_plain(a[:M].contiguous(), w, out[:M], code)
+    torch.cuda.synchronize()
+    ops.check_kernel_status()
+    assert torch.equal(out[:M], whole[:M]) and bool((out[M] == 7.0).all())
