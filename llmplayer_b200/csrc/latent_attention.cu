@@ -1021,7 +1021,7 @@ latent_absorb_tc_kernel(const float* __restrict__ q, int ldq, const __nv_bfloat1
             float ss = 0.f;
             for (int c = tid * 4; c < rank; c += AB_WARPS * 128) {
                 const float4 v = *(const float4*)(kv + c);
-                ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;      // (in the order of latent_prepare_vec4_kernel: the same bits)
             }
             const float factor = 1.0f / sqrtf(lp_block_sum(ss, scratch) / (float)rank + k.eps);
             for (int c = tid * 4; c < rank; c += AB_WARPS * 128) {
@@ -1306,7 +1306,8 @@ bool absorb_on_tensor_cores(int w_dtype, int dn, int dr, int rank, const void* u
 }  // namespace
 
 // What lp_latent_prepare and lp_latent_absorb do one after the other, in one launch, for a 16-bit cache and 16-bit weights; see there for
-// the operands. Returns LP_NOT_SERVED for sizes and addresses that it does not take.
+// the operands. Returns LP_NOT_SERVED for sizes and addresses that it does not take: those that lp_latent_prepare refuses or serves value by
+// value are left to it, so that a cached row has the same bits whichever wrote it (a rank of up to 512, as the cache's readers take).
 extern "C" int lp_latent_queries(const float* proj, int ld, int q_off, int kv_off, const float* gain, float eps, const float* inv_freq,
                                  int rot, const int* positions, const int* seq_ids, const int* page_table, int pt_stride, void* pages,
                                  int kv_dtype, int T, int H, int dn, int dr, int rank, int page_size, const float* q_sep, int ldq,
@@ -1314,7 +1315,7 @@ extern "C" int lp_latent_queries(const float* proj, int ld, int q_off, int kv_of
     if (T <= 0) return 0;
     const float* q = q_sep ? q_sep : proj + q_off;
     if (!q_sep) ldq = ld;
-    if (H <= 0 || H >= 65535 || page_size <= 0 || kv_dtype != LP_BF16 || rot < 0 || (rot & 1) || rot > dr || (rot > 0 && !inv_freq) || q_off < 0 ||
+    if (H <= 0 || H >= 65535 || page_size <= 0 || kv_dtype != LP_BF16 || rot < 0 || rot % 8 || rot > dr || rot > 256 || (rot > 0 && !inv_freq) || q_off < 0 ||
         kv_off < 0 || kv_off + rank + dr > ld || (q_sep ? 0 : q_off) + H * (dn + dr) > ldq || !absorb_on_tensor_cores(w_dtype, dn, dr, rank, uk, qa) ||
         ld % 4 || ldq % 4 || kv_off % 4 || dr % 4 || (((uintptr_t)q | (uintptr_t)proj | (uintptr_t)gain | (uintptr_t)pages) & 15) != 0)
         return LP_NOT_SERVED;
