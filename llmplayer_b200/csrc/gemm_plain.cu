@@ -2,15 +2,15 @@
 // Every output element is summed in one fixed way whatever M is, so a row's result does not depend on which other rows share the
 // launch: K is cut into eighths (rounded up to 32 products), each eighth is a sum of its own, the eighths of each half are
 // added in increasing order, then the halves. Two ways of forming an eighth:
-//   * rows of 64 float32 and more that can be read 16 bytes at a time: on the tensor cores, float32 numbers as three bfloat16 parts
+//   * rows of 32 float32 and more that can be read 16 bytes at a time: on the tensor cores, float32 numbers as three bfloat16 parts
 //     (gemm_f32_few_kernel and gemm_f32_rows_kernel up to 16 rows, gemm_f32_split_kernel from 17 on: the same bits);
 //   * any other types, sizes and alignments: a chain of multiply-adds in increasing k that starts at zero (gemm_plain_kernel, which
 //     adds all eighths in order).
 // Errors against 64 bits, root mean square in units of 2^-24 of the sum of the products' magnitudes, in parts / by multiply-adds, at
-// K = 64, 256, 2048, 8192: normal numbers 0.17 / 0.35, 0.11 / 0.19, 0.05 / 0.17, 0.04 / 0.17; numbers in [1, 2) 0.82 / 1.21, 0.90 / 0.96,
-// 0.92 / 1.62, 1.02 / 2.94; numbers of very different sizes (normal times e^(2 normal)) 0.62 / 1.02, 0.62 / 0.92, 0.54 / 1.58, 0.55 / 2.30; mantissas
-// of ones 1.16 / 1.63, 1.22 / 2.22, 1.43 / 2.38, 1.64 / 115, but 1.17 / 0.87 at K = 16: hence the line at 64. A product that stands alone in its sum is off
-// by 0.63 (3.5 at most) where a rounded one is by 0.42 (1.0).
+// K = 32, 64, 256, 2048, 8192: normal numbers 0.20 / 0.47, 0.17 / 0.35, 0.11 / 0.19, 0.05 / 0.17, 0.04 / 0.17; numbers in [1, 2) 0.65 / 1.46, 0.82 / 1.21,
+// 0.90 / 0.96, 0.92 / 1.62, 1.02 / 2.94; numbers of very different sizes (normal times e^(2 normal)) 0.61 / 1.08, 0.62 / 1.02, 0.62 / 0.92, 0.54 / 1.58,
+// 0.55 / 2.30; mantissas of ones 1.25 / 1.89, 1.16 / 1.63, 1.22 / 2.22, 1.43 / 2.38, 1.64 / 115, but 1.16 / 0.87 at K = 16: hence the line at 32 (behind it
+// these alone came out worse, at 40: 1.59 / 1.11). A product that stands alone in its sum is off by 0.63 (3.7 at most) where a rounded one is by 0.42 (1.0).
 // It is the product of the float32 path and the comparison twin of the bfloat16 kernels.
 //
 // Counterparts in the reference (src/main/resources/kernels/cuda/): matmul_f32.cu:6-39,
@@ -149,7 +149,7 @@ gemm_plain_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __rest
 // rows: 16384 x 2048 (gated) 820 -> 222 us, 2048 x 8192 407 -> 105, 3072 x 2048 163 -> 53, 2048 x 2048 111 -> 39; the four one behind the other
 // (243 MB of weights, cold) 1499 -> 420. 64 rows: 130 -> 60, 121 -> 53, 34 -> 22, 34 -> 26; together 359 -> 177. 17 rows: together 301 -> 170.
 constexpr int SPLIT_K = 32;                     // products of a block
-constexpr int SPLIT_MIN_K = 64;                 // shorter sums run on gemm_plain_kernel
+constexpr int SPLIT_MIN_K = 32;                 // shorter sums run on gemm_plain_kernel (300 x 2048, K = 16: 4.7 us, 9.8 in parts)
 constexpr float SPLIT_SCALE = 16777216.f, SUM_SCALE = 1.f / (SPLIT_SCALE * SPLIT_SCALE);      // 2^24 of an operand, 2^-48 of a sum
 
 template <int TOK> struct SplitTile {

@@ -36,7 +36,7 @@ def draw(kind, g, *shape):
 
 
 @pytest.mark.parametrize("M", ROWS)
-@pytest.mark.parametrize("K", [64, 260, 1024, 2048])
+@pytest.mark.parametrize("K", [32, 36, 64, 260, 1024, 2048])
 @pytest.mark.parametrize("kind", ["normal", "one sign", "worst mantissas", "many sizes"])
 def test_no_further_from_64_bits_than_multiply_adds(kind, K, M):
     g = torch.Generator(device=DEV).manual_seed(K + M)
@@ -48,7 +48,7 @@ def test_no_further_from_64_bits_than_multiply_adds(kind, K, M):
 
 
 @pytest.mark.parametrize("M", ROWS)
-@pytest.mark.parametrize("K", [64, 260, 2048])
+@pytest.mark.parametrize("K", [32, 64, 260, 2048])
 def test_exact_sums_stay_exact(K, M):
     """Whole numbers whose sums float32 holds (2^11 terms of up to 60 x 60), and rows of one 1 that pick any values out."""
     g = torch.Generator(device=DEV).manual_seed(K + M)
@@ -95,7 +95,7 @@ def test_the_ends_of_the_range(of_a, of_w, M):
 
 
 @pytest.mark.parametrize("mode", ["store", "accumulate", "swiglu"])
-@pytest.mark.parametrize("N,K,M", [(7, 64, 1), (40, 8192, 2), (40, 8192, 5), (2391, 100, 1), (2391, 512, 3), (5000, 2048, 4), (2391, 2048, 8), (2391, 4096, 8)])
+@pytest.mark.parametrize("N,K,M", [(7, 32, 1), (7, 64, 1), (40, 8192, 2), (40, 8192, 5), (2391, 100, 1), (2391, 512, 3), (5000, 2048, 4), (2391, 2048, 8), (2391, 4096, 8)])
 def test_a_few_rows_in_every_form(N, K, M, mode):
     """A tile of features per SM or fewer, several for each of two groups of warps, the short ring beside many tokens, tokens that fit no
     shared memory; chains of odd numbers of blocks, ragged last tiles: the bits of the same rows in a tile of 64."""
